@@ -201,6 +201,8 @@ typedef enum {
                                       8), 0 = automatic (none); the slicing of chunk c + 1 runs
                                       beside the GEMM of chunk c. */,
   SSBLAS_PATH_F16_TCGEN05 = 11,     /* fp16 inputs (SSBLAS_EXT_R16F row) on tcgen05.mma kind::f16 */
+  SSBLAS_PATH_F32_TCGEN05 = 13,    /* plain fp32 on tcgen05.mma kind::f16: three BF16 parts per operand
+                                      (exact), six products, FP32 sums of 32 k added in registers */
   SSBLAS_PATH_GROUPED_OZAKI_TILE = 12 /* not a path: ssblasSetKernelConfig / tuning key of the tile
                                       shape of a grouped call's Ozaki instances per size bucket
                                       (batch 1): 0 = 128 x 64 tiles, one accumulator; 1 (default)

@@ -34,7 +34,7 @@ SSBLAS_COMPUTE_DEFAULT = 0
 # extensions
 SSBLAS_MATH_PLAIN, SSBLAS_MATH_FP64_OZAKI, SSBLAS_MATH_FP32_BF16X3 = 0, 1, 2
 PATH_NAMES = {0: "none", 1: "simt", 2: "i8_tcgen05", 3: "ozaki_tcgen05", 4: "bf16x3_tcgen05", 5: "grouped",
-              6: "dmma", 11: "f16_tcgen05"}
+              6: "dmma", 11: "f16_tcgen05", 13: "f32_tcgen05"}
 # type and semantics extensions (ssblasSetExtensions)
 SSBLAS_EXT_NONE, SSBLAS_EXT_R16F, SSBLAS_EXT_R8U, SSBLAS_EXT_OP_C, SSBLAS_EXT_K0_BETA, SSBLAS_EXT_COMPUTE_TYPE = (
     0, 1, 2, 4, 8, 16)

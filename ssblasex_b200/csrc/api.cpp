@@ -587,6 +587,13 @@ static cudaError_t dispatch(const BatchDesc& d, cudaStream_t st) {
       if (e == cudaSuccess) note_path(SSBLAS_PATH_BF16X3_TCGEN05);
       return e;
     }
+  } else if (d.row == ROW_F32 && !d.exact_f32 && simt_config(d) == kSimtF32Split) {
+    // plain fp32 on the BF16 tensor cores, operands split in three parts
+    cudaError_t e = launch_f32_split(d, 3, st);
+    if (e != cudaErrorNotSupported) {
+      if (e == cudaSuccess) note_path(SSBLAS_PATH_F32_TCGEN05);
+      return e;
+    }
   }
   note_path(SSBLAS_PATH_SIMT);
   return launch_simt_gemm(d, st);

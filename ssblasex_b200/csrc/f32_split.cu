@@ -1,0 +1,599 @@
+// FP32 batched GEMM on the BF16 tensor cores (tcgen05.mma kind::f16), the operands split into BF16
+// parts inside the kernel. Two forms of the fp32 row share it:
+//   plain (NP = 3)    x = hi + mid + lo exactly (8 + 8 + 8 significand bits), six products
+//                     hi hi, hi mid, mid hi, mid mid, hi lo, lo hi: what is left out is below
+//                     2^-25 of a product, so the result is an FP32 GEMM's;
+//   3xBF16 (NP = 2)   x ~ hi + lo, three products (the emulation mode of the fp32 row).
+// Semantics follow the reference (hirokitokura/ssblasEx): C <- beta*C, not read when beta == 0
+// (src/include/CScale/Xgemm_scale_kernel.hpp:164-176), then C <- C + acc*alpha with one fused
+// multiply-add (src/include/GemmCore/Xgemm_kernel_sve_v4x5_1.hpp:93-127).
+//
+// Accuracy of the plain form. The tensor core adds a K step of 16 products and the accumulator
+// exactly enough, but truncates the sum to FP32: over a long K that bias would exceed the error of a
+// chain of fused multiply-adds (k = 1024, U[-1,1): 1.25e-6 against 5.6e-7 of the 2-norm). So an
+// accumulator only lives for one chunk of 32 k -- the small products first, then the two steps of
+// hi hi, the only truncations at full magnitude -- and the epilogue warps add the chunks in
+// registers, rounding to nearest. The ends of the range: both operands are scaled by 2^24 before they
+// are split (exact, and the lo part of the smallest subnormal is then a BF16 number; the tensor
+// core takes and gives subnormals), and every sum that is not finite (Inf and NaN operands,
+// |x| >= 2^104, sums of 2^80 and more), or is below 2^-100 and not zero, is computed again by a chain
+// of fused multiply-adds over the operands, so those behave as FP32 arithmetic does.
+//
+// Design: persistent CTAs over (instance, 128 x BN tile) items, K in chunks of 32:
+//   warps 8-15   converters: each thread loads 16 bytes of op(A) / op(B) straight from the
+//                caller's matrices (any alignment: 4-byte loads where 16-byte ones are not possible),
+//                DEPTH chunks ahead in registers, splits, and writes the parts in the layout the
+//                tensor core reads -- K-major (64-byte swizzle) where K is contiguous in memory,
+//                MN-major (128-byte swizzle) where M or N is, so nothing is transposed
+//   warp 16      tensor memory, MMA issue from one lane
+//   warps 0-7    chunk sums from tensor memory into registers, then alpha * acc + beta * C
+// Operands cross HBM once as fp32 and no plane is written back: the operands of a tile are split
+// again for every tile that shares them, which is cheaper than the 10 bytes per element of a split
+// pass. What bounds it (16 x 1024^3): a 128 x 128 chunk takes about 1850 cycles; its 12 MMAs alone take
+// 1100 (each reads 8 KB of shared memory in the 64 cycles of its products), the parts' writes (48 KB)
+// share that memory's 128 B per cycle, and the 32 KB a chunk loads come from L2 at 4.6 TB/s over the
+// GPU. Measured (ms, FFMA kernels -> this one): 16 x 1024^3 NN 0.829 -> 0.215; 4 x 2048^3 TN 1.73 ->
+// 0.41; 64 x 128^3 NN 0.0145 -> 0.0120; 8 x (777 x 555 x 333) 0.103 -> 0.040; 2 x 128^2 x 4096 0.19 ->
+// 0.09. 3xBF16 (split pass and tiled GEMM -> this kernel): 256 x 256^3 0.130 -> 0.053.
+#include <cuda_bf16.h>
+#include <cuda_runtime.h>
+#include <stdint.h>
+
+#include "internal.h"
+#include "ptx.cuh"
+
+namespace ssb {
+namespace {
+
+constexpr int kKC = 32;                      // K elements per chunk
+constexpr int kConvThreads = 256;            // warps 8-15
+constexpr int kSplitThreads = 32 * 20;       // the last warpgroup's first warp issues the MMAs
+// registers per thread: 640 x 96 at launch = 61,440; 4 x 128 x 112 + 128 x 32 = 61,440 after the split
+constexpr int kWorkRegs = 112, kIssueRegs = 32;
+// Plain form: scale of the operands, of their sums, and the magnitude below which a sum that is not
+// zero is computed again
+constexpr float kScale = 0x1p24f, kUnscale = 0x1p-48f;
+constexpr uint32_t kSmallestBits = 0x0d800000u;   // 2^-100
+
+// NP parts per operand, AR rows of op(A) converted per tile (64 when m <= 64), BN columns
+template <int NP_, int AR_, int BN_>
+struct Split {
+  static constexpr int NP = NP_, AR = AR_, BN = BN_;
+  static constexpr int A_PLANE = AR * kKC * 2;
+  static constexpr int B_PLANE = BN * kKC * 2;
+  static constexpr int STAGE = NP * (A_PLANE + B_PLANE);
+  static constexpr int STAGES = (200 * 1024) / STAGE > 8 ? 8 : (200 * 1024) / STAGE;
+  static constexpr int NACC = 4;             // accumulators in flight
+  static constexpr int TMEM_COLS = NACC * BN;
+  static constexpr int UA = AR * kKC / 4 / kConvThreads, UB = BN * kKC / 4 / kConvThreads;   // 16-byte units per thread
+  static constexpr int DEPTH = (UA + UB) >= 6 ? 2 : 3;                                       // chunks held in registers
+  // the MMA reads 128 rows of every A part: with AR = 64 the upper 64 come from whatever follows
+  // (within the stage, since B follows A), and their products are never read
+  static constexpr int SMEM = 1024 + STAGES * STAGE + 512;
+  static constexpr bool PROMOTE = NP == 3;
+  static_assert(STAGE % 1024 == 0 && NP * B_PLANE >= 4096 && SMEM <= 232448, "stages");
+};
+
+struct SplitArgs {
+  long m, n, k, lda, ldb, ldc;
+  const float* const* A;
+  const float* const* B;
+  float* const* C;
+  float alpha, beta;
+  int a_mn, b_mn;          // op(A) rows / op(B) columns contiguous in memory
+  uint32_t tiles_m, tiles_mn, total;
+  int* err;
+  uint32_t wait_limit;
+  int skip;                // injected fault: CTA 0 never signals its first chunk
+};
+
+// One work item: the tile at (m0, n0) of instance b.
+struct SplitTile {
+  uint32_t b;
+  long m0, n0;
+};
+template <class F>
+__device__ __forceinline__ SplitTile split_tile(const SplitArgs& a, uint32_t t) {
+  const uint32_t b = t / a.tiles_mn, r = t - b * a.tiles_mn;
+  const uint32_t nt = r / a.tiles_m;
+  return {b, (long)(r - nt * a.tiles_m) * 128, (long)nt * F::BN};
+}
+
+// One operand as a converter thread sees it: its unit i (4 consecutive elements along the contiguous
+// dimension) of the next chunk is at p + i * step.
+//   mn: a unit is 4 rows at one k; a warp takes whole k lines of ROWS; unit i is 256 / (ROWS / 4) k on
+//   else a unit is 4 k of one row, 8 lanes a row; unit i is 32 rows on
+struct SplitOperand {
+  const float* p;
+  int step, adv;           // elements between units, between chunks (ld < 2^25)
+  int rows, k;             // valid rows from this thread's unit 0 on; valid k from the next chunk on
+  bool mn, vec, full;      // full: every unit of the tile's whole chunks is inside the matrix
+};
+template <int ROWS>
+__device__ __forceinline__ SplitOperand split_operand(const float* X, long rows, long K, long ld, bool mn, long r0,
+                                                      int t) {
+  constexpr int RG = ROWS / 4;
+  SplitOperand o;
+  o.mn = mn;
+  o.vec = ((uintptr_t)X % 16) == 0 && ld % 4 == 0;
+  o.full = o.vec && rows - r0 >= ROWS;
+  const int rr = mn ? 4 * (t % RG) : t / 8, kk = mn ? t / RG : 4 * (t % 8);
+  o.p = X + (mn ? r0 + rr + kk * ld : (r0 + rr) * ld + kk);
+  o.step = (mn ? kConvThreads / RG : 32) * (int)ld;
+  o.adv = mn ? kKC * (int)ld : kKC;
+  o.rows = (int)(rows - r0 < ROWS ? rows - r0 : ROWS) - rr;
+  o.k = (int)K;
+  return o;
+}
+
+// The units of the next chunk; the operand moves on to the one after it.
+template <int ROWS, int U>
+__device__ __forceinline__ void split_load(SplitOperand& o, int t, float4 (&x)[U]) {
+  constexpr int RG = ROWS / 4;
+  const float* src = o.p;
+  if (o.full && o.k >= kKC) {
+#pragma unroll
+    for (int i = 0; i < U; ++i, src += o.step) x[i] = __ldg((const float4*)src);
+  } else {
+#pragma unroll
+    for (int i = 0; i < U; ++i, src += o.step) {
+      const int kk = o.mn ? t / RG + i * (kConvThreads / RG) : 4 * (t % 8);
+      const int n = o.mn ? (o.k > kk ? o.rows : 0) : (o.rows > 32 * i ? o.k - kk : 0);
+      x[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (o.vec && n >= 4) {
+        x[i] = __ldg((const float4*)src);
+      } else {
+        if (n > 0) x[i].x = __ldg(src);
+        if (n > 1) x[i].y = __ldg(src + 1);
+        if (n > 2) x[i].z = __ldg(src + 2);
+        if (n > 3) x[i].w = __ldg(src + 3);
+      }
+    }
+  }
+  o.p += o.adv;
+  o.k -= kKC;
+}
+
+// Packed FP32 arithmetic (two values per instruction): d = a * b + c, and a + b
+__device__ __forceinline__ uint64_t pack2(float x, float y) {
+  uint64_t r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(x), "f"(y));
+  return r;
+}
+__device__ __forceinline__ void unpack2(uint64_t v, float& x, float& y) {
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(x), "=f"(y) : "l"(v));
+}
+__device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) {
+  uint64_t d;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+  return d;
+}
+__device__ __forceinline__ uint64_t mul2(uint64_t a, uint64_t b) {
+  uint64_t d;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+  return d;
+}
+__device__ __forceinline__ uint64_t add2(uint64_t a, uint64_t b) {
+  uint64_t d;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+  return d;
+}
+
+// Two values rounded to bf16 (low half = first), and (REST) what rounding left of them.
+template <bool REST>
+__device__ __forceinline__ uint32_t take_bf16(uint64_t& v) {
+  float x, y;
+  unpack2(v, x, y);
+  const __nv_bfloat162 h = __floats2bfloat162_rn(x, y);
+  const uint32_t w = *(const uint32_t*)&h;
+  if (REST) v = fma2(pack2(__uint_as_float(w << 16), __uint_as_float(w & 0xffff0000u)), pack2(-1.f, -1.f), v);
+  return w;
+}
+
+// Splits the units and writes the NP parts of the operand.
+template <int NP, int ROWS, int U>
+__device__ __forceinline__ void split_store(uint32_t dst, bool mn, int t, float4 (&x)[U]) {
+  constexpr int PLANE = ROWS * kKC * 2;
+  constexpr int RG = ROWS / 4;
+  uint32_t off, step;
+  if (mn) {
+    // blocks of 64 rows x 32 k lines of 128 bytes; lines kk, kk + 8q: the swizzle (kk % 8) is fixed
+    const uint32_t rg = t % RG, kk = t / RG;
+    off = (rg >> 4) * (kKC * 128u) + kk * 128u + ((((rg & 15u) >> 1) ^ (kk & 7u)) << 4) + ((rg & 1u) << 3);
+    step = (kConvThreads / RG) * 128u;
+  } else {
+    // lines of 64 bytes; rows rr + 32 i: the swizzle ((rr / 2) % 4) is fixed
+    const uint32_t rr = t / 8, kq = t % 8;
+    off = rr * 64u + (((kq >> 1) ^ ((rr >> 1) & 3u)) << 4) + ((kq & 1u) << 3);
+    step = 32 * 64u;
+  }
+#pragma unroll
+  for (int i = 0; i < U; ++i) {
+    const uint32_t d = dst + off + i * step;
+    uint64_t v0 = pack2(x[i].x, x[i].y), v1 = pack2(x[i].z, x[i].w);
+    if constexpr (NP == 3) {
+      v0 = mul2(v0, pack2(kScale, kScale));
+      v1 = mul2(v1, pack2(kScale, kScale));
+    }
+#pragma unroll
+    for (int p = 0; p < NP; ++p) {
+      const uint32_t w0 = p + 1 < NP ? take_bf16<true>(v0) : take_bf16<false>(v0);
+      const uint32_t w1 = p + 1 < NP ? take_bf16<true>(v1) : take_bf16<false>(v1);
+      asm volatile("st.shared.v2.b32 [%0], {%1, %2};" ::"r"(d + p * PLANE), "r"(w0), "r"(w1) : "memory");
+    }
+  }
+}
+
+// The sums of one lane's row again, for 16 columns, by a chain of fused multiply-adds over the operands
+// in k order: op(A)(i, k) = pa[k * ak], op(B)(k, j) = pb[j * bc + k * bk]; columns from n on repeat
+// column n - 1. Eight k are in flight at a time, so that this rare path runs near the speed of an
+// ordinary FP32 kernel.
+__device__ __noinline__ void split_redo(const float* pa, long ak, const float* pb, long bc, long bk, int n, int k,
+                                        float* v) {
+  float acc[16];
+#pragma unroll
+  for (int j = 0; j < 16; ++j) acc[j] = 0.f;
+  int kk = 0;
+#pragma unroll 1
+  for (; kk + 8 <= k; kk += 8, pa += 8 * ak, pb += 8 * bk) {
+    float x[8];
+#pragma unroll
+    for (int u = 0; u < 8; ++u) x[u] = __ldg(pa + u * ak);
+#pragma unroll
+    for (int j = 0; j < 16; ++j) {
+      const float* q = pb + (j < n ? j : n - 1) * bc;
+      float y[8];
+#pragma unroll
+      for (int u = 0; u < 8; ++u) y[u] = __ldg(q + u * bk);
+#pragma unroll
+      for (int u = 0; u < 8; ++u) acc[j] = fmaf(x[u], y[u], acc[j]);
+    }
+  }
+#pragma unroll 1
+  for (; kk < k; ++kk, pa += ak, pb += bk) {
+    const float x = __ldg(pa);
+#pragma unroll
+    for (int j = 0; j < 16; ++j) acc[j] = fmaf(x, __ldg(pb + (j < n ? j : n - 1) * bc), acc[j]);
+  }
+#pragma unroll
+  for (int j = 0; j < 16; ++j) v[j] = acc[j];
+}
+
+template <class F>
+__global__ void __launch_bounds__(kSplitThreads, 1) f32_split_kernel(const SplitArgs a) {
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t* stages = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
+  uint64_t* full = (uint64_t*)(stages + F::STAGES * F::STAGE);   // parts written (converter warps)
+  uint64_t* empty = full + F::STAGES;                            // parts read by the MMAs (commit)
+  uint64_t* acc_full = empty + F::STAGES;                        // [NACC] sums complete (commit)
+  uint64_t* acc_empty = acc_full + F::NACC;                      // [NACC] sums read (8 warps)
+  uint64_t* drain = acc_empty + F::NACC;
+  uint32_t* tmem_slot = (uint32_t*)(drain + 1);
+  static_assert((2 * F::STAGES + 2 * F::NACC + 1) * 8 + 4 <= 512, "barrier area");
+
+  const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
+  const uint32_t wl = a.wait_limit ? a.wait_limit : ptx::kWaitLimit;
+  int* err = a.err;
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < F::STAGES; ++s) {
+      ptx::mbar_init(ptx::smem_u32(&full[s]), kConvThreads / 32);
+      ptx::mbar_init(ptx::smem_u32(&empty[s]), 1);
+    }
+    for (int q = 0; q < F::NACC; ++q) {
+      ptx::mbar_init(ptx::smem_u32(&acc_full[q]), 1);
+      ptx::mbar_init(ptx::smem_u32(&acc_empty[q]), 8);
+    }
+    ptx::mbar_init(ptx::smem_u32(drain), 1);
+    ptx::fence_mbar_init();
+  }
+  if (warp == 16) {
+    ptx::tmem_alloc(ptx::smem_u32(tmem_slot), F::TMEM_COLS);
+    ptx::tmem_relinquish();
+  }
+  ptx::tc_fence_before();
+  __syncthreads();
+  ptx::tc_fence_after();
+  const uint32_t tmem = __shfl_sync(0xffffffffu, *tmem_slot, 0);   // known to be warp-uniform
+  // under a programmatic launch the set-up above overlaps the end of the kernel before
+  ptx::grid_dep_wait();
+  ptx::grid_dep_launch();
+  const uint32_t nkc = (uint32_t)((a.k + kKC - 1) / kKC);
+
+  if (warp >= 8 && warp < 16) {
+    // ------------------------------------------------------------------ converters --------
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kWorkRegs));
+    const int t = threadIdx.x - 256;
+    const uint32_t stages0 = ptx::smem_u32(stages);
+    struct Pos {
+      uint32_t t, kc;
+      SplitOperand A, B;
+    };
+    Pos ld;                      // next chunk to load
+    ld.t = blockIdx.x;
+    ld.kc = 0;
+    auto enter = [&]() {
+      if (ld.t >= a.total) return;
+      const SplitTile ti = split_tile<F>(a, ld.t);
+      ld.A = split_operand<F::AR>(a.A[ti.b], a.m, a.k, a.lda, a.a_mn != 0, ti.m0, t);
+      ld.B = split_operand<F::BN>(a.B[ti.b], a.n, a.k, a.ldb, a.b_mn != 0, ti.n0, t);
+    };
+    float4 xa[F::DEPTH][F::UA], xb[F::DEPTH][F::UB];
+    auto load = [&](float4 (&va)[F::UA], float4 (&vb)[F::UB]) {
+      if (ld.t >= a.total) return;
+      split_load<F::AR, F::UA>(ld.A, t, va);
+      split_load<F::BN, F::UB>(ld.B, t, vb);
+      if (++ld.kc == nkc) {
+        ld.kc = 0;
+        ld.t += gridDim.x;
+        enter();
+      }
+    };
+    enter();
+#pragma unroll
+    for (int d = 0; d < F::DEPTH; ++d) load(xa[d], xb[d]);
+    uint32_t c = 0, kc = 0;
+    uint32_t cur = blockIdx.x;
+    bool ok = true;
+    while (ok && cur < a.total) {
+#pragma unroll
+      for (int d = 0; d < F::DEPTH; ++d) {
+        if (!ok || cur >= a.total) break;
+        const uint32_t s = c % F::STAGES;
+        if (!ptx::mbar_wait(ptx::smem_u32(&empty[s]), ((c / F::STAGES) & 1) ^ 1, err, 81, wl)) {
+          ok = false;
+          break;
+        }
+        const uint32_t st = stages0 + s * F::STAGE;
+        split_store<F::NP, F::AR, F::UA>(st, a.a_mn != 0, t, xa[d]);
+        split_store<F::NP, F::BN, F::UB>(st + F::NP * F::A_PLANE, a.b_mn != 0, t, xb[d]);
+        ptx::fence_proxy_async_smem();   // generic-proxy writes -> the tensor core's reads
+        __syncwarp();
+        if (lane == 0 && !(a.skip && c == 0 && blockIdx.x == 0)) ptx::mbar_arrive(ptx::smem_u32(&full[s]));
+        load(xa[d], xb[d]);
+        ++c;
+        if (++kc == nkc) {
+          kc = 0;
+          cur += gridDim.x;
+        }
+      }
+    }
+  } else if (warp >= 16) {
+    // ------------------------------------------------------------------ MMA ---------------
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kIssueRegs));
+    if (warp == 16) {
+      const uint32_t idesc = ptx::idesc_bf16(128, F::BN, a.a_mn != 0, a.b_mn != 0);
+      // descriptors of stage 0's first part, and their step along K: 16 k are 32 bytes of a K-major
+      // line, 16 lines of an MN-major block (addresses count 16 bytes). The whole warp runs the loop
+      // and one lane's predicate is on the MMA itself, so descriptors stay in uniform registers:
+      // under a branch on the lane each MMA cost four moves into them, 90 cycles a MMA.
+      const uint32_t lead = ptx::elect_one();
+      const uint32_t st0 = ptx::smem_u32(stages);
+      const uint64_t a0 = a.a_mn ? ptx::smem_desc_mnmajor(st0, kKC * 128) : ptx::smem_desc_kmajor(st0, 64);
+      const uint64_t b0 = a.b_mn ? ptx::smem_desc_mnmajor(st0 + F::NP * F::A_PLANE, kKC * 128)
+                                 : ptx::smem_desc_kmajor(st0 + F::NP * F::A_PLANE, 64);
+      const uint64_t ka = a.a_mn ? 128 : 2, kb = a.b_mn ? 128 : 2;
+      static_assert(kKC == 32, "two K steps per chunk");
+      uint32_t c = 0, q = 0;     // chunks, accumulators
+      bool ok = true;
+      for (uint32_t t = blockIdx.x; t < a.total && ok; t += gridDim.x) {
+        for (uint32_t kc = 0; kc < nkc; ++kc, ++c) {
+          const uint32_t s = c % F::STAGES;
+          if (F::PROMOTE || kc == 0) {
+            if (!ptx::mbar_wait(ptx::smem_u32(&acc_empty[q % F::NACC]), ((q / F::NACC) & 1) ^ 1, err, 82, wl)) {
+              ok = false;
+              break;
+            }
+          }
+          if (!ptx::mbar_wait(ptx::smem_u32(&full[s]), (c / F::STAGES) & 1, err, 83, wl)) {
+            ok = false;
+            break;
+          }
+          ptx::tc_fence_after();
+          const uint32_t d = tmem + (q % F::NACC) * F::BN;
+          const uint64_t sa = a0 + (uint64_t)(s * (uint32_t)(F::STAGE >> 4)), sb = b0 + (uint64_t)(s * (uint32_t)(F::STAGE >> 4));
+          uint32_t acc = F::PROMOTE || kc == 0 ? 0u : 1u;
+          // smallest products first
+#pragma unroll
+          for (int sum = F::NP - 1; sum >= 0; --sum)
+#pragma unroll
+            for (int p = 0; p <= sum; ++p) {
+              const uint64_t ad = sa + (uint64_t)(p * (F::A_PLANE >> 4)), bd = sb + (uint64_t)((sum - p) * (F::B_PLANE >> 4));
+              ptx::mma_f16_if(lead, d, ad, bd, idesc, acc);
+              ptx::mma_f16_if(lead, d, ad + ka, bd + kb, idesc, 1u);
+              acc = 1u;
+            }
+          ptx::mma_commit_if(lead, ptx::smem_u32(&empty[s]));
+          if (F::PROMOTE || kc + 1 == nkc) {
+            ptx::mma_commit_if(lead, ptx::smem_u32(&acc_full[q % F::NACC]));
+            ++q;
+          }
+        }
+      }
+      // every MMA issued has finished before the tensor memory is released
+      ptx::mma_commit_if(lead, ptx::smem_u32(drain));
+      ptx::mbar_wait(ptx::smem_u32(drain), 0, err, 84, wl);
+    }
+  } else {
+    // ------------------------------------------------------------------ epilogue ----------
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kWorkRegs));
+    constexpr int HALF = F::BN / 2;
+    const int quarter = warp % 4, half = warp / 4;
+    const uint32_t t_row = tmem + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(half * HALF);
+    const bool active = quarter * 32 < F::AR;      // rows past AR hold no results
+    uint32_t q = 0, item = 0;
+    bool ok = true;
+    for (uint32_t t = blockIdx.x; t < a.total && ok; t += gridDim.x, ++item) {
+      const SplitTile ti = split_tile<F>(a, t);
+      const long gi = ti.m0 + quarter * 32 + lane, gj0 = ti.n0 + half * HALF;
+      float* C = a.C[ti.b] + gi + gj0 * a.ldc;
+      const bool row_ok = active && gi < a.m;
+      const int cols = gj0 < a.n ? (a.n - gj0 < HALF ? (int)(a.n - gj0) : HALF) : 0;
+      const bool read_c = a.beta != 0.0f;
+      // narrow tiles: C is in flight while the products run
+      constexpr bool EARLY_C = HALF == 32;
+      constexpr int G = EARLY_C ? 32 : 16;     // columns per group
+      float cv[G];
+      // (the walking pointers are opaque to the compiler: it would keep an address per column otherwise)
+      auto load_c = [&](int j0) {
+        const float* cp = C + (long)j0 * a.ldc;
+        asm volatile("" : "+l"(cp));
+        if (row_ok && cols == HALF) {
+#pragma unroll
+          for (int j = 0; j < G; ++j, cp += a.ldc) cv[j] = __ldcs(cp);
+        } else {
+#pragma unroll
+          for (int j = 0; j < G; ++j, cp += a.ldc) cv[j] = (row_ok && j0 + j < cols) ? __ldcs(cp) : 0.0f;
+        }
+      };
+      if (EARLY_C && read_c) load_c(0);
+      uint64_t sum[HALF / 2];                  // pairs of columns
+#pragma unroll
+      for (int j = 0; j < HALF / 2; ++j) sum[j] = 0;
+      const uint32_t parts = F::PROMOTE ? nkc : 1;
+      for (uint32_t p = 0; p < parts; ++p, ++q) {
+        const uint32_t buf = q % F::NACC;
+        if (!ptx::mbar_wait(ptx::smem_u32(&acc_full[buf]), (q / F::NACC) & 1, err, 85, wl)) {
+          ok = false;
+          break;
+        }
+        ptx::tc_fence_after();
+        if (active) {
+#pragma unroll
+          for (int g = 0; g < HALF; g += 16) {
+            uint32_t raw[16];
+            ptx::tmem_ld16(t_row + buf * F::BN + g, raw);
+            ptx::tmem_wait_ld();
+#pragma unroll
+            for (int j = 0; j < 8; ++j)
+              sum[g / 2 + j] = add2(sum[g / 2 + j], pack2(__uint_as_float(raw[2 * j]), __uint_as_float(raw[2 * j + 1])));
+          }
+        }
+        ptx::tc_fence_before();
+        __syncwarp();
+        if (lane == 0) ptx::mbar_arrive(ptx::smem_u32(&acc_empty[buf]));
+      }
+      if (!ok) break;
+      float acc[HALF];
+#pragma unroll
+      for (int j = 0; j < HALF / 2; ++j)
+        unpack2(F::NP == 3 ? mul2(sum[j], pack2(kUnscale, kUnscale)) : sum[j], acc[2 * j], acc[2 * j + 1]);
+      if constexpr (F::NP == 3) {
+        // sums to compute again: not finite, or below the smallest and not zero (2 bits - 1 drops the
+        // sign and wraps zero to the largest value)
+        constexpr uint32_t LO = 2u * kSmallestBits - 1u;
+        uint32_t low = 0xffffffffu;
+        float high = 0.f;
+#pragma unroll
+        for (int j = 0; j < HALF; ++j) {
+          low = min(low, 2u * __float_as_uint(acc[j]) - 1u);
+          asm("max.NaN.f32 %0, %0, %1;" : "+f"(high) : "f"(fabsf(acc[j])));
+        }
+        if (row_ok && (low < LO || !(high < INFINITY))) {
+          const float* pa = a.A[ti.b] + (a.a_mn ? gi : gi * a.lda);
+          const float* pb = a.B[ti.b] + (a.b_mn ? gj0 : gj0 * a.ldb);
+          const long ak = a.a_mn ? a.lda : 1, bc = a.b_mn ? 1 : a.ldb, bk = a.b_mn ? a.ldb : 1;
+#pragma unroll
+          for (int g = 0; g < HALF; g += 16) {
+            uint32_t mask = 0;
+#pragma unroll
+            for (int j = 0; j < 16; ++j) {
+              if (g + j < cols && (2u * __float_as_uint(acc[g + j]) - 1u < LO || !(fabsf(acc[g + j]) < INFINITY)))
+                mask |= 1u << j;
+            }
+            if (mask == 0) continue;
+            float v[16];
+            split_redo(pa, ak, pb + g * bc, bc, bk, cols - g, (int)a.k, v);
+#pragma unroll
+            for (int j = 0; j < 16; ++j)
+              if ((mask >> j) & 1u) acc[g + j] = v[j];
+          }
+        }
+      }
+#pragma unroll
+      for (int g = 0; g < HALF; g += G) {
+        if (!EARLY_C && read_c) load_c(g);
+        float* cp = C + (long)g * a.ldc;
+        asm volatile("" : "+l"(cp));
+#pragma unroll
+        for (int j = 0; j < G; ++j) acc[g + j] = fmaf(acc[g + j], a.alpha, read_c ? a.beta * cv[j] : 0.0f);
+        if (!row_ok) continue;
+        if (cols == HALF) {
+#pragma unroll
+          for (int j = 0; j < G; ++j, cp += a.ldc) __stcs(cp, acc[g + j]);
+        } else {
+#pragma unroll
+          for (int j = 0; j < G; ++j, cp += a.ldc)
+            if (g + j < cols) __stcs(cp, acc[g + j]);
+        }
+      }
+    }
+  }
+  ptx::tc_fence_before();
+  __syncthreads();
+  if (warp == 16) {
+    ptx::tc_fence_after();
+    ptx::tmem_dealloc(tmem, F::TMEM_COLS);
+  }
+}
+
+template <class F>
+cudaError_t launch_split(const BatchDesc& d, cudaStream_t st) {
+  SplitArgs a{};
+  a.m = d.m; a.n = d.n; a.k = d.k; a.lda = d.lda; a.ldb = d.ldb; a.ldc = d.ldc;
+  a.A = (const float* const*)d.A;
+  a.B = (const float* const*)d.B;
+  a.C = (float* const*)d.C;
+  a.alpha = d.alpha_f;
+  a.beta = d.beta_f;
+  a.a_mn = d.transa == SSBLAS_OP_N;
+  a.b_mn = d.transb == SSBLAS_OP_T;
+  const long tm = (d.m + 127) / 128, tn = (d.n + F::BN - 1) / F::BN;
+  a.tiles_m = (uint32_t)tm;
+  a.tiles_mn = (uint32_t)(tm * tn);
+  a.total = (uint32_t)(tm * tn * d.batch);
+  a.err = device_error_flag();
+  if (settings().fault == SSBLAS_FAULT_SKIP_COPY) {
+    settings().fault = SSBLAS_FAULT_NONE;
+    a.skip = 1;
+    a.wait_limit = 1u << 10;
+  }
+  auto kern = f32_split_kernel<F>;
+  static bool attr[kMaxDevices] = {};
+  if (cudaError_t e = smem_attr_once(attr, kern, F::SMEM)) return e;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(a.total < (uint32_t)num_sms() ? a.total : (unsigned)num_sms(), 1, 1);
+  cfg.blockDim = dim3(kSplitThreads, 1, 1);
+  cfg.dynamicSmemBytes = F::SMEM;
+  cfg.stream = st;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  ProfScope prof(F::NP == 3 ? "f32_split" : "bf16x3_split", st);
+  note_launch();
+  return cudaLaunchKernelEx(&cfg, kern, a);
+}
+
+template <int NP>
+cudaError_t launch_split_np(const BatchDesc& d, cudaStream_t st) {
+  if (!tcgen05_available()) return cudaErrorNotSupported;
+  if (d.k >= (1L << 31) || d.m >= (1L << 31) || d.n >= (1L << 31) || d.lda >= (1L << 25) || d.ldb >= (1L << 25))
+    return cudaErrorNotSupported;
+  const long tm = (d.m + 127) / 128, t64 = tm * ((d.n + 63) / 64) * d.batch, t128 = tm * ((d.n + 127) / 128) * d.batch;
+  if (t64 >= (1L << 31)) return cudaErrorNotSupported;
+  const long sms = num_sms();
+  if (d.m <= 64 && d.n <= 64) return launch_split<Split<NP, 64, 64>>(d, st);
+  // a 64-column chunk takes about two thirds of a 128-column one (measured: 1250 against 1900
+  // cycles), so the narrow tile is taken where it saves a third of the waves or more
+  const bool narrow = d.n <= 64 || (t64 + sms - 1) / sms * 2 < (t128 + sms - 1) / sms * 3;
+  return narrow ? launch_split<Split<NP, 128, 64>>(d, st) : launch_split<Split<NP, 128, 128>>(d, st);
+}
+
+}  // namespace
+
+cudaError_t launch_f32_split(const BatchDesc& d, int parts, cudaStream_t st) {
+  return parts == 3 ? launch_split_np<3>(d, st) : launch_split_np<2>(d, st);
+}
+
+}  // namespace ssb

@@ -260,13 +260,24 @@ SimtArgs<T> make_args(const BatchDesc& d) {
 
 }  // namespace
 
-cudaError_t launch_simt_gemm(const BatchDesc& d, cudaStream_t stream) {
+int simt_config(const BatchDesc& d) {
   // Large tiles when both dimensions fill them and there is enough work to occupy the GPU with
   // them, small tiles otherwise (the tuning table or a forced configuration can override).
   const long big_tiles = ((d.m + 127) / 128) * ((d.n + 127) / 128) * d.batch;
   const bool big_default = d.m >= 128 && d.n >= 128 && big_tiles >= 2L * num_sms();
-  const int cfg = choose_config(SSBLAS_PATH_SIMT, d.m, d.n, d.k, d.batch,
-                                d.row == ROW_F32 ? (big_default ? 4 : d.k <= 64 ? 5 : 3) : (big_default ? 1 : 0));
+  const int cores = d.row == ROW_F32 ? (big_default ? 4 : d.k <= 64 ? 5 : 3) : (big_default ? 1 : 0);
+  // Plain fp32 takes the BF16 tensor cores from k = 128 on. Below, its error against 64 bits can be
+  // larger than that of the FFMA kernels (a truncated sum of 16 products against chains of so few
+  // rounded ones: entries with outliers, k = 64: 7.0e-8 against 6.4e-8; k = 128: 7.4e-8 against
+  // 8.0e-8; k = 1024: 1.2e-7 against 2.0e-7; U[-1,1), k = 1024: 1.2e-7 against 5.8e-7). The line
+  // depends on k alone, so a result does not depend on how many instances share the call.
+  const int best = d.row == ROW_F32 && d.k >= 128 && !d.exact_f32 ? kSimtF32Split : cores;
+  const int cfg = choose_config(SSBLAS_PATH_SIMT, d.m, d.n, d.k, d.batch, best);
+  return cfg == kSimtF32Split && (d.row != ROW_F32 || d.exact_f32) ? cores : cfg;
+}
+
+cudaError_t launch_simt_gemm(const BatchDesc& d, cudaStream_t stream) {
+  const int cfg = simt_config(d);
   // fp32: configurations 3, 4 and 5 are the cp.async-pipelined kernels (gemm_sgemm.cu)
   if (d.row == ROW_F32 && cfg >= 3) return launch_sgemm_async(d, cfg, stream);
   const bool big = cfg == 1;

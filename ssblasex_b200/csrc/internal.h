@@ -97,6 +97,13 @@ int* device_error_flag();
 
 // ---- kernel entry points (each returns a CUDA error code; launches on `stream`) ----
 cudaError_t launch_simt_gemm(const BatchDesc& d, cudaStream_t stream);
+// configuration of the plain fp32 / fp64 / int8 fallback kernels for this call; kSimtF32Split = the
+// fp32 row takes the tensor cores (launch_f32_split)
+constexpr int kSimtF32Split = 14;
+int simt_config(const BatchDesc& d);
+// fp32 on the BF16 tensor cores with the operands split in the kernel: parts = 3 (plain fp32) or
+// 2 (the 3xBF16 emulation); cudaErrorNotSupported where the sizes do not fit
+cudaError_t launch_f32_split(const BatchDesc& d, int parts, cudaStream_t stream);
 // plain fp32 with a cp.async pipeline (config 3: 64 x 64 tiles, 4: 128 x 128)
 cudaError_t launch_sgemm_async(const BatchDesc& d, int config, cudaStream_t stream);
 // plain fp32 with TMA staging (gemm_sgemm_tma.cu); cudaErrorNotSupported unless the instances are

@@ -583,15 +583,21 @@ cudaError_t launch_ozaki_gemm_on(const BatchDesc& d, int S, const int8_t* pa, co
 cudaError_t launch_bf16x3_f32(const BatchDesc& d, cudaStream_t st) {
   if (!is_sm100() || !encoder()) return cudaErrorNotSupported;
   if (d.m > (1L << 31) || d.n > (1L << 31) || d.k > (1L << 31)) return cudaErrorNotSupported;
-  // configurations: 0 / 1 = split pass then tiled GEMM with 64- / 128-column tiles; 2 = one
-  // kernel that splits in shared memory, for equally spaced instances of at most 128 x 128 (the
-  // others take configuration 0 / 1) -- the default where it applies: on 4096 x 64^3 TT it takes
-  // 0.069 ms against 0.084 + 0.072 ms for the split pass and the tiled GEMM
-  const int fallback = bf16x3_small_fits(d) ? 2 : d.n <= 64 ? 0 : 1;
+  // configurations: 0 / 1 = split pass then tiled GEMM with 64- / 128-column tiles; 2 = one kernel
+  // fed by TMA that splits in shared memory, for equally spaced instances of at most 128 x 128 (the
+  // others take configuration 0 / 1); 3 = one kernel that splits the tiles of any instances as it
+  // loads them (f32_split.cu). Default: 2 where it applies (4096 x 64^3 TT: 0.057 ms against
+  // 0.084 + 0.072 ms for the split pass and the tiled GEMM), else 3 (256 x 256^3 NT: 0.053 against
+  // 0.130 ms; 16 x 1024^3: 0.170 ms).
+  const int fallback = bf16x3_small_fits(d) ? 2 : 3;
   const int cfg = choose_config(SSBLAS_PATH_BF16X3_TCGEN05, d.m, d.n, d.k, d.batch, fallback);
   cudaError_t e;
   if (cfg == 2 && bf16x3_small_fits(d)) {
     e = launch_bf16x3_small(d, st);
+    if (e != cudaErrorNotSupported) return e;
+  }
+  if (cfg == 3) {
+    e = launch_f32_split(d, 2, st);
     if (e != cudaErrorNotSupported) return e;
   }
   const long Kp = round_up(d.k, 8);

@@ -1,0 +1,155 @@
+"""Plain fp32 and 3xBF16 on the BF16 tensor cores with the operands split inside the kernel
+(f32_split.cu), against the FP64-exact oracle.
+
+Tolerance of the plain form, derived from its arithmetic, in units of u = 2^-24 times
+|alpha| |op(A)||op(B)| + |beta||C|: per chunk of 32 k two truncations at full magnitude (2 u each) and
+the rounding of the small products (below 2^-7 of it) make at most 5 u, left-out products at most
+1 u, every chunk sum is rounded once when it is added (k / 32 u), alpha and beta 2 u: k / 32 + 8."""
+import ctypes as ct
+
+import numpy as np
+import pytest
+
+from oracle import oracle as O
+
+pytestmark = pytest.mark.gpu
+U = 2.0 ** -24
+
+
+@pytest.fixture(scope="module")
+def S():
+    import torch
+    assert torch.cuda.is_available()
+    import ssblasex_b200 as S
+    S.set_math_mode(S.SSBLAS_MATH_PLAIN)
+    S.set_sync_mode(True)
+    yield S
+    S.set_math_mode(S.SSBLAS_MATH_PLAIN)
+
+
+def problem(ta, tb, m, n, k, batch, beta, pads, seed, dist="uniform"):
+    from ssblasex_b200 import workloads as W
+    ar, br = (m if ta == 0 else k), (k if tb == 0 else n)
+    return W.make_problem("f32", ta, tb, m, n, k, batch, 0.75, beta, lda=ar + pads[0], ldb=br + pads[1],
+                          ldc=m + pads[2], seed=seed, dist=dist)
+
+
+def run(S, p, pad=0, C=None):
+    """One call with host arrays of device pointers; each instance starts `pad` floats further on, so odd
+    pads break the 16-byte alignment and the spacing."""
+    import torch
+    bufs, ptrs = [], []
+    for X in (p.A, p.B, p.C if C is None else C):
+        per = X[0].size + pad
+        flat = torch.full((pad + per * p.batch,), float("nan"), dtype=torch.float32, device="cuda")
+        for b in range(p.batch):
+            flat[pad + b * per: pad + b * per + X[b].size] = torch.from_numpy(X[b].reshape(-1)).cuda()
+        bufs.append(flat)
+        ptrs.append((ct.c_void_p * p.batch)(*[flat.data_ptr() + 4 * (pad + b * per) for b in range(p.batch)]))
+    al, be = np.array([p.alpha], np.float32), np.array([p.beta], np.float32)
+    st = S.lib().ssblasGemmBatchedEx(p.transa, p.transb, p.m, p.n, p.k, al.ctypes.data, ptrs[0], S.SSBLAS_R_32F, p.lda,
+                                     ptrs[1], S.SSBLAS_R_32F, p.ldb, be.ctypes.data, ptrs[2], S.SSBLAS_R_32F, p.ldc,
+                                     p.batch, 0, 0)
+    assert st == 0
+    flat, per = bufs[2].cpu().numpy(), p.C[0].size + pad
+    return np.stack([flat[pad + b * per: pad + b * per + p.C[0].size] for b in range(p.batch)]).reshape(p.C.shape)
+
+
+@pytest.mark.parametrize("ta,tb", [(0, 0), (0, 1), (1, 0), (1, 1)])
+@pytest.mark.parametrize("shape", [(64, 64, 128, 5), (65, 63, 129, 3), (128, 128, 160, 2), (129, 65, 191, 2),
+                                   (1, 1, 128, 3), (127, 257, 255, 2), (300, 200, 161, 40), (40, 30, 300, 700)])
+@pytest.mark.parametrize("pads,pad,beta", [((0, 0, 0), 0, 0.0), ((4, 8, 4), 0, 0.25), ((3, 1, 2), 1, -1.5)])
+def test_plain_against_exact(S, ta, tb, shape, pads, pad, beta):
+    m, n, k, batch = shape
+    p = problem(ta, tb, m, n, k, batch, beta, pads, 31 + m + 2 * ta + tb, "outliers" if m == 300 else "uniform")
+    C0 = p.C.copy()
+    if beta == 0.0:                       # beta == 0 never reads C
+        C0.reshape(batch, n, -1)[:, :, :m] = np.nan
+    C = run(S, p, pad, C0)
+    assert S.last_run_info()["path"] == "f32_tcgen05"
+    for b in range(0, batch, max(1, batch // 3)):
+        ex, nrm = O.exact_f64(p, b)
+        err = np.abs(p.c_view(C, b).astype(np.float64) - ex)
+        assert np.all(err <= (k / 32 + 8) * U * nrm)
+    np.testing.assert_array_equal(C.reshape(batch, n, -1)[:, :, m:], C0.reshape(batch, n, -1)[:, :, m:])
+
+
+@pytest.mark.parametrize("ta,tb", [(0, 0), (1, 1)])
+@pytest.mark.parametrize("kind", ["inf", "nan", "huge", "tiny", "zero"])
+def test_plain_ends_of_the_range(S, ta, tb, kind):
+    """Inf, NaN, values that round to Inf in BF16 or overflow when scaled, subnormals and elements
+    whose low bits are below BF16's range: what an FFMA chain gives. Inf and NaN exactly; the others within
+    the FP32 bound of the exact product, with FP32's own underflow (2^-149 per term)."""
+    m, n, k = 70, 90, 140
+    p = problem(ta, tb, m, n, k, 2, 0.0, (0, 0, 0), 5)
+    rng = np.random.default_rng(3)
+    opa, opb = p.op_a(0), p.op_b(0)
+    if kind == "inf":
+        opa[3, 7], opb[9, 11], opb[:, 20] = np.inf, -np.inf, 0.0
+    elif kind == "nan":
+        opa[69, 139], opb[0, 0] = np.nan, np.nan
+    elif kind == "huge":
+        opa[5, :], opb[:, 6] = 3.395e38 * np.sign(opa[5, :]), opb[:, 6] * np.float32(2.0 ** -100)
+        opa[6, :] = opa[6, :] * np.float32(2.0 ** 110)
+    elif kind == "tiny":
+        opa[2, :] = (rng.integers(-2 ** 20, 2 ** 20, k) * 2.0 ** -149).astype(np.float32)
+        opb[:, 4] = (rng.standard_normal(k) * 2.0 ** -115).astype(np.float32)
+        opa[8, :] = 0.0
+        opa[8, 1], opb[1, 5] = np.float32(1.2345678e-35), 1.0
+    else:
+        opa[:], opb[:, ::2] = 0.0, 0.0
+    C = run(S, p)
+    S.set_kernel_config("simt", 3)
+    try:
+        R = run(S, p)
+    finally:
+        S.set_kernel_config("simt", -1)
+    got, ref = p.c_view(C, 0), p.c_view(R, 0)
+    if kind in ("inf", "nan"):
+        np.testing.assert_array_equal(np.isnan(got), np.isnan(ref))
+        np.testing.assert_array_equal(got[np.isinf(ref)], ref[np.isinf(ref)])
+        np.testing.assert_array_equal(np.isinf(got), np.isinf(ref))
+    ok = np.isfinite(ref)
+    A, B = opa.astype(np.float64), opb.astype(np.float64)
+    A, B = np.where(np.isfinite(A), A, 0.0), np.where(np.isfinite(B), B, 0.0)
+    ex, nrm = 0.75 * (A @ B), 0.75 * (np.abs(A) @ np.abs(B))
+    with np.errstate(over="ignore", invalid="ignore"):
+        fine = ok & (nrm < 2.0 ** 127)
+        assert np.all(np.abs(got.astype(np.float64) - ex)[fine] <= (4 * k * U * nrm + k * 2.0 ** -149)[fine])
+    np.testing.assert_array_equal(np.isfinite(got), ok)
+
+
+@pytest.mark.parametrize("ta,tb", [(0, 0), (0, 1), (1, 0), (1, 1)])
+@pytest.mark.parametrize("shape", [(200, 130, 31, 3), (129, 64, 33, 2), (50, 300, 100, 4), (64, 64, 1, 3)])
+@pytest.mark.parametrize("pad", [0, 1])
+def test_bf16x3_split_in_kernel(S, ta, tb, shape, pad):
+    """Configuration 3 of the 3xBF16 mode: the products of the emulation oracle, accumulated in FP32."""
+    m, n, k, batch = shape
+    p = problem(ta, tb, m, n, k, batch, 0.25, (pad, pad, 3), 77 + m + 2 * ta + tb, "outliers")
+    S.set_math_mode(S.SSBLAS_MATH_FP32_BF16X3)
+    S.set_kernel_config("bf16x3_tcgen05", 3)
+    try:
+        C = run(S, p, pad)
+        info = S.last_run_info()
+    finally:
+        S.set_kernel_config("bf16x3_tcgen05", -1)
+        S.set_math_mode(S.SSBLAS_MATH_PLAIN)
+    assert info["path"] == "bf16x3_tcgen05" and info["kernel_launches"] == 1
+    for b in range(batch):
+        emu = O.bf16x3_f32(p, b)
+        _, nrm = O.exact_f64(p, b)
+        assert np.max(np.abs(p.c_view(C, b).astype(np.float64) - emu) / nrm) <= 4 * k * U
+    np.testing.assert_array_equal(C.reshape(batch, n, -1)[:, :, m:], p.C.reshape(batch, n, -1)[:, :, m:])
+
+
+def test_skipped_chunk_is_reported(S):
+    """A converter signal that never comes: the waits run out, the call reports it, the next is right."""
+    p = problem(0, 0, 200, 200, 200, 3, 0.0, (0, 0, 0), 9)
+    assert S.set_fault_injection(S.SSBLAS_FAULT_SKIP_COPY) == 0
+    from ssblasex_b200 import runner
+    dp = runner.DeviceProblem(p)
+    st, _ = runner.call(p, mode="host_array", dp=dp)
+    assert st == S.SSBLAS_STATUS_INTERNAL_ERROR and S.last_run_info()["device_error"] != 0
+    C = run(S, p)
+    ex, nrm = O.exact_f64(p, 0)
+    assert np.all(np.abs(p.c_view(C, 0).astype(np.float64) - ex) <= (200 / 32 + 8) * U * nrm)
