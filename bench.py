@@ -325,7 +325,7 @@ def run_reference_arm(args):
 def grouped_leg(S, count: int, steps: int, warmup: int, stream):
     """10,000 uneven GEMMs (m, n, k log-uniform in [8, 512]; half fp64 in the Ozaki mode, half
     fp32 in the 3xBF16 mode) through one ssblasGemmGroupedBatchedEx call per step (pre-pass and
-    persistent GEMM launches replayed from a CUDA graph), against the same instances as one plain
+    persistent GEMM launches of a cached plan), against the same instances as one plain
     ssblasGemmBatchedEx launch each (asynchronous, back to back). Both on the library stream,
     timed with CUDA events."""
     import torch

@@ -619,65 +619,88 @@ ssblasStatus_t check_device_error(cudaStream_t st) {
 static ssblasStatus_t map_err(cudaError_t e);
 static void* pinned(size_t bytes, cudaError_t* err);
 
-// Grouped call with device-resident matrices: validation of every group (the batched call's
-// rules), pointer arrays made device-resident, then grouped_run (grouped.cu). Returns
-// SSBLAS_STATUS_NOT_COMPUTED_ERROR when the matrices are in host memory, which the caller then
-// stages group by group.
-static ssblasStatus_t grouped_device(
-    const ssblasOperation_t transa_array[], const ssblasOperation_t transb_array[],
-    const SSINT m_array[], const SSINT n_array[], const SSINT k_array[],
-    const void* const alpha_array[], const void* const A[], const ssblasDataType_t Atype_array[],
-    const SSINT lda_array[], const void* const B[], const ssblasDataType_t Btype_array[],
-    const SSINT ldb_array[], const void* const beta_array[], void* const C[],
-    const ssblasDataType_t Ctype_array[], const SSINT ldc_array[], SSINT group_count,
-    const SSINT group_size[]) {
-  GroupedDesc g;
+// The scalars of the groups by value; false where an alpha or beta is missing or C has a type that no row
+// has (the validation then answers).
+static bool grouped_scalars(const void* const alpha_array[], const void* const beta_array[], GroupedArgs& a) {
+  a.scalars.assign(2 * (size_t)a.groups, 0);
+  for (SSINT gi = 0; gi < a.groups; ++gi) {
+    const ssblasDataType_t c = a.ctype[gi];
+    if (!alpha_array[gi] || !beta_array[gi] || (c != SSBLAS_R_64F && c != SSBLAS_R_32F && c != SSBLAS_R_32I)) return false;
+    const size_t bytes = c == SSBLAS_R_64F ? 8 : 4;
+    memcpy(&a.scalars[2 * gi], alpha_array[gi], bytes);
+    memcpy(&a.scalars[2 * gi + 1], beta_array[gi], bytes);
+  }
+  return true;
+}
+
+// Validation of every group (the batched call's rules), and its instances.
+static ssblasStatus_t grouped_instances(const GroupedArgs& a, const void* const alpha_array[],
+                                        const void* const beta_array[], GroupedDesc& g) {
   long total = 0;
-  for (SSINT gi = 0; gi < group_count; ++gi) {
-    Rowsel rs = select_row(Atype_array[gi], Btype_array[gi], Ctype_array[gi]);
+  for (SSINT gi = 0; gi < a.groups; ++gi) {
+    Rowsel rs = select_row(a.atype[gi], a.btype[gi], a.ctype[gi]);
     if (!rs.ok) return SSBLAS_STATUS_INVALID_VALUE;
-    const int ta = transa_array[gi], tb = transb_array[gi];
+    const int ta = a.transa[gi], tb = a.transb[gi];
     if ((ta != SSBLAS_OP_N && ta != SSBLAS_OP_T) || (tb != SSBLAS_OP_N && tb != SSBLAS_OP_T))
       return SSBLAS_STATUS_INVALID_VALUE;
-    const long m = m_array[gi], n = n_array[gi], k = k_array[gi];
-    if (m <= 0 || n <= 0 || group_size[gi] <= 0) return SSBLAS_STATUS_INTERNAL_ERROR;
+    const long m = a.m[gi], n = a.n[gi], k = a.k[gi];
+    if (m <= 0 || n <= 0 || a.group_size[gi] <= 0) return SSBLAS_STATUS_INTERNAL_ERROR;
     if (!alpha_array[gi] || !beta_array[gi]) return SSBLAS_STATUS_INVALID_VALUE;
     const long arows = (ta == SSBLAS_OP_N) ? m : k, brows = (tb == SSBLAS_OP_N) ? k : n;
-    if (k > 0 && (lda_array[gi] < arows || ldb_array[gi] < brows)) return SSBLAS_STATUS_INVALID_VALUE;
-    if (ldc_array[gi] < m) return SSBLAS_STATUS_INVALID_VALUE;
+    if (k > 0 && (a.lda[gi] < arows || a.ldb[gi] < brows)) return SSBLAS_STATUS_INVALID_VALUE;
+    if (a.ldc[gi] < m) return SSBLAS_STATUS_INVALID_VALUE;
     GroupedInst in{};
     in.row = rs.row; in.transa = ta; in.transb = tb;
-    in.m = m; in.n = n; in.k = k; in.lda = lda_array[gi]; in.ldb = ldb_array[gi]; in.ldc = ldc_array[gi];
+    in.m = m; in.n = n; in.k = k; in.lda = a.lda[gi]; in.ldb = a.ldb[gi]; in.ldc = a.ldc[gi];
     if (rs.row == ROW_F32) { in.alpha_f = *(const float*)alpha_array[gi]; in.beta_f = *(const float*)beta_array[gi]; }
     else if (rs.row == ROW_F64) { in.alpha_d = *(const double*)alpha_array[gi]; in.beta_d = *(const double*)beta_array[gi]; }
     else { in.alpha_i = *(const int32_t*)alpha_array[gi]; in.beta_i = *(const int32_t*)beta_array[gi]; }
-    for (SSINT j = 0; j < group_size[gi]; ++j) {
+    for (SSINT j = 0; j < a.group_size[gi]; ++j) {
       in.idx = total++;
       g.inst.push_back(in);
     }
   }
+  return SSBLAS_STATUS_SUCCESS;
+}
+
+// Grouped call with device-resident matrices. A call that repeats the shapes and scalars of a cached
+// plan (compared value by value: they were valid then) skips the validation and the tables; the
+// pointer arrays are its own. Returns SSBLAS_STATUS_NOT_COMPUTED_ERROR when the matrices are in host
+// memory, which the caller then stages group by group.
+static ssblasStatus_t grouped_device(GroupedArgs& args, const void* const alpha_array[],
+                                     const void* const beta_array[], const void* const A[], const void* const B[],
+                                     void* const C[]) {
   std::lock_guard<std::mutex> lock(g_mutex);
+  GroupedPlan* plan = grouped_scalars(alpha_array, beta_array, args) ? grouped_find(args) : nullptr;
+  GroupedDesc g;
+  if (!plan) {
+    const ssblasStatus_t v = grouped_instances(args, alpha_array, beta_array, g);
+    if (v != SSBLAS_STATUS_SUCCESS) return v;
+  }
   g_info = ssblasRunInfo_t{};
   if (settings().math_mode & SSBLAS_MATH_FP64_OZAKI) {
     // the grouped kernels are built for 7 slices: a fixed other count, or a tolerance that needs
     // 8, cannot be honoured (a looser tolerance is met by 7 slices as well)
-    bool any_f64 = false;
+    bool any_f64 = plan && grouped_has_f64(*plan);
     for (const GroupedInst& in : g.inst) any_f64 |= in.row == ROW_F64;
     const int S = ozaki_slices_for_call();
     if (any_f64 && (settings().ozaki_slices != 0 ? S != 7 : S > 7)) return SSBLAS_STATUS_NOTIMPLEMENTED_ERROR;
   }
   cudaStream_t st = settings().stream;
   cudaError_t e;
+  GroupedPtrs ptrs;
   const bool dev_arrays = kind_of((const void*)A) == PK_DEVICE;
   if (dev_arrays) {
     if (kind_of((const void*)B) != PK_DEVICE || kind_of((const void*)C) != PK_DEVICE)
       return SSBLAS_STATUS_INVALID_VALUE;
-    g.A = A; g.B = B; g.C = C;
+    ptrs = {A, B, C};
   } else {
     if (kind_of((const void*)B) == PK_DEVICE || kind_of((const void*)C) == PK_DEVICE)
       return SSBLAS_STATUS_INVALID_VALUE;
     if (kind_of(A[0]) != PK_DEVICE) return SSBLAS_STATUS_NOT_COMPUTED_ERROR;
     if (kind_of(B[0]) != PK_DEVICE || kind_of(C[0]) != PK_DEVICE) return SSBLAS_STATUS_INVALID_VALUE;
+    long total = 0;
+    for (SSINT gi = 0; gi < args.groups; ++gi) total += args.group_size[gi];
     void* h = pinned(3 * sizeof(void*) * total, &e);
     if (!h) return map_err(e);
     void** hp = (void**)h;
@@ -688,11 +711,10 @@ static ssblasStatus_t grouped_device(
     if (!dp) return map_err(e);
     if ((e = cudaMemcpyAsync(dp, hp, 3 * sizeof(void*) * total, cudaMemcpyHostToDevice, st))) return map_err(e);
     pinned_done(st);
-    g.A = (const void* const*)dp;
-    g.B = (const void* const*)(dp + total);
-    g.C = (void* const*)(dp + 2 * total);
+    ptrs = {(const void* const*)dp, (const void* const*)(dp + total), (void* const*)(dp + 2 * total)};
   }
-  if ((e = grouped_run(g, st)) != cudaSuccess) return map_err(e);
+  if (!plan && (e = grouped_make(g, args, st, &plan)) != cudaSuccess) return map_err(e);
+  if ((e = grouped_launch(*plan, ptrs, st)) != cudaSuccess) return map_err(e);
   if (settings().synchronous) {
     if ((e = cudaStreamSynchronize(st)) != cudaSuccess) return map_err(e);
     return check_device_error(st);
@@ -992,9 +1014,8 @@ ssblasStatus_t ssblasGemmBatchedEx_64(ssblasOperation_t transa, ssblasOperation_
   return st;
 }
 
-// Grouped batched GEMM. Validation follows the batched call for each group; groups run in order
-// on the library stream. (The persistent single-launch scheduler replaces this loop when all
-// groups are device-resident; see grouped.cu.)
+// Grouped batched GEMM. Validation follows the batched call for each group; device-resident groups
+// run together (grouped.cu), groups of host matrices in order on the library stream.
 ssblasStatus_t ssblasGemmGroupedBatchedEx(
     const ssblasOperation_t transa_array[], const ssblasOperation_t transb_array[],
     const SSINT m_array[], const SSINT n_array[], const SSINT k_array[],
@@ -1009,10 +1030,9 @@ ssblasStatus_t ssblasGemmGroupedBatchedEx(
       !Atype_array || !lda_array || !B || !Btype_array || !ldb_array || !beta_array || !C ||
       !Ctype_array || !ldc_array || !group_size)
     return SSBLAS_STATUS_INVALID_VALUE;
-  ssblasStatus_t st = grouped_device(transa_array, transb_array, m_array, n_array, k_array,
-                                     alpha_array, A, Atype_array, lda_array, B, Btype_array,
-                                     ldb_array, beta_array, C, Ctype_array, ldc_array, group_count,
-                                     group_size);
+  GroupedArgs args{transa_array, transb_array, m_array, n_array, k_array, lda_array, ldb_array, ldc_array,
+                   group_size, Atype_array, Btype_array, Ctype_array, group_count, {}};
+  ssblasStatus_t st = grouped_device(args, alpha_array, beta_array, A, B, C);
   if (st != SSBLAS_STATUS_NOT_COMPUTED_ERROR) return st;
   // host matrices (the reference's convention): each group through the batched path
   long off = 0;

@@ -239,14 +239,14 @@ cudaError_t launch_layout(const DmmaArgs& a, bool a_mn, bool b_mn, cudaStream_t 
 }
 
 template <bool A_MN, bool B_MN>
-cudaError_t launch_grouped_layout(const GroupedSimt& s, int lay, cudaStream_t st) {
+cudaError_t launch_grouped_layout(const GroupedSimt& s, const GroupedPtrs& p, int lay, cudaStream_t st) {
   constexpr int SMEM = kGST * DmmaSmem<kGBM, kGBM, kGBK>::STAGE * 8;
   auto kern = dmma_grouped_kernel<A_MN, B_MN>;
   static bool attr[kMaxDevices] = {};
   if (cudaError_t e = smem_attr_once(attr, kern, SMEM)) return e;
   kern<<<(unsigned)s.ndmma[lay], (kGBM / kGW) * (kGBM / kGW) * 32, SMEM, st>>>(
-      (const SimtGInst*)s.inst64, (const int*)s.dmma_tiles[lay], (const double* const*)s.A,
-      (const double* const*)s.B, (double* const*)s.C);
+      (const SimtGInst*)s.inst64, (const int*)s.dmma_tiles[lay], (const double* const*)p.A,
+      (const double* const*)p.B, (double* const*)p.C);
   note_launch();
   return cudaGetLastError();
 }
@@ -255,17 +255,17 @@ cudaError_t launch_grouped_layout(const GroupedSimt& s, int lay, cudaStream_t st
 
 // The plain fp64 tiles of a grouped call, one launch per op(A) / op(B) layout present
 // (layout index = 2 * (op(A) rows contiguous) + (op(B) columns contiguous)).
-cudaError_t launch_dmma_grouped(const GroupedSimt& s, cudaStream_t st) {
+cudaError_t launch_dmma_grouped(const GroupedSimt& s, const GroupedPtrs& p, cudaStream_t st) {
   if (!s.ndmma[0] && !s.ndmma[1] && !s.ndmma[2] && !s.ndmma[3]) return cudaSuccess;
   ProfScope prof("dmma_grouped", st);
   cudaError_t e = cudaSuccess;
   for (int lay = 0; lay < 4 && e == cudaSuccess; ++lay) {
     if (!s.ndmma[lay]) continue;
     switch (lay) {
-      case 3: e = launch_grouped_layout<true, true>(s, lay, st); break;
-      case 2: e = launch_grouped_layout<true, false>(s, lay, st); break;
-      case 1: e = launch_grouped_layout<false, true>(s, lay, st); break;
-      default: e = launch_grouped_layout<false, false>(s, lay, st); break;
+      case 3: e = launch_grouped_layout<true, true>(s, p, lay, st); break;
+      case 2: e = launch_grouped_layout<true, false>(s, p, lay, st); break;
+      case 1: e = launch_grouped_layout<false, true>(s, p, lay, st); break;
+      default: e = launch_grouped_layout<false, false>(s, p, lay, st); break;
     }
   }
   return e;

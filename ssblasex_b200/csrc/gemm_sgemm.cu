@@ -647,31 +647,31 @@ cudaError_t launch_sl(const SgemmArgs& a, bool a_mn, bool b_mn, cudaStream_t st)
 }  // namespace
 
 template <bool A_MN, bool B_MN>
-cudaError_t launch_sgemm_grouped_layout(const GroupedSimt& s, int lay, cudaStream_t st) {
+cudaError_t launch_sgemm_grouped_layout(const GroupedSimt& s, const GroupedPtrs& p, int lay, cudaStream_t st) {
   constexpr int SMEM = kGST * kGBK * (2 * kGT + 8) * 4;
   auto kern = sgemm_grouped_kernel<A_MN, B_MN>;
   static bool attr[kMaxDevices] = {};
   if (cudaError_t e = smem_attr_once(attr, kern, SMEM)) return e;
   kern<<<(unsigned)s.nsg[lay], (kGT / kGTM) * (kGT / kGTM), SMEM, st>>>(
-      (const SimtGInst*)s.inst32, (const int*)s.sg_tiles[lay], (const float* const*)s.A, (const float* const*)s.B,
-      (float* const*)s.C);
+      (const SimtGInst*)s.inst32, (const int*)s.sg_tiles[lay], (const float* const*)p.A, (const float* const*)p.B,
+      (float* const*)p.C);
   note_launch();
   return cudaGetLastError();
 }
 
 // The plain fp32 tiles of a grouped call, one launch per op(A) / op(B) layout present (layout
 // index = 2 * (op(A) rows contiguous) + (op(B) columns contiguous)).
-cudaError_t launch_sgemm_grouped(const GroupedSimt& s, cudaStream_t st) {
+cudaError_t launch_sgemm_grouped(const GroupedSimt& s, const GroupedPtrs& p, cudaStream_t st) {
   if (!s.nsg[0] && !s.nsg[1] && !s.nsg[2] && !s.nsg[3]) return cudaSuccess;
   ProfScope prof("sgemm_grouped", st);
   cudaError_t e = cudaSuccess;
   for (int lay = 0; lay < 4 && e == cudaSuccess; ++lay) {
     if (!s.nsg[lay]) continue;
     switch (lay) {
-      case 3: e = launch_sgemm_grouped_layout<true, true>(s, lay, st); break;
-      case 2: e = launch_sgemm_grouped_layout<true, false>(s, lay, st); break;
-      case 1: e = launch_sgemm_grouped_layout<false, true>(s, lay, st); break;
-      default: e = launch_sgemm_grouped_layout<false, false>(s, lay, st); break;
+      case 3: e = launch_sgemm_grouped_layout<true, true>(s, p, lay, st); break;
+      case 2: e = launch_sgemm_grouped_layout<true, false>(s, p, lay, st); break;
+      case 1: e = launch_sgemm_grouped_layout<false, true>(s, p, lay, st); break;
+      default: e = launch_sgemm_grouped_layout<false, false>(s, p, lay, st); break;
     }
   }
   return e;

@@ -387,7 +387,6 @@ cudaError_t plan_simt_grouped(const GroupedDesc& g, const std::vector<int>& memb
       return e;
   out.ntiles32 = (long)t32.size() / 3;
   out.ntiles64 = (long)t64.size() / 3;
-  out.A = g.A; out.B = g.B; out.C = g.C;
   out.launches = (out.ntiles32 ? 1 : 0) + (out.ntiles64 ? 1 : 0);
   for (int l = 0; l < 4; ++l) {
     out.ndmma[l] = (long)tdl[l].size() / 3;
@@ -397,19 +396,19 @@ cudaError_t plan_simt_grouped(const GroupedDesc& g, const std::vector<int>& memb
   return cudaStreamSynchronize(st);
 }
 
-cudaError_t launch_simt_grouped(const GroupedSimt& s, cudaStream_t st) {
+cudaError_t launch_simt_grouped(const GroupedSimt& s, const GroupedPtrs& p, cudaStream_t st) {
   if (!s.ntiles32 && !s.ntiles64) return cudaSuccess;
   ProfScope prof("simt_grouped", st);
   if (s.ntiles32) {
     simt_grouped_kernel<float, 64, 64, 16, 4, 4><<<(unsigned)s.ntiles32, 256, 0, st>>>(
-        (const SimtGInst*)s.inst32, (const int*)s.tiles32, (const float* const*)s.A, (const float* const*)s.B,
-        (float* const*)s.C);
+        (const SimtGInst*)s.inst32, (const int*)s.tiles32, (const float* const*)p.A, (const float* const*)p.B,
+        (float* const*)p.C);
     note_launch();
   }
   if (s.ntiles64) {
     simt_grouped_kernel<double, 64, 64, 16, 4, 4><<<(unsigned)s.ntiles64, 256, 0, st>>>(
-        (const SimtGInst*)s.inst64, (const int*)s.tiles64, (const double* const*)s.A, (const double* const*)s.B,
-        (double* const*)s.C);
+        (const SimtGInst*)s.inst64, (const int*)s.tiles64, (const double* const*)p.A, (const double* const*)p.B,
+        (double* const*)p.C);
     note_launch();
   }
   return cudaGetLastError();

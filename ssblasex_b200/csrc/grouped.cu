@@ -13,7 +13,9 @@
 // Plain fp32 instances run on the cp.async FFMA tiles (gemm_sgemm.cu), plain fp64 ones on the FP64
 // tensor cores (gemm_dmma.cu), one launch per op(A) / op(B) layout present.
 //
-// The sequence is captured once per distinct call signature into a CUDA graph and replayed.
+// The tables of a call (instances, tiles, work items, buffer offsets) depend on its shapes only and
+// are kept as a plan; a call whose shapes, scalars and settings equal a cached plan's launches it on its
+// own pointer arrays.
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 #include <stdint.h>
@@ -43,7 +45,8 @@ __device__ __forceinline__ uint32_t swz(int r, int c, int KB) {
 }
 
 struct GPrepInst {
-  const void* const* X;  // pointer array (A or B) of the call
+  int from_b;            // the matrix is in the call's B array (else A)
+  int pad_;
   long idx;              // instance position in the pointer array
   long rows, K, ld;
   int kcontig;
@@ -76,6 +79,8 @@ template <> struct GElem<2> { using T = double; };
 
 template <int MODE, int S, int KB, int RTILE_A, int RTILE_B>
 __global__ void __launch_bounds__(GNT, MODE == 2 ? 6 : MODE == 0 ? 6 : 8) gprep_kernel(const GPrepInst* __restrict__ items, const uint2* __restrict__ work,
+                                                    const void* const* __restrict__ ptrA,
+                                                    const void* const* __restrict__ ptrB,
                                                     uint8_t* __restrict__ outA, uint8_t* __restrict__ outB,
                                                     int32_t* __restrict__ exps) {
   using T = typename GElem<MODE>::T;
@@ -101,7 +106,7 @@ __global__ void __launch_bounds__(GNT, MODE == 2 ? 6 : MODE == 0 ? 6 : 8) gprep_
   const bool is_b = (wk.x & 1) != 0;
   const int RTILE = is_b ? RTILE_B : RTILE_A;
   uint8_t* out = (is_b ? outB : outA) + it.off;
-  const T* X = (const T*)it.X[it.idx];
+  const T* X = (const T*)(it.from_b ? ptrB : ptrA)[it.idx];
   const long gr0 = (long)wk.y * GRT;                        // first row (of the padded range)
   const int rt = (int)(gr0 / RTILE), rr0 = (int)(gr0 % RTILE);
   const long K = it.K, ld = it.ld;
@@ -317,8 +322,8 @@ void plan_kind(const GroupedDesc& g, const std::vector<int>& members, KindPlan<C
     for (int a = 0; a < tm; ++a)
       for (int b = 0; b < tn; ++b) kp.tiles.push_back(GTile{li, a, b});
     // op(A) as rows x K (K contiguous when A is transposed), op(B)^T likewise
-    const GPrepInst opa{g.A, in.idx, in.m, in.k, in.lda, in.transa == SSBLAS_OP_T, 0, gi.nk, 0, 0};
-    const GPrepInst opb{(const void* const*)g.B, in.idx, in.n, in.k, in.ldb, in.transb == SSBLAS_OP_N, 0, gi.nk, 0, 0};
+    const GPrepInst opa{0, 0, in.idx, in.m, in.k, in.lda, in.transa == SSBLAS_OP_T, 0, gi.nk, 0, 0};
+    const GPrepInst opb{1, 0, in.idx, in.n, in.k, in.ldb, in.transb == SSBLAS_OP_N, 0, gi.nk, 0, 0};
     GPrepInst pa = swap ? opb : opa, pb = swap ? opa : opb;   // tile rows, tile columns
     pa.tiles = tm; pa.off = gi.offA; pa.eoff = gi.offEA;
     pb.tiles = tn; pb.off = gi.offB; pb.eoff = gi.offEB;
@@ -370,14 +375,14 @@ cudaError_t upload_kind(const KindPlan<Cfg>& kp, KindDev& kd, cudaStream_t st) {
 }
 
 template <class Cfg, int MODE, int S>
-cudaError_t launch_kind(const KindDev& kd, void* const* C, cudaStream_t st, const char* prep_name,
+cudaError_t launch_kind(const KindDev& kd, const GroupedPtrs& ptrs, cudaStream_t st, const char* prep_name,
                         const char* gemm_name, bool dynamic_order) {
   if (kd.ninst == 0) return cudaSuccess;
   {
     ProfScope prof(prep_name, st);
     if (kd.nwork >= (1L << 31)) return cudaErrorInvalidValue;
     gprep_kernel<MODE, S, Cfg::KB, Cfg::BM, Cfg::BN><<<(unsigned)kd.nwork, GNT, 0, st>>>(
-        (const GPrepInst*)kd.prep.p, (const uint2*)kd.work.p, (uint8_t*)kd.packA.p, (uint8_t*)kd.packB.p,
+        (const GPrepInst*)kd.prep.p, (const uint2*)kd.work.p, ptrs.A, ptrs.B, (uint8_t*)kd.packA.p, (uint8_t*)kd.packB.p,
         (int32_t*)kd.exps.p);
     note_launch();
     cudaError_t e = cudaGetLastError();
@@ -388,7 +393,7 @@ cudaError_t launch_kind(const KindDev& kd, void* const* C, cudaStream_t st, cons
   tc::Params prm{};
   prm.total_tiles = kd.ntiles;
   prm.tiles_m = prm.tiles_n = 1;
-  prm.C = C;
+  prm.C = ptrs.C;
   prm.exp_a = (const int32_t*)kd.exps.p;
   prm.exp_b = (const int32_t*)kd.exps.p;
   prm.exp_shift = -12;
@@ -399,7 +404,7 @@ cudaError_t launch_kind(const KindDev& kd, void* const* C, cudaStream_t st, cons
   prm.packA = (const uint8_t*)kd.packA.p;
   prm.packB = (const uint8_t*)kd.packB.p;
   prm.queue = dynamic_order ? (unsigned long long*)kd.queue.p : nullptr;
-  // the device-side tile queue starts at tile 0 on every launch (a memset node when captured)
+  // the device-side tile queue starts at tile 0 on every launch
   if (dynamic_order) {
     cudaError_t e = cudaMemsetAsync(kd.queue.p, 0, sizeof(unsigned long long), st);
     if (e != cudaSuccess) return e;
@@ -421,24 +426,38 @@ using GCfgOz32 = tc::Config<tc::KIND_I8, 7, 7, 32, 32, 6, 7, 2, tc::EPI_OZAKI, 2
 using GCfgBf = tc::Config<tc::KIND_BF16, 2, 2, 64, 128, 4, 1, 2, tc::EPI_F32, 1>;
 using GCfgI8 = tc::Config<tc::KIND_I8, 1, 1, 128, 128, 6, 1, 2, tc::EPI_I32, 0>;
 
-// A prepared grouped call: device tables and packed buffers per kind, the plain-instance batch,
-// and (after the first replay request) the captured CUDA graph of all its launches.
-struct Plan {
-  std::vector<uint64_t> key;
+}  // namespace
+
+// A prepared grouped call: device tables and packed buffers per kind, and the plain-instance batch.
+// The packed buffers are scratch of the calls that run it, so those are ordered: an event follows each
+// use, and a call on another stream waits for it.
+struct GroupedPlan {
+  std::vector<char> shapes;            // the argument arrays, back to back
+  std::vector<uint64_t> scalars, settings;
   bool dynamic = true;       // tiles from the device-side queue (else the static stride)
+  bool has_f64 = false;
   // Ozaki instances by tile shape: oz on 128 x 32 tiles with two accumulators, oz_wide on
   // 128 x 64 tiles with one (chosen per instance size bucket)
   KindDev oz, oz_wide, bf, i8;
   std::unique_ptr<GroupedSimt> simt;
-  void* const* C = nullptr;
-  cudaGraphExec_t exec = nullptr;
-  int launches = 0;
-  ~Plan() {
-    if (exec) cudaGraphExecDestroy(exec);
+  size_t scratch = 0;        // bytes of packed operand buffers
+  cudaEvent_t used = nullptr;
+  cudaStream_t last_stream = nullptr;
+  bool in_use = false;
+  unsigned long tick = 0;
+  ~GroupedPlan() {
+    if (used) cudaEventDestroy(used);
   }
 };
 
-std::map<int, std::unique_ptr<Plan>> g_plans;   // one cached plan per device
+namespace {
+
+// Cached plans per device: at most kMaxPlans, and beyond the newest one only as long as their scratch
+// stays within kMaxScratch. Host access is under the library lock.
+constexpr size_t kMaxPlans = 4;
+constexpr size_t kMaxScratch = (size_t)2 << 30;
+std::map<int, std::vector<std::unique_ptr<GroupedPlan>>> g_plans;
+unsigned long g_plan_tick = 0;
 
 // Tile shape of one Ozaki instance: 128 x 64 tiles with one accumulator read the slice planes from
 // shared memory a third more efficiently per product than 128 x 32 tiles with two, whose gain is
@@ -453,49 +472,52 @@ bool ozaki_wide_tiles(const GroupedInst& in, int gcfg) {
   return choose_config(SSBLAS_PATH_GROUPED_OZAKI_TILE, in.m, in.n, in.k, 1, 1) == 0;
 }
 
-std::vector<uint64_t> signature(const GroupedDesc& g, int mode, int oz_cfg) {
-  std::vector<uint64_t> k;
-  k.reserve(g.inst.size() * 12 + 8);
-  k.push_back((uint64_t)mode | ((uint64_t)oz_cfg << 32));
-  // a forced DMMA configuration decides whether plain fp64 instances take the tensor cores
-  k.push_back((uint64_t)(int64_t)forced_config(SSBLAS_PATH_DMMA));
-  k.push_back((uint64_t)(int64_t)forced_config(SSBLAS_PATH_SIMT));
-  k.push_back((uint64_t)(uintptr_t)g.A);
-  k.push_back((uint64_t)(uintptr_t)g.B);
-  k.push_back((uint64_t)(uintptr_t)g.C);
-  for (const auto& in : g.inst) {
-    uint64_t f[12];
-    f[0] = (uint64_t)in.row | ((uint64_t)in.transa << 8) | ((uint64_t)in.transb << 16);
-    f[1] = in.m; f[2] = in.n; f[3] = in.k; f[4] = in.lda; f[5] = in.ldb; f[6] = in.ldc; f[7] = in.idx;
-    memcpy(&f[8], &in.alpha_d, 8);
-    memcpy(&f[9], &in.beta_d, 8);
-    uint64_t t;
-    memcpy(&t, &in.alpha_f, 4);
-    f[10] = t | ((uint64_t)(uint32_t)in.alpha_i << 32);
-    memcpy(&t, &in.beta_f, 4);
-    f[11] = (t & 0xffffffffu) | ((uint64_t)(uint32_t)in.beta_i << 32);
-    k.insert(k.end(), f, f + 12);
-  }
+// Settings a plan depends on besides its arguments.
+std::vector<uint64_t> plan_settings() {
+  std::vector<uint64_t> k{(uint64_t)settings().math_mode, (uint64_t)tuning_generation()};
+  for (int path : {(int)SSBLAS_PATH_GROUPED, (int)SSBLAS_PATH_GROUPED_OZAKI_TILE, (int)SSBLAS_PATH_DMMA,
+                   (int)SSBLAS_PATH_SIMT})
+    k.push_back((uint64_t)(int64_t)forced_config(path));
   return k;
 }
 
-cudaError_t run_plan(Plan& pl, cudaStream_t st) {
-  cudaError_t e;
-  if ((e = launch_kind<GCfgOz, 2, 7>(pl.oz_wide, pl.C, st, "grouped_ozaki_slice", "grouped_ozaki_gemm", pl.dynamic)))
-    return e;
-  if ((e = launch_kind<GCfgOz32, 2, 7>(pl.oz, pl.C, st, "grouped_ozaki_slice", "grouped_ozaki_gemm", pl.dynamic)))
-    return e;
-  if ((e = launch_kind<GCfgBf, 1, 1>(pl.bf, pl.C, st, "grouped_split_bf16", "grouped_bf16x3_gemm", pl.dynamic))) return e;
-  if ((e = launch_kind<GCfgI8, 0, 1>(pl.i8, pl.C, st, "grouped_pack_i8", "grouped_i8_gemm", pl.dynamic))) return e;
-  if (pl.simt && (e = launch_simt_grouped(*pl.simt, st))) return e;
-  if (pl.simt && (e = launch_dmma_grouped(*pl.simt, st))) return e;
-  if (pl.simt && (e = launch_sgemm_grouped(*pl.simt, st))) return e;
-  return cudaSuccess;
+// f(array, bytes) over the argument arrays until it returns false
+template <class F>
+bool each_array(const GroupedArgs& a, F f) {
+  const size_t g = (size_t)a.groups;
+  for (const SSINT* v : {a.m, a.n, a.k, a.lda, a.ldb, a.ldc, a.group_size})
+    if (!f((const char*)v, g * sizeof(SSINT))) return false;
+  for (const ssblasOperation_t* v : {a.transa, a.transb})
+    if (!f((const char*)v, g * sizeof(*v))) return false;
+  for (const ssblasDataType_t* v : {a.atype, a.btype, a.ctype})
+    if (!f((const char*)v, g * sizeof(*v))) return false;
+  return true;
 }
 
 }  // namespace
 
-cudaError_t grouped_run(const GroupedDesc& g, cudaStream_t st) {
+GroupedPlan* grouped_find(const GroupedArgs& a) {
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess) return nullptr;
+  auto it = g_plans.find(dev);
+  if (it == g_plans.end()) return nullptr;
+  const std::vector<uint64_t> key = plan_settings();
+  for (auto& p : it->second) {
+    if (p->scalars != a.scalars || p->settings != key) continue;
+    size_t at = 0;
+    const bool same = each_array(a, [&](const char* v, size_t n) {
+      if (at + n > p->shapes.size() || memcmp(p->shapes.data() + at, v, n) != 0) return false;
+      at += n;
+      return true;
+    });
+    if (same && at == p->shapes.size()) return p.get();
+  }
+  return nullptr;
+}
+
+bool grouped_has_f64(const GroupedPlan& plan) { return plan.has_f64; }
+
+cudaError_t grouped_make(const GroupedDesc& g, const GroupedArgs& a, cudaStream_t st, GroupedPlan** out) {
   const int mode = settings().math_mode;
   int dev = 0;
   cudaError_t e = cudaGetDevice(&dev);
@@ -504,46 +526,18 @@ cudaError_t grouped_run(const GroupedDesc& g, cudaStream_t st) {
   // the tile shape of each Ozaki instance from its size bucket (SSBLAS_PATH_GROUPED_OZAKI_TILE),
   // dynamic tile queue; 2 = every Ozaki instance on 128 x 32 tiles, static tile order
   const int gcfg = choose_config(SSBLAS_PATH_GROUPED, 0, 0, 0, 0, 1);
-  const bool dynamic_order = gcfg != 2;
-  std::vector<uint64_t> key = signature(g, mode, gcfg);
-  auto it = g_plans.find(dev);
-  if (it != g_plans.end() && it->second->key == key) {
-    Plan& pl = *it->second;
-    if (pl.exec == nullptr) {
-      // second call with this signature: capture the launch sequence into a graph
-      cudaStream_t cs;
-      if ((e = cudaStreamCreateWithFlags(&cs, cudaStreamNonBlocking))) return e;
-      cudaGraph_t graph;
-      const int before = 0;
-      (void)before;
-      if ((e = cudaStreamBeginCapture(cs, cudaStreamCaptureModeThreadLocal))) {
-        cudaStreamDestroy(cs);
-        return e;
-      }
-      cudaError_t er = run_plan(pl, cs);
-      e = cudaStreamEndCapture(cs, &graph);
-      cudaStreamDestroy(cs);
-      if (er) return er;
-      if (e) return e;
-      e = cudaGraphInstantiate(&pl.exec, graph, 0);
-      cudaGraphDestroy(graph);
-      if (e) return e;
-    }
-    ProfScope prof("grouped_graph", st);
-    e = cudaGraphLaunch(pl.exec, st);
-    note_launch(pl.launches);
-    note_path(SSBLAS_PATH_GROUPED, 7);
-    return e;
-  }
-
-  // new signature: build the plan
-  auto pl = std::make_unique<Plan>();
-  pl->key = std::move(key);
-  pl->dynamic = dynamic_order;
-  pl->C = g.C;
+  auto pl = std::make_unique<GroupedPlan>();
+  pl->settings = plan_settings();
+  pl->scalars = a.scalars;
+  each_array(a, [&](const char* v, size_t n) {
+    pl->shapes.insert(pl->shapes.end(), v, v + n);
+    return true;
+  });
+  pl->dynamic = gcfg != 2;
   std::vector<int> oz, oz_wide, bf, i8, plain;
   for (int i = 0; i < (int)g.inst.size(); ++i) {
     const GroupedInst& in = g.inst[i];
+    pl->has_f64 |= in.row == ROW_F64;
     if (in.k <= 0) continue;   // C untouched, as in the reference
     if (in.row == ROW_I8) i8.push_back(i);
     else if (in.row == ROW_F64 && (mode & SSBLAS_MATH_FP64_OZAKI) && in.k <= 16384)
@@ -551,30 +545,70 @@ cudaError_t grouped_run(const GroupedDesc& g, cudaStream_t st) {
     else if (in.row == ROW_F32 && (mode & SSBLAS_MATH_FP32_BF16X3)) bf.push_back(i);
     else plain.push_back(i);
   }
+  // make room first: the evicted plans' buffers may be what the new one needs (cudaFree waits for
+  // the work that reads them)
+  auto& plans = g_plans[dev];
+  auto evict_oldest = [&] {
+    size_t old = 0;
+    for (size_t i = 1; i < plans.size(); ++i)
+      if (plans[i]->tick < plans[old]->tick) old = i;
+    plans.erase(plans.begin() + (long)old);
+  };
+  if (plans.size() >= kMaxPlans) evict_oldest();
   {
     KindPlan<GCfgOz32> k1;
     plan_kind(g, oz, k1);
-    if ((e = upload_kind(k1, pl->oz, st))) return e;
     KindPlan<GCfgOz> k0;
     plan_kind(g, oz_wide, k0);
-    if ((e = upload_kind(k0, pl->oz_wide, st))) return e;
     KindPlan<GCfgBf> k2;
     plan_kind(g, bf, k2);
-    if ((e = upload_kind(k2, pl->bf, st))) return e;
     KindPlan<GCfgI8> k3;
     plan_kind(g, i8, k3);
+    pl->scratch = (size_t)(k0.bytesA + k0.bytesB + k1.bytesA + k1.bytesB + k2.bytesA + k2.bytesB + k3.bytesA + k3.bytesB);
+    auto total = [&] {
+      size_t s = pl->scratch;
+      for (auto& p : plans) s += p->scratch;
+      return s;
+    };
+    while (!plans.empty() && total() > kMaxScratch) evict_oldest();
+    if ((e = upload_kind(k1, pl->oz, st))) return e;
+    if ((e = upload_kind(k0, pl->oz_wide, st))) return e;
+    if ((e = upload_kind(k2, pl->bf, st))) return e;
     if ((e = upload_kind(k3, pl->i8, st))) return e;
   }
   if (!plain.empty()) {
     pl->simt = std::make_unique<GroupedSimt>();
     if ((e = plan_simt_grouped(g, plain, *pl->simt, st))) return e;
   }
-  pl->launches = (pl->oz.ninst ? 2 : 0) + (pl->oz_wide.ninst ? 2 : 0) + (pl->bf.ninst ? 2 : 0) +
-                 (pl->i8.ninst ? 2 : 0) + (pl->simt ? pl->simt->launches : 0);
-  g_plans[dev] = std::move(pl);
-  Plan& p = *g_plans[dev];
-  note_path(SSBLAS_PATH_GROUPED, (p.oz.ninst || p.oz_wide.ninst) ? 7 : 0);
-  return run_plan(p, st);
+  if ((e = cudaEventCreateWithFlags(&pl->used, cudaEventDisableTiming)) != cudaSuccess) return e;
+  plans.push_back(std::move(pl));
+  *out = plans.back().get();
+  return cudaSuccess;
+}
+
+cudaError_t grouped_launch(GroupedPlan& pl, const GroupedPtrs& p, cudaStream_t st) {
+  cudaError_t e;
+  pl.tick = ++g_plan_tick;
+  note_path(SSBLAS_PATH_GROUPED, (pl.oz.ninst || pl.oz_wide.ninst) ? 7 : 0);
+  // (a stream that is being captured runs later, and in the order that the caller gives its graph)
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(st, &cap) != cudaSuccess) cudaGetLastError();
+  const bool captured = cap != cudaStreamCaptureStatusNone;
+  if (!captured && pl.in_use && pl.last_stream != st && (e = cudaStreamWaitEvent(st, pl.used, 0)) != cudaSuccess) return e;
+  if ((e = launch_kind<GCfgOz, 2, 7>(pl.oz_wide, p, st, "grouped_ozaki_slice", "grouped_ozaki_gemm", pl.dynamic)))
+    return e;
+  if ((e = launch_kind<GCfgOz32, 2, 7>(pl.oz, p, st, "grouped_ozaki_slice", "grouped_ozaki_gemm", pl.dynamic)))
+    return e;
+  if ((e = launch_kind<GCfgBf, 1, 1>(pl.bf, p, st, "grouped_split_bf16", "grouped_bf16x3_gemm", pl.dynamic))) return e;
+  if ((e = launch_kind<GCfgI8, 0, 1>(pl.i8, p, st, "grouped_pack_i8", "grouped_i8_gemm", pl.dynamic))) return e;
+  if (pl.simt && (e = launch_simt_grouped(*pl.simt, p, st))) return e;
+  if (pl.simt && (e = launch_dmma_grouped(*pl.simt, p, st))) return e;
+  if (pl.simt && (e = launch_sgemm_grouped(*pl.simt, p, st))) return e;
+  if (captured) return cudaSuccess;
+  if ((e = cudaEventRecord(pl.used, st)) != cudaSuccess) return e;
+  pl.in_use = true;
+  pl.last_stream = st;
+  return cudaSuccess;
 }
 
 void grouped_release() { g_plans.clear(); }

@@ -22,10 +22,18 @@ struct GroupedInst {
 
 struct GroupedDesc {
   std::vector<GroupedInst> inst;
-  const void* const* A;      // device arrays of device pointers
-  const void* const* B;
-  void* const* C;
 };
+
+// The shape arguments of a grouped call as the caller passes them (no pointer array), and the scalars
+// of its groups by value (the bits of alpha, then beta, of each group).
+struct GroupedArgs {
+  const ssblasOperation_t *transa, *transb;
+  const SSINT *m, *n, *k, *lda, *ldb, *ldc, *group_size;
+  const ssblasDataType_t *atype, *btype, *ctype;
+  SSINT groups;
+  std::vector<uint64_t> scalars;
+};
+struct GroupedPlan;
 
 // plain fp32/fp64 instances of a grouped call (64 x 64 tiles: FFMA / DMMA kernels, or the SIMT
 // kernel where a forced configuration asks for it)
@@ -46,21 +54,31 @@ struct GroupedSimt {
   // fp32 tiles for the cp.async FFMA kernel (gemm_sgemm.cu), the same way; instances in inst32
   void* sg_tiles[4] = {};
   long nsg[4] = {};
-  const void* const* A = nullptr;
-  const void* const* B = nullptr;
-  void* const* C = nullptr;
   int launches = 0;
   ~GroupedSimt();
 };
 cudaError_t plan_simt_grouped(const GroupedDesc& g, const std::vector<int>& members, GroupedSimt& out,
                               cudaStream_t st);
-cudaError_t launch_simt_grouped(const GroupedSimt& s, cudaStream_t st);
-cudaError_t launch_dmma_grouped(const GroupedSimt& s, cudaStream_t st);
-cudaError_t launch_sgemm_grouped(const GroupedSimt& s, cudaStream_t st);
+// the pointer arrays (device arrays of device pointers) of a grouped call
+struct GroupedPtrs {
+  const void* const* A;
+  const void* const* B;
+  void* const* C;
+};
+cudaError_t launch_simt_grouped(const GroupedSimt& s, const GroupedPtrs& p, cudaStream_t st);
+cudaError_t launch_dmma_grouped(const GroupedSimt& s, const GroupedPtrs& p, cudaStream_t st);
+cudaError_t launch_sgemm_grouped(const GroupedSimt& s, const GroupedPtrs& p, cudaStream_t st);
 
-// Runs all instances with device-resident operands: one pre-pass and one persistent GEMM launch per
-// kind, replayed from a captured CUDA graph when the same call signature repeats.
-cudaError_t grouped_run(const GroupedDesc& g, cudaStream_t st);
+// A grouped call's device tables depend on its shapes, scalars and the settings only, so a plan serves
+// every call that repeats those values, whatever matrices it points to. grouped_find: the cached plan
+// of the current device for these arguments (compared value by value), nullptr if there is none.
+// grouped_make: a new plan (the arguments were validated), cached in place of the least recently
+// used one. grouped_launch: all instances with device-resident operands, one pre-pass and one
+// persistent GEMM launch per kind. grouped_has_f64: whether any instance is fp64.
+GroupedPlan* grouped_find(const GroupedArgs& a);
+cudaError_t grouped_make(const GroupedDesc& g, const GroupedArgs& a, cudaStream_t st, GroupedPlan** out);
+cudaError_t grouped_launch(GroupedPlan& plan, const GroupedPtrs& p, cudaStream_t st);
+bool grouped_has_f64(const GroupedPlan& plan);
 void grouped_release();
 
 }  // namespace ssb

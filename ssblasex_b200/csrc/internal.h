@@ -154,6 +154,8 @@ bool make_tiled_map(CUtensorMap* map, CUtensorMapDataType dt, int rank, const vo
 int choose_config(int path, long m, long n, long k, long batch, int fallback);
 // the configuration forced by ssblasSetKernelConfig for `path`, -1 if none
 int forced_config(int path);
+// number of times the tuning table was read again (ssblasReloadTuning)
+int tuning_generation();
 
 // Optional per-kernel CUDA-event timing (ssblasSetProfiling): records an event pair around each
 // launch on its stream; ssblasGetProfile resolves them. Each launch is also an NVTX range of the

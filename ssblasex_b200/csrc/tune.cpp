@@ -21,6 +21,7 @@ namespace {
 
 std::mutex g_tune_mutex;
 bool g_loaded = false;
+int g_generation = 0;   // how often the table was read again
 std::map<std::pair<int, std::string>, int> g_table;
 constexpr int kKeys = 16;
 int g_forced[kKeys] = {-1, -1, -1, -1, -1, -1, -1, -1, -1, -1, -1, -1, -1, -1, -1, -1};
@@ -80,6 +81,11 @@ int forced_config(int path) {
   return (path >= 0 && path < kKeys) ? g_forced[path] : -1;
 }
 
+int tuning_generation() {
+  std::lock_guard<std::mutex> lock(g_tune_mutex);
+  return g_generation;
+}
+
 }  // namespace ssb
 
 extern "C" ssblasStatus_t ssblasSetKernelConfig(int path, int config) {
@@ -92,6 +98,7 @@ extern "C" ssblasStatus_t ssblasSetKernelConfig(int path, int config) {
 extern "C" ssblasStatus_t ssblasReloadTuning(void) {
   std::lock_guard<std::mutex> lock(ssb::g_tune_mutex);
   ssb::g_table.clear();
+  ++ssb::g_generation;
   ssb::load_table();
   return SSBLAS_STATUS_SUCCESS;
 }
