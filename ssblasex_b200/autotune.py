@@ -61,7 +61,7 @@ FAMILIES = {
         dict(row="i8", transa=1, transb=0, m=256, n=256, k=1024, batch=512, alpha=1, beta=0,
              lda=1024, ldb=1024, ldc=256),
     ]),
-    "dmma": (SSBLAS_MATH_PLAIN, [0, 1, 3, 4], "dmma_gemm", [
+    "dmma": (SSBLAS_MATH_PLAIN, [0, 2], "(all)", [
         dict(row="f64", transa=0, transb=1, m=1024, n=1024, k=1024, batch=32, alpha=1.0, beta=0.0,
              lda=1032, ldb=1032, ldc=1032, dist="expspread"),
         dict(row="f64", transa=1, transb=0, m=128, n=128, k=128, batch=256, alpha=1.0, beta=0.5),

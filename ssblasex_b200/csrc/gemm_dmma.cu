@@ -6,7 +6,7 @@
 // multiply-add (src/include/GemmCore/Xgemm_kernel_sve_v4x5_1.hpp:93-127). The reference adds
 // alpha*acc once per 512-wide K block; here it is added once, which differs only by rounding.
 //
-// Design: one CTA per (BM x BN tile, instance). op(A) and op(B) tiles are copied into shared
+// Design: one CTA per (64 x 64 tile, instance). op(A) and op(B) tiles are copied into shared
 // memory by cp.async in a STAGES-deep ring (the copies for K step kt + STAGES - 1 are in flight
 // while step kt is multiplied), each in the orientation it has in global memory -- the copy
 // absorbs op(A)/op(B): an operand whose rows (m or n) are contiguous is staged [k][mn], one whose
@@ -64,39 +64,85 @@ struct DmmaSmem {
   static constexpr int STAGE = A_MAX + B_MAX;
 };
 
-// Copies the (rows x BK) slab of one operand at (r0, k0) into a stage buffer.
-// MN: rows contiguous in global memory (element (r, k) at X[r + k*ld]) -> staged [k][r];
-// otherwise element (r, k) at X[r*ld + k] -> staged [r][k].
+// One operand's copies by this thread: chunk q (two doubles along the contiguous dimension) of the next
+// K slab comes from src + q * step and goes to dst + q * DSTEP of the slab's buffer, so that a slab
+// inside the matrix costs one copy and one addition per chunk (with the position of every chunk
+// worked out again the copies took as many issue slots as the products' loads).
+//   MN: rows contiguous in global memory (element (r, k) at X[r + k*ld]) -> staged [k][r];
+//   otherwise element (r, k) at X[r*ld + k] -> staged [r][k].
 template <int ROWS, int BK, int NT, bool MN>
-__device__ __forceinline__ void load_slab(double* dst, const double* __restrict__ X, long nrows, long K, long ld,
-                                          long r0, long k0, bool vec) {
-  constexpr int P = MN ? ROWS + 4 : BK + 4;
-  constexpr int CHUNKS = ROWS * BK / 2;   // pairs of doubles
-  static_assert(CHUNKS % NT == 0, "slab/threads mismatch");
-  const int t = threadIdx.x;
-#pragma unroll
-  for (int q = 0; q < CHUNKS / NT; ++q) {
-    const int idx = t + q * NT;
-    int rr, kk;       // first element of the pair: pair runs along r (MN) or along k
-    if (MN) { kk = idx / (ROWS / 2); rr = 2 * (idx % (ROWS / 2)); }
-    else { rr = idx / (BK / 2); kk = 2 * (idx % (BK / 2)); }
-    const long gr = r0 + rr, gk = k0 + kk;
-    double* s = MN ? dst + kk * P + rr : dst + rr * P + kk;
-    // valid elements of the pair
-    long nvalid;
-    if (MN) nvalid = (gk < K) ? (nrows - gr < 2 ? nrows - gr : 2) : 0;
-    else nvalid = (gr < nrows) ? (K - gk < 2 ? K - gk : 2) : 0;
-    if (nvalid < 0) nvalid = 0;
-    const double* g = (nvalid > 0) ? (MN ? X + gr + gk * ld : X + gr * ld + gk) : X;
-    if (vec) {
-      cp16(smem_addr(s), g, (int)(8 * nvalid));
-    } else {
-      cp8(smem_addr(s), g, nvalid > 0 ? 8 : 0);
-      const double* g1 = (nvalid > 1) ? g + 1 : X;
-      cp8(smem_addr(s + 1), g1, nvalid > 1 ? 8 : 0);
-    }
+struct Slab {
+  static constexpr int P = MN ? ROWS + 4 : BK + 4;
+  static constexpr int CPL = (MN ? ROWS : BK) / 2;        // chunks per contiguous line
+  static constexpr int NQ = ROWS * BK / 2 / NT;           // chunks per thread
+  static constexpr int LSTEP = NT / CPL;                  // lines between a thread's chunks
+  static constexpr int DSTEP = LSTEP * P;                 // doubles between their places
+  static_assert(NT % CPL == 0 && NQ * NT == ROWS * BK / 2 && NQ * LSTEP == (MN ? BK : ROWS), "slab/threads mismatch");
+  const double* src;
+  const double* X;
+  long step, adv;            // doubles between chunks, between slabs
+  int k, kk;                 // valid k from the next slab on; k of this thread's first chunk in a slab
+  int lines, bytes;          // chunks of this thread inside the rows, and valid bytes of each (MN)
+  uint32_t dst;              // byte offset of its place
+  bool vec;
+  __device__ __forceinline__ void init(const double* __restrict__ X_, long nrows, long K, long ld, long r0) {
+    const int t = threadIdx.x;
+    X = X_;
+    vec = ((uintptr_t)X % 16 == 0) && (ld % 2 == 0);
+    const int rr = MN ? 2 * (t % CPL) : t / CPL;
+    kk = MN ? t / CPL : 2 * (t % CPL);
+    src = X + (MN ? r0 + rr + kk * ld : (r0 + rr) * ld + kk);
+    step = LSTEP * ld;
+    adv = MN ? BK * ld : BK;
+    const long left = nrows - r0 - rr;    // valid rows from this thread's first chunk on
+    lines = MN ? NQ : left >= ROWS ? NQ : left > 0 ? min(NQ, (int)((left + LSTEP - 1) / LSTEP)) : 0;
+    bytes = MN ? (left >= 2 ? 16 : left == 1 ? 8 : 0) : 16;
+    if (bytes == 0) lines = 0;
+    k = (int)K;
+    dst = 8u * (uint32_t)(MN ? kk * P + rr : rr * P + kk);
   }
-}
+  // The next slab into `buf` (shared-space address); moves on to the one after it. A slab with all of
+  // its k inside the matrix asks for fixed lines and bytes per thread; only the last one, where k runs
+  // out, looks at each chunk.
+  __device__ __forceinline__ void copy(uint32_t buf) {
+    const uint32_t d = buf + dst;
+    const double* s = src;
+    if (k >= BK) {
+      if (vec && lines == NQ && bytes == 16) {
+#pragma unroll
+        for (int q = 0; q < NQ; ++q, s += step) cp16(d + 8u * (uint32_t)(q * DSTEP), s, 16);
+      } else if (vec) {
+#pragma unroll
+        for (int q = 0; q < NQ; ++q, s += step)
+          cp16(d + 8u * (uint32_t)(q * DSTEP), q < lines ? s : X, q < lines ? bytes : 0);
+      } else {
+        const int b0 = bytes < 8 ? bytes : 8, b1 = bytes - b0;
+#pragma unroll
+        for (int q = 0; q < NQ; ++q, s += step) {
+          const bool ok = q < lines;
+          cp8(d + 8u * (uint32_t)(q * DSTEP), ok ? s : X, ok ? b0 : 0);
+          cp8(d + 8u * (uint32_t)(q * DSTEP + 1), ok && b1 ? s + 1 : X, ok ? b1 : 0);
+        }
+      }
+    } else {
+#pragma unroll
+      for (int q = 0; q < NQ; ++q, s += step) {
+        // valid elements of the chunk, which runs along r (MN) or along k
+        int nv = MN ? (kk + q * LSTEP < k ? bytes / 8 : 0) : (q < lines ? k - kk : 0);
+        nv = nv < 0 ? 0 : (nv > 2 ? 2 : nv);
+        const double* g = nv > 0 ? s : X;
+        if (vec) {
+          cp16(d + 8u * (uint32_t)(q * DSTEP), g, 8 * nv);
+        } else {
+          cp8(d + 8u * (uint32_t)(q * DSTEP), g, nv > 0 ? 8 : 0);
+          cp8(d + 8u * (uint32_t)(q * DSTEP + 1), nv > 1 ? g + 1 : X, nv > 1 ? 8 : 0);
+        }
+      }
+    }
+    src += adv;
+    k -= BK;
+  }
+};
 
 // One BM x BN tile of C = alpha op(A) op(B) + beta C for one instance, by the whole CTA: the K loop
 // over the stage ring, then the epilogue. Leaves the stage buffers free (every copy has landed and
@@ -112,8 +158,10 @@ __device__ __forceinline__ void dmma_tile(const double* __restrict__ A, const do
   const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
   const int wm = warp % NWM, wn = warp / NWM;
   const int fr = lane >> 2, fk = lane & 3;    // fragment row (m or n) and k within an 8x4 block
-  const bool vecA = ((uintptr_t)A % 16 == 0) && (lda % 2 == 0);
-  const bool vecB = ((uintptr_t)B % 16 == 0) && (ldb % 2 == 0);
+  Slab<BM, BK, NT, A_MN> ca;
+  Slab<BN, BK, NT, B_MN> cb;
+  ca.init(A, m, k, lda, m0);
+  cb.init(B, n, k, ldb, n0);
 
   double acc[MI][NI][2];
 #pragma unroll
@@ -121,19 +169,19 @@ __device__ __forceinline__ void dmma_tile(const double* __restrict__ A, const do
 #pragma unroll
     for (int j = 0; j < NI; ++j) acc[i][j][0] = acc[i][j][1] = 0.0;
 
-  const long ktiles = (k + BK - 1) / BK;
-  auto issue = [&](long kt) {
-    double* sa = smem + (kt % STAGES) * Sm::STAGE;
-    double* sb = sa + Sm::A_MAX;
-    load_slab<BM, BK, NT, A_MN>(sa, A, m, k, lda, m0, kt * BK, vecA);
-    load_slab<BN, BK, NT, B_MN>(sb, B, n, k, ldb, n0, kt * BK, vecB);
+  const int ktiles = (int)((k + BK - 1) / BK);
+  const uint32_t smem0 = smem_addr(smem);
+  auto issue = [&](int kt) {     // slabs in order, kt counts them
+    const uint32_t sa = smem0 + 8u * (uint32_t)((kt % STAGES) * Sm::STAGE);
+    ca.copy(sa);
+    cb.copy(sa + 8u * Sm::A_MAX);
   };
 #pragma unroll
   for (int s = 0; s < STAGES - 1; ++s) {
     if (s < ktiles) issue(s);
     cp_commit();
   }
-  for (long kt = 0; kt < ktiles; ++kt) {
+  for (int kt = 0; kt < ktiles; ++kt) {
     cp_wait<STAGES - 2>();
     __syncthreads();
     if (kt + STAGES - 1 < ktiles) issue(kt + STAGES - 1);
@@ -189,62 +237,62 @@ __device__ __forceinline__ void dmma_tile(const double* __restrict__ A, const do
   }
 }
 
-template <int BM, int BN, int BK, int WM, int WN, int STAGES, int MINB, bool A_MN, bool B_MN>
-__global__ void __launch_bounds__((BM / WM) * (BN / WN) * 32, MINB) dmma_gemm_kernel(DmmaArgs args) {
+// Tiles: 64 x 64, 4 warps of 32 x 32, three 16-deep K slabs in flight (52 KB): with at most 170
+// registers a thread three CTAs share an SM, and one's barrier, copies and epilogue run beside the
+// others' products. 128 x 128 tiles with one CTA per SM left the FP64 pipe idle a third of the time (every
+// warp of the SM at the same barrier) and padded small and ragged sizes more. The pipe's own peak, measured
+// with operands in registers, is 36.9 TFLOP/s for every mma.sync f64 shape. Before -> after:
+// 32 x 1024^3 NT 2.39 -> 2.05 ms (33.6 TFLOP/s), 64 x (500 x 300 x 700) TN 0.867 -> 0.467 ms,
+// 100 x (200 x 150 x 300) NN with odd ld 0.197 -> 0.121 ms, 256 x 128^3 TN 0.0735 -> 0.061 ms.
+// Four slabs: 2.10, 0.518, 0.141, 0.073 ms; four CTAs of 128 registers: 2.13, 0.492, 0.124, 0.061 ms.
+constexpr int kBM = 64, kBN = 64, kBK = 16, kW = 32, kStages = 3, kMinBlocks = 3;
+constexpr int kDmmaThreads = (kBM / kW) * (kBN / kW) * 32;
+constexpr int kDmmaSmem = kStages * DmmaSmem<kBM, kBN, kBK>::STAGE * 8;
+
+template <bool A_MN, bool B_MN>
+__global__ void __launch_bounds__(kDmmaThreads, kMinBlocks) dmma_gemm_kernel(DmmaArgs args) {
   extern __shared__ __align__(16) double smem[];
-  const long tiles_m = (args.m + BM - 1) / BM;
-  const long m0 = (blockIdx.x % tiles_m) * BM;
-  const long n0 = (blockIdx.x / tiles_m) * BN;
+  const long tiles_m = (args.m + kBM - 1) / kBM;
+  const long m0 = (blockIdx.x % tiles_m) * kBM;
+  const long n0 = (blockIdx.x / tiles_m) * kBN;
   for (long b = blockIdx.y; b < args.batch; b += gridDim.y)
-    dmma_tile<BM, BN, BK, WM, WN, STAGES, A_MN, B_MN>(args.A[b], args.B[b], args.C[b], args.m, args.n, args.k,
-                                                       args.lda, args.ldb, args.ldc, args.alpha, args.beta, m0, n0,
-                                                       smem);
+    dmma_tile<kBM, kBN, kBK, kW, kW, kStages, A_MN, B_MN>(args.A[b], args.B[b], args.C[b], args.m, args.n, args.k,
+                                                         args.lda, args.ldb, args.ldc, args.alpha, args.beta, m0, n0,
+                                                         smem);
 }
 
 // Grouped form (plain fp64 instances of ssblasGemmGroupedBatchedEx): one CTA per (instance,
 // 64 x 64 tile) entry of a tile table whose instances all have this op(A) / op(B) layout.
-constexpr int kGBM = 64, kGBK = 16, kGW = 32, kGST = 4;
 template <bool A_MN, bool B_MN>
-__global__ void __launch_bounds__((kGBM / kGW) * (kGBM / kGW) * 32, 2)
+__global__ void __launch_bounds__(kDmmaThreads, kMinBlocks)
 dmma_grouped_kernel(const SimtGInst* __restrict__ inst, const int* __restrict__ tiles, const double* const* A,
                     const double* const* B, double* const* C) {
   extern __shared__ __align__(16) double smem[];
   const int* t = tiles + 3 * (long)blockIdx.x;
   const SimtGInst g = inst[t[0]];
-  dmma_tile<kGBM, kGBM, kGBK, kGW, kGW, kGST, A_MN, B_MN>(A[g.idx], B[g.idx], C[g.idx], g.m, g.n, g.k, g.lda, g.ldb,
-                                                          g.ldc, g.alpha_d, g.beta_d, (long)t[1] * kGBM,
-                                                          (long)t[2] * kGBM, smem);
+  dmma_tile<kBM, kBN, kBK, kW, kW, kStages, A_MN, B_MN>(A[g.idx], B[g.idx], C[g.idx], g.m, g.n, g.k, g.lda, g.ldb,
+                                                       g.ldc, g.alpha_d, g.beta_d, (long)t[1] * kBM,
+                                                       (long)t[2] * kBN, smem);
 }
 
-template <int BM, int BN, int BK, int WM, int WN, int STAGES, int MINB, bool A_MN, bool B_MN>
+template <bool A_MN, bool B_MN>
 cudaError_t launch_cfg(const DmmaArgs& a, cudaStream_t st) {
-  constexpr int NT = (BM / WM) * (BN / WN) * 32;
-  constexpr int SMEM = STAGES * DmmaSmem<BM, BN, BK>::STAGE * 8;
-  auto kern = dmma_gemm_kernel<BM, BN, BK, WM, WN, STAGES, MINB, A_MN, B_MN>;
+  auto kern = dmma_gemm_kernel<A_MN, B_MN>;
   static bool attr[kMaxDevices] = {};
-  if (cudaError_t e = smem_attr_once(attr, kern, SMEM)) return e;
-  const long tiles = ((a.m + BM - 1) / BM) * ((a.n + BN - 1) / BN);
+  if (cudaError_t e = smem_attr_once(attr, kern, kDmmaSmem)) return e;
+  const long tiles = ((a.m + kBM - 1) / kBM) * ((a.n + kBN - 1) / kBN);
   if (tiles > 0x7fffffffL) return cudaErrorInvalidValue;
   dim3 grid((unsigned)tiles, (unsigned)(a.batch < 65535 ? a.batch : 65535));
-  kern<<<grid, NT, SMEM, st>>>(a);
+  kern<<<grid, kDmmaThreads, kDmmaSmem, st>>>(a);
   return cudaGetLastError();
-}
-
-template <int BM, int BN, int BK, int WM, int WN, int STAGES, int MINB>
-cudaError_t launch_layout(const DmmaArgs& a, bool a_mn, bool b_mn, cudaStream_t st) {
-  if (a_mn && b_mn) return launch_cfg<BM, BN, BK, WM, WN, STAGES, MINB, true, true>(a, st);
-  if (a_mn) return launch_cfg<BM, BN, BK, WM, WN, STAGES, MINB, true, false>(a, st);
-  if (b_mn) return launch_cfg<BM, BN, BK, WM, WN, STAGES, MINB, false, true>(a, st);
-  return launch_cfg<BM, BN, BK, WM, WN, STAGES, MINB, false, false>(a, st);
 }
 
 template <bool A_MN, bool B_MN>
 cudaError_t launch_grouped_layout(const GroupedSimt& s, const GroupedPtrs& p, int lay, cudaStream_t st) {
-  constexpr int SMEM = kGST * DmmaSmem<kGBM, kGBM, kGBK>::STAGE * 8;
   auto kern = dmma_grouped_kernel<A_MN, B_MN>;
   static bool attr[kMaxDevices] = {};
-  if (cudaError_t e = smem_attr_once(attr, kern, SMEM)) return e;
-  kern<<<(unsigned)s.ndmma[lay], (kGBM / kGW) * (kGBM / kGW) * 32, SMEM, st>>>(
+  if (cudaError_t e = smem_attr_once(attr, kern, kDmmaSmem)) return e;
+  kern<<<(unsigned)s.ndmma[lay], kDmmaThreads, kDmmaSmem, st>>>(
       (const SimtGInst*)s.inst64, (const int*)s.dmma_tiles[lay], (const double* const*)p.A,
       (const double* const*)p.B, (double* const*)p.C);
   note_launch();
@@ -281,25 +329,13 @@ cudaError_t launch_dmma_f64(const BatchDesc& d, cudaStream_t st) {
   a.beta = d.beta_d;
   const bool a_mn = d.transa == SSBLAS_OP_N;   // op(A) rows (m) contiguous
   const bool b_mn = d.transb == SSBLAS_OP_T;   // op(B) columns (n) contiguous
-  // Configurations (ssblasSetKernelConfig(SSBLAS_PATH_DMMA, c)):
-  //   0: 64 x 64 tiles, 4 warps of 32 x 32, 16-deep K stages x 4
-  //   1: 128 x 128 tiles, 8 warps of 64 x 32, 16-deep K stages x 4
-  //   3: 128 x 128 tiles, 16 warps of 32 x 32, 16-deep K stages x 4
-  //   4: 128 x 128 tiles, 16 warps of 32 x 32, 32-deep K stages x 3
-  // (2 selects the DFMA SIMT kernel, handled by the caller). Default: configuration 4 when there
-  // are enough 128 x 128 tiles to fill the GPU (fastest on 32 x 1024^3: 2.40 ms against 2.54 for
-  // 3 and 2.60 for 1), else 0.
-  const long big_tiles = ((d.m + 127) / 128) * ((d.n + 127) / 128) * d.batch;
-  const bool big_default = d.m >= 128 && d.n >= 128 && big_tiles >= 2L * num_sms();
-  const int cfg = choose_config(SSBLAS_PATH_DMMA, d.m, d.n, d.k, d.batch, big_default ? 4 : 0);
+  // One configuration (2 selects the DFMA SIMT kernel, handled by the caller): see the tile constants.
   ProfScope prof("dmma_gemm", st);
   cudaError_t e;
-  switch (cfg) {
-    case 1: e = launch_layout<128, 128, 16, 64, 32, 4, 1>(a, a_mn, b_mn, st); break;
-    case 3: e = launch_layout<128, 128, 16, 32, 32, 4, 1>(a, a_mn, b_mn, st); break;
-    case 4: e = launch_layout<128, 128, 32, 32, 32, 3, 1>(a, a_mn, b_mn, st); break;
-    default: e = launch_layout<64, 64, 16, 32, 32, 4, 2>(a, a_mn, b_mn, st); break;
-  }
+  if (a_mn && b_mn) e = launch_cfg<true, true>(a, st);
+  else if (a_mn) e = launch_cfg<true, false>(a, st);
+  else if (b_mn) e = launch_cfg<false, true>(a, st);
+  else e = launch_cfg<false, false>(a, st);
   note_launch();
   return e;
 }
