@@ -2,7 +2,7 @@
 // through the caller's pointer array -- any transpose, any leading dimension -- and writes
 // K-major "planes" [instance][plane][rows][Kp] that the GEMM kernel stages with TMA.
 //
-//   pack_i8      one plane: the int8 values themselves (int8 row, layouts other than TN)
+//   align_i8     int8 operands off the 16-byte grid, copied line by line onto it (order kept)
 //   split_bf16   two planes: hi = bf16(x), lo = bf16(x - hi) of an fp32 value (both operands of a
 //                call in one launch)
 //   ozaki_slice  S planes of balanced int8 digits of an fp64 value under a per-row power-of-two
@@ -102,78 +102,75 @@ __device__ __forceinline__ void write_out(const uint8_t* st, uint8_t* out, long 
   write_rows<P, KT * BPE>(st, out, plane_stride, rows, Kp_bytes, row0, kbyte0);
 }
 
-// int8 -> K-major plane. A CTA takes 128 rows x 128 k of one instance (blocks: k tile fastest,
-// then row tile, then instance). K contiguous: already K-major, each thread copies 16-byte row
-// segments to the plane's pitch. Rows contiguous (element (r, k) at X[r + k*ld]): each thread
-// loads four 4 x 4 byte blocks as 32-bit words -- lane l of a warp takes rows 4l .. 4l+3, so one
-// load instruction reads 128 contiguous bytes -- transposes them in registers (byte permutes),
-// stages the 4-byte k runs of its rows in shared memory, and the CTA writes 16-byte row segments.
-// Positions past K (up to Kp) get zero bytes.
-constexpr int PKR = 128, PKK = 128;          // rows and k per CTA
-constexpr int PKP = PKK + 4;                 // staged row pitch (bytes)
-__global__ void __launch_bounds__(NTH) pack_i8_kernel(PlaneArgs a, long ktiles, long rtiles) {
-  __shared__ __align__(16) uint8_t st[PKR * PKP];
-  const long blk = blockIdx.x;
-  const long kt = blk % ktiles, rt = (blk / ktiles) % rtiles, b = blk / (ktiles * rtiles);
-  const long r0 = rt * PKR, k0 = kt * PKK;
-  const int8_t* X = (const int8_t*)a.X[b];
-  uint8_t* out = (uint8_t*)a.out + b * a.batch_stride;
-  const int t = threadIdx.x;
-  if (a.kcontig) {
-    const bool vec = ((uintptr_t)X % 16) == 0 && a.ld % 16 == 0;
+// An aligned 16-byte vector, or zeros without a load (a predicated load: a selection after it would wait
+// for the vector).
+__device__ __forceinline__ uint4 vector_if(bool ok, const uint8_t* p) {
+  uint4 v;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "setp.ne.u32 p, %5, 0;\n\t"
+      "mov.u32 %0, 0;\n\tmov.u32 %1, 0;\n\tmov.u32 %2, 0;\n\tmov.u32 %3, 0;\n\t"
+      "@p ld.global.nc.v4.u32 {%0, %1, %2, %3}, [%4];\n\t}"
+      : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
+      : "l"(p), "r"((uint32_t)ok));
+  return v;
+}
+__device__ __forceinline__ uint32_t keep_bytes(uint32_t w, int n) {   // the first n bytes of w, the others zero
+  return n >= 4 ? w : n > 0 ? w & ((1u << (8 * n)) - 1u) : 0u;
+}
+// bytes [off, off + 16) of the 32 bytes lo, hi (off in [0, 16))
+__device__ __forceinline__ uint4 bytes_from(const uint4 lo, const uint4 hi, uint32_t off) {
+  const bool two = off & 8u, one = off & 4u;
+  const uint32_t a0 = two ? lo.z : lo.x, a1 = two ? lo.w : lo.y, a2 = two ? hi.x : lo.z, a3 = two ? hi.y : lo.w,
+                 a4 = two ? hi.z : hi.x, a5 = two ? hi.w : hi.y;
+  const uint32_t b0 = one ? a1 : a0, b1 = one ? a2 : a1, b2 = one ? a3 : a2, b3 = one ? a4 : a3, b4 = one ? a5 : a4;
+  const uint32_t s = 8u * (off & 3u);
+  return make_uint4(__funnelshift_r(b0, b1, s), __funnelshift_r(b1, b2, s), __funnelshift_r(b2, b3, s),
+                    __funnelshift_r(b3, b4, s));
+}
+
+// int8 operands that TMA cannot address, copied line by line to a 16-byte grid: stored column c of the
+// instance at X + c * ld, `len` bytes, becomes the line out + c * pitch (pitch = len rounded up to 16), the
+// rest of the line zero. The order of the matrix is kept -- the GEMM reads either major -- so this is a
+// plain copy. Each thread makes four 16-byte vectors from the (up to) eight aligned vectors that hold
+// their bytes, all loads first; only vectors that hold a byte of the line are read. Blocks
+// [0, n0) of x copy the first operand, the others the second; y strides over the instances.
+// Bound by memory: 64 x (501 x 517 x 509) NN with ld + 2, both operands (66 MB moved) 18.6 us; the two
+// launches that made K-major planes, with byte loads off the word grid and a transpose, took 49.
+constexpr int AV = 4;                       // vectors per thread
+__global__ void __launch_bounds__(NTH) align_i8_kernel(LineCopy a0, LineCopy a1, uint32_t n0, long batch) {
+  ptx::grid_dep_launch();                   // the GEMM's set-up may overlap this kernel; it waits for its end
+  const bool second = blockIdx.x >= n0;
+  const LineCopy a = second ? a1 : a0;
+  const uint32_t first = (second ? blockIdx.x - n0 : blockIdx.x) * (uint32_t)(AV * NTH) + threadIdx.x;
+  const uint32_t vpl = (uint32_t)(a.pitch / 16), total = (uint32_t)a.lines * vpl;
+  for (long b = blockIdx.y; b < batch; b += gridDim.y) {
+    const uint8_t* X = (const uint8_t*)a.X[b];
+    uint8_t* out = (uint8_t*)a.out + b * a.lines * a.pitch;
+    uint4 lo[AV], hi[AV];
+    uint32_t off[AV];
+    int bytes[AV];
 #pragma unroll
-    for (int q = 0; q < PKR * PKK / 16 / NTH; ++q) {
-      const int id = t + q * NTH, r = id / (PKK / 16), c = id % (PKK / 16);
-      const long gr = r0 + r, gk = k0 + 16 * c;
-      if (gr >= a.rows || gk >= a.Kp) continue;
-      uint4 w = make_uint4(0u, 0u, 0u, 0u);
-      const int8_t* src = X + gr * a.ld + gk;
-      if (vec && gk + 16 <= a.K) {
-        w = __ldg((const uint4*)src);
-      } else {
-        uint8_t by[16];
-#pragma unroll
-        for (int i = 0; i < 16; ++i) by[i] = gk + i < a.K ? (uint8_t)__ldg(src + i) : 0;
-        memcpy(&w, by, 16);
-      }
-      *(uint4*)(out + gr * a.Kp + gk) = w;
+    for (int q = 0; q < AV; ++q) {
+      const uint32_t i = first + q * NTH, line = i / vpl, v = i - line * vpl;
+      const uint8_t* src = X + (long)line * a.ld + 16 * v;
+      bytes[q] = i < total ? (int)(a.len - 16 * (long)v < 16 ? a.len - 16 * (long)v : 16) : 0;
+      off[q] = (uint32_t)(uintptr_t)src & 15u;
+      lo[q] = vector_if(bytes[q] > 0, src - off[q]);
+      hi[q] = vector_if(off[q] + bytes[q] > 16, src - off[q] + 16);
     }
-    return;
-  }
-  const bool vec = ((uintptr_t)X % 4) == 0 && a.ld % 4 == 0;
-  const int rg = t % 32;                       // rows 4 rg .. 4 rg + 3 of the tile
-  const long gr = r0 + 4 * rg;
 #pragma unroll
-  for (int q = 0; q < PKK / 4 / (NTH / 32); ++q) {
-    const int kg = t / 32 + (NTH / 32) * q;    // k 4 kg .. 4 kg + 3 of the tile
-    uint32_t w[4], o[4];
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      const long gk = k0 + 4 * kg + i;
-      const int8_t* src = X + gr + gk * a.ld;
-      w[i] = 0u;
-      if (gk < a.K) {
-        if (vec && gr + 4 <= a.rows) {
-          w[i] = __ldg((const uint32_t*)src);
-        } else {
-#pragma unroll
-          for (int j = 0; j < 4; ++j)
-            if (gr + j < a.rows) w[i] |= (uint32_t)(uint8_t)__ldg(src + j) << (8 * j);
-        }
+    for (int q = 0; q < AV; ++q) {
+      if (bytes[q] <= 0) continue;
+      uint4 w = bytes_from(lo[q], hi[q], off[q]);
+      if (bytes[q] < 16) {
+        w.x = keep_bytes(w.x, bytes[q]);
+        w.y = keep_bytes(w.y, bytes[q] - 4);
+        w.z = keep_bytes(w.z, bytes[q] - 8);
+        w.w = keep_bytes(w.w, bytes[q] - 12);
       }
+      *(uint4*)(out + 16 * (long)(first + q * NTH)) = w;
     }
-    byte_transpose4(w, o);                     // o[j]: k 4 kg .. 4 kg + 3 of row 4 rg + j
-#pragma unroll
-    for (int j = 0; j < 4; ++j) *(uint32_t*)(st + (4 * rg + j) * PKP + 4 * kg) = o[j];
-  }
-  __syncthreads();
-#pragma unroll
-  for (int q = 0; q < PKR * PKK / 16 / NTH; ++q) {
-    const int id = t + q * NTH, r = id / (PKK / 16), c = id % (PKK / 16);
-    const long gr2 = r0 + r, gk = k0 + 16 * c;
-    if (gr2 >= a.rows || gk >= a.Kp) continue;
-    const uint32_t* src = (const uint32_t*)(st + r * PKP + 16 * c);
-    *(uint4*)(out + gr2 * a.Kp + gk) = make_uint4(src[0], src[1], src[2], src[3]);
   }
 }
 
@@ -1087,12 +1084,14 @@ cudaError_t launch_ozaki_cluster(const PlaneArgs& a0, int32_t* e0, const PlaneAr
 }
 
 
-cudaError_t launch_pack_i8(const PlaneArgs& a, cudaStream_t st) {
-  const long ktiles = (a.Kp + PKK - 1) / PKK, rtiles = (a.rows + PKR - 1) / PKR;
-  const long blocks = ktiles * rtiles * a.batch;
-  if (blocks >= (1L << 31)) return cudaErrorInvalidValue;
-  ProfScope prof("pack_i8", st);
-  pack_i8_kernel<<<(unsigned)blocks, NTH, 0, st>>>(a, ktiles, rtiles);
+cudaError_t launch_align_i8(const LineCopy* a, const LineCopy* b, long batch, cudaStream_t st) {
+  auto blocks = [](const LineCopy* x) { return x ? (x->lines * (x->pitch / 16) + AV * NTH - 1) / (AV * NTH) : 0; };
+  const long n0 = blocks(a), n1 = blocks(b);
+  // 32-bit vector counts per instance
+  if (n0 * AV * NTH >= (1L << 32) || n1 * AV * NTH >= (1L << 32) || n0 + n1 < 1) return cudaErrorInvalidValue;
+  ProfScope prof("align_i8", st);
+  const dim3 grid((unsigned)(n0 + n1), (unsigned)(batch < 65535 ? batch : 65535));
+  align_i8_kernel<<<grid, NTH, 0, st>>>(a ? *a : *b, b ? *b : *a, (uint32_t)n0, batch);
   note_launch();
   return cudaGetLastError();
 }

@@ -23,7 +23,16 @@ struct PlaneArgs {
   long xstride = 0;
 };
 
-cudaError_t launch_pack_i8(const PlaneArgs& a, cudaStream_t st);
+// an operand copied line by line onto the 16-byte grid (align_i8)
+struct LineCopy {
+  const void* const* X;   // device array of per-instance operand pointers
+  long ld;                // bytes between lines (stored columns)
+  long lines, len;        // lines, and bytes of each
+  void* out;              // [batch][lines][pitch]
+  long pitch;             // len rounded up to 16
+};
+// one or both (nullptr = none) operands of one call in one launch
+cudaError_t launch_align_i8(const LineCopy* a, const LineCopy* b, long batch, cudaStream_t st);
 // both operands of one call in one launch
 cudaError_t launch_split_bf16_pair(const PlaneArgs& a, const PlaneArgs& b, cudaStream_t st);
 cudaError_t launch_ozaki_slice(const PlaneArgs& a, int slices, int32_t* exps, cudaStream_t st);

@@ -185,21 +185,6 @@ tc::Params base_params(const BatchDesc& d) {
 
 inline long round_up(long x, long a) { return (x + a - 1) / a * a; }
 
-// int8 planes of op(A) and op(B), K-major, through the pack pre-pass.
-cudaError_t pack_operands_i8(const BatchDesc& d, cudaStream_t st, int8_t** pa, int8_t** pb, long* Kp) {
-  cudaError_t e;
-  *Kp = round_up(d.k, 16);
-  const long sa = d.m * *Kp, sb = d.n * *Kp;
-  *pa = (int8_t*)workspace(WS_PACK_A, (size_t)sa * d.batch, &e);
-  if (!*pa) return e;
-  *pb = (int8_t*)workspace(WS_PACK_B, (size_t)sb * d.batch, &e);
-  if (!*pb) return e;
-  PlaneArgs a{d.A, d.m, d.k, d.lda, d.transa == SSBLAS_OP_T, d.batch, *pa, *Kp, sa, sa};
-  if ((e = launch_pack_i8(a, st)) != cudaSuccess) return e;
-  PlaneArgs b{d.B, d.n, d.k, d.ldb, d.transb == SSBLAS_OP_N, d.batch, *pb, *Kp, sb, sb};
-  return launch_pack_i8(b, st);
-}
-
 using CfgBf64 = tc::Config<tc::KIND_BF16, 2, 2, 64, 128, 4, 1, 2, tc::EPI_F32, 1>;
 using CfgBf128 = tc::Config<tc::KIND_BF16, 2, 2, 128, 128, 3, 1, 2, tc::EPI_F32, 1>;
 template <int S> struct OzCfg;
@@ -357,10 +342,11 @@ namespace {
 // bases, strides and leading dimensions): each op(X) is K-major where it is stored K-contiguous
 // (op(A) = A^T, op(B) = B) and MN-major where it is stored M- (N-)contiguous (op(A) = A,
 // op(B) = B^T), so no layout needs a transposing pass. `elem` = bytes per element.
+bool operand_direct(const void* X0, long stride, long ld, long batch, int elem) {
+  return X0 && (batch == 1 || stride > 0) && (ld * elem) % 16 == 0 && ((uintptr_t)X0 % 16) == 0 && stride % 16 == 0;
+}
 bool direct_eligible(const BatchDesc& d, int elem) {
-  const bool uniform = d.batch == 1 || (d.strideA > 0 && d.strideB > 0);
-  return uniform && (d.lda * elem) % 16 == 0 && (d.ldb * elem) % 16 == 0 && ((uintptr_t)d.A0 % 16) == 0 &&
-         ((uintptr_t)d.B0 % 16) == 0 && d.strideA % 16 == 0 && d.strideB % 16 == 0;
+  return operand_direct(d.A0, d.strideA, d.lda, d.batch, elem) && operand_direct(d.B0, d.strideB, d.ldb, d.batch, elem);
 }
 
 // 4-D maps {inner, outer, 1, batch} of op(A) and op(B) for one 128-byte K stage: K-major tiles are
@@ -385,10 +371,11 @@ using CfgI8 = tc::Config<tc::KIND_I8, 1, 1, BN, 128, BN == 256 ? 4 : 6, 1, 2, tc
 template <int BN>
 cudaError_t run_i8(const CUtensorMap& ta, const CUtensorMap& tb, const tc::Params& prm, bool amn, bool bmn,
                    cudaStream_t st, const SplitPlan& plan) {
-  if (amn && bmn) return run_gemm<CfgI8<BN, 1, 1>>(ta, tb, prm, st, "i8_gemm", plan);
-  if (amn) return run_gemm<CfgI8<BN, 1, 0>>(ta, tb, prm, st, "i8_gemm", plan);
-  if (bmn) return run_gemm<CfgI8<BN, 0, 1>>(ta, tb, prm, st, "i8_gemm", plan);
-  return run_gemm<CfgI8<BN, 0, 0>>(ta, tb, prm, st, "i8_gemm", plan);
+  // programmatic launch: the set-up overlaps the end of the kernel before
+  if (amn && bmn) return run_gemm<CfgI8<BN, 1, 1>>(ta, tb, prm, st, "i8_gemm", plan, nullptr, true);
+  if (amn) return run_gemm<CfgI8<BN, 1, 0>>(ta, tb, prm, st, "i8_gemm", plan, nullptr, true);
+  if (bmn) return run_gemm<CfgI8<BN, 0, 1>>(ta, tb, prm, st, "i8_gemm", plan, nullptr, true);
+  return run_gemm<CfgI8<BN, 0, 0>>(ta, tb, prm, st, "i8_gemm", plan, nullptr, true);
 }
 
 }  // namespace
@@ -397,22 +384,43 @@ cudaError_t launch_i8_tcgen05(const BatchDesc& d, cudaStream_t st) {
   if (!is_sm100() || !encoder()) return cudaErrorNotSupported;
   if (d.k > (1L << 31) || d.m > (1L << 31) || d.n > (1L << 31)) return cudaErrorNotSupported;
   CUtensorMap ta, tb;
-  const int BN = choose_config(SSBLAS_PATH_I8_TCGEN05, d.m, d.n, d.k, d.batch, d.n <= 128 ? 1 : 0) == 1 ? 128 : 256;
-  bool amn = false, bmn = false, ok;
-  if (direct_eligible(d, 1)) {
-    amn = d.transa == SSBLAS_OP_N;
-    bmn = d.transb == SSBLAS_OP_T;
-    ok = direct_maps(d, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, BN, &ta, &tb);
-  } else {
-    // odd leading dimensions or unevenly spaced instances: K-major planes from the pack pre-pass
-    int8_t *pa, *pb;
-    long Kp;
-    cudaError_t e = pack_operands_i8(d, st, &pa, &pb, &Kp);
-    if (e != cudaSuccess) return e;
-    ok = make_map(&ta, pa, CU_TENSOR_MAP_DATA_TYPE_UINT8, d.k, d.m, 1, d.batch, Kp, d.m * Kp, d.m * Kp, 128, 128, 1, 128) &&
-         make_map(&tb, pb, CU_TENSOR_MAP_DATA_TYPE_UINT8, d.k, d.n, 1, d.batch, Kp, d.n * Kp, d.n * Kp, 128, BN, 1, 128);
+  // 128 x 128 tiles (configuration 1) or 128 x 256 (0). The wide tile reads a third less shared memory per
+  // product and is the faster one where the products bound the call (8 x 4096^3: 2570 TOPS against
+  // 1890); where bytes do, the narrow one is, whose shorter epilogues leave the memory idle for less. The
+  // line lies at 240 operations per byte of operands and C, between the measured sides (ms, narrow
+  // and wide): 512 x 512^3 beta = 1 (102 per byte) 0.221, 0.257; beta = 0 (171) 0.136, 0.145;
+  // 16 x 1024^3 off the 16-byte grid (341) 0.0424, 0.0408; 8 x 4096^3 (1365) 0.583, 0.429. Few wide
+  // tiles also take the narrow form.
+  const double ops = 2.0 * d.m * d.n * d.k;
+  const double bytes = (double)d.m * d.k + (double)d.n * d.k + (d.beta_i ? 8.0 : 4.0) * d.m * d.n;
+  const long wide = ((d.m + 127) / 128) * ((d.n + 255) / 256) * d.batch;
+  const bool narrow = d.n <= 128 || ops < 240.0 * bytes || wide < num_sms();
+  const int BN = choose_config(SSBLAS_PATH_I8_TCGEN05, d.m, d.n, d.k, d.batch, narrow ? 1 : 0) == 1 ? 128 : 256;
+  const bool amn = d.transa == SSBLAS_OP_N, bmn = d.transb == SSBLAS_OP_T;
+  // operands with odd leading dimensions or bases, or unevenly spaced instances, are first copied onto
+  // the 16-byte grid, in the order in which they are stored
+  BatchDesc x = d;
+  LineCopy ca, cb;
+  const LineCopy *pa = nullptr, *pb = nullptr;
+  cudaError_t e;
+  if (!operand_direct(d.A0, d.strideA, d.lda, d.batch, 1)) {
+    const long len = amn ? d.m : d.k, lines = amn ? d.k : d.m, pitch = round_up(len, 16);
+    void* w = workspace(WS_PACK_A, (size_t)(lines * pitch) * (size_t)d.batch, &e);
+    if (!w) return e;
+    ca = LineCopy{d.A, d.lda, lines, len, w, pitch};
+    pa = &ca;
+    x.A0 = w; x.lda = pitch; x.strideA = d.batch > 1 ? lines * pitch : 0;
   }
-  if (!ok) return cudaErrorNotSupported;
+  if (!operand_direct(d.B0, d.strideB, d.ldb, d.batch, 1)) {
+    const long len = bmn ? d.n : d.k, lines = bmn ? d.k : d.n, pitch = round_up(len, 16);
+    void* w = workspace(WS_PACK_B, (size_t)(lines * pitch) * (size_t)d.batch, &e);
+    if (!w) return e;
+    cb = LineCopy{d.B, d.ldb, lines, len, w, pitch};
+    pb = &cb;
+    x.B0 = w; x.ldb = pitch; x.strideB = d.batch > 1 ? lines * pitch : 0;
+  }
+  if (!direct_maps(x, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, BN, &ta, &tb)) return cudaErrorNotSupported;
+  if ((pa || pb) && (e = launch_align_i8(pa, pb, d.batch, st)) != cudaSuccess) return e;
   tc::Params prm = base_params(d);
   prm.ab_unsigned = (d.a_unsigned ? 1 : 0) | (d.b_unsigned ? 2 : 0);
   note_path(SSBLAS_PATH_I8_TCGEN05);
