@@ -39,6 +39,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "f32x2.cuh"
 #include "internal.h"
 #include "ptx.cuh"
 
@@ -154,31 +155,6 @@ __device__ __forceinline__ void split_load(SplitOperand& o, int t, float4 (&x)[U
   o.k -= kKC;
 }
 
-// Packed FP32 arithmetic (two values per instruction): d = a * b + c, and a + b
-__device__ __forceinline__ uint64_t pack2(float x, float y) {
-  uint64_t r;
-  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(x), "f"(y));
-  return r;
-}
-__device__ __forceinline__ void unpack2(uint64_t v, float& x, float& y) {
-  asm("mov.b64 {%0, %1}, %2;" : "=f"(x), "=f"(y) : "l"(v));
-}
-__device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) {
-  uint64_t d;
-  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
-  return d;
-}
-__device__ __forceinline__ uint64_t mul2(uint64_t a, uint64_t b) {
-  uint64_t d;
-  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
-  return d;
-}
-__device__ __forceinline__ uint64_t add2(uint64_t a, uint64_t b) {
-  uint64_t d;
-  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
-  return d;
-}
-
 // Two values rounded to bf16 (low half = first), and (REST) what rounding left of them.
 template <bool REST>
 __device__ __forceinline__ uint32_t take_bf16(uint64_t& v) {
@@ -224,12 +200,12 @@ __device__ __forceinline__ void split_store(uint32_t dst, bool mn, int t, float4
   }
 }
 
-// The sums of one lane's row again, for 16 columns, by a chain of fused multiply-adds over the operands
-// in k order: op(A)(i, k) = pa[k * ak], op(B)(k, j) = pb[j * bc + k * bk]; columns from n on repeat
-// column n - 1. Eight k are in flight at a time, so that this rare path runs near the speed of an
-// ordinary FP32 kernel.
+// One lane's row of C again, for the columns of the mask among 16 from `C` on: C <- alpha * acc + beta * C
+// with acc a chain of fused multiply-adds over the operands in k order, op(A)(i, k) = pa[k * ak],
+// op(B)(k, j) = pb[j * bc + k * bk]; columns from n on repeat column n - 1. Eight k are in flight at a time,
+// so that this rare path runs near the speed of an ordinary FP32 kernel.
 __device__ __noinline__ void split_redo(const float* pa, long ak, const float* pb, long bc, long bk, int n, int k,
-                                        float* v) {
+                                        uint32_t mask, float* C, long ldc, float alpha, float beta) {
   float acc[16];
 #pragma unroll
   for (int j = 0; j < 16; ++j) acc[j] = 0.f;
@@ -256,7 +232,8 @@ __device__ __noinline__ void split_redo(const float* pa, long ak, const float* p
     for (int j = 0; j < 16; ++j) acc[j] = fmaf(x, __ldg(pb + (j < n ? j : n - 1) * bc), acc[j]);
   }
 #pragma unroll
-  for (int j = 0; j < 16; ++j) v[j] = acc[j];
+  for (int j = 0; j < 16; ++j)
+    if ((mask >> j) & 1u) C[j * ldc] = fmaf(acc[j], alpha, beta != 0.0f ? beta * C[j * ldc] : 0.0f);
 }
 
 template <class F>
@@ -477,10 +454,11 @@ __global__ void __launch_bounds__(kSplitThreads, 1) f32_split_kernel(const Split
 #pragma unroll
       for (int j = 0; j < HALF / 2; ++j)
         unpack2(F::NP == 3 ? mul2(sum[j], pack2(kUnscale, kUnscale)) : sum[j], acc[2 * j], acc[2 * j + 1]);
+      // sums to compute again (plain form): not finite, or below the smallest and not zero (2 bits - 1
+      // drops the sign and wraps zero to the largest value)
+      constexpr uint32_t LO = 2u * kSmallestBits - 1u;
+      bool redo = false;
       if constexpr (F::NP == 3) {
-        // sums to compute again: not finite, or below the smallest and not zero (2 bits - 1 drops the
-        // sign and wraps zero to the largest value)
-        constexpr uint32_t LO = 2u * kSmallestBits - 1u;
         uint32_t low = 0xffffffffu;
         float high = 0.f;
 #pragma unroll
@@ -488,42 +466,46 @@ __global__ void __launch_bounds__(kSplitThreads, 1) f32_split_kernel(const Split
           low = min(low, 2u * __float_as_uint(acc[j]) - 1u);
           asm("max.NaN.f32 %0, %0, %1;" : "+f"(high) : "f"(fabsf(acc[j])));
         }
-        if (row_ok && (low < LO || !(high < INFINITY))) {
-          const float* pa = a.A[ti.b] + (a.a_mn ? gi : gi * a.lda);
-          const float* pb = a.B[ti.b] + (a.b_mn ? gj0 : gj0 * a.ldb);
-          const long ak = a.a_mn ? a.lda : 1, bc = a.b_mn ? 1 : a.ldb, bk = a.b_mn ? a.ldb : 1;
+        redo = __any_sync(0xffffffffu, row_ok && (low < LO || !(high < INFINITY)));
+      }
+      if (!redo) {
 #pragma unroll
-          for (int g = 0; g < HALF; g += 16) {
-            uint32_t mask = 0;
+        for (int g = 0; g < HALF; g += G) {
+          if (!EARLY_C && read_c) load_c(g);
+          float* cp = C + (long)g * a.ldc;
+          asm volatile("" : "+l"(cp));
 #pragma unroll
-            for (int j = 0; j < 16; ++j) {
-              if (g + j < cols && (2u * __float_as_uint(acc[g + j]) - 1u < LO || !(fabsf(acc[g + j]) < INFINITY)))
-                mask |= 1u << j;
-            }
-            if (mask == 0) continue;
-            float v[16];
-            split_redo(pa, ak, pb + g * bc, bc, bk, cols - g, (int)a.k, v);
+          for (int j = 0; j < G; ++j) acc[g + j] = fmaf(acc[g + j], a.alpha, read_c ? a.beta * cv[j] : 0.0f);
+          if (!row_ok) continue;
+          if (cols == HALF) {
 #pragma unroll
-            for (int j = 0; j < 16; ++j)
-              if ((mask >> j) & 1u) acc[g + j] = v[j];
+            for (int j = 0; j < G; ++j, cp += a.ldc) __stcs(cp, acc[g + j]);
+          } else {
+#pragma unroll
+            for (int j = 0; j < G; ++j, cp += a.ldc)
+              if (g + j < cols) __stcs(cp, acc[g + j]);
           }
         }
-      }
+      } else if (row_ok) {
+        // the sound columns, then the others
+        uint64_t mask = 0;
 #pragma unroll
-      for (int g = 0; g < HALF; g += G) {
-        if (!EARLY_C && read_c) load_c(g);
-        float* cp = C + (long)g * a.ldc;
-        asm volatile("" : "+l"(cp));
-#pragma unroll
-        for (int j = 0; j < G; ++j) acc[g + j] = fmaf(acc[g + j], a.alpha, read_c ? a.beta * cv[j] : 0.0f);
-        if (!row_ok) continue;
-        if (cols == HALF) {
-#pragma unroll
-          for (int j = 0; j < G; ++j, cp += a.ldc) __stcs(cp, acc[g + j]);
-        } else {
-#pragma unroll
-          for (int j = 0; j < G; ++j, cp += a.ldc)
-            if (g + j < cols) __stcs(cp, acc[g + j]);
+        for (int j = 0; j < HALF; ++j) {
+          if (j >= cols) break;
+          if (2u * __float_as_uint(acc[j]) - 1u < LO || !(fabsf(acc[j]) < INFINITY)) {
+            mask |= 1ull << j;
+          } else {
+            float* cp = C + (long)j * a.ldc;
+            *cp = fmaf(acc[j], a.alpha, read_c ? a.beta * *cp : 0.0f);
+          }
+        }
+        const float* pa = a.A[ti.b] + (a.a_mn ? gi : gi * a.lda);
+        const float* pb = a.B[ti.b] + (a.b_mn ? gj0 : gj0 * a.ldb);
+        const long ak = a.a_mn ? a.lda : 1, bc = a.b_mn ? 1 : a.ldb, bk = a.b_mn ? a.ldb : 1;
+#pragma unroll 1
+        for (int g = 0; g < cols; g += 16) {
+          const uint32_t mk = (uint32_t)(mask >> g) & 0xffffu;
+          if (mk) split_redo(pa, ak, pb + g * bc, bc, bk, cols - g, (int)a.k, mk, C + (long)g * a.ldc, a.ldc, a.alpha, a.beta);
         }
       }
     }
