@@ -19,22 +19,26 @@
 // |x| >= 2^104, sums of 2^80 and more), or is below 2^-100 and not zero, is computed again by a chain
 // of fused multiply-adds over the operands, so those behave as FP32 arithmetic does.
 //
-// Design: persistent CTAs over (instance, 128 x BN tile) items, K in chunks of 32:
-//   warps 8-15   converters: each thread loads 16 bytes of op(A) / op(B) straight from the
-//                caller's matrices (any alignment: 4-byte loads where 16-byte ones are not possible),
-//                DEPTH chunks ahead in registers, splits, and writes the parts in the layout the
-//                tensor core reads -- K-major (64-byte swizzle) where K is contiguous in memory,
-//                MN-major (128-byte swizzle) where M or N is, so nothing is transposed
-//   warp 16      tensor memory, MMA issue from one lane
+// Design: persistent CTAs over (instance, tile) items, K in chunks of 32:
+//   warps 8-15   converters: each thread copies its own 16-byte units of op(A) and op(B), two to four chunks
+//                ahead, from the caller's matrices to its own places in shared memory (cp.async; any
+//                alignment: 4-byte copies where 16-byte ones are not possible), reads them back, splits
+//                them and writes the parts in the layout the tensor core reads -- K-major (64-byte
+//                swizzle) where K is contiguous in memory, MN-major (128-byte swizzle) where M or N is, so
+//                nothing is transposed
+//   warp 16      tensor memory, MMA issue
 //   warps 0-7    chunk sums from tensor memory into registers, then alpha * acc + beta * C
-// Operands cross HBM once as fp32 and no plane is written back: the operands of a tile are split
-// again for every tile that shares them, which is cheaper than the 10 bytes per element of a split
-// pass. What bounds it (16 x 1024^3): a 128 x 128 chunk takes about 1850 cycles; its 12 MMAs alone take
-// 1100 (each reads 8 KB of shared memory in the 64 cycles of its products), the parts' writes (48 KB)
-// share that memory's 128 B per cycle, and the 32 KB a chunk loads come from L2 at 4.6 TB/s over the
-// GPU. Measured (ms, FFMA kernels -> this one): 16 x 1024^3 NN 0.829 -> 0.215; 4 x 2048^3 TN 1.73 ->
-// 0.41; 64 x 128^3 NN 0.0145 -> 0.0120; 8 x (777 x 555 x 333) 0.103 -> 0.040; 2 x 128^2 x 4096 0.19 ->
-// 0.09. 3xBF16 (split pass and tiled GEMM -> this kernel): 256 x 256^3 0.130 -> 0.053.
+// For large tiles two CTAs share a 256 x 256 tile (tcgen05 cta_group::2): each loads, splits and writes
+// 128 of its rows and 128 of its columns, half as much per product as alone, and arrives on the leader's
+// barriers. Operands cross HBM once as fp32 and no plane is written back: the operands of a tile are split
+// again for every tile that shares them, which is cheaper than the 10 bytes per element of a split pass.
+// What bounds it (16 x 1024^3 plain, a pair's chunk of 1940 cycles): the 128 B per cycle of shared memory
+// (units in and out 64 KB, parts in 48 KB, 12 MMAs reading 96 KB: 1660 cycles; the MMAs alone 1540). With
+// the units in registers, as before, the wait for a stage queued behind the loads and a chunk of a 128 x 128
+// tile took 1850 cycles; so did one of a pair while its arrivals asked for a cluster-wide release.
+// Measured (ms, FFMA kernels -> this one): 16 x 1024^3 NN 0.829 -> 0.166 (207 TFLOP/s); 4 x 2048^3 1.73 ->
+// 0.297; 64 x 128^3 NN 0.0145 -> 0.0125; 8 x (777 x 555 x 333) 0.103 -> 0.041; 2 x 128^2 x 4096 0.19 -> 0.094.
+// 3xBF16 (split pass and tiled GEMM -> this kernel): 256 x 256^3 0.130 -> 0.039, 16 x 1024^3 0.096.
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 #include <stdint.h>
@@ -49,30 +53,41 @@ namespace {
 constexpr int kKC = 32;                      // K elements per chunk
 constexpr int kConvThreads = 256;            // warps 8-15
 constexpr int kSplitThreads = 32 * 20;       // the last warpgroup's first warp issues the MMAs
-// registers per thread: 640 x 96 at launch = 61,440; 4 x 128 x 112 + 128 x 32 = 61,440 after the split
-constexpr int kWorkRegs = 112, kIssueRegs = 32;
+constexpr int kIssueRegs = 32;               // registers per thread of that warpgroup
+constexpr int kUnitRow = 16 * kConvThreads;  // bytes of one unit of every converter thread
 // Plain form: scale of the operands, of their sums, and the magnitude below which a sum that is not
 // zero is computed again
 constexpr float kScale = 0x1p24f, kUnscale = 0x1p-48f;
 constexpr uint32_t kSmallestBits = 0x0d800000u;   // 2^-100
 
-// NP parts per operand, AR rows of op(A) converted per tile (64 when m <= 64), BN columns
-template <int NP_, int AR_, int BN_>
+// NP parts per operand, AR rows of op(A) (64 when m <= 64) and BN columns of op(B) converted per CTA and
+// chunk. PAIR: two CTAs (a cluster) share a 256 x 256 tile -- each converts 128 of its rows and 128 of its
+// columns and holds 128 rows of the result, and the leader's MMAs (cta_group::2) read both CTAs'
+// parts -- so per product a CTA loads, splits, writes and reads half as much.
+template <int NP_, int AR_, int BN_, bool PAIR_ = false>
 struct Split {
   static constexpr int NP = NP_, AR = AR_, BN = BN_;
+  static constexpr bool PAIR = PAIR_;
   static constexpr int A_PLANE = AR * kKC * 2;
   static constexpr int B_PLANE = BN * kKC * 2;
   static constexpr int STAGE = NP * (A_PLANE + B_PLANE);
-  static constexpr int STAGES = (200 * 1024) / STAGE > 8 ? 8 : (200 * 1024) / STAGE;
-  static constexpr int NACC = 4;             // accumulators in flight
-  static constexpr int TMEM_COLS = NACC * BN;
   static constexpr int UA = AR * kKC / 4 / kConvThreads, UB = BN * kKC / 4 / kConvThreads;   // 16-byte units per thread
-  static constexpr int DEPTH = (UA + UB) >= 6 ? 2 : 3;                                       // chunks held in registers
+  // chunks of fp32 units in flight, and stages of parts, in 224 KB
+  static constexpr int RAW_STAGE = (UA + UB) * kUnitRow;
+  static constexpr int RAW = RAW_STAGE > 24 * 1024 ? (NP == 3 ? 2 : 3) : 4;
+  static constexpr int STAGES = (224 * 1024 - RAW * RAW_STAGE) / STAGE > 6 ? 6 : (224 * 1024 - RAW * RAW_STAGE) / STAGE;
+  static constexpr int TM = PAIR ? 256 : 128, TN = PAIR ? 2 * BN : BN;   // the tile
+  static constexpr int NACC = PAIR ? 2 : 4;  // accumulators in flight, TN columns each
+  static constexpr int TMEM_COLS = NACC * TN;
+  static constexpr bool PROMOTE = NP == 3;
+  // registers of the converters and epilogue warps: 640 threads x 96 at launch = 61,440 = 256 x (conv +
+  // epilogue) + 128 x 32; the plain form's epilogue holds a sum per output, 128 a thread in a pair
+  static constexpr int CONV_REGS = PAIR && PROMOTE ? 56 : 104, EPI_REGS = 224 - CONV_REGS;
   // the MMA reads 128 rows of every A part: with AR = 64 the upper 64 come from whatever follows
   // (within the stage, since B follows A), and their products are never read
-  static constexpr int SMEM = 1024 + STAGES * STAGE + 512;
-  static constexpr bool PROMOTE = NP == 3;
-  static_assert(STAGE % 1024 == 0 && NP * B_PLANE >= 4096 && SMEM <= 232448, "stages");
+  static constexpr int SMEM = 1024 + STAGES * STAGE + RAW * RAW_STAGE + 512;
+  static_assert(STAGE % 1024 == 0 && NP * B_PLANE >= 4096 && SMEM <= 232448 && TMEM_COLS <= 512, "stages");
+  static_assert(256 * (CONV_REGS + EPI_REGS) + 128 * kIssueRegs <= kSplitThreads * 96, "registers");
 };
 
 struct SplitArgs {
@@ -97,7 +112,7 @@ template <class F>
 __device__ __forceinline__ SplitTile split_tile(const SplitArgs& a, uint32_t t) {
   const uint32_t b = t / a.tiles_mn, r = t - b * a.tiles_mn;
   const uint32_t nt = r / a.tiles_m;
-  return {b, (long)(r - nt * a.tiles_m) * 128, (long)nt * F::BN};
+  return {b, (long)(r - nt * a.tiles_m) * F::TM, (long)nt * F::TN};
 }
 
 // One operand as a converter thread sees it: its unit i (4 consecutive elements along the contiguous
@@ -105,7 +120,7 @@ __device__ __forceinline__ SplitTile split_tile(const SplitArgs& a, uint32_t t) 
 //   mn: a unit is 4 rows at one k; a warp takes whole k lines of ROWS; unit i is 256 / (ROWS / 4) k on
 //   else a unit is 4 k of one row, 8 lanes a row; unit i is 32 rows on
 struct SplitOperand {
-  const float* p;
+  const float *p, *base;
   int step, adv;           // elements between units, between chunks (ld < 2^25)
   int rows, k;             // valid rows from this thread's unit 0 on; valid k from the next chunk on
   bool mn, vec, full;      // full: every unit of the tile's whole chunks is inside the matrix
@@ -115,6 +130,7 @@ __device__ __forceinline__ SplitOperand split_operand(const float* X, long rows,
                                                       int t) {
   constexpr int RG = ROWS / 4;
   SplitOperand o;
+  o.base = X;
   o.mn = mn;
   o.vec = ((uintptr_t)X % 16) == 0 && ld % 4 == 0;
   o.full = o.vec && rows - r0 >= ROWS;
@@ -127,27 +143,33 @@ __device__ __forceinline__ SplitOperand split_operand(const float* X, long rows,
   return o;
 }
 
-// The units of the next chunk; the operand moves on to the one after it.
+__device__ __forceinline__ void copy16(uint32_t dst, const float* src, int bytes) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(dst), "l"(src), "r"(bytes) : "memory");
+}
+__device__ __forceinline__ void copy4(uint32_t dst, const float* src, bool ok) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;\n" ::"r"(dst), "l"(src), "r"(ok ? 4 : 0) : "memory");
+}
+// Copies the units of the next chunk to this thread's places, unit i at dst + i * 4096 (zeros outside the
+// matrix); the operand moves on to the chunk after it.
 template <int ROWS, int U>
-__device__ __forceinline__ void split_load(SplitOperand& o, int t, float4 (&x)[U]) {
+__device__ __forceinline__ void split_copy(SplitOperand& o, int t, uint32_t dst) {
   constexpr int RG = ROWS / 4;
   const float* src = o.p;
   if (o.full && o.k >= kKC) {
 #pragma unroll
-    for (int i = 0; i < U; ++i, src += o.step) x[i] = __ldg((const float4*)src);
+    for (int i = 0; i < U; ++i, src += o.step) copy16(dst + i * kUnitRow, src, 16);
   } else {
 #pragma unroll
     for (int i = 0; i < U; ++i, src += o.step) {
       const int kk = o.mn ? t / RG + i * (kConvThreads / RG) : 4 * (t % 8);
-      const int n = o.mn ? (o.k > kk ? o.rows : 0) : (o.rows > 32 * i ? o.k - kk : 0);
-      x[i] = make_float4(0.f, 0.f, 0.f, 0.f);
-      if (o.vec && n >= 4) {
-        x[i] = __ldg((const float4*)src);
+      int n = o.mn ? (o.k > kk ? o.rows : 0) : (o.rows > 32 * i ? o.k - kk : 0);   // valid elements
+      n = n < 0 ? 0 : n > 4 ? 4 : n;
+      const float* q = n > 0 ? src : o.base;
+      if (o.vec) {
+        copy16(dst + i * kUnitRow, q, 4 * n);
       } else {
-        if (n > 0) x[i].x = __ldg(src);
-        if (n > 1) x[i].y = __ldg(src + 1);
-        if (n > 2) x[i].z = __ldg(src + 2);
-        if (n > 3) x[i].w = __ldg(src + 3);
+#pragma unroll
+        for (int e = 0; e < 4; ++e) copy4(dst + i * kUnitRow + 4 * e, n > e ? q + e : q, n > e);
       }
     }
   }
@@ -166,9 +188,9 @@ __device__ __forceinline__ uint32_t take_bf16(uint64_t& v) {
   return w;
 }
 
-// Splits the units and writes the NP parts of the operand.
+// Splits this thread's units (unit i at raw + i * 4096) and writes the NP parts of the operand.
 template <int NP, int ROWS, int U>
-__device__ __forceinline__ void split_store(uint32_t dst, bool mn, int t, float4 (&x)[U]) {
+__device__ __forceinline__ void split_store(uint32_t raw, uint32_t dst, bool mn, int t) {
   constexpr int PLANE = ROWS * kKC * 2;
   constexpr int RG = ROWS / 4;
   uint32_t off, step;
@@ -183,20 +205,28 @@ __device__ __forceinline__ void split_store(uint32_t dst, bool mn, int t, float4
     off = rr * 64u + (((kq >> 1) ^ ((rr >> 1) & 3u)) << 4) + ((kq & 1u) << 3);
     step = 32 * 64u;
   }
+  // all reads before the first write: the units' conversions then overlap
+  uint64_t v[U][2];
 #pragma unroll
-  for (int i = 0; i < U; ++i) {
-    const uint32_t d = dst + off + i * step;
-    uint64_t v0 = pack2(x[i].x, x[i].y), v1 = pack2(x[i].z, x[i].w);
-    if constexpr (NP == 3) {
-      v0 = mul2(v0, pack2(kScale, kScale));
-      v1 = mul2(v1, pack2(kScale, kScale));
-    }
+  for (int i = 0; i < U; ++i)
+    asm volatile("ld.shared.v2.b64 {%0, %1}, [%2];" : "=l"(v[i][0]), "=l"(v[i][1]) : "r"(raw + i * kUnitRow) : "memory");
+  if constexpr (NP == 3) {
 #pragma unroll
-    for (int p = 0; p < NP; ++p) {
-      const uint32_t w0 = p + 1 < NP ? take_bf16<true>(v0) : take_bf16<false>(v0);
-      const uint32_t w1 = p + 1 < NP ? take_bf16<true>(v1) : take_bf16<false>(v1);
-      asm volatile("st.shared.v2.b32 [%0], {%1, %2};" ::"r"(d + p * PLANE), "r"(w0), "r"(w1) : "memory");
-    }
+    for (int i = 0; i < U; ++i)
+#pragma unroll
+      for (int h = 0; h < 2; ++h) v[i][h] = mul2(v[i][h], pack2(kScale, kScale));
+  }
+#pragma unroll
+  for (int p = 0; p < NP; ++p) {
+    uint32_t w[U][2];
+#pragma unroll
+    for (int i = 0; i < U; ++i)
+#pragma unroll
+      for (int h = 0; h < 2; ++h) w[i][h] = p + 1 < NP ? take_bf16<true>(v[i][h]) : take_bf16<false>(v[i][h]);
+#pragma unroll
+    for (int i = 0; i < U; ++i)
+      asm volatile("st.shared.v2.b32 [%0], {%1, %2};" ::"r"(dst + off + i * step + p * PLANE), "r"(w[i][0]), "r"(w[i][1])
+                   : "memory");
   }
 }
 
@@ -240,7 +270,8 @@ template <class F>
 __global__ void __launch_bounds__(kSplitThreads, 1) f32_split_kernel(const SplitArgs a) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t* stages = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
-  uint64_t* full = (uint64_t*)(stages + F::STAGES * F::STAGE);   // parts written (converter warps)
+  uint8_t* raw = stages + F::STAGES * F::STAGE;                  // [RAW] fp32 units, a place per thread
+  uint64_t* full = (uint64_t*)(raw + F::RAW * F::RAW_STAGE);     // parts written (converter warps)
   uint64_t* empty = full + F::STAGES;                            // parts read by the MMAs (commit)
   uint64_t* acc_full = empty + F::STAGES;                        // [NACC] sums complete (commit)
   uint64_t* acc_empty = acc_full + F::NACC;                      // [NACC] sums read (8 warps)
@@ -251,24 +282,33 @@ __global__ void __launch_bounds__(kSplitThreads, 1) f32_split_kernel(const Split
   const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
   const uint32_t wl = a.wait_limit ? a.wait_limit : ptx::kWaitLimit;
   int* err = a.err;
+  // this CTA's place: worker `me` of `workers` (a worker is a CTA or a pair), rank in the pair
+  constexpr uint32_t CT = F::PAIR ? 2 : 1;
+  const uint32_t rank = F::PAIR ? ptx::cluster_rank() : 0;
+  const uint32_t me = blockIdx.x / CT, workers = gridDim.x / CT;
   if (threadIdx.x == 0) {
     for (int s = 0; s < F::STAGES; ++s) {
-      ptx::mbar_init(ptx::smem_u32(&full[s]), kConvThreads / 32);
+      ptx::mbar_init(ptx::smem_u32(&full[s]), CT * kConvThreads / 32);
       ptx::mbar_init(ptx::smem_u32(&empty[s]), 1);
     }
     for (int q = 0; q < F::NACC; ++q) {
       ptx::mbar_init(ptx::smem_u32(&acc_full[q]), 1);
-      ptx::mbar_init(ptx::smem_u32(&acc_empty[q]), 8);
+      ptx::mbar_init(ptx::smem_u32(&acc_empty[q]), CT * 8);
     }
     ptx::mbar_init(ptx::smem_u32(drain), 1);
     ptx::fence_mbar_init();
   }
   if (warp == 16) {
-    ptx::tmem_alloc(ptx::smem_u32(tmem_slot), F::TMEM_COLS);
-    ptx::tmem_relinquish();
+    if constexpr (F::PAIR) {
+      ptx::tmem_alloc_pair(ptx::smem_u32(tmem_slot), F::TMEM_COLS);
+    } else {
+      ptx::tmem_alloc(ptx::smem_u32(tmem_slot), F::TMEM_COLS);
+      ptx::tmem_relinquish();
+    }
   }
   ptx::tc_fence_before();
   __syncthreads();
+  if constexpr (F::PAIR) ptx::cluster_sync();   // both CTAs' barriers and tensor memory are there
   ptx::tc_fence_after();
   const uint32_t tmem = __shfl_sync(0xffffffffu, *tmem_slot, 0);   // known to be warp-uniform
   // under a programmatic launch the set-up above overlaps the end of the kernel before
@@ -276,69 +316,72 @@ __global__ void __launch_bounds__(kSplitThreads, 1) f32_split_kernel(const Split
   ptx::grid_dep_launch();
   const uint32_t nkc = (uint32_t)((a.k + kKC - 1) / kKC);
 
+  // a pair's `full` and `acc_empty` are the leader's, and collect both CTAs' arrivals
+  auto arrive = [&](uint64_t* bar) {
+    if constexpr (F::PAIR) ptx::mbar_arrive_at(ptx::smem_u32(bar), 0);
+    else ptx::mbar_arrive(ptx::smem_u32(bar));
+  };
+
   if (warp >= 8 && warp < 16) {
     // ------------------------------------------------------------------ converters --------
-    asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kWorkRegs));
+    if constexpr (F::CONV_REGS > 96) asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(F::CONV_REGS));
+    else asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(F::CONV_REGS));
     const int t = threadIdx.x - 256;
     const uint32_t stages0 = ptx::smem_u32(stages);
-    struct Pos {
-      uint32_t t, kc;
-      SplitOperand A, B;
-    };
-    Pos ld;                      // next chunk to load
-    ld.t = blockIdx.x;
-    ld.kc = 0;
+    const uint32_t raw0 = ptx::smem_u32(raw) + 16 * t;
+    uint32_t lt = me, lkc = 0, lr = 0;     // next chunk to copy: tile, chunk of it, place
+    SplitOperand A, B;
     auto enter = [&]() {
-      if (ld.t >= a.total) return;
-      const SplitTile ti = split_tile<F>(a, ld.t);
-      ld.A = split_operand<F::AR>(a.A[ti.b], a.m, a.k, a.lda, a.a_mn != 0, ti.m0, t);
-      ld.B = split_operand<F::BN>(a.B[ti.b], a.n, a.k, a.ldb, a.b_mn != 0, ti.n0, t);
+      if (lt >= a.total) return;
+      const SplitTile ti = split_tile<F>(a, lt);
+      A = split_operand<F::AR>(a.A[ti.b], a.m, a.k, a.lda, a.a_mn != 0, ti.m0 + rank * 128, t);
+      B = split_operand<F::BN>(a.B[ti.b], a.n, a.k, a.ldb, a.b_mn != 0, ti.n0 + rank * F::BN, t);
     };
-    float4 xa[F::DEPTH][F::UA], xb[F::DEPTH][F::UB];
-    auto load = [&](float4 (&va)[F::UA], float4 (&vb)[F::UB]) {
-      if (ld.t >= a.total) return;
-      split_load<F::AR, F::UA>(ld.A, t, va);
-      split_load<F::BN, F::UB>(ld.B, t, vb);
-      if (++ld.kc == nkc) {
-        ld.kc = 0;
-        ld.t += gridDim.x;
-        enter();
+    auto copy = [&]() {
+      if (lt < a.total) {
+        const uint32_t dst = raw0 + lr * F::RAW_STAGE;
+        split_copy<F::AR, F::UA>(A, t, dst);
+        split_copy<F::BN, F::UB>(B, t, dst + F::UA * kUnitRow);
+        if (++lkc == nkc) {
+          lkc = 0;
+          lt += workers;
+          enter();
+        }
       }
+      if (++lr == F::RAW) lr = 0;
+      asm volatile("cp.async.commit_group;" ::: "memory");
     };
     enter();
 #pragma unroll
-    for (int d = 0; d < F::DEPTH; ++d) load(xa[d], xb[d]);
-    uint32_t c = 0, kc = 0;
-    uint32_t cur = blockIdx.x;
+    for (int d = 0; d < F::RAW; ++d) copy();
+    uint32_t c = 0, s = 0, r = 0;
     bool ok = true;
-    while (ok && cur < a.total) {
-#pragma unroll
-      for (int d = 0; d < F::DEPTH; ++d) {
-        if (!ok || cur >= a.total) break;
-        const uint32_t s = c % F::STAGES;
+    for (uint32_t cur = me; ok && cur < a.total; cur += workers) {
+      for (uint32_t kc = 0; kc < nkc; ++kc, ++c) {
+        // the stage is waited for before the next copies are queued: behind them the answer would take
+        // hundreds of cycles
         if (!ptx::mbar_wait(ptx::smem_u32(&empty[s]), ((c / F::STAGES) & 1) ^ 1, err, 81, wl)) {
           ok = false;
           break;
         }
-        const uint32_t st = stages0 + s * F::STAGE;
-        split_store<F::NP, F::AR, F::UA>(st, a.a_mn != 0, t, xa[d]);
-        split_store<F::NP, F::BN, F::UB>(st + F::NP * F::A_PLANE, a.b_mn != 0, t, xb[d]);
+        if (c > 0) copy();                   // into the place of the chunk before, which this thread has read
+        asm volatile("cp.async.wait_group %0;" ::"n"(F::RAW - 1) : "memory");   // (each thread reads its own units)
+        const uint32_t st = stages0 + s * F::STAGE, rw = raw0 + r * F::RAW_STAGE;
+        split_store<F::NP, F::AR, F::UA>(rw, st, a.a_mn != 0, t);
+        split_store<F::NP, F::BN, F::UB>(rw + F::UA * kUnitRow, st + F::NP * F::A_PLANE, a.b_mn != 0, t);
         ptx::fence_proxy_async_smem();   // generic-proxy writes -> the tensor core's reads
         __syncwarp();
-        if (lane == 0 && !(a.skip && c == 0 && blockIdx.x == 0)) ptx::mbar_arrive(ptx::smem_u32(&full[s]));
-        load(xa[d], xb[d]);
-        ++c;
-        if (++kc == nkc) {
-          kc = 0;
-          cur += gridDim.x;
-        }
+        if (lane == 0 && !(a.skip && c == 0 && blockIdx.x == 0)) arrive(&full[s]);
+        if (++s == F::STAGES) s = 0;
+        if (++r == F::RAW) r = 0;
       }
     }
+    asm volatile("cp.async.wait_group 0;" ::: "memory");   // no copy is in flight when the CTA exits
   } else if (warp >= 16) {
     // ------------------------------------------------------------------ MMA ---------------
     asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kIssueRegs));
-    if (warp == 16) {
-      const uint32_t idesc = ptx::idesc_bf16(128, F::BN, a.a_mn != 0, a.b_mn != 0);
+    if (warp == 16 && rank == 0) {
+      const uint32_t idesc = ptx::idesc_bf16(F::TM, F::TN, a.a_mn != 0, a.b_mn != 0);
       // descriptors of stage 0's first part, and their step along K: 16 k are 32 bytes of a K-major
       // line, 16 lines of an MN-major block (addresses count 16 bytes). The whole warp runs the loop
       // and one lane's predicate is on the MMA itself, so descriptors stay in uniform registers:
@@ -352,7 +395,11 @@ __global__ void __launch_bounds__(kSplitThreads, 1) f32_split_kernel(const Split
       static_assert(kKC == 32, "two K steps per chunk");
       uint32_t c = 0, q = 0;     // chunks, accumulators
       bool ok = true;
-      for (uint32_t t = blockIdx.x; t < a.total && ok; t += gridDim.x) {
+      auto commit = [&](uint64_t* bar) {
+        if constexpr (F::PAIR) ptx::mma_commit_pair_if(lead, ptx::smem_u32(bar));
+        else ptx::mma_commit_if(lead, ptx::smem_u32(bar));
+      };
+      for (uint32_t t = me; t < a.total && ok; t += workers) {
         for (uint32_t kc = 0; kc < nkc; ++kc, ++c) {
           const uint32_t s = c % F::STAGES;
           if (F::PROMOTE || kc == 0) {
@@ -366,7 +413,7 @@ __global__ void __launch_bounds__(kSplitThreads, 1) f32_split_kernel(const Split
             break;
           }
           ptx::tc_fence_after();
-          const uint32_t d = tmem + (q % F::NACC) * F::BN;
+          const uint32_t d = tmem + (q % F::NACC) * F::TN;
           const uint64_t sa = a0 + (uint64_t)(s * (uint32_t)(F::STAGE >> 4)), sb = b0 + (uint64_t)(s * (uint32_t)(F::STAGE >> 4));
           uint32_t acc = F::PROMOTE || kc == 0 ? 0u : 1u;
           // smallest products first
@@ -375,40 +422,47 @@ __global__ void __launch_bounds__(kSplitThreads, 1) f32_split_kernel(const Split
 #pragma unroll
             for (int p = 0; p <= sum; ++p) {
               const uint64_t ad = sa + (uint64_t)(p * (F::A_PLANE >> 4)), bd = sb + (uint64_t)((sum - p) * (F::B_PLANE >> 4));
-              ptx::mma_f16_if(lead, d, ad, bd, idesc, acc);
-              ptx::mma_f16_if(lead, d, ad + ka, bd + kb, idesc, 1u);
+              if constexpr (F::PAIR) {
+                ptx::mma_f16_pair_if(lead, d, ad, bd, idesc, acc);
+                ptx::mma_f16_pair_if(lead, d, ad + ka, bd + kb, idesc, 1u);
+              } else {
+                ptx::mma_f16_if(lead, d, ad, bd, idesc, acc);
+                ptx::mma_f16_if(lead, d, ad + ka, bd + kb, idesc, 1u);
+              }
               acc = 1u;
             }
-          ptx::mma_commit_if(lead, ptx::smem_u32(&empty[s]));
+          commit(&empty[s]);
           if (F::PROMOTE || kc + 1 == nkc) {
-            ptx::mma_commit_if(lead, ptx::smem_u32(&acc_full[q % F::NACC]));
+            commit(&acc_full[q % F::NACC]);
             ++q;
           }
         }
       }
       // every MMA issued has finished before the tensor memory is released
-      ptx::mma_commit_if(lead, ptx::smem_u32(drain));
+      commit(drain);
       ptx::mbar_wait(ptx::smem_u32(drain), 0, err, 84, wl);
+    } else if (warp == 16) {
+      ptx::mbar_wait(ptx::smem_u32(drain), 0, err, 84, wl);   // the leader's last arrival here
     }
   } else {
     // ------------------------------------------------------------------ epilogue ----------
-    asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kWorkRegs));
-    constexpr int HALF = F::BN / 2;
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(F::EPI_REGS));
+    constexpr int HALF = F::TN / 2;
     const int quarter = warp % 4, half = warp / 4;
     const uint32_t t_row = tmem + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(half * HALF);
     const bool active = quarter * 32 < F::AR;      // rows past AR hold no results
-    uint32_t q = 0, item = 0;
+    uint32_t q = 0;
     bool ok = true;
-    for (uint32_t t = blockIdx.x; t < a.total && ok; t += gridDim.x, ++item) {
+    for (uint32_t t = me; t < a.total && ok; t += workers) {
       const SplitTile ti = split_tile<F>(a, t);
-      const long gi = ti.m0 + quarter * 32 + lane, gj0 = ti.n0 + half * HALF;
+      const long gi = ti.m0 + rank * 128 + quarter * 32 + lane, gj0 = ti.n0 + half * HALF;
       float* C = a.C[ti.b] + gi + gj0 * a.ldc;
       const bool row_ok = active && gi < a.m;
       const int cols = gj0 < a.n ? (a.n - gj0 < HALF ? (int)(a.n - gj0) : HALF) : 0;
       const bool read_c = a.beta != 0.0f;
       // narrow tiles: C is in flight while the products run
       constexpr bool EARLY_C = HALF == 32;
-      constexpr int G = EARLY_C ? 32 : 16;     // columns per group
+      constexpr int G = EARLY_C || !F::PROMOTE ? 32 : 16;     // columns per group
       float cv[G];
       // (the walking pointers are opaque to the compiler: it would keep an address per column otherwise)
       auto load_c = [&](int j0) {
@@ -423,11 +477,46 @@ __global__ void __launch_bounds__(kSplitThreads, 1) f32_split_kernel(const Split
         }
       };
       if (EARLY_C && read_c) load_c(0);
+      if constexpr (!F::PROMOTE) {
+        // one accumulator per tile: groups of columns straight from it to C
+        const uint32_t buf = q % F::NACC;
+        if (!ptx::mbar_wait(ptx::smem_u32(&acc_full[buf]), (q / F::NACC) & 1, err, 85, wl)) break;
+        ptx::tc_fence_after();
+        if (active) {
+#pragma unroll 1
+          for (int g = 0; g < HALF; g += G) {
+            uint32_t raw[G / 16][16];
+#pragma unroll
+            for (int i = 0; i < G / 16; ++i) ptx::tmem_ld16(t_row + buf * F::TN + g + 16 * i, raw[i]);
+            if (!EARLY_C && read_c) load_c(g);
+            ptx::tmem_wait_ld();
+            float* cp = C + (long)g * a.ldc;
+            asm volatile("" : "+l"(cp));
+            if (!row_ok) continue;
+#pragma unroll
+            for (int j = 0; j < G; ++j)
+              raw[j / 16][j % 16] =
+                  __float_as_uint(fmaf(__uint_as_float(raw[j / 16][j % 16]), a.alpha, read_c ? a.beta * cv[j] : 0.0f));
+            if (cols == HALF) {
+#pragma unroll
+              for (int j = 0; j < G; ++j, cp += a.ldc) __stcs(cp, __uint_as_float(raw[j / 16][j % 16]));
+            } else {
+#pragma unroll
+              for (int j = 0; j < G; ++j, cp += a.ldc)
+                if (g + j < cols) __stcs(cp, __uint_as_float(raw[j / 16][j % 16]));
+            }
+          }
+        }
+        ptx::tc_fence_before();
+        __syncwarp();
+        if (lane == 0) arrive(&acc_empty[buf]);
+        ++q;
+        continue;
+      }
       uint64_t sum[HALF / 2];                  // pairs of columns
 #pragma unroll
       for (int j = 0; j < HALF / 2; ++j) sum[j] = 0;
-      const uint32_t parts = F::PROMOTE ? nkc : 1;
-      for (uint32_t p = 0; p < parts; ++p, ++q) {
+      for (uint32_t p = 0; p < nkc; ++p, ++q) {
         const uint32_t buf = q % F::NACC;
         if (!ptx::mbar_wait(ptx::smem_u32(&acc_full[buf]), (q / F::NACC) & 1, err, 85, wl)) {
           ok = false;
@@ -438,7 +527,7 @@ __global__ void __launch_bounds__(kSplitThreads, 1) f32_split_kernel(const Split
 #pragma unroll
           for (int g = 0; g < HALF; g += 16) {
             uint32_t raw[16];
-            ptx::tmem_ld16(t_row + buf * F::BN + g, raw);
+            ptx::tmem_ld16(t_row + buf * F::TN + g, raw);
             ptx::tmem_wait_ld();
 #pragma unroll
             for (int j = 0; j < 8; ++j)
@@ -447,27 +536,24 @@ __global__ void __launch_bounds__(kSplitThreads, 1) f32_split_kernel(const Split
         }
         ptx::tc_fence_before();
         __syncwarp();
-        if (lane == 0) ptx::mbar_arrive(ptx::smem_u32(&acc_empty[buf]));
+        if (lane == 0) arrive(&acc_empty[buf]);
       }
       if (!ok) break;
       float acc[HALF];
 #pragma unroll
       for (int j = 0; j < HALF / 2; ++j)
-        unpack2(F::NP == 3 ? mul2(sum[j], pack2(kUnscale, kUnscale)) : sum[j], acc[2 * j], acc[2 * j + 1]);
-      // sums to compute again (plain form): not finite, or below the smallest and not zero (2 bits - 1
+        unpack2(mul2(sum[j], pack2(kUnscale, kUnscale)), acc[2 * j], acc[2 * j + 1]);
+      // sums to compute again: not finite, or below the smallest and not zero (2 bits - 1
       // drops the sign and wraps zero to the largest value)
       constexpr uint32_t LO = 2u * kSmallestBits - 1u;
-      bool redo = false;
-      if constexpr (F::NP == 3) {
-        uint32_t low = 0xffffffffu;
-        float high = 0.f;
+      uint32_t low = 0xffffffffu;
+      float high = 0.f;
 #pragma unroll
-        for (int j = 0; j < HALF; ++j) {
-          low = min(low, 2u * __float_as_uint(acc[j]) - 1u);
-          asm("max.NaN.f32 %0, %0, %1;" : "+f"(high) : "f"(fabsf(acc[j])));
-        }
-        redo = __any_sync(0xffffffffu, row_ok && (low < LO || !(high < INFINITY)));
+      for (int j = 0; j < HALF; ++j) {
+        low = min(low, 2u * __float_as_uint(acc[j]) - 1u);
+        asm("max.NaN.f32 %0, %0, %1;" : "+f"(high) : "f"(fabsf(acc[j])));
       }
+      const bool redo = __any_sync(0xffffffffu, row_ok && (low < LO || !(high < INFINITY)));
       if (!redo) {
 #pragma unroll
         for (int g = 0; g < HALF; g += G) {
@@ -488,12 +574,12 @@ __global__ void __launch_bounds__(kSplitThreads, 1) f32_split_kernel(const Split
         }
       } else if (row_ok) {
         // the sound columns, then the others
-        uint64_t mask = 0;
+        uint32_t mask[HALF / 32] = {};
 #pragma unroll
         for (int j = 0; j < HALF; ++j) {
           if (j >= cols) break;
           if (2u * __float_as_uint(acc[j]) - 1u < LO || !(fabsf(acc[j]) < INFINITY)) {
-            mask |= 1ull << j;
+            mask[j / 32] |= 1u << (j % 32);
           } else {
             float* cp = C + (long)j * a.ldc;
             *cp = fmaf(acc[j], a.alpha, read_c ? a.beta * *cp : 0.0f);
@@ -502,9 +588,9 @@ __global__ void __launch_bounds__(kSplitThreads, 1) f32_split_kernel(const Split
         const float* pa = a.A[ti.b] + (a.a_mn ? gi : gi * a.lda);
         const float* pb = a.B[ti.b] + (a.b_mn ? gj0 : gj0 * a.ldb);
         const long ak = a.a_mn ? a.lda : 1, bc = a.b_mn ? 1 : a.ldb, bk = a.b_mn ? a.ldb : 1;
-#pragma unroll 1
-        for (int g = 0; g < cols; g += 16) {
-          const uint32_t mk = (uint32_t)(mask >> g) & 0xffffu;
+#pragma unroll
+        for (int g = 0; g < HALF; g += 16) {
+          const uint32_t mk = (mask[g / 32] >> (g % 32)) & 0xffffu;
           if (mk) split_redo(pa, ak, pb + g * bc, bc, bk, cols - g, (int)a.k, mk, C + (long)g * a.ldc, a.ldc, a.alpha, a.beta);
         }
       }
@@ -512,9 +598,12 @@ __global__ void __launch_bounds__(kSplitThreads, 1) f32_split_kernel(const Split
   }
   ptx::tc_fence_before();
   __syncthreads();
+  // neither CTA of a pair leaves, or gives up its tensor memory, while the other may still reach it
+  if constexpr (F::PAIR) ptx::cluster_sync();
   if (warp == 16) {
     ptx::tc_fence_after();
-    ptx::tmem_dealloc(tmem, F::TMEM_COLS);
+    if constexpr (F::PAIR) ptx::tmem_dealloc_pair(tmem, F::TMEM_COLS);
+    else ptx::tmem_dealloc(tmem, F::TMEM_COLS);
   }
 }
 
@@ -529,7 +618,7 @@ cudaError_t launch_split(const BatchDesc& d, cudaStream_t st) {
   a.beta = d.beta_f;
   a.a_mn = d.transa == SSBLAS_OP_N;
   a.b_mn = d.transb == SSBLAS_OP_T;
-  const long tm = (d.m + 127) / 128, tn = (d.n + F::BN - 1) / F::BN;
+  const long tm = (d.m + F::TM - 1) / F::TM, tn = (d.n + F::TN - 1) / F::TN;
   a.tiles_m = (uint32_t)tm;
   a.tiles_mn = (uint32_t)(tm * tn);
   a.total = (uint32_t)(tm * tn * d.batch);
@@ -542,16 +631,22 @@ cudaError_t launch_split(const BatchDesc& d, cudaStream_t st) {
   auto kern = f32_split_kernel<F>;
   static bool attr[kMaxDevices] = {};
   if (cudaError_t e = smem_attr_once(attr, kern, F::SMEM)) return e;
+  constexpr unsigned CT = F::PAIR ? 2 : 1;
+  const unsigned workers = (unsigned)num_sms() / CT;
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(a.total < (uint32_t)num_sms() ? a.total : (unsigned)num_sms(), 1, 1);
+  cfg.gridDim = dim3(CT * (a.total < workers ? a.total : workers), 1, 1);
   cfg.blockDim = dim3(kSplitThreads, 1, 1);
   cfg.dynamicSmemBytes = F::SMEM;
   cfg.stream = st;
-  cudaLaunchAttribute at[1];
+  cudaLaunchAttribute at[2];
   at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   at[0].val.programmaticStreamSerializationAllowed = 1;
+  at[1].id = cudaLaunchAttributeClusterDimension;
+  at[1].val.clusterDim.x = CT;
+  at[1].val.clusterDim.y = 1;
+  at[1].val.clusterDim.z = 1;
   cfg.attrs = at;
-  cfg.numAttrs = 1;
+  cfg.numAttrs = F::PAIR ? 2 : 1;
   ProfScope prof(F::NP == 3 ? "f32_split" : "bf16x3_split", st);
   note_launch();
   return cudaLaunchKernelEx(&cfg, kern, a);
@@ -562,14 +657,33 @@ cudaError_t launch_split_np(const BatchDesc& d, cudaStream_t st) {
   if (!tcgen05_available()) return cudaErrorNotSupported;
   if (d.k >= (1L << 31) || d.m >= (1L << 31) || d.n >= (1L << 31) || d.lda >= (1L << 25) || d.ldb >= (1L << 25))
     return cudaErrorNotSupported;
-  const long tm = (d.m + 127) / 128, t64 = tm * ((d.n + 63) / 64) * d.batch, t128 = tm * ((d.n + 127) / 128) * d.batch;
-  if (t64 >= (1L << 31)) return cudaErrorNotSupported;
-  const long sms = num_sms();
+  if ((d.m + 127) / 128 * ((d.n + 63) / 64) * d.batch >= (1L << 31)) return cudaErrorNotSupported;
   if (d.m <= 64 && d.n <= 64) return launch_split<Split<NP, 64, 64>>(d, st);
-  // a 64-column chunk takes about two thirds of a 128-column one (measured: 1250 against 1900
-  // cycles), so the narrow tile is taken where it saves a third of the waves or more
-  const bool narrow = d.n <= 64 || (t64 + sms - 1) / sms * 2 < (t128 + sms - 1) / sms * 3;
-  return narrow ? launch_split<Split<NP, 128, 64>>(d, st) : launch_split<Split<NP, 128, 128>>(d, st);
+  // 128 x 64, 128 x 128 or (a pair of CTAs) 256 x 256 tiles: the one whose waves end first, from the time
+  // of a chunk and of a tile's end that each was measured to take (ns; fitted to 16 x 1024^3 and
+  // 4 x 2048^3, checked on 16 other shapes). All give the same results bit for bit. Measured (us, 64 / 128 /
+  // pair): plain 16 x 1024^3 328 / 194 / 166, 256 x 256^3 98 / 62 / 74, 1 x 1024^3 32 / 34 / 47,
+  // 64 x (1024 x 64 x 512) 52 / 69 / 93; 3xBF16 16 x 1024^3 209 / 131 / 96, 256 x 256^3 65 / 44 / 39.
+  struct Cost {
+    long tm, tn, ctas, chunk, tile;
+  };
+  constexpr Cost cost[3] = {{128, 64, 1, NP == 3 ? 750 : 430, NP == 3 ? 300 : 1100},
+                            {128, 128, 1, NP == 3 ? 780 : 520, NP == 3 ? 2600 : 2100},
+                            {256, 256, 2, NP == 3 ? 1030 : 610, NP == 3 ? 8500 : 4400}};
+  const long nkc = (d.k + kKC - 1) / kKC;
+  int best = 0;
+  long least = 0;
+  for (int i = 0; i < 3; ++i) {
+    const Cost& c = cost[i];
+    const long tiles = (d.m + c.tm - 1) / c.tm * ((d.n + c.tn - 1) / c.tn) * d.batch, workers = num_sms() / c.ctas;
+    const long t = (tiles + workers - 1) / workers * (nkc * c.chunk + c.tile);
+    if (i == 0 || t < least) {
+      best = i;
+      least = t;
+    }
+  }
+  if (best == 2) return launch_split<Split<NP, 128, 128, true>>(d, st);
+  return best == 1 ? launch_split<Split<NP, 128, 128>>(d, st) : launch_split<Split<NP, 128, 64>>(d, st);
 }
 
 }  // namespace

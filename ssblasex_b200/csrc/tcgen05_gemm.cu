@@ -595,8 +595,8 @@ cudaError_t launch_bf16x3_f32(const BatchDesc& d, cudaStream_t st) {
   // fed by TMA that splits in shared memory, for equally spaced instances of at most 128 x 128 (the
   // others take configuration 0 / 1); 3 = one kernel that splits the tiles of any instances as it
   // loads them (f32_split.cu). Default: 2 where it applies (4096 x 64^3 TT: 0.057 ms against
-  // 0.084 + 0.072 ms for the split pass and the tiled GEMM), else 3 (256 x 256^3 NT: 0.053 against
-  // 0.130 ms; 16 x 1024^3: 0.170 ms).
+  // 0.084 + 0.072 ms for the split pass and the tiled GEMM), else 3 (256 x 256^3 NT: 0.039 against
+  // 0.130 ms).
   const int fallback = bf16x3_small_fits(d) ? 2 : 3;
   const int cfg = choose_config(SSBLAS_PATH_BF16X3_TCGEN05, d.m, d.n, d.k, d.batch, fallback);
   cudaError_t e;

@@ -6,6 +6,7 @@ Tolerance of the plain form, derived from its arithmetic, in units of u = 2^-24 
 the rounding of the small products (below 2^-7 of it) make at most 5 u, left-out products at most
 1 u, every chunk sum is rounded once when it is added (k / 32 u), alpha and beta 2 u: k / 32 + 8."""
 import ctypes as ct
+import dataclasses
 
 import numpy as np
 import pytest
@@ -72,6 +73,27 @@ def test_plain_against_exact(S, ta, tb, shape, pads, pad, beta):
         err = np.abs(p.c_view(C, b).astype(np.float64) - ex)
         assert np.all(err <= (k / 32 + 8) * U * nrm)
     np.testing.assert_array_equal(C.reshape(batch, n, -1)[:, :, m:], C0.reshape(batch, n, -1)[:, :, m:])
+
+
+@pytest.mark.parametrize("mode", [0, 2])
+@pytest.mark.parametrize("ta,tb,pad", [(0, 0, 0), (0, 1, 3), (1, 0, 4), (1, 1, 1)])
+def test_pair_tiles(S, mode, ta, tb, pad):
+    """Ragged 256 x 256 tiles of CTA pairs (one per instance, 70 for 74 pairs), beside the same instances
+    one by one, whose tiles are a single CTA's: equal bit for bit, and within the bound."""
+    m, n, k, batch = 250, 255, 1000, 70
+    p = problem(ta, tb, m, n, k, batch, 0.25, (pad, pad, pad), 91 + ta, "outliers")
+    S.set_math_mode(mode)
+    try:
+        C = run(S, p)
+        for b in (0, 37, 69):
+            one = dataclasses.replace(p, batch=1, A=p.A[b:b + 1], B=p.B[b:b + 1], C=p.C[b:b + 1])
+            np.testing.assert_array_equal(run(S, one).view(np.uint32), C[b:b + 1].view(np.uint32))
+            ex, nrm = O.exact_f64(one, 0)
+            bound = (k / 32 + 8) * U if mode == 0 else 2.0 ** -14
+            assert np.all(np.abs(p.c_view(C, b).astype(np.float64) - ex) <= bound * nrm)
+    finally:
+        S.set_math_mode(0)
+    np.testing.assert_array_equal(C.reshape(batch, n, -1)[:, :, m:], p.C.reshape(batch, n, -1)[:, :, m:])
 
 
 @pytest.mark.parametrize("ta,tb", [(0, 0), (1, 1)])
