@@ -38,12 +38,14 @@
 // tile took 1850 cycles; so did one of a pair while its arrivals asked for a cluster-wide release.
 // Measured (ms, FFMA kernels -> this one): 16 x 1024^3 NN 0.829 -> 0.166 (207 TFLOP/s); 4 x 2048^3 1.73 ->
 // 0.297; 64 x 128^3 NN 0.0145 -> 0.0125; 8 x (777 x 555 x 333) 0.103 -> 0.041; 2 x 128^2 x 4096 0.19 -> 0.094.
-// 3xBF16 (split pass and tiled GEMM -> this kernel): 256 x 256^3 0.130 -> 0.039, 16 x 1024^3 0.096.
+// 3xBF16 (split pass and tiled GEMM -> this kernel): 256 x 256^3 0.130 -> 0.039, 16 x 1024^3 0.096; a grouped
+// call's 5000 instances of 8 to 512 each way 0.564 -> 0.39.
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 #include <stdint.h>
 
 #include "f32x2.cuh"
+#include "grouped.h"
 #include "internal.h"
 #include "ptx.cuh"
 
@@ -90,6 +92,18 @@ struct Split {
   static_assert(256 * (CONV_REGS + EPI_REGS) + 128 * kIssueRegs <= kSplitThreads * 96, "registers");
 };
 
+// One tile of a grouped launch as a worker's warps see it: its record and its instance's matrices. A
+// scheduler warp reads both up to kRing tiles ahead of the others, eight at a time (a lane per tile, so a
+// batch costs one chain of dependent loads), into a ring in shared memory.
+struct SplitItem {
+  SplitRec r;
+  const float* A;
+  const float* B;
+  float* C;
+  int valid, pad;            // valid = 0 ends the worker's tiles
+};
+constexpr uint32_t kRing = 16;
+
 struct SplitArgs {
   long m, n, k, lda, ldb, ldc;
   const float* const* A;
@@ -101,6 +115,7 @@ struct SplitArgs {
   int* err;
   uint32_t wait_limit;
   int skip;                // injected fault: CTA 0 never signals its first chunk
+  const SplitRec* recs;    // grouped launches: one per tile
 };
 
 // One work item: the tile at (m0, n0) of instance b.
@@ -123,8 +138,15 @@ struct SplitOperand {
   const float *p, *base;
   int step, adv;           // elements between units, between chunks (ld < 2^25)
   int rows, k;             // valid rows from this thread's unit 0 on; valid k from the next chunk on
+  int units, bytes;        // units with a row inside the matrix, and the valid bytes of one inside K
   bool mn, vec, full;      // full: every unit of the tile's whole chunks is inside the matrix
 };
+// A thread's units with a row inside the matrix, `rows` of which are left from its unit 0 on.
+template <int ROWS>
+__device__ __forceinline__ int split_units(int rows, bool mn) {
+  constexpr int U = ROWS * kKC / 4 / kConvThreads;
+  return rows <= 0 ? 0 : mn ? U : min(U, (rows + 31) / 32);
+}
 template <int ROWS>
 __device__ __forceinline__ SplitOperand split_operand(const float* X, long rows, long K, long ld, bool mn, long r0,
                                                       int t) {
@@ -140,27 +162,39 @@ __device__ __forceinline__ SplitOperand split_operand(const float* X, long rows,
   o.adv = mn ? kKC * (int)ld : kKC;
   o.rows = (int)(rows - r0 < ROWS ? rows - r0 : ROWS) - rr;
   o.k = (int)K;
+  o.units = split_units<ROWS>(o.rows, mn);
+  o.bytes = mn && o.rows < 4 ? 4 * o.rows : 16;
   return o;
 }
 
 __device__ __forceinline__ void copy16(uint32_t dst, const float* src, int bytes) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(dst), "l"(src), "r"(bytes) : "memory");
 }
+__device__ __forceinline__ void copy16_if(bool on, uint32_t dst, const float* src, int bytes) {
+  asm volatile("{\n.reg .pred p;\nsetp.ne.b32 p, %3, 0;\n@p cp.async.cg.shared.global [%0], [%1], 16, %2;\n}" ::"r"(dst),
+               "l"(src), "r"(bytes), "r"((int)on)
+               : "memory");
+}
 __device__ __forceinline__ void copy4(uint32_t dst, const float* src, bool ok) {
   asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;\n" ::"r"(dst), "l"(src), "r"(ok ? 4 : 0) : "memory");
 }
 // Copies the units of the next chunk to this thread's places, unit i at dst + i * 4096 (zeros outside the
-// matrix); the operand moves on to the chunk after it.
-template <int ROWS, int U>
+// matrix); the operand moves on to the chunk after it. SKIP: units past the matrix's rows stay as they are.
+template <int ROWS, int U, bool SKIP>
 __device__ __forceinline__ void split_copy(SplitOperand& o, int t, uint32_t dst) {
   constexpr int RG = ROWS / 4;
   const float* src = o.p;
   if (o.full && o.k >= kKC) {
 #pragma unroll
     for (int i = 0; i < U; ++i, src += o.step) copy16(dst + i * kUnitRow, src, 16);
+  } else if (SKIP && o.vec && o.k >= kKC) {
+#pragma unroll
+    for (int i = 0; i < U; ++i, src += o.step)
+      copy16_if(i < o.units, dst + i * kUnitRow, src, o.bytes);
   } else {
 #pragma unroll
     for (int i = 0; i < U; ++i, src += o.step) {
+      if (SKIP && i >= o.units) break;
       const int kk = o.mn ? t / RG + i * (kConvThreads / RG) : 4 * (t % 8);
       int n = o.mn ? (o.k > kk ? o.rows : 0) : (o.rows > 32 * i ? o.k - kk : 0);   // valid elements
       n = n < 0 ? 0 : n > 4 ? 4 : n;
@@ -188,9 +222,10 @@ __device__ __forceinline__ uint32_t take_bf16(uint64_t& v) {
   return w;
 }
 
-// Splits this thread's units (unit i at raw + i * 4096) and writes the NP parts of the operand.
-template <int NP, int ROWS, int U>
-__device__ __forceinline__ void split_store(uint32_t raw, uint32_t dst, bool mn, int t) {
+// Splits this thread's units (unit i at raw + i * 4096; SOME: the first `units` of them) and writes the NP
+// parts of the operand.
+template <int NP, int ROWS, int U, bool SOME>
+__device__ __forceinline__ void split_store(uint32_t raw, uint32_t dst, bool mn, int t, int units) {
   constexpr int PLANE = ROWS * kKC * 2;
   constexpr int RG = ROWS / 4;
   uint32_t off, step;
@@ -205,11 +240,18 @@ __device__ __forceinline__ void split_store(uint32_t raw, uint32_t dst, bool mn,
     off = rr * 64u + (((kq >> 1) ^ ((rr >> 1) & 3u)) << 4) + ((kq & 1u) << 3);
     step = 32 * 64u;
   }
-  // all reads before the first write: the units' conversions then overlap
-  uint64_t v[U][2];
+  // all reads before the first write: the units' conversions then overlap. (SOME: by predicates, since a
+  // branch per unit would take that overlap away and measured 1.8 times as long on whole tiles)
+  uint64_t v[U][2] = {};
 #pragma unroll
   for (int i = 0; i < U; ++i)
-    asm volatile("ld.shared.v2.b64 {%0, %1}, [%2];" : "=l"(v[i][0]), "=l"(v[i][1]) : "r"(raw + i * kUnitRow) : "memory");
+    if (SOME)
+      asm volatile("{\n.reg .pred p;\nsetp.lt.s32 p, %3, %4;\n@p ld.shared.v2.b64 {%0, %1}, [%2];\n}"
+                   : "+l"(v[i][0]), "+l"(v[i][1])
+                   : "r"(raw + i * kUnitRow), "r"(i), "r"(units)
+                   : "memory");
+    else
+      asm volatile("ld.shared.v2.b64 {%0, %1}, [%2];" : "=l"(v[i][0]), "=l"(v[i][1]) : "r"(raw + i * kUnitRow) : "memory");
   if constexpr (NP == 3) {
 #pragma unroll
     for (int i = 0; i < U; ++i)
@@ -225,8 +267,14 @@ __device__ __forceinline__ void split_store(uint32_t raw, uint32_t dst, bool mn,
       for (int h = 0; h < 2; ++h) w[i][h] = p + 1 < NP ? take_bf16<true>(v[i][h]) : take_bf16<false>(v[i][h]);
 #pragma unroll
     for (int i = 0; i < U; ++i)
-      asm volatile("st.shared.v2.b32 [%0], {%1, %2};" ::"r"(dst + off + i * step + p * PLANE), "r"(w[i][0]), "r"(w[i][1])
-                   : "memory");
+      if (SOME)
+        asm volatile("{\n.reg .pred p;\nsetp.lt.s32 p, %3, %4;\n@p st.shared.v2.b32 [%0], {%1, %2};\n}" ::"r"(
+                         dst + off + i * step + p * PLANE),
+                     "r"(w[i][0]), "r"(w[i][1]), "r"(i), "r"(units)
+                     : "memory");
+      else
+        asm volatile("st.shared.v2.b32 [%0], {%1, %2};" ::"r"(dst + off + i * step + p * PLANE), "r"(w[i][0]), "r"(w[i][1])
+                     : "memory");
   }
 }
 
@@ -266,8 +314,13 @@ __device__ __noinline__ void split_redo(const float* pa, long ak, const float* p
     if ((mask >> j) & 1u) C[j * ldc] = fmaf(acc[j], alpha, beta != 0.0f ? beta * C[j * ldc] : 0.0f);
 }
 
-template <class F>
+// GROUPED: the tiles, their shapes and scalars come from a.recs. What bounds it on mixed small shapes (8 to 512
+// each way: 875 MB in 0.39 ms, 2.2 TB/s) is the converters' own instructions, 1 us a chunk whether it is
+// whole or not: a second group of converter warps (which took them below 64 registers) made it 1.8 times
+// as long, so the units of rows outside the matrix are left out instead (0.403 -> 0.390 ms).
+template <class F, bool GROUPED>
 __global__ void __launch_bounds__(kSplitThreads, 1) f32_split_kernel(const SplitArgs a) {
+  static_assert(!GROUPED || (!F::PAIR && !F::PROMOTE), "grouped launches: 3xBF16, one CTA per tile");
   extern __shared__ uint8_t smem_raw[];
   uint8_t* stages = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
   uint8_t* raw = stages + F::STAGES * F::STAGE;                  // [RAW] fp32 units, a place per thread
@@ -276,8 +329,11 @@ __global__ void __launch_bounds__(kSplitThreads, 1) f32_split_kernel(const Split
   uint64_t* acc_full = empty + F::STAGES;                        // [NACC] sums complete (commit)
   uint64_t* acc_empty = acc_full + F::NACC;                      // [NACC] sums read (8 warps)
   uint64_t* drain = acc_empty + F::NACC;
-  uint32_t* tmem_slot = (uint32_t*)(drain + 1);
-  static_assert((2 * F::STAGES + 2 * F::NACC + 1) * 8 + 4 <= 512, "barrier area");
+  uint64_t* ring_full = drain + 1;                               // [kRing] record written (scheduler)
+  uint64_t* ring_empty = ring_full + kRing;                      // [kRing] record read (17 warps)
+  uint32_t* tmem_slot = (uint32_t*)(ring_empty + kRing);
+  SplitItem* ring = (SplitItem*)((uint8_t*)full + 512);
+  static_assert((2 * F::STAGES + 2 * F::NACC + 1 + 2 * kRing) * 8 + 4 <= 512, "barrier area");
 
   const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
   const uint32_t wl = a.wait_limit ? a.wait_limit : ptx::kWaitLimit;
@@ -296,6 +352,12 @@ __global__ void __launch_bounds__(kSplitThreads, 1) f32_split_kernel(const Split
       ptx::mbar_init(ptx::smem_u32(&acc_empty[q]), CT * 8);
     }
     ptx::mbar_init(ptx::smem_u32(drain), 1);
+    if (GROUPED) {
+      for (uint32_t q = 0; q < kRing; ++q) {
+        ptx::mbar_init(ptx::smem_u32(&ring_full[q]), 1);
+        ptx::mbar_init(ptx::smem_u32(&ring_empty[q]), 17);
+      }
+    }
     ptx::fence_mbar_init();
   }
   if (warp == 16) {
@@ -314,7 +376,16 @@ __global__ void __launch_bounds__(kSplitThreads, 1) f32_split_kernel(const Split
   // under a programmatic launch the set-up above overlaps the end of the kernel before
   ptx::grid_dep_wait();
   ptx::grid_dep_launch();
-  const uint32_t nkc = (uint32_t)((a.k + kKC - 1) / kKC);
+  const uint32_t nkc_all = (uint32_t)((a.k + kKC - 1) / kKC);   // chunks of every tile of a batched launch
+  // the worker's i-th tile: whether there is one (grouped: once its record has arrived)
+  auto tile_ready = [&](uint32_t i, int code) -> bool {
+    if constexpr (GROUPED) {
+      const uint32_t q = i % kRing;
+      return ptx::mbar_wait(ptx::smem_u32(&ring_full[q]), (i / kRing) & 1, err, code, wl) && ring[q].valid;
+    } else {
+      return me + i * workers < a.total;
+    }
+  };
 
   // a pair's `full` and `acc_empty` are the leader's, and collect both CTAs' arrivals
   auto arrive = [&](uint64_t* bar) {
@@ -329,22 +400,33 @@ __global__ void __launch_bounds__(kSplitThreads, 1) f32_split_kernel(const Split
     const int t = threadIdx.x - 256;
     const uint32_t stages0 = ptx::smem_u32(stages);
     const uint32_t raw0 = ptx::smem_u32(raw) + 16 * t;
-    uint32_t lt = me, lkc = 0, lr = 0;     // next chunk to copy: tile, chunk of it, place
+    // next chunk to copy: tile, chunk of it, place
+    uint32_t li = 0, lkc = 0, lr = 0;
+    uint32_t lnkc = nkc_all;               // chunks of that tile
+    bool more = true;                      // there is such a tile
     SplitOperand A, B;
     auto enter = [&]() {
-      if (lt >= a.total) return;
-      const SplitTile ti = split_tile<F>(a, lt);
-      A = split_operand<F::AR>(a.A[ti.b], a.m, a.k, a.lda, a.a_mn != 0, ti.m0 + rank * 128, t);
-      B = split_operand<F::BN>(a.B[ti.b], a.n, a.k, a.ldb, a.b_mn != 0, ti.n0 + rank * F::BN, t);
+      more = tile_ready(li, 88);
+      if (!more) return;
+      if constexpr (GROUPED) {
+        const SplitItem& it = ring[li % kRing];
+        A = split_operand<F::AR>(it.A, it.r.m, it.r.k, it.r.lda, it.r.a_mn != 0, it.r.m0, t);
+        B = split_operand<F::BN>(it.B, it.r.n, it.r.k, it.r.ldb, it.r.b_mn != 0, it.r.n0, t);
+        lnkc = (uint32_t)it.r.nkc;
+      } else {
+        const SplitTile ti = split_tile<F>(a, me + li * workers);
+        A = split_operand<F::AR>(a.A[ti.b], a.m, a.k, a.lda, a.a_mn != 0, ti.m0 + rank * 128, t);
+        B = split_operand<F::BN>(a.B[ti.b], a.n, a.k, a.ldb, a.b_mn != 0, ti.n0 + rank * F::BN, t);
+      }
     };
     auto copy = [&]() {
-      if (lt < a.total) {
+      if (more) {
         const uint32_t dst = raw0 + lr * F::RAW_STAGE;
-        split_copy<F::AR, F::UA>(A, t, dst);
-        split_copy<F::BN, F::UB>(B, t, dst + F::UA * kUnitRow);
-        if (++lkc == nkc) {
+        split_copy<F::AR, F::UA, GROUPED>(A, t, dst);
+        split_copy<F::BN, F::UB, GROUPED>(B, t, dst + F::UA * kUnitRow);
+        if (++lkc == lnkc) {
           lkc = 0;
-          lt += workers;
+          ++li;
           enter();
         }
       }
@@ -356,7 +438,20 @@ __global__ void __launch_bounds__(kSplitThreads, 1) f32_split_kernel(const Split
     for (int d = 0; d < F::RAW; ++d) copy();
     uint32_t c = 0, s = 0, r = 0;
     bool ok = true;
-    for (uint32_t cur = me; ok && cur < a.total; cur += workers) {
+    for (uint32_t i = 0; ok && (i < li || more); ++i) {   // the copies are at tile i or past it
+      bool amn = a.a_mn != 0, bmn = a.b_mn != 0;
+      uint32_t nkc = nkc_all;
+      // a grouped call's tiles are often mostly outside their matrices: what stands in the rows past one
+      // (any bits) reaches only results that are not stored
+      int ua = F::UA, ub = F::UB;
+      if constexpr (GROUPED) {
+        const SplitItem& it = ring[i % kRing];
+        ua = split_units<F::AR>(it.r.m - it.r.m0 - (it.r.a_mn ? 4 * (t % (F::AR / 4)) : t / 8), it.r.a_mn != 0);
+        ub = split_units<F::BN>(it.r.n - it.r.n0 - (it.r.b_mn ? 4 * (t % (F::BN / 4)) : t / 8), it.r.b_mn != 0);
+        amn = it.r.a_mn != 0;
+        bmn = it.r.b_mn != 0;
+        nkc = (uint32_t)it.r.nkc;
+      }
       for (uint32_t kc = 0; kc < nkc; ++kc, ++c) {
         // the stage is waited for before the next copies are queued: behind them the answer would take
         // hundreds of cycles
@@ -367,13 +462,16 @@ __global__ void __launch_bounds__(kSplitThreads, 1) f32_split_kernel(const Split
         if (c > 0) copy();                   // into the place of the chunk before, which this thread has read
         asm volatile("cp.async.wait_group %0;" ::"n"(F::RAW - 1) : "memory");   // (each thread reads its own units)
         const uint32_t st = stages0 + s * F::STAGE, rw = raw0 + r * F::RAW_STAGE;
-        split_store<F::NP, F::AR, F::UA>(rw, st, a.a_mn != 0, t);
-        split_store<F::NP, F::BN, F::UB>(rw + F::UA * kUnitRow, st + F::NP * F::A_PLANE, a.b_mn != 0, t);
+        split_store<F::NP, F::AR, F::UA, GROUPED>(rw, st, amn, t, ua);
+        split_store<F::NP, F::BN, F::UB, GROUPED>(rw + F::UA * kUnitRow, st + F::NP * F::A_PLANE, bmn, t, ub);
         ptx::fence_proxy_async_smem();   // generic-proxy writes -> the tensor core's reads
         __syncwarp();
         if (lane == 0 && !(a.skip && c == 0 && blockIdx.x == 0)) arrive(&full[s]);
         if (++s == F::STAGES) s = 0;
         if (++r == F::RAW) r = 0;
+      }
+      if constexpr (GROUPED) {
+        if (lane == 0) ptx::mbar_arrive(ptx::smem_u32(&ring_empty[i % kRing]));
       }
     }
     asm volatile("cp.async.wait_group 0;" ::: "memory");   // no copy is in flight when the CTA exits
@@ -381,17 +479,12 @@ __global__ void __launch_bounds__(kSplitThreads, 1) f32_split_kernel(const Split
     // ------------------------------------------------------------------ MMA ---------------
     asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kIssueRegs));
     if (warp == 16 && rank == 0) {
-      const uint32_t idesc = ptx::idesc_bf16(F::TM, F::TN, a.a_mn != 0, a.b_mn != 0);
       // descriptors of stage 0's first part, and their step along K: 16 k are 32 bytes of a K-major
       // line, 16 lines of an MN-major block (addresses count 16 bytes). The whole warp runs the loop
       // and one lane's predicate is on the MMA itself, so descriptors stay in uniform registers:
       // under a branch on the lane each MMA cost four moves into them, 90 cycles a MMA.
       const uint32_t lead = ptx::elect_one();
       const uint32_t st0 = ptx::smem_u32(stages);
-      const uint64_t a0 = a.a_mn ? ptx::smem_desc_mnmajor(st0, kKC * 128) : ptx::smem_desc_kmajor(st0, 64);
-      const uint64_t b0 = a.b_mn ? ptx::smem_desc_mnmajor(st0 + F::NP * F::A_PLANE, kKC * 128)
-                                 : ptx::smem_desc_kmajor(st0 + F::NP * F::A_PLANE, 64);
-      const uint64_t ka = a.a_mn ? 128 : 2, kb = a.b_mn ? 128 : 2;
       static_assert(kKC == 32, "two K steps per chunk");
       uint32_t c = 0, q = 0;     // chunks, accumulators
       bool ok = true;
@@ -399,7 +492,21 @@ __global__ void __launch_bounds__(kSplitThreads, 1) f32_split_kernel(const Split
         if constexpr (F::PAIR) ptx::mma_commit_pair_if(lead, ptx::smem_u32(bar));
         else ptx::mma_commit_if(lead, ptx::smem_u32(bar));
       };
-      for (uint32_t t = me; t < a.total && ok; t += workers) {
+      for (uint32_t i = 0; ok && tile_ready(i, 89); ++i) {
+        bool amn = a.a_mn != 0, bmn = a.b_mn != 0;
+        uint32_t nkc = nkc_all;
+        if constexpr (GROUPED) {
+          const SplitItem& it = ring[i % kRing];
+          amn = __shfl_sync(0xffffffffu, it.r.a_mn, 0) != 0;
+          bmn = __shfl_sync(0xffffffffu, it.r.b_mn, 0) != 0;
+          nkc = (uint32_t)__shfl_sync(0xffffffffu, it.r.nkc, 0);
+          if (lane == 0) ptx::mbar_arrive(ptx::smem_u32(&ring_empty[i % kRing]));
+        }
+        const uint32_t idesc = ptx::idesc_bf16(F::TM, F::TN, amn, bmn);
+        const uint64_t a0 = amn ? ptx::smem_desc_mnmajor(st0, kKC * 128) : ptx::smem_desc_kmajor(st0, 64);
+        const uint64_t b0 = bmn ? ptx::smem_desc_mnmajor(st0 + F::NP * F::A_PLANE, kKC * 128)
+                                : ptx::smem_desc_kmajor(st0 + F::NP * F::A_PLANE, 64);
+        const uint64_t ka = amn ? 128 : 2, kb = bmn ? 128 : 2;
         for (uint32_t kc = 0; kc < nkc; ++kc, ++c) {
           const uint32_t s = c % F::STAGES;
           if (F::PROMOTE || kc == 0) {
@@ -443,6 +550,26 @@ __global__ void __launch_bounds__(kSplitThreads, 1) f32_split_kernel(const Split
       ptx::mbar_wait(ptx::smem_u32(drain), 0, err, 84, wl);
     } else if (warp == 16) {
       ptx::mbar_wait(ptx::smem_u32(drain), 0, err, 84, wl);   // the leader's last arrival here
+    } else if (GROUPED && warp == 17) {
+      // ---------------------------------------------------------------- scheduler ---------
+      constexpr uint32_t kBatch = kRing / 2;
+      for (uint32_t i = 0;; i += kBatch) {
+        const uint32_t rec = i + lane, q = rec % kRing, t = me + rec * workers;
+        bool last = false;
+        if (lane < kBatch) {
+          last = !ptx::mbar_wait(ptx::smem_u32(&ring_empty[q]), ((rec / kRing) & 1) ^ 1, err, 80, wl) || t >= a.total;
+          SplitItem& it = ring[q];
+          if (!last) {
+            it.r = a.recs[t];
+            it.A = a.A[it.r.idx];
+            it.B = a.B[it.r.idx];
+            it.C = a.C[it.r.idx];
+          }
+          it.valid = last ? 0 : 1;
+          ptx::mbar_arrive(ptx::smem_u32(&ring_full[q]));
+        }
+        if (__any_sync(0xffffffffu, last)) break;
+      }
     }
   } else {
     // ------------------------------------------------------------------ epilogue ----------
@@ -453,56 +580,87 @@ __global__ void __launch_bounds__(kSplitThreads, 1) f32_split_kernel(const Split
     const bool active = quarter * 32 < F::AR;      // rows past AR hold no results
     uint32_t q = 0;
     bool ok = true;
-    for (uint32_t t = me; t < a.total && ok; t += workers) {
-      const SplitTile ti = split_tile<F>(a, t);
-      const long gi = ti.m0 + rank * 128 + quarter * 32 + lane, gj0 = ti.n0 + half * HALF;
-      float* C = a.C[ti.b] + gi + gj0 * a.ldc;
-      const bool row_ok = active && gi < a.m;
-      const int cols = gj0 < a.n ? (a.n - gj0 < HALF ? (int)(a.n - gj0) : HALF) : 0;
-      const bool read_c = a.beta != 0.0f;
-      // narrow tiles: C is in flight while the products run
+    for (uint32_t i = 0; ok && tile_ready(i, 90); ++i) {
+      long gi = rank * 128 + quarter * 32 + lane, gj0 = half * HALF, m = a.m, n = a.n, ldc = a.ldc;
+      float alpha = a.alpha, beta = a.beta;
+      float* C;
+      uint32_t b = 0;
+      if constexpr (GROUPED) {
+        const SplitItem& it = ring[i % kRing];
+        gi += it.r.m0;
+        gj0 += it.r.n0;
+        m = it.r.m;
+        n = it.r.n;
+        ldc = it.r.ldc;
+        alpha = it.r.alpha;
+        beta = it.r.beta;
+        C = it.C;
+        __syncwarp();
+        if (lane == 0) ptx::mbar_arrive(ptx::smem_u32(&ring_empty[i % kRing]));
+      } else {
+        const SplitTile ti = split_tile<F>(a, me + i * workers);
+        b = ti.b;
+        gi += ti.m0;
+        gj0 += ti.n0;
+        C = a.C[b];
+      }
+      C += gi + gj0 * ldc;
+      const bool row_ok = active && gi < m;
+      const int cols = gj0 < n ? (n - gj0 < HALF ? (int)(n - gj0) : HALF) : 0;
+      const bool read_c = beta != 0.0f;
+      if constexpr (GROUPED) {
+        // the next tile's C: short tiles leave the reads no other time to cross HBM
+        if (tile_ready(i + 1, 91) && ring[(i + 1) % kRing].r.beta != 0.0f) {
+          const SplitItem& nx = ring[(i + 1) % kRing];
+          const int r0 = nx.r.m0 + quarter * 32, c0 = nx.r.n0 + half * HALF;
+#pragma unroll
+          for (int h = 0; h < HALF; h += 32)
+            if (r0 < nx.r.m && c0 + h + lane < nx.r.n) ptx::prefetch_l2(nx.C + r0 + (c0 + h + lane) * nx.r.ldc);
+        }
+      }
+      // narrow tiles, and those of one accumulator: C is in flight while the products run
       constexpr bool EARLY_C = HALF == 32;
       constexpr int G = EARLY_C || !F::PROMOTE ? 32 : 16;     // columns per group
       float cv[G];
       // (the walking pointers are opaque to the compiler: it would keep an address per column otherwise)
       auto load_c = [&](int j0) {
-        const float* cp = C + (long)j0 * a.ldc;
+        const float* cp = C + (long)j0 * ldc;
         asm volatile("" : "+l"(cp));
-        if (row_ok && cols == HALF) {
+        if (row_ok && cols >= j0 + G) {
 #pragma unroll
-          for (int j = 0; j < G; ++j, cp += a.ldc) cv[j] = __ldcs(cp);
+          for (int j = 0; j < G; ++j, cp += ldc) cv[j] = __ldcs(cp);
         } else {
 #pragma unroll
-          for (int j = 0; j < G; ++j, cp += a.ldc) cv[j] = (row_ok && j0 + j < cols) ? __ldcs(cp) : 0.0f;
+          for (int j = 0; j < G; ++j, cp += ldc) cv[j] = (row_ok && j0 + j < cols) ? __ldcs(cp) : 0.0f;
         }
       };
-      if (EARLY_C && read_c) load_c(0);
+      if ((EARLY_C || !F::PROMOTE) && read_c) load_c(0);
       if constexpr (!F::PROMOTE) {
         // one accumulator per tile: groups of columns straight from it to C
         const uint32_t buf = q % F::NACC;
         if (!ptx::mbar_wait(ptx::smem_u32(&acc_full[buf]), (q / F::NACC) & 1, err, 85, wl)) break;
         ptx::tc_fence_after();
-        if (active) {
+        if (active && gi - lane < m) {
 #pragma unroll 1
-          for (int g = 0; g < HALF; g += G) {
+          for (int g = 0; g < cols; g += G) {
             uint32_t raw[G / 16][16];
 #pragma unroll
-            for (int i = 0; i < G / 16; ++i) ptx::tmem_ld16(t_row + buf * F::TN + g + 16 * i, raw[i]);
-            if (!EARLY_C && read_c) load_c(g);
+            for (int h = 0; h < G / 16; ++h) ptx::tmem_ld16(t_row + buf * F::TN + g + 16 * h, raw[h]);
             ptx::tmem_wait_ld();
-            float* cp = C + (long)g * a.ldc;
-            asm volatile("" : "+l"(cp));
-            if (!row_ok) continue;
 #pragma unroll
             for (int j = 0; j < G; ++j)
               raw[j / 16][j % 16] =
-                  __float_as_uint(fmaf(__uint_as_float(raw[j / 16][j % 16]), a.alpha, read_c ? a.beta * cv[j] : 0.0f));
-            if (cols == HALF) {
+                  __float_as_uint(fmaf(__uint_as_float(raw[j / 16][j % 16]), alpha, read_c ? beta * cv[j] : 0.0f));
+            if (read_c && g + G < cols) load_c(g + G);
+            float* cp = C + (long)g * ldc;
+            asm volatile("" : "+l"(cp));
+            if (!row_ok) continue;
+            if (cols >= g + G) {
 #pragma unroll
-              for (int j = 0; j < G; ++j, cp += a.ldc) __stcs(cp, __uint_as_float(raw[j / 16][j % 16]));
+              for (int j = 0; j < G; ++j, cp += ldc) __stcs(cp, __uint_as_float(raw[j / 16][j % 16]));
             } else {
 #pragma unroll
-              for (int j = 0; j < G; ++j, cp += a.ldc)
+              for (int j = 0; j < G; ++j, cp += ldc)
                 if (g + j < cols) __stcs(cp, __uint_as_float(raw[j / 16][j % 16]));
             }
           }
@@ -516,7 +674,7 @@ __global__ void __launch_bounds__(kSplitThreads, 1) f32_split_kernel(const Split
       uint64_t sum[HALF / 2];                  // pairs of columns
 #pragma unroll
       for (int j = 0; j < HALF / 2; ++j) sum[j] = 0;
-      for (uint32_t p = 0; p < nkc; ++p, ++q) {
+      for (uint32_t p = 0; p < nkc_all; ++p, ++q) {
         const uint32_t buf = q % F::NACC;
         if (!ptx::mbar_wait(ptx::smem_u32(&acc_full[buf]), (q / F::NACC) & 1, err, 85, wl)) {
           ok = false;
@@ -558,17 +716,17 @@ __global__ void __launch_bounds__(kSplitThreads, 1) f32_split_kernel(const Split
 #pragma unroll
         for (int g = 0; g < HALF; g += G) {
           if (!EARLY_C && read_c) load_c(g);
-          float* cp = C + (long)g * a.ldc;
+          float* cp = C + (long)g * ldc;
           asm volatile("" : "+l"(cp));
 #pragma unroll
-          for (int j = 0; j < G; ++j) acc[g + j] = fmaf(acc[g + j], a.alpha, read_c ? a.beta * cv[j] : 0.0f);
+          for (int j = 0; j < G; ++j) acc[g + j] = fmaf(acc[g + j], alpha, read_c ? beta * cv[j] : 0.0f);
           if (!row_ok) continue;
           if (cols == HALF) {
 #pragma unroll
-            for (int j = 0; j < G; ++j, cp += a.ldc) __stcs(cp, acc[g + j]);
+            for (int j = 0; j < G; ++j, cp += ldc) __stcs(cp, acc[g + j]);
           } else {
 #pragma unroll
-            for (int j = 0; j < G; ++j, cp += a.ldc)
+            for (int j = 0; j < G; ++j, cp += ldc)
               if (g + j < cols) __stcs(cp, acc[g + j]);
           }
         }
@@ -581,17 +739,17 @@ __global__ void __launch_bounds__(kSplitThreads, 1) f32_split_kernel(const Split
           if (2u * __float_as_uint(acc[j]) - 1u < LO || !(fabsf(acc[j]) < INFINITY)) {
             mask[j / 32] |= 1u << (j % 32);
           } else {
-            float* cp = C + (long)j * a.ldc;
-            *cp = fmaf(acc[j], a.alpha, read_c ? a.beta * *cp : 0.0f);
+            float* cp = C + (long)j * ldc;
+            *cp = fmaf(acc[j], alpha, read_c ? beta * *cp : 0.0f);
           }
         }
-        const float* pa = a.A[ti.b] + (a.a_mn ? gi : gi * a.lda);
-        const float* pb = a.B[ti.b] + (a.b_mn ? gj0 : gj0 * a.ldb);
+        const float* pa = a.A[b] + (a.a_mn ? gi : gi * a.lda);
+        const float* pb = a.B[b] + (a.b_mn ? gj0 : gj0 * a.ldb);
         const long ak = a.a_mn ? a.lda : 1, bc = a.b_mn ? 1 : a.ldb, bk = a.b_mn ? a.ldb : 1;
 #pragma unroll
         for (int g = 0; g < HALF; g += 16) {
           const uint32_t mk = (mask[g / 32] >> (g % 32)) & 0xffffu;
-          if (mk) split_redo(pa, ak, pb + g * bc, bc, bk, cols - g, (int)a.k, mk, C + (long)g * a.ldc, a.ldc, a.alpha, a.beta);
+          if (mk) split_redo(pa, ak, pb + g * bc, bc, bk, cols - g, (int)a.k, mk, C + (long)g * ldc, ldc, alpha, beta);
         }
       }
     }
@@ -605,6 +763,41 @@ __global__ void __launch_bounds__(kSplitThreads, 1) f32_split_kernel(const Split
     if constexpr (F::PAIR) ptx::tmem_dealloc_pair(tmem, F::TMEM_COLS);
     else ptx::tmem_dealloc(tmem, F::TMEM_COLS);
   }
+}
+
+// One launch over a.total tiles.
+template <class F, bool GROUPED>
+cudaError_t launch_tiles(SplitArgs a, const char* name, cudaStream_t st) {
+  a.err = device_error_flag();
+  if (!GROUPED && settings().fault == SSBLAS_FAULT_SKIP_COPY) {
+    settings().fault = SSBLAS_FAULT_NONE;
+    a.skip = 1;
+    a.wait_limit = 1u << 10;
+  }
+  auto kern = f32_split_kernel<F, GROUPED>;
+  constexpr int smem = F::SMEM + (GROUPED ? kRing * (int)sizeof(SplitItem) : 0);
+  static_assert(smem <= 232448, "shared memory");
+  static bool attr[kMaxDevices] = {};
+  if (cudaError_t e = smem_attr_once(attr, kern, smem)) return e;
+  constexpr unsigned CT = F::PAIR ? 2 : 1;
+  const unsigned workers = (unsigned)num_sms() / CT;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(CT * (a.total < workers ? a.total : workers), 1, 1);
+  cfg.blockDim = dim3(kSplitThreads, 1, 1);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cudaLaunchAttribute at[2];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = 1;
+  at[1].id = cudaLaunchAttributeClusterDimension;
+  at[1].val.clusterDim.x = CT;
+  at[1].val.clusterDim.y = 1;
+  at[1].val.clusterDim.z = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = F::PAIR ? 2 : 1;
+  ProfScope prof(name, st);
+  note_launch();
+  return cudaLaunchKernelEx(&cfg, kern, a);
 }
 
 template <class F>
@@ -622,34 +815,7 @@ cudaError_t launch_split(const BatchDesc& d, cudaStream_t st) {
   a.tiles_m = (uint32_t)tm;
   a.tiles_mn = (uint32_t)(tm * tn);
   a.total = (uint32_t)(tm * tn * d.batch);
-  a.err = device_error_flag();
-  if (settings().fault == SSBLAS_FAULT_SKIP_COPY) {
-    settings().fault = SSBLAS_FAULT_NONE;
-    a.skip = 1;
-    a.wait_limit = 1u << 10;
-  }
-  auto kern = f32_split_kernel<F>;
-  static bool attr[kMaxDevices] = {};
-  if (cudaError_t e = smem_attr_once(attr, kern, F::SMEM)) return e;
-  constexpr unsigned CT = F::PAIR ? 2 : 1;
-  const unsigned workers = (unsigned)num_sms() / CT;
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(CT * (a.total < workers ? a.total : workers), 1, 1);
-  cfg.blockDim = dim3(kSplitThreads, 1, 1);
-  cfg.dynamicSmemBytes = F::SMEM;
-  cfg.stream = st;
-  cudaLaunchAttribute at[2];
-  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  at[0].val.programmaticStreamSerializationAllowed = 1;
-  at[1].id = cudaLaunchAttributeClusterDimension;
-  at[1].val.clusterDim.x = CT;
-  at[1].val.clusterDim.y = 1;
-  at[1].val.clusterDim.z = 1;
-  cfg.attrs = at;
-  cfg.numAttrs = F::PAIR ? 2 : 1;
-  ProfScope prof(F::NP == 3 ? "f32_split" : "bf16x3_split", st);
-  note_launch();
-  return cudaLaunchKernelEx(&cfg, kern, a);
+  return launch_tiles<F, false>(a, F::NP == 3 ? "f32_split" : "bf16x3_split", st);
 }
 
 template <int NP>
@@ -687,6 +853,40 @@ cudaError_t launch_split_np(const BatchDesc& d, cudaStream_t st) {
 }
 
 }  // namespace
+
+using GroupedSplit = Split<2, 128, 128>;
+
+bool f32_split_records(const GroupedInst& in, std::vector<SplitRec>& out) {
+  if (in.k == 0 || in.m >= (1L << 31) || in.n >= (1L << 31) || in.k >= (1L << 31) || in.lda >= (1L << 25) || in.ldb >= (1L << 25) ||
+      in.idx >= (1L << 31))
+    return false;
+  SplitRec r{};
+  r.m = (int)in.m; r.n = (int)in.n; r.k = (int)in.k;
+  r.idx = (int)in.idx;
+  r.a_mn = in.transa == SSBLAS_OP_N;
+  r.b_mn = in.transb == SSBLAS_OP_T;
+  r.lda = (int)in.lda; r.ldb = (int)in.ldb; r.ldc = in.ldc;
+  r.alpha = in.alpha_f; r.beta = in.beta_f;
+  r.nkc = (int)((in.k + kKC - 1) / kKC);
+  for (long m0 = 0; m0 < in.m; m0 += GroupedSplit::TM)
+    for (long n0 = 0; n0 < in.n; n0 += GroupedSplit::TN) {
+      r.m0 = (int)m0;
+      r.n0 = (int)n0;
+      out.push_back(r);
+    }
+  return true;
+}
+
+cudaError_t launch_f32_split_grouped(const SplitRec* recs, long tiles, const GroupedPtrs& p, cudaStream_t st) {
+  if (!tcgen05_available()) return cudaErrorNotSupported;
+  SplitArgs a{};
+  a.A = (const float* const*)p.A;
+  a.B = (const float* const*)p.B;
+  a.C = (float* const*)p.C;
+  a.recs = recs;
+  a.total = (uint32_t)tiles;
+  return launch_tiles<GroupedSplit, true>(a, "grouped_bf16x3_gemm", st);
+}
 
 cudaError_t launch_f32_split(const BatchDesc& d, int parts, cudaStream_t st) {
   return parts == 3 ? launch_split_np<3>(d, st) : launch_split_np<2>(d, st);

@@ -2,21 +2,22 @@
 // persistent launch per phase.
 //
 // Phase 1 (pre-pass, one launch per kind): every instance's op(A) and op(B) are converted -- into
-//   Ozaki int8 slices (fp64 rows, SSBLAS_MATH_FP64_OZAKI), BF16 hi/lo parts (fp32 rows,
-//   SSBLAS_MATH_FP32_BF16X3) or plain int8 (int8 row) -- and written as ready-to-use tensor-core
-//   operand tiles: for each (row tile, K block) one contiguous chunk holding all planes, already in
+//   Ozaki int8 slices (fp64 rows, SSBLAS_MATH_FP64_OZAKI) or plain int8 (int8 row) -- and written as
+//   ready-to-use tensor-core operand tiles: for each (row tile, K block) one contiguous chunk holding all planes, already in
 //   the 128B/64B/32B-swizzled K-major layout the MMA reads, zero-padded to whole tiles. Each
 //   instance's chunks start at its own offset (a prefix sum over the instances).
 // Phase 2 (GEMM, one launch per kind): the persistent tcgen05 kernel walks a device-side tile
 //   table (instance, row tile, column tile), longest K first; its producer stages each chunk with a
 //   single plain bulk copy, so no per-instance tensor map is needed.
+// fp32 instances in the 3xBF16 mode take one launch: the kernel of f32_split.cu splits the tiles as it
+// loads them (5000 of 8 to 512 each way: 0.564 ms as a split pass and a GEMM, 0.39 ms so; uniform
+// 128 x 128 x 128: 0.141 ms, the 0.87 GB at 6.2 TB/s).
 // Plain fp32 instances run on the cp.async FFMA tiles (gemm_sgemm.cu), plain fp64 ones on the FP64
 // tensor cores (gemm_dmma.cu), one launch per op(A) / op(B) layout present.
 //
 // The tables of a call (instances, tiles, work items, buffer offsets) depend on its shapes only and
 // are kept as a plan; a call whose shapes, scalars and settings equal a cached plan's launches it on its
 // own pointer arrays.
-#include <cuda_bf16.h>
 #include <cuda_runtime.h>
 #include <stdint.h>
 
@@ -61,7 +62,7 @@ constexpr int GNT = 256;
 
 // One CTA per work item = (operand of an instance, block of 32 rows of it). Only rows and K
 // blocks of the matrix are written; the tile padding around them was zeroed when the plan was made.
-// MODE 0: int8 copy (1 plane); 1: BF16 hi/lo (2 planes); 2: Ozaki slices (S planes).
+// MODE 0: int8 copy (1 plane); 2: Ozaki slices (S planes).
 //
 // The item's rows are converted in K chunks of KC elements. Each thread handles runs of 4
 // consecutive k of one row; with the rows contiguous in memory (element (r, k) at X[r + k*ld]) the
@@ -74,19 +75,17 @@ constexpr int GNT = 256;
 // [RTILE rows][KB bytes], 16-byte chunks permuted by the hardware swizzle of a KB-byte span.
 template <int MODE> struct GElem;
 template <> struct GElem<0> { using T = int8_t; };
-template <> struct GElem<1> { using T = float; };
 template <> struct GElem<2> { using T = double; };
 
 template <int MODE, int S, int KB, int RTILE_A, int RTILE_B>
-__global__ void __launch_bounds__(GNT, MODE == 2 ? 6 : MODE == 0 ? 6 : 8) gprep_kernel(const GPrepInst* __restrict__ items, const uint2* __restrict__ work,
+__global__ void __launch_bounds__(GNT, 6) gprep_kernel(const GPrepInst* __restrict__ items, const uint2* __restrict__ work,
                                                     const void* const* __restrict__ ptrA,
                                                     const void* const* __restrict__ ptrB,
                                                     uint8_t* __restrict__ outA, uint8_t* __restrict__ outB,
                                                     int32_t* __restrict__ exps) {
   using T = typename GElem<MODE>::T;
-  constexpr int P = MODE == 0 ? 1 : MODE == 1 ? 2 : S;
-  constexpr int OB = MODE == 1 ? 2 : 1;                     // output bytes per element and plane
-  constexpr int KE = KB / OB;                               // K elements per block
+  constexpr int P = MODE == 0 ? 1 : S;
+  constexpr int KE = KB;                                    // K elements (a byte each) per block and plane
   constexpr int KC = MODE == 0 ? 128 : 64;                  // K elements per chunk
   constexpr int NKB = KC / KE;                              // K blocks per chunk
   constexpr int RPR = KC / 4;                               // runs of 4 k per row and chunk
@@ -141,9 +140,6 @@ __global__ void __launch_bounds__(GNT, MODE == 2 ? 6 : MODE == 0 ? 6 : 8) gprep_
         if constexpr (sizeof(T) == 8) {
           const double2 a = __ldg((const double2*)p), b = __ldg((const double2*)p + 1);
           x[0] = a.x; x[1] = a.y; x[2] = b.x; x[3] = b.y;
-        } else if constexpr (sizeof(T) == 4) {
-          const float4 a = __ldg((const float4*)p);
-          x[0] = a.x; x[1] = a.y; x[2] = a.z; x[3] = a.w;
         } else {
           const char4 a = __ldg((const char4*)p);
           x[0] = a.x; x[1] = a.y; x[2] = a.z; x[3] = a.w;
@@ -218,16 +214,14 @@ __global__ void __launch_bounds__(GNT, MODE == 2 ? 6 : MODE == 0 ? 6 : 8) gprep_
 #pragma unroll
     for (int q = 0; q < PER; ++q) {
       const int r = rq[q], kl = kq[q];
-      const int kb = kl / KE, cbyte = (kl % KE) * OB;
+      const int kb = kl / KE, cbyte = kl % KE;
       uint8_t* row = stage + (kb * P) * GRT * PB + r * PB + cbyte;
       // rows past the matrix are never written out; a run past K is zero in every plane (the
-      // digits, BF16 parts and int8 copy of 0 are all zero bytes)
+      // digits and the int8 copy of 0 are all zero bytes)
       if (!rv[q]) continue;
       if (k0 + kl >= K) {
 #pragma unroll
-        for (int p = 0; p < P; ++p)
-#pragma unroll
-          for (int w = 0; w < OB; ++w) *(uint32_t*)(row + p * GRT * PB + 4 * w) = 0u;
+        for (int p = 0; p < P; ++p) *(uint32_t*)(row + p * GRT * PB) = 0u;
         continue;
       }
       T x[4];
@@ -237,16 +231,6 @@ __global__ void __launch_bounds__(GNT, MODE == 2 ? 6 : MODE == 0 ? 6 : 8) gprep_
 #pragma unroll
         for (int i = 0; i < 4; ++i) w |= ((uint32_t)(uint8_t)x[i]) << (8 * i);
         *(uint32_t*)row = w;
-      } else if constexpr (MODE == 1) {
-        // paired conversions, each value rounded to nearest even as a single conversion would be
-        const __nv_bfloat162 h01 = __floats2bfloat162_rn(x[0], x[1]), h23 = __floats2bfloat162_rn(x[2], x[3]);
-        const float2 f01 = __bfloat1622float2(h01), f23 = __bfloat1622float2(h23);
-        const __nv_bfloat162 l01 = __floats2bfloat162_rn(x[0] - f01.x, x[1] - f01.y);
-        const __nv_bfloat162 l23 = __floats2bfloat162_rn(x[2] - f23.x, x[3] - f23.y);
-        *(__nv_bfloat162*)row = h01;
-        *(__nv_bfloat162*)(row + 4) = h23;
-        *(__nv_bfloat162*)(row + GRT * PB) = l01;
-        *(__nv_bfloat162*)(row + GRT * PB + 4) = l23;
       } else {
         // rows holding an Inf or a NaN (zero scale) have zero digits
         double xd[4] = {x[0], x[1], x[2], x[3]};
@@ -423,7 +407,6 @@ cudaError_t launch_kind(const KindDev& kd, const GroupedPtrs& ptrs, cudaStream_t
 // default: most tiles of an uneven batch are short in K, and their epilogues dominate)
 using GCfgOz = tc::Config<tc::KIND_I8, 7, 7, 64, 32, 5, 7, 1, tc::EPI_OZAKI, 2>;
 using GCfgOz32 = tc::Config<tc::KIND_I8, 7, 7, 32, 32, 6, 7, 2, tc::EPI_OZAKI, 2>;
-using GCfgBf = tc::Config<tc::KIND_BF16, 2, 2, 64, 128, 4, 1, 2, tc::EPI_F32, 1>;
 using GCfgI8 = tc::Config<tc::KIND_I8, 1, 1, 128, 128, 6, 1, 2, tc::EPI_I32, 0>;
 
 }  // namespace
@@ -438,7 +421,9 @@ struct GroupedPlan {
   bool has_f64 = false;
   // Ozaki instances by tile shape: oz on 128 x 32 tiles with two accumulators, oz_wide on
   // 128 x 64 tiles with one (chosen per instance size bucket)
-  KindDev oz, oz_wide, bf, i8;
+  KindDev oz, oz_wide, i8;
+  DevBuf bf;                 // SplitRec per tile of the 3xBF16 instances, longest K first
+  long bf_tiles = 0;
   std::unique_ptr<GroupedSimt> simt;
   size_t scratch = 0;        // bytes of packed operand buffers
   cudaEvent_t used = nullptr;
@@ -534,7 +519,8 @@ cudaError_t grouped_make(const GroupedDesc& g, const GroupedArgs& a, cudaStream_
     return true;
   });
   pl->dynamic = gcfg != 2;
-  std::vector<int> oz, oz_wide, bf, i8, plain;
+  std::vector<int> oz, oz_wide, i8, plain;
+  std::vector<SplitRec> bf;
   for (int i = 0; i < (int)g.inst.size(); ++i) {
     const GroupedInst& in = g.inst[i];
     pl->has_f64 |= in.row == ROW_F64;
@@ -542,7 +528,7 @@ cudaError_t grouped_make(const GroupedDesc& g, const GroupedArgs& a, cudaStream_
     if (in.row == ROW_I8) i8.push_back(i);
     else if (in.row == ROW_F64 && (mode & SSBLAS_MATH_FP64_OZAKI) && in.k <= 16384)
       (ozaki_wide_tiles(in, gcfg) ? oz_wide : oz).push_back(i);
-    else if (in.row == ROW_F32 && (mode & SSBLAS_MATH_FP32_BF16X3)) bf.push_back(i);
+    else if (in.row == ROW_F32 && (mode & SSBLAS_MATH_FP32_BF16X3) && f32_split_records(in, bf)) continue;
     else plain.push_back(i);
   }
   // make room first: the evicted plans' buffers may be what the new one needs (cudaFree waits for
@@ -560,11 +546,9 @@ cudaError_t grouped_make(const GroupedDesc& g, const GroupedArgs& a, cudaStream_
     plan_kind(g, oz, k1);
     KindPlan<GCfgOz> k0;
     plan_kind(g, oz_wide, k0);
-    KindPlan<GCfgBf> k2;
-    plan_kind(g, bf, k2);
     KindPlan<GCfgI8> k3;
     plan_kind(g, i8, k3);
-    pl->scratch = (size_t)(k0.bytesA + k0.bytesB + k1.bytesA + k1.bytesB + k2.bytesA + k2.bytesB + k3.bytesA + k3.bytesB);
+    pl->scratch = (size_t)(k0.bytesA + k0.bytesB + k1.bytesA + k1.bytesB + k3.bytesA + k3.bytesB);
     auto total = [&] {
       size_t s = pl->scratch;
       for (auto& p : plans) s += p->scratch;
@@ -573,8 +557,15 @@ cudaError_t grouped_make(const GroupedDesc& g, const GroupedArgs& a, cudaStream_
     while (!plans.empty() && total() > kMaxScratch) evict_oldest();
     if ((e = upload_kind(k1, pl->oz, st))) return e;
     if ((e = upload_kind(k0, pl->oz_wide, st))) return e;
-    if ((e = upload_kind(k2, pl->bf, st))) return e;
     if ((e = upload_kind(k3, pl->i8, st))) return e;
+  }
+  if (!bf.empty()) {
+    std::stable_sort(bf.begin(), bf.end(), [](const SplitRec& x, const SplitRec& y) { return x.nkc > y.nkc; });
+    pl->bf_tiles = (long)bf.size();
+    if ((e = pl->bf.alloc(sizeof(SplitRec) * bf.size())) ||
+        (e = cudaMemcpyAsync(pl->bf.p, bf.data(), sizeof(SplitRec) * bf.size(), cudaMemcpyHostToDevice, st)) ||
+        (e = cudaStreamSynchronize(st)))   // the host table is a temporary
+      return e;
   }
   if (!plain.empty()) {
     pl->simt = std::make_unique<GroupedSimt>();
@@ -599,7 +590,7 @@ cudaError_t grouped_launch(GroupedPlan& pl, const GroupedPtrs& p, cudaStream_t s
     return e;
   if ((e = launch_kind<GCfgOz32, 2, 7>(pl.oz, p, st, "grouped_ozaki_slice", "grouped_ozaki_gemm", pl.dynamic)))
     return e;
-  if ((e = launch_kind<GCfgBf, 1, 1>(pl.bf, p, st, "grouped_split_bf16", "grouped_bf16x3_gemm", pl.dynamic))) return e;
+  if (pl.bf_tiles && (e = launch_f32_split_grouped((const SplitRec*)pl.bf.p, pl.bf_tiles, p, st))) return e;
   if ((e = launch_kind<GCfgI8, 0, 1>(pl.i8, p, st, "grouped_pack_i8", "grouped_i8_gemm", pl.dynamic))) return e;
   if (pl.simt && (e = launch_simt_grouped(*pl.simt, p, st))) return e;
   if (pl.simt && (e = launch_dmma_grouped(*pl.simt, p, st))) return e;

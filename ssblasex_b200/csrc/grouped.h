@@ -69,6 +69,19 @@ cudaError_t launch_simt_grouped(const GroupedSimt& s, const GroupedPtrs& p, cuda
 cudaError_t launch_dmma_grouped(const GroupedSimt& s, const GroupedPtrs& p, cudaStream_t st);
 cudaError_t launch_sgemm_grouped(const GroupedSimt& s, const GroupedPtrs& p, cudaStream_t st);
 
+// One 128 x 128 tile of an fp32 instance in the 3xBF16 mode (f32_split.cu).
+struct SplitRec {
+  int m, n, k, m0, n0, idx;  // the instance's shape, the tile's first row and column, place in the arrays
+  int a_mn, b_mn;            // op(A) rows / op(B) columns contiguous in memory
+  int lda, ldb;
+  long ldc;
+  float alpha, beta;
+  int nkc, pad;              // K chunks
+};
+// appends the instance's tiles; false (none appended) where its sizes are beyond the records
+bool f32_split_records(const GroupedInst& in, std::vector<SplitRec>& out);
+cudaError_t launch_f32_split_grouped(const SplitRec* recs, long tiles, const GroupedPtrs& p, cudaStream_t st);
+
 // A grouped call's device tables depend on its shapes, scalars and the settings only, so a plan serves
 // every call that repeats those values, whatever matrices it points to. grouped_find: the cached plan
 // of the current device for these arguments (compared value by value), nullptr if there is none.
