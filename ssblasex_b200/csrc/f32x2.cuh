@@ -33,13 +33,13 @@ static __device__ __forceinline__ uint64_t add2(uint64_t a, uint64_t b) {
 }
 
 // acc (TM x TN, pairs of rows) += a (TM values, k-th line of op(A) at pa) x b (TN values at pb); pa and pb
-// are 16-byte aligned, TM and TN multiples of 4.
-template <int TM, int TN>
+// are 16-byte aligned, TM and TN multiples of 4; the rows are groups of 4, STEP apart.
+template <int TM, int TN, int STEP = 4>
 static __device__ __forceinline__ void outer2(uint64_t (&acc)[TM / 2][TN], const float* pa, const float* pb) {
   uint64_t a[TM / 2];
 #pragma unroll
   for (int i = 0; i < TM / 4; ++i) {
-    const ulonglong2 x = *(const ulonglong2*)(pa + 4 * i);
+    const ulonglong2 x = *(const ulonglong2*)(pa + STEP * i);
     a[2 * i] = x.x;
     a[2 * i + 1] = x.y;
   }

@@ -17,8 +17,7 @@
 // Each thread owns a TM x TN block of C (rows tx*TM.., columns ty*TN..); a warp covers 4 x 8
 // threads, so its A reads are 4 distinct 16-byte vectors and its B reads 8 (broadcasts). The products are
 // packed fused multiply-adds over pairs of rows (f32x2.cuh), the same results in half the issue slots
-// (4096 x 64^3 TT, configuration 9: 0.0785 -> 0.0735 ms, where the loads from shared memory, 75% of their
-// pipe's wavefronts, are what is left; NN, configuration 3: 0.078 -> 0.076).
+// (4096 x 64^3 TT, configuration 9: 0.0785 -> 0.0735 ms; NN, configuration 3: 0.078 -> 0.076).
 #include <cuda_runtime.h>
 #include <stdint.h>
 
@@ -219,132 +218,19 @@ sgemm_grouped_kernel(const SimtGInst* __restrict__ inst, const int* __restrict__
                                                          (long)t[2] * kGT, sm);
 }
 
-// Persistent form for K <= KS * BK (the whole K of a work item fits the KS stages of one buffer):
-// work item w = (instance w / tiles, tile w % tiles), CTA c takes items c, c + G, c + 2G, ... and
-// double-buffers them -- the next item's operands are in flight while the current one is computed
-// and written -- so a batch of thousands of small instances keeps HBM busy instead of paying one
-// load latency per CTA. C of the item (when beta != 0) is read into registers before the
-// products, so that read overlaps them too.
-template <int BM, int BN, int BK, int TM, int TN, int KS, int MINB, bool A_MN, bool B_MN>
-__global__ void __launch_bounds__((BM / TM) * (BN / TN), MINB) sgemm_small_kernel(SgemmArgs args, uint32_t tiles_m,
-                                                                                   uint32_t tiles, uint32_t total) {
-  constexpr int TX = BM / TM, TY = BN / TN, NT = TX * TY;
-  constexpr int PA = BM + 4, PB = BN + 4;
-  constexpr int STAGE = BK * (PA + PB);
-  constexpr int BUF = KS * STAGE;
-  extern __shared__ __align__(16) float sm[];
-  const int lane = threadIdx.x % 32, warp = threadIdx.x / 32;
-  constexpr int WX = TX / 4;   // warps along m (a warp = 4 (m) x 8 (n) threads)
-  const int tx = (warp % WX) * 4 + lane % 4;
-  const int ty = (warp / WX) * 8 + lane / 4;
-  const long ktiles = (args.k + BK - 1) / BK;   // <= KS (checked by the launcher)
-  const bool read_c = args.beta != 0.0f;
-
-  // work item w -> (instance b, tile t) -> (m0, n0), in 32-bit arithmetic (the launcher keeps the
-  // item count below 2^31): a 64-bit division costs dozens of instructions per item
-  auto item = [&](uint32_t w, long& b, long& m0, long& n0) {
-    const uint32_t bb = w / tiles, t = w - bb * tiles;
-    const uint32_t tn = t / tiles_m;
-    b = bb;
-    m0 = (long)(t - tn * tiles_m) * BM;
-    n0 = (long)tn * BN;
-  };
-  auto issue = [&](uint32_t w, int buf) {
-    long b, m0, n0;
-    item(w, b, m0, n0);
-    const float* __restrict__ A = args.A[b];
-    const float* __restrict__ B = args.B[b];
-    const bool vecA = ((uintptr_t)A % 16 == 0) && (args.lda % 4 == 0);
-    const bool vecB = ((uintptr_t)B % 16 == 0) && (args.ldb % 4 == 0);
-#pragma unroll
-    for (int kt = 0; kt < KS; ++kt) {
-      if (kt >= ktiles) break;
-      float* sa = sm + buf * BUF + kt * STAGE;
-      sload<BM, BK, NT, A_MN>(sa, A, args.m, args.k, args.lda, m0, kt * BK, vecA);
-      sload<BN, BK, NT, B_MN>(sa + BK * PA, B, args.n, args.k, args.ldb, n0, kt * BK, vecB);
-    }
-  };
-
-  uint32_t w = blockIdx.x;
-  if (w < total) issue(w, 0);
-  commit_s();
-  for (int buf = 0; w < total; w += gridDim.x, buf ^= 1) {
-    // the next item's operands go into the other buffer (free since the previous iteration's
-    // closing barrier)
-    if (w + gridDim.x < total) issue(w + gridDim.x, buf ^ 1);
-    commit_s();
-    long b, m0, n0;
-    item(w, b, m0, n0);
-    float* __restrict__ C = args.C[b];
-    const long gi0 = m0 + tx * TM;
-    const bool cvec = (((uintptr_t)C) % 16 == 0) && (args.ldc % 4 == 0) && gi0 + TM <= args.m;
-    float cv[TN][TM];
-#pragma unroll
-    for (int j = 0; j < TN; ++j) {
-      const long gj = n0 + ty * TN + j;
-      const float* cp = C + gi0 + gj * args.ldc;
-#pragma unroll
-      for (int i = 0; i < TM; i += 4) {
-        if (read_c && gj < args.n && cvec) {
-          const float4 x = *(const float4*)(cp + i);
-          cv[j][i] = x.x; cv[j][i + 1] = x.y; cv[j][i + 2] = x.z; cv[j][i + 3] = x.w;
-        } else {
-#pragma unroll
-          for (int q = 0; q < 4; ++q) cv[j][i + q] = (read_c && gj < args.n && gi0 + i + q < args.m) ? cp[i + q] : 0.0f;
-        }
-      }
-    }
-    wait_s<1>();   // this item's group has landed (the next item's may still be in flight)
-    __syncthreads();
-    uint64_t acc2[TM / 2][TN];
-#pragma unroll
-    for (int i = 0; i < TM / 2; ++i)
-#pragma unroll
-      for (int j = 0; j < TN; ++j) acc2[i][j] = 0;
-    for (int kt = 0; kt < ktiles; ++kt) {
-      const float* sa = sm + buf * BUF + kt * STAGE;
-      const float* sb = sa + BK * PA;
-#pragma unroll 4
-      for (int kk = 0; kk < BK; ++kk) outer2<TM, TN>(acc2, sa + kk * PA + tx * TM, sb + kk * PB + ty * TN);
-    }
-    float acc[TM][TN];
-    unpack_acc<TM, TN>(acc2, acc);
-#pragma unroll
-    for (int j = 0; j < TN; ++j) {
-      const long gj = n0 + ty * TN + j;
-      if (gj >= args.n) continue;
-      float* cp = C + gi0 + gj * args.ldc;
-      if (cvec) {
-#pragma unroll
-        for (int i = 0; i < TM; i += 4) {
-          float4 o;
-          o.x = fmaf(acc[i][j], args.alpha, read_c ? args.beta * cv[j][i] : 0.0f);
-          o.y = fmaf(acc[i + 1][j], args.alpha, read_c ? args.beta * cv[j][i + 1] : 0.0f);
-          o.z = fmaf(acc[i + 2][j], args.alpha, read_c ? args.beta * cv[j][i + 2] : 0.0f);
-          o.w = fmaf(acc[i + 3][j], args.alpha, read_c ? args.beta * cv[j][i + 3] : 0.0f);
-          *(float4*)(cp + i) = o;
-        }
-      } else {
-#pragma unroll
-        for (int i = 0; i < TM; ++i)
-          if (gi0 + i < args.m) cp[i] = fmaf(acc[i][j], args.alpha, read_c ? args.beta * cv[j][i] : 0.0f);
-      }
-    }
-    __syncthreads();   // this buffer is refilled by the next iteration's copies
-  }
-  wait_s<0>();
-}
-
 // Register-heavy form for K <= KMAX: one 64 x 64 tile of one instance per CTA of 64 threads, each
-// thread an 8 x 8 block of C (rows 8 tx.., columns 8 ty.., tx = t % 8, ty = t / 8). The whole K of
-// the tile is requested at once (16-deep slices of the cp.async copies above, both operands
-// staged [k][rows]), C (beta != 0) is read into registers while the copies land, and the inner
-// loop issues 4 shared-memory vector loads per 64 FFMAs -- a quarter of the per-product overhead
-// of the 4 x 4 threads. Several CTAs per SM overlap one tile's loads with another's products.
-// (Staging a K-contiguous operand as it lies, [rows][k] with 16-byte copies, measured slower on
-// 4096 x 64^3 TT: 0.105 ms against 0.084 ms -- its rows 8 apart per thread turn the C stores
-// into 4-byte ones.)
-template <int KMAX, int MINB, bool A_MN, bool B_MN>
+// thread an 8 x 8 block of C (tx = t % 8, ty = t / 8: rows 4 tx.. and 32 + 4 tx.., columns 8 ty..). The
+// whole K of the tile is requested at once (16-deep slices of the cp.async copies above, both operands
+// staged [k][rows]), C (READ_C) is read into registers while the copies land, and the inner
+// loop issues 4 shared-memory vector loads per 64 FFMAs. Several CTAs per SM overlap one tile's loads with
+// another's products: six without the 64 registers of C, else four.
+// The rows as two groups of four, 32 apart: eight lanes then read 128 contiguous bytes, where rows
+// 8 tx.. took two passes of the shared memory each, and they read and write whole lines of C. What bounds
+// it is those loads (64 bytes per thread and k, 16 passes per warp against 16 of the products' pipe).
+// Measured, 4096 x 64^3: TT with C read 0.0735 -> 0.069 ms (0.041 of HBM time), NN 0.079 -> 0.070.
+// (Staging a K-contiguous operand as it lies, [rows][k] with 16-byte copies: 0.105 ms against 0.084 then;
+// C through L2 prefetches instead of registers, six CTAs: 0.084 against 0.069.)
+template <int KMAX, int MINB, bool READ_C, bool A_MN, bool B_MN>
 __global__ void __launch_bounds__(64, MINB) sgemm_reg8_kernel(SgemmArgs args, uint32_t tiles_m, uint32_t tiles) {
   constexpr int P = 64 + 4;
   extern __shared__ __align__(16) float sm[];
@@ -369,22 +255,26 @@ __global__ void __launch_bounds__(64, MINB) sgemm_reg8_kernel(SgemmArgs args, ui
   commit_s();
 
   const int tx = threadIdx.x % 8, ty = threadIdx.x / 8;
-  const long gi0 = m0 + tx * 8;
-  const bool read_c = args.beta != 0.0f;
-  const bool cvec = (((uintptr_t)C) % 16 == 0) && (args.ldc % 4 == 0) && gi0 + 8 <= args.m;
+  const long gi0 = m0 + 4 * tx;   // and gi0 + 32
+  const bool vecC = (((uintptr_t)C) % 16 == 0) && (args.ldc % 4 == 0);
+  const bool cvec[2] = {vecC && gi0 + 4 <= args.m, vecC && gi0 + 36 <= args.m};
   // C of this thread's block, in flight while the operand copies land
-  float cv[8][8];
+  float cv[READ_C ? 8 : 1][8];
+  if constexpr (READ_C) {
 #pragma unroll
-  for (int j = 0; j < 8; ++j) {
-    const long gj = n0 + ty * 8 + j;
-    const float* cp = C + gi0 + gj * args.ldc;
-    if (read_c && gj < args.n && cvec) {
-      const float4 x0 = *(const float4*)cp, x1 = *(const float4*)(cp + 4);
-      cv[j][0] = x0.x; cv[j][1] = x0.y; cv[j][2] = x0.z; cv[j][3] = x0.w;
-      cv[j][4] = x1.x; cv[j][5] = x1.y; cv[j][6] = x1.z; cv[j][7] = x1.w;
-    } else {
+    for (int j = 0; j < 8; ++j) {
+      const long gj = n0 + ty * 8 + j;
+      const float* cp = C + gi0 + gj * args.ldc;
 #pragma unroll
-      for (int i = 0; i < 8; ++i) cv[j][i] = (read_c && gj < args.n && gi0 + i < args.m) ? cp[i] : 0.0f;
+      for (int h = 0; h < 2; ++h) {
+        if (gj < args.n && cvec[h]) {
+          const float4 x = *(const float4*)(cp + 32 * h);
+          cv[j][4 * h] = x.x; cv[j][4 * h + 1] = x.y; cv[j][4 * h + 2] = x.z; cv[j][4 * h + 3] = x.w;
+        } else {
+#pragma unroll
+          for (int i = 0; i < 4; ++i) cv[j][4 * h + i] = (gj < args.n && gi0 + 32 * h + i < args.m) ? cp[32 * h + i] : 0.0f;
+        }
+      }
     }
   }
   wait_s<0>();
@@ -396,7 +286,7 @@ __global__ void __launch_bounds__(64, MINB) sgemm_reg8_kernel(SgemmArgs args, ui
 #pragma unroll
     for (int j = 0; j < 8; ++j) acc2[i][j] = 0;
 #pragma unroll 4
-  for (int kk = 0; kk < K; ++kk) outer2<8, 8>(acc2, sa + kk * P + tx * 8, sb + kk * P + ty * 8);
+  for (int kk = 0; kk < K; ++kk) outer2<8, 8, 32>(acc2, sa + kk * P + 4 * tx, sb + kk * P + ty * 8);
   float acc[8][8];
   unpack_acc<8, 8>(acc2, acc);
 
@@ -405,24 +295,27 @@ __global__ void __launch_bounds__(64, MINB) sgemm_reg8_kernel(SgemmArgs args, ui
     const long gj = n0 + ty * 8 + j;
     if (gj >= args.n) continue;
     float* cp = C + gi0 + gj * args.ldc;
-    float o[8];
 #pragma unroll
-    for (int i = 0; i < 8; ++i) o[i] = fmaf(acc[i][j], args.alpha, read_c ? args.beta * cv[j][i] : 0.0f);
-    if (cvec) {
-      *(float4*)cp = make_float4(o[0], o[1], o[2], o[3]);
-      *(float4*)(cp + 4) = make_float4(o[4], o[5], o[6], o[7]);
-    } else {
+    for (int h = 0; h < 2; ++h) {
+      float o[4];
 #pragma unroll
-      for (int i = 0; i < 8; ++i)
-        if (gi0 + i < args.m) cp[i] = o[i];
+      for (int i = 0; i < 4; ++i)
+        o[i] = fmaf(acc[4 * h + i][j], args.alpha, READ_C ? args.beta * cv[READ_C ? j : 0][4 * h + i] : 0.0f);
+      if (cvec[h]) {
+        *(float4*)(cp + 32 * h) = make_float4(o[0], o[1], o[2], o[3]);
+      } else {
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+          if (gi0 + 32 * h + i < args.m) cp[32 * h + i] = o[i];
+      }
     }
   }
 }
 
-template <int KMAX, int MINB, bool A_MN, bool B_MN>
+template <int KMAX, int MINB, bool READ_C, bool A_MN, bool B_MN>
 cudaError_t launch_reg8(const SgemmArgs& a, cudaStream_t st) {
   constexpr int SMEM = 2 * KMAX * (64 + 4) * 4;
-  auto kern = sgemm_reg8_kernel<KMAX, MINB, A_MN, B_MN>;
+  auto kern = sgemm_reg8_kernel<KMAX, MINB, READ_C, A_MN, B_MN>;
   static bool attr[kMaxDevices] = {};
   if (cudaError_t e = smem_attr_once(attr, kern, SMEM)) return e;
   const long tiles_m = (a.m + 63) / 64;
@@ -433,12 +326,12 @@ cudaError_t launch_reg8(const SgemmArgs& a, cudaStream_t st) {
   return cudaGetLastError();
 }
 
-template <int KMAX, int MINB>
+template <int KMAX, int MINB, bool READ_C>
 cudaError_t launch_reg8_l(const SgemmArgs& a, bool a_mn, bool b_mn, cudaStream_t st) {
-  if (a_mn && b_mn) return launch_reg8<KMAX, MINB, true, true>(a, st);
-  if (a_mn) return launch_reg8<KMAX, MINB, true, false>(a, st);
-  if (b_mn) return launch_reg8<KMAX, MINB, false, true>(a, st);
-  return launch_reg8<KMAX, MINB, false, false>(a, st);
+  if (a_mn && b_mn) return launch_reg8<KMAX, MINB, READ_C, true, true>(a, st);
+  if (a_mn) return launch_reg8<KMAX, MINB, READ_C, true, false>(a, st);
+  if (b_mn) return launch_reg8<KMAX, MINB, READ_C, false, true>(a, st);
+  return launch_reg8<KMAX, MINB, READ_C, false, false>(a, st);
 }
 
 // K split inside the CTA, for k <= KMAX: one 64 x 64 tile per CTA of 256 threads, four groups of
@@ -496,16 +389,16 @@ __global__ void __launch_bounds__(256, MINB) sgemm_ksplit_kernel(SgemmArgs args,
 #pragma unroll
     for (int j = 0; j < 8; ++j) acc2[i][j] = 0;
 #pragma unroll 2
-  for (int kk = k0; kk < k1; ++kk) outer2<8, 8>(acc2, sa + kk * P + tx * 8, sb + kk * P + ty * 8);
+  for (int kk = k0; kk < k1; ++kk) outer2<8, 8, 32>(acc2, sa + kk * P + 4 * tx, sb + kk * P + ty * 8);
   float acc[8][8];
   unpack_acc<8, 8>(acc2, acc);
   __syncthreads();   // every group is done with the operand buffers
   float* part = red + g * 64 * P;
 #pragma unroll
   for (int j = 0; j < 8; ++j) {
-    float* q = part + (ty * 8 + j) * P + tx * 8;
+    float* q = part + (ty * 8 + j) * P + 4 * tx;
     *(float4*)q = make_float4(acc[0][j], acc[1][j], acc[2][j], acc[3][j]);
-    *(float4*)(q + 4) = make_float4(acc[4][j], acc[5][j], acc[6][j], acc[7][j]);
+    *(float4*)(q + 32) = make_float4(acc[4][j], acc[5][j], acc[6][j], acc[7][j]);
   }
   __syncthreads();
 
@@ -557,31 +450,6 @@ cudaError_t launch_ksplit_l(const SgemmArgs& a, bool a_mn, bool b_mn, cudaStream
   if (a_mn) return launch_ksplit<KMAX, MINB, true, false>(a, st);
   if (b_mn) return launch_ksplit<KMAX, MINB, false, true>(a, st);
   return launch_ksplit<KMAX, MINB, false, false>(a, st);
-}
-
-template <int BM, int BN, int BK, int TM, int TN, int KS, int MINB, bool A_MN, bool B_MN>
-cudaError_t launch_small(const SgemmArgs& a, cudaStream_t st) {
-  constexpr int NT = (BM / TM) * (BN / TN);
-  constexpr int SMEM = 2 * KS * BK * (BM + 4 + BN + 4) * 4;
-  auto kern = sgemm_small_kernel<BM, BN, BK, TM, TN, KS, MINB, A_MN, B_MN>;
-  static int per_sm_dev[kMaxDevices] = {};
-  const int dev = current_device();
-  if (dev < 0) return cudaErrorInvalidDevice;
-  int& per_sm = per_sm_dev[dev];
-  if (!per_sm) {
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM);
-    if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, NT, SMEM);
-    if (e != cudaSuccess) return e;
-    if (per_sm < 1) per_sm = 1;
-  }
-  const long tiles_m = (a.m + BM - 1) / BM;
-  const long tiles = tiles_m * ((a.n + BN - 1) / BN);
-  const long total = tiles * a.batch;
-  if (total >= (1L << 31)) return cudaErrorNotSupported;   // the caller takes the tiled kernel
-  const long cap = (long)per_sm * num_sms();
-  kern<<<(unsigned)(total < cap ? total : cap), NT, SMEM, st>>>(a, (uint32_t)tiles_m, (uint32_t)tiles,
-                                                                 (uint32_t)total);
-  return cudaGetLastError();
 }
 
 template <int BM, int BN, int BK, int TM, int TN, int STAGES, int MINB, bool A_MN, bool B_MN>
@@ -659,33 +527,20 @@ cudaError_t launch_sgemm_async(const BatchDesc& d, int config, cudaStream_t st) 
   ProfScope prof("sgemm_async", st);
   // 3: 64 x 64 tiles, 256 threads of 4 x 4, 32-deep K stages x 2 (k <= 64 entirely in flight)
   // 4: 128 x 128 tiles, 256 threads of 8 x 8, 16-deep K stages x 3
-  // 5 (k <= 64): 64 x 64 tiles, persistent CTAs that double-buffer their work items, 256 threads
-  //   of 4 x 4
-  // 6 (k <= 64): as 5 with 128 threads of 8 x 4 (twice the products per thread for the same
-  //   per-item index, copy and epilogue work)
   // 7: 32 x 64 tiles, 128 threads of 4 x 4, 32-deep K stages x 4 (k <= 128 entirely in flight):
   //   four times the CTAs of configuration 3, for batches whose 64 x 64 tiles fill under a wave
   // 8: 32 x 32 tiles, 64 threads of 4 x 4, 16-deep K stages x 8
-  // 9 (k <= 64) / 10 (k <= 128): 64 x 64 tiles, 64 threads of 8 x 8, the whole K at once
+  // 9 (k <= 64) / 10 (k <= 128): 64 x 64 tiles, 64 threads of 8 x 8, the whole K at once (5 and 6,
+  //   forced or in a tuning file: 9)
   // 11 (k <= 128): 64 x 64 tiles, 256 threads: four 8 x 8 groups over quarters of K, summed in
   //   shared memory
   e = cudaErrorNotSupported;
-  if (config == 9 && d.k <= 64) {
-    e = launch_reg8_l<64, 4>(a, a_mn, b_mn, st);
+  if ((config == 9 || config == 5 || config == 6) && d.k <= 64) {
+    e = a.beta != 0.0f ? launch_reg8_l<64, 4, true>(a, a_mn, b_mn, st) : launch_reg8_l<64, 6, false>(a, a_mn, b_mn, st);
   } else if (config == 10 && d.k <= 128) {
-    e = launch_reg8_l<128, 3>(a, a_mn, b_mn, st);
+    e = a.beta != 0.0f ? launch_reg8_l<128, 3, true>(a, a_mn, b_mn, st) : launch_reg8_l<128, 3, false>(a, a_mn, b_mn, st);
   } else if (config == 11 && d.k <= 128) {
     e = launch_ksplit_l<128, 2>(a, a_mn, b_mn, st);
-  } else if (config == 5 && d.k <= 64) {
-    if (a_mn && b_mn) e = launch_small<64, 64, 32, 4, 4, 2, 3, true, true>(a, st);
-    else if (a_mn) e = launch_small<64, 64, 32, 4, 4, 2, 3, true, false>(a, st);
-    else if (b_mn) e = launch_small<64, 64, 32, 4, 4, 2, 3, false, true>(a, st);
-    else e = launch_small<64, 64, 32, 4, 4, 2, 3, false, false>(a, st);
-  } else if (config == 6 && d.k <= 64) {
-    if (a_mn && b_mn) e = launch_small<64, 64, 32, 8, 4, 2, 3, true, true>(a, st);
-    else if (a_mn) e = launch_small<64, 64, 32, 8, 4, 2, 3, true, false>(a, st);
-    else if (b_mn) e = launch_small<64, 64, 32, 8, 4, 2, 3, false, true>(a, st);
-    else e = launch_small<64, 64, 32, 8, 4, 2, 3, false, false>(a, st);
   } else if (config == 4) {
     e = launch_sl<128, 128, 16, 8, 8, 3, 1>(a, a_mn, b_mn, st);
   } else if (config == 7) {
@@ -693,7 +548,7 @@ cudaError_t launch_sgemm_async(const BatchDesc& d, int config, cudaStream_t st) 
   } else if (config == 8) {
     e = launch_sl<32, 32, 16, 4, 4, 8, 8>(a, a_mn, b_mn, st);
   }
-  // configuration 3 serves the rest (and item counts of 2^31 or more for 5 and 6)
+  // configuration 3 serves the rest (and tile counts of 2^31 or more for 9 to 11)
   if (e == cudaErrorNotSupported) e = launch_sl<64, 64, 32, 4, 4, 2, 3>(a, a_mn, b_mn, st);
   note_launch();
   return e;

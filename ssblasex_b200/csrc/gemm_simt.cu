@@ -265,7 +265,15 @@ int simt_config(const BatchDesc& d) {
   // them, small tiles otherwise (the tuning table or a forced configuration can override).
   const long big_tiles = ((d.m + 127) / 128) * ((d.n + 127) / 128) * d.batch;
   const bool big_default = d.m >= 128 && d.n >= 128 && big_tiles >= 2L * num_sms();
-  const int cores = d.row == ROW_F32 ? (big_default ? 4 : d.k <= 64 ? 5 : 3) : (big_default ? 1 : 0);
+  // fp32, k <= 64: the 8 x 8 threads on 64 x 64 tiles (9), or 32 x 32 tiles (8) where those cover at most
+  // half the area. Measured (ms; 9, 8, before = the persistent 4 x 4 threads or 128 x 128 tiles):
+  // 500 x (128 x 128 x 32) TT, beta: 0.025, 0.057, 0.049; 16 x (1024 x 1024 x 48) 0.047, 0.074, 0.062;
+  // 4 x (2000 x 2000 x 64) 0.063, 0.095, 0.073; 500 x (130 x 140 x 33), odd strides 0.069, 0.100, 0.213;
+  // 4000 x (20 x 30 x 40) 0.053, 0.026, 0.088; 2000 x (48 x 16 x 64) 0.038, 0.032, 0.041. Every one sums in k
+  // order in one chain: the results are the same.
+  auto area = [&](long t) { return ((d.m + t - 1) / t * t) * ((d.n + t - 1) / t * t); };
+  const int short_k = area(64) >= 2 * area(32) ? 8 : 9;
+  const int cores = d.row == ROW_F32 ? (d.k <= 64 ? short_k : big_default ? 4 : 3) : (big_default ? 1 : 0);
   // Plain fp32 takes the BF16 tensor cores from k = 128 on. Below, its error against 64 bits can be
   // larger than that of the FFMA kernels (a truncated sum of 16 products against chains of so few
   // rounded ones: entries with outliers, k = 64: 7.0e-8 against 6.4e-8; k = 128: 7.4e-8 against
@@ -278,7 +286,7 @@ int simt_config(const BatchDesc& d) {
 
 cudaError_t launch_simt_gemm(const BatchDesc& d, cudaStream_t stream) {
   const int cfg = simt_config(d);
-  // fp32: configurations 3, 4 and 5 are the cp.async-pipelined kernels (gemm_sgemm.cu)
+  // fp32: configurations 3 to 13 are the cp.async-pipelined kernels (gemm_sgemm.cu)
   if (d.row == ROW_F32 && cfg >= 3) return launch_sgemm_async(d, cfg, stream);
   const bool big = cfg == 1;
   switch (d.row) {
