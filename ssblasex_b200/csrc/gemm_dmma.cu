@@ -21,6 +21,7 @@
 
 #include "grouped.h"
 #include "internal.h"
+#include "ptx.cuh"
 
 namespace ssb {
 namespace {
@@ -268,11 +269,13 @@ __global__ void __launch_bounds__(kDmmaThreads, kMinBlocks)
 dmma_grouped_kernel(const SimtGInst* __restrict__ inst, const int* __restrict__ tiles, const double* const* A,
                     const double* const* B, double* const* C) {
   extern __shared__ __align__(16) double smem[];
+  ptx::grid_dep_launch();
   const int* t = tiles + 3 * (long)blockIdx.x;
   const SimtGInst g = inst[t[0]];
   dmma_tile<kBM, kBN, kBK, kW, kW, kStages, A_MN, B_MN>(A[g.idx], B[g.idx], C[g.idx], g.m, g.n, g.k, g.lda, g.ldb,
                                                        g.ldc, g.alpha_d, g.beta_d, (long)t[1] * kBM,
                                                        (long)t[2] * kBN, smem);
+  ptx::grid_chain_end();
 }
 
 template <bool A_MN, bool B_MN>
@@ -288,32 +291,31 @@ cudaError_t launch_cfg(const DmmaArgs& a, cudaStream_t st) {
 }
 
 template <bool A_MN, bool B_MN>
-cudaError_t launch_grouped_layout(const GroupedSimt& s, const GroupedPtrs& p, int lay, cudaStream_t st) {
+cudaError_t launch_grouped_layout(const GroupedSimt& s, const GroupedPtrs& p, int lay, cudaStream_t st, bool& follows) {
   auto kern = dmma_grouped_kernel<A_MN, B_MN>;
   static bool attr[kMaxDevices] = {};
   if (cudaError_t e = smem_attr_once(attr, kern, kDmmaSmem)) return e;
-  kern<<<(unsigned)s.ndmma[lay], kDmmaThreads, kDmmaSmem, st>>>(
-      (const SimtGInst*)s.inst64, (const int*)s.dmma_tiles[lay], (const double* const*)p.A,
-      (const double* const*)p.B, (double* const*)p.C);
   note_launch();
-  return cudaGetLastError();
+  return launch_chained(kern, (unsigned)s.ndmma[lay], kDmmaThreads, kDmmaSmem, st, follows, (const SimtGInst*)s.inst64,
+                        (const int*)s.dmma_tiles[lay], (const double* const*)p.A, (const double* const*)p.B,
+                        (double* const*)p.C);
 }
 
 }  // namespace
 
 // The plain fp64 tiles of a grouped call, one launch per op(A) / op(B) layout present
 // (layout index = 2 * (op(A) rows contiguous) + (op(B) columns contiguous)).
-cudaError_t launch_dmma_grouped(const GroupedSimt& s, const GroupedPtrs& p, cudaStream_t st) {
+cudaError_t launch_dmma_grouped(const GroupedSimt& s, const GroupedPtrs& p, cudaStream_t st, bool& follows) {
   if (!s.ndmma[0] && !s.ndmma[1] && !s.ndmma[2] && !s.ndmma[3]) return cudaSuccess;
   ProfScope prof("dmma_grouped", st);
   cudaError_t e = cudaSuccess;
   for (int lay = 0; lay < 4 && e == cudaSuccess; ++lay) {
     if (!s.ndmma[lay]) continue;
     switch (lay) {
-      case 3: e = launch_grouped_layout<true, true>(s, p, lay, st); break;
-      case 2: e = launch_grouped_layout<true, false>(s, p, lay, st); break;
-      case 1: e = launch_grouped_layout<false, true>(s, p, lay, st); break;
-      default: e = launch_grouped_layout<false, false>(s, p, lay, st); break;
+      case 3: e = launch_grouped_layout<true, true>(s, p, lay, st, follows); break;
+      case 2: e = launch_grouped_layout<true, false>(s, p, lay, st, follows); break;
+      case 1: e = launch_grouped_layout<false, true>(s, p, lay, st, follows); break;
+      default: e = launch_grouped_layout<false, false>(s, p, lay, st, follows); break;
     }
   }
   return e;

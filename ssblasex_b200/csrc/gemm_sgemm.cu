@@ -24,6 +24,7 @@
 #include "f32x2.cuh"
 #include "grouped.h"
 #include "internal.h"
+#include "ptx.cuh"
 
 namespace ssb {
 namespace {
@@ -211,11 +212,13 @@ __global__ void __launch_bounds__((kGT / kGTM) * (kGT / kGTM), 3)
 sgemm_grouped_kernel(const SimtGInst* __restrict__ inst, const int* __restrict__ tiles, const float* const* A,
                      const float* const* B, float* const* C) {
   extern __shared__ __align__(16) float sm[];
+  ptx::grid_dep_launch();
   const int* t = tiles + 3 * (long)blockIdx.x;
   const SimtGInst g = inst[t[0]];
   sgemm_tile<kGT, kGT, kGBK, kGTM, kGTM, kGST, A_MN, B_MN>(A[g.idx], B[g.idx], C[g.idx], g.m, g.n, g.k, g.lda, g.ldb,
                                                          g.ldc, g.alpha_f, g.beta_f, (long)t[1] * kGT,
                                                          (long)t[2] * kGT, sm);
+  ptx::grid_chain_end();
 }
 
 // Register-heavy form for K <= KMAX: one 64 x 64 tile of one instance per CTA of 64 threads, each
@@ -477,31 +480,30 @@ cudaError_t launch_sl(const SgemmArgs& a, bool a_mn, bool b_mn, cudaStream_t st)
 }  // namespace
 
 template <bool A_MN, bool B_MN>
-cudaError_t launch_sgemm_grouped_layout(const GroupedSimt& s, const GroupedPtrs& p, int lay, cudaStream_t st) {
+cudaError_t launch_sgemm_grouped_layout(const GroupedSimt& s, const GroupedPtrs& p, int lay, cudaStream_t st, bool& follows) {
   constexpr int SMEM = kGST * kGBK * (2 * kGT + 8) * 4;
   auto kern = sgemm_grouped_kernel<A_MN, B_MN>;
   static bool attr[kMaxDevices] = {};
   if (cudaError_t e = smem_attr_once(attr, kern, SMEM)) return e;
-  kern<<<(unsigned)s.nsg[lay], (kGT / kGTM) * (kGT / kGTM), SMEM, st>>>(
-      (const SimtGInst*)s.inst32, (const int*)s.sg_tiles[lay], (const float* const*)p.A, (const float* const*)p.B,
-      (float* const*)p.C);
   note_launch();
-  return cudaGetLastError();
+  return launch_chained(kern, (unsigned)s.nsg[lay], (kGT / kGTM) * (kGT / kGTM), SMEM, st, follows,
+                        (const SimtGInst*)s.inst32, (const int*)s.sg_tiles[lay], (const float* const*)p.A,
+                        (const float* const*)p.B, (float* const*)p.C);
 }
 
 // The plain fp32 tiles of a grouped call, one launch per op(A) / op(B) layout present (layout
 // index = 2 * (op(A) rows contiguous) + (op(B) columns contiguous)).
-cudaError_t launch_sgemm_grouped(const GroupedSimt& s, const GroupedPtrs& p, cudaStream_t st) {
+cudaError_t launch_sgemm_grouped(const GroupedSimt& s, const GroupedPtrs& p, cudaStream_t st, bool& follows) {
   if (!s.nsg[0] && !s.nsg[1] && !s.nsg[2] && !s.nsg[3]) return cudaSuccess;
   ProfScope prof("sgemm_grouped", st);
   cudaError_t e = cudaSuccess;
   for (int lay = 0; lay < 4 && e == cudaSuccess; ++lay) {
     if (!s.nsg[lay]) continue;
     switch (lay) {
-      case 3: e = launch_sgemm_grouped_layout<true, true>(s, p, lay, st); break;
-      case 2: e = launch_sgemm_grouped_layout<true, false>(s, p, lay, st); break;
-      case 1: e = launch_sgemm_grouped_layout<false, true>(s, p, lay, st); break;
-      default: e = launch_sgemm_grouped_layout<false, false>(s, p, lay, st); break;
+      case 3: e = launch_sgemm_grouped_layout<true, true>(s, p, lay, st, follows); break;
+      case 2: e = launch_sgemm_grouped_layout<true, false>(s, p, lay, st, follows); break;
+      case 1: e = launch_sgemm_grouped_layout<false, true>(s, p, lay, st, follows); break;
+      default: e = launch_sgemm_grouped_layout<false, false>(s, p, lay, st, follows); break;
     }
   }
   return e;

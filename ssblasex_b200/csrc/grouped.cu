@@ -593,8 +593,9 @@ cudaError_t grouped_launch(GroupedPlan& pl, const GroupedPtrs& p, cudaStream_t s
   if (pl.bf_tiles && (e = launch_f32_split_grouped((const SplitRec*)pl.bf.p, pl.bf_tiles, p, st))) return e;
   if ((e = launch_kind<GCfgI8, 0, 1>(pl.i8, p, st, "grouped_pack_i8", "grouped_i8_gemm", pl.dynamic))) return e;
   if (pl.simt && (e = launch_simt_grouped(*pl.simt, p, st))) return e;
-  if (pl.simt && (e = launch_dmma_grouped(*pl.simt, p, st))) return e;
-  if (pl.simt && (e = launch_sgemm_grouped(*pl.simt, p, st))) return e;
+  bool follows = false;
+  if (pl.simt && (e = launch_dmma_grouped(*pl.simt, p, st, follows))) return e;
+  if (pl.simt && (e = launch_sgemm_grouped(*pl.simt, p, st, follows))) return e;
   if (captured) return cudaSuccess;
   if ((e = cudaEventRecord(pl.used, st)) != cudaSuccess) return e;
   pl.in_use = true;

@@ -66,8 +66,27 @@ struct GroupedPtrs {
   void* const* C;
 };
 cudaError_t launch_simt_grouped(const GroupedSimt& s, const GroupedPtrs& p, cudaStream_t st);
-cudaError_t launch_dmma_grouped(const GroupedSimt& s, const GroupedPtrs& p, cudaStream_t st);
-cudaError_t launch_sgemm_grouped(const GroupedSimt& s, const GroupedPtrs& p, cudaStream_t st);
+// One launch per layout. The layouts' launches have nothing to do with each other, and run into each other:
+// `follows` says that the launch before on the stream is one of this call's chain (grid_chain_end in ptx.cuh), and is set for the next.
+cudaError_t launch_dmma_grouped(const GroupedSimt& s, const GroupedPtrs& p, cudaStream_t st, bool& follows);
+cudaError_t launch_sgemm_grouped(const GroupedSimt& s, const GroupedPtrs& p, cudaStream_t st, bool& follows);
+#ifdef __CUDACC__
+template <class K, class... Args>
+cudaError_t launch_chained(K kern, unsigned grid, unsigned block, int smem, cudaStream_t st, bool& follows, Args... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(grid, 1, 1);
+  cfg.blockDim = dim3(block, 1, 1);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = follows ? 1 : 0;   // the first of a chain waits for all before it
+  follows = true;
+  return cudaLaunchKernelEx(&cfg, kern, args...);
+}
+#endif
 
 // One 128 x 128 tile of an fp32 instance in the 3xBF16 mode (f32_split.cu).
 struct SplitRec {

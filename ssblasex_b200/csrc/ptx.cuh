@@ -129,6 +129,12 @@ __device__ __forceinline__ void prefetch_tmap(const CUtensorMap* map) {
 // frees; it changes nothing for a next kernel launched the ordinary way.
 __device__ __forceinline__ void grid_dep_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void grid_dep_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+// A chain of grids without dependences among them (their first grid_dep_launch() is at their start, so that
+// the next grid's CTAs fill the SMs that this one's last leave): one CTA of each waits for the grid before
+// when its work is done, so a grid has completed only after all before it.
+__device__ __forceinline__ void grid_chain_end() {
+  if (blockIdx.x == gridDim.x - 1) grid_dep_wait();
+}
 
 // ------------------------------------------------------------------------------ tcgen05 -----
 __device__ __forceinline__ void tmem_alloc(uint32_t dst_smem, uint32_t ncols) {
