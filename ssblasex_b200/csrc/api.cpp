@@ -974,10 +974,10 @@ static ssblasStatus_t gemm_batched(ssblasOperation_t transa, ssblasOperation_t t
 
 static void log_call(const char* entry, ssblasStatus_t st, long m, long n, long k, long batch) {
   static const char* const names[] = {"none", "simt", "i8_tcgen05", "ozaki_tcgen05", "bf16x3_tcgen05", "grouped",
-                                      "dmma", "", "", "", "", "f16_tcgen05"};
+                                      "dmma", "", "", "", "", "f16_tcgen05", "", "f32_tcgen05"};
   const int p = g_info.path;
   fprintf(stderr, "ssblas: %s m=%ld n=%ld k=%ld batch=%ld status=%d path=%s slices=%d launches=%d split_k=%d%s\n",
-          entry, m, n, k, batch, (int)st, (p >= 0 && p < 12 && names[p][0]) ? names[p] : "?", g_info.slices,
+          entry, m, n, k, batch, (int)st, (p >= 0 && p < 14 && names[p][0]) ? names[p] : "?", g_info.slices,
           g_info.kernel_launches, g_info.split_k, g_info.device_error ? " device_error" : "");
 }
 

@@ -21,6 +21,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <type_traits>
+
 #include <algorithm>
 #include <cstring>
 #include <map>
@@ -73,6 +75,10 @@ constexpr int GNT = 256;
 // (conflict-free word stores) and leave as 16-byte vectors into the pre-swizzled tile layout the
 // grouped GEMM stages with bulk copies: for each (row tile, K block) of the instance, P planes of
 // [RTILE rows][KB bytes], 16-byte chunks permuted by the hardware swizzle of a KB-byte span.
+// What bounds the Ozaki form is its instructions (64% of the issue slots, 87 per value with the idle lanes
+// of ragged blocks; 1.16 GB read and 1.0 GB written in 0.60 ms): 32-bit K indices and the write-out's
+// places worked out once per item took 0.625 -> 0.604 ms on 5000 instances of 8 to 512 each way. Six CTAs per
+// SM: four 0.696 ms, five 0.632, seven and eight 0.61.
 template <int MODE> struct GElem;
 template <> struct GElem<0> { using T = int8_t; };
 template <> struct GElem<2> { using T = double; };
@@ -108,7 +114,10 @@ __global__ void __launch_bounds__(GNT, 6) gprep_kernel(const GPrepInst* __restri
   const T* X = (const T*)(it.from_b ? ptrB : ptrA)[it.idx];
   const long gr0 = (long)wk.y * GRT;                        // first row (of the padded range)
   const int rt = (int)(gr0 / RTILE), rr0 = (int)(gr0 % RTILE);
-  const long K = it.K, ld = it.ld;
+  // (the Ozaki instances of a plan have K <= 16384)
+  using KT = typename std::conditional<MODE == 2, int, long>::type;
+  const KT K = (KT)it.K;
+  const long ld = it.ld;
   const bool kc = it.kcontig != 0;
   const int t = threadIdx.x, lane = t % 32, warp = t / 32;
 
@@ -129,12 +138,12 @@ __global__ void __launch_bounds__(GNT, 6) gprep_kernel(const GPrepInst* __restri
   }
   // 4 consecutive k of a row in one vector load when the row starts are aligned for it
   const bool vec = kc && ((uintptr_t)X % (sizeof(T) == 1 ? 4 : 16)) == 0 && ld % (sizeof(T) == 8 ? 2 : 4) == 0;
-  auto load4 = [&](int q, long k0, T (&x)[4]) {
+  auto load4 = [&](int q, KT k0, T (&x)[4]) {
 #pragma unroll
     for (int i = 0; i < 4; ++i) x[i] = T(0);
     if (!rv[q]) return;
     const T* p = pq[q] + k0 * estep;
-    const long kk = k0 + kq[q];
+    const KT kk = k0 + kq[q];
     if (kk + 4 <= K) {
       if (vec) {
         if constexpr (sizeof(T) == 8) {
@@ -163,7 +172,7 @@ __global__ void __launch_bounds__(GNT, 6) gprep_kernel(const GPrepInst* __restri
       uint32_t mh[PER], ml[PER];
 #pragma unroll
       for (int q = 0; q < PER; ++q) mh[q] = ml[q] = 0;
-      for (long k0 = 0; k0 < K; k0 += KC) {
+      for (KT k0 = 0; k0 < K; k0 += KC) {
 #pragma unroll
         for (int q = 0; q < PER; ++q) {
           T x[4];
@@ -207,10 +216,21 @@ __global__ void __launch_bounds__(GNT, 6) gprep_kernel(const GPrepInst* __restri
   const bool wrow = gr0 + wr < it.rows;
   const uint32_t soff = (uint32_t)(wr * PB + 16 * wc);
   const uint32_t doff = swz(rr0 + wr, 16 * wc, KB);
-  const long tile_bytes = (long)P * RTILE * KB;             // one (row tile, K block) chunk, all planes
+  const int tile_bytes = P * RTILE * KB;                    // one (row tile, K block) chunk, all planes
+  // the (K block, plane) blocks that this thread writes: bp0, bp0 + BPP, ...
+  constexpr int NW = (NBP + BPP - 1) / BPP;
+  const int bp0 = t / CHT;
+  uint32_t woff[NW];                                        // their places past the chunk's first K block
+#pragma unroll
+  for (int i = 0; i < NW; ++i) {
+    const int kb = (bp0 + i * BPP) / P, pl = bp0 + i * BPP - kb * P;
+    woff[i] = (uint32_t)(kb * tile_bytes + pl * RTILE * KB) + doff;
+  }
+  uint8_t* outk = out + (long)rt * it.nk * tile_bytes;
+  const uint8_t* src0 = stage + bp0 * GRT * PB + soff;
 
   // K blocks at or past K are padding, zero since the plan was created: chunks start below K
-  for (long k0 = 0; k0 < K; k0 += KC) {
+  for (KT k0 = 0; k0 < K; k0 += KC, outk += (long)NKB * tile_bytes) {
 #pragma unroll
     for (int q = 0; q < PER; ++q) {
       const int r = rq[q], kl = kq[q];
@@ -245,13 +265,12 @@ __global__ void __launch_bounds__(GNT, 6) gprep_kernel(const GPrepInst* __restri
     // write-out: per (K block, plane), 32 rows x KB bytes of the tile, 16-byte chunks swizzled
     if (wrow) {
 #pragma unroll
-      for (int bp = t / CHT; bp < NBP; bp += BPP) {
-        const int kb = bp / P, pl = bp - kb * P;
-        const long kbg = k0 / KE + kb;
-        if (kbg * KE >= K) continue;
-        const uint32_t* src = (const uint32_t*)(stage + bp * GRT * PB + soff);
-        const uint4 w = make_uint4(src[0], src[1], src[2], src[3]);
-        *(uint4*)(out + ((long)rt * it.nk + kbg) * tile_bytes + (long)pl * RTILE * KB + doff) = w;
+      for (int i = 0; i < NW; ++i) {
+        const int bp = bp0 + i * BPP;
+        if (NBP % BPP != 0 && i == NW - 1 && bp >= NBP) break;
+        if (k0 + bp / P * KE >= K) break;                   // padding: and so are the blocks after it
+        const uint32_t* src = (const uint32_t*)(src0 + i * BPP * GRT * PB);
+        *(uint4*)(outk + woff[i]) = make_uint4(src[0], src[1], src[2], src[3]);
       }
     }
     __syncthreads();

@@ -1,5 +1,5 @@
 // Host launchers of the tcgen05 paths: int8 -> int32 (direct TMA from the caller's matrices, or
-// through the int8 pack pre-pass), FP64 via Ozaki int8 slices, FP32 via three BF16 products.
+// from copies on the 16-byte grid), FP64 via Ozaki int8 slices, FP32 via three BF16 products.
 #include <cuda.h>
 #include <cuda_runtime.h>
 #include <stdint.h>
