@@ -3,9 +3,9 @@
 //
 // Phase 1 (pre-pass, one launch per kind): every instance's op(A) and op(B) are converted -- into
 //   Ozaki int8 slices (fp64 rows, SSBLAS_MATH_FP64_OZAKI) or plain int8 (int8 row) -- and written as
-//   ready-to-use tensor-core operand tiles: for each (row tile, K block) one contiguous chunk holding all planes, already in
-//   the 128B/64B/32B-swizzled K-major layout the MMA reads, zero-padded to whole tiles. Each
-//   instance's chunks start at its own offset (a prefix sum over the instances).
+//   ready-to-use tensor-core operand tiles: for each (row tile, K block) one contiguous chunk holding
+//   all planes, already in the 128B/64B/32B-swizzled K-major layout the MMA reads, zero-padded to whole
+//   tiles. Each instance's chunks start at its own offset (a prefix sum over the instances).
 // Phase 2 (GEMM, one launch per kind): the persistent tcgen05 kernel walks a device-side tile
 //   table (instance, row tile, column tile), longest K first; its producer stages each chunk with a
 //   single plain bulk copy, so no per-instance tensor map is needed.
