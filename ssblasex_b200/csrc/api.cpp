@@ -577,7 +577,8 @@ static cudaError_t dispatch(const BatchDesc& d, cudaStream_t st) {
   } else if (d.row == ROW_F64 && (mode & SSBLAS_MATH_FP64_OZAKI)) {
     cudaError_t e = launch_ozaki_f64(d, ozaki_slices_for_call(), st);
     if (e != cudaErrorNotSupported) return e;
-  } else if (d.row == ROW_F64 && choose_config(SSBLAS_PATH_DMMA, d.m, d.n, d.k, d.batch, 0) != 2) {
+  } else if (d.row == ROW_F64 && d.k < kDmmaMaxK &&
+             choose_config(SSBLAS_PATH_DMMA, d.m, d.n, d.k, d.batch, 0) != 2) {
     // plain fp64: DMMA tiles (configuration 2 selects the DFMA SIMT kernel instead)
     note_path(SSBLAS_PATH_DMMA);
     return launch_dmma_f64(d, st);

@@ -19,6 +19,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "dmma_slab.h"
 #include "grouped.h"
 #include "internal.h"
 #include "ptx.cuh"
@@ -38,12 +39,14 @@ __device__ __forceinline__ uint32_t smem_addr(const void* p) {
   return (uint32_t)__cvta_generic_to_shared(p);
 }
 // cp.async of `bytes` valid bytes (0, 8 or 16) into a 16- or 8-byte slot; the rest is zero-filled
-__device__ __forceinline__ void cp16(uint32_t dst, const void* src, int bytes) {
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(dst), "l"(src), "r"(bytes) : "memory");
-}
-__device__ __forceinline__ void cp8(uint32_t dst, const void* src, int bytes) {
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;\n" ::"r"(dst), "l"(src), "r"(bytes) : "memory");
-}
+struct CpAsync {
+  __device__ __forceinline__ void cp16(uint32_t dst, const void* src, int bytes) const {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(dst), "l"(src), "r"(bytes) : "memory");
+  }
+  __device__ __forceinline__ void cp8(uint32_t dst, const void* src, int bytes) const {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;\n" ::"r"(dst), "l"(src), "r"(bytes) : "memory");
+  }
+};
 __device__ __forceinline__ void cp_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
 template <int N>
 __device__ __forceinline__ void cp_wait() { asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory"); }
@@ -65,86 +68,6 @@ struct DmmaSmem {
   static constexpr int STAGE = A_MAX + B_MAX;
 };
 
-// One operand's copies by this thread: chunk q (two doubles along the contiguous dimension) of the next
-// K slab comes from src + q * step and goes to dst + q * DSTEP of the slab's buffer, so that a slab
-// inside the matrix costs one copy and one addition per chunk (with the position of every chunk
-// worked out again the copies took as many issue slots as the products' loads).
-//   MN: rows contiguous in global memory (element (r, k) at X[r + k*ld]) -> staged [k][r];
-//   otherwise element (r, k) at X[r*ld + k] -> staged [r][k].
-template <int ROWS, int BK, int NT, bool MN>
-struct Slab {
-  static constexpr int P = MN ? ROWS + 4 : BK + 4;
-  static constexpr int CPL = (MN ? ROWS : BK) / 2;        // chunks per contiguous line
-  static constexpr int NQ = ROWS * BK / 2 / NT;           // chunks per thread
-  static constexpr int LSTEP = NT / CPL;                  // lines between a thread's chunks
-  static constexpr int DSTEP = LSTEP * P;                 // doubles between their places
-  static_assert(NT % CPL == 0 && NQ * NT == ROWS * BK / 2 && NQ * LSTEP == (MN ? BK : ROWS), "slab/threads mismatch");
-  const double* src;
-  const double* X;
-  long step, adv;            // doubles between chunks, between slabs
-  int k, kk;                 // valid k from the next slab on; k of this thread's first chunk in a slab
-  int lines, bytes;          // chunks of this thread inside the rows, and valid bytes of each (MN)
-  uint32_t dst;              // byte offset of its place
-  bool vec;
-  __device__ __forceinline__ void init(const double* __restrict__ X_, long nrows, long K, long ld, long r0) {
-    const int t = threadIdx.x;
-    X = X_;
-    vec = ((uintptr_t)X % 16 == 0) && (ld % 2 == 0);
-    const int rr = MN ? 2 * (t % CPL) : t / CPL;
-    kk = MN ? t / CPL : 2 * (t % CPL);
-    src = X + (MN ? r0 + rr + kk * ld : (r0 + rr) * ld + kk);
-    step = LSTEP * ld;
-    adv = MN ? BK * ld : BK;
-    const long left = nrows - r0 - rr;    // valid rows from this thread's first chunk on
-    lines = MN ? NQ : left >= ROWS ? NQ : left > 0 ? min(NQ, (int)((left + LSTEP - 1) / LSTEP)) : 0;
-    bytes = MN ? (left >= 2 ? 16 : left == 1 ? 8 : 0) : 16;
-    if (bytes == 0) lines = 0;
-    k = (int)K;
-    dst = 8u * (uint32_t)(MN ? kk * P + rr : rr * P + kk);
-  }
-  // The next slab into `buf` (shared-space address); moves on to the one after it. A slab with all of
-  // its k inside the matrix asks for fixed lines and bytes per thread; only the last one, where k runs
-  // out, looks at each chunk.
-  __device__ __forceinline__ void copy(uint32_t buf) {
-    const uint32_t d = buf + dst;
-    const double* s = src;
-    if (k >= BK) {
-      if (vec && lines == NQ && bytes == 16) {
-#pragma unroll
-        for (int q = 0; q < NQ; ++q, s += step) cp16(d + 8u * (uint32_t)(q * DSTEP), s, 16);
-      } else if (vec) {
-#pragma unroll
-        for (int q = 0; q < NQ; ++q, s += step)
-          cp16(d + 8u * (uint32_t)(q * DSTEP), q < lines ? s : X, q < lines ? bytes : 0);
-      } else {
-        const int b0 = bytes < 8 ? bytes : 8, b1 = bytes - b0;
-#pragma unroll
-        for (int q = 0; q < NQ; ++q, s += step) {
-          const bool ok = q < lines;
-          cp8(d + 8u * (uint32_t)(q * DSTEP), ok ? s : X, ok ? b0 : 0);
-          cp8(d + 8u * (uint32_t)(q * DSTEP + 1), ok && b1 ? s + 1 : X, ok ? b1 : 0);
-        }
-      }
-    } else {
-#pragma unroll
-      for (int q = 0; q < NQ; ++q, s += step) {
-        // valid elements of the chunk, which runs along r (MN) or along k
-        int nv = MN ? (kk + q * LSTEP < k ? bytes / 8 : 0) : (q < lines ? k - kk : 0);
-        nv = nv < 0 ? 0 : (nv > 2 ? 2 : nv);
-        const double* g = nv > 0 ? s : X;
-        if (vec) {
-          cp16(d + 8u * (uint32_t)(q * DSTEP), g, 8 * nv);
-        } else {
-          cp8(d + 8u * (uint32_t)(q * DSTEP), g, nv > 0 ? 8 : 0);
-          cp8(d + 8u * (uint32_t)(q * DSTEP + 1), nv > 1 ? g + 1 : X, nv > 1 ? 8 : 0);
-        }
-      }
-    }
-    src += adv;
-    k -= BK;
-  }
-};
-
 // One BM x BN tile of C = alpha op(A) op(B) + beta C for one instance, by the whole CTA: the K loop
 // over the stage ring, then the epilogue. Leaves the stage buffers free (every copy has landed and
 // every thread has passed a barrier after its last read).
@@ -156,13 +79,14 @@ __device__ __forceinline__ void dmma_tile(const double* __restrict__ A, const do
   constexpr int NT = NWM * NWN * 32;
   constexpr int MI = WM / 8, NI = WN / 8;
   using Sm = DmmaSmem<BM, BN, BK>;
+  static_assert(Slab<BM, BK, NT, A_MN>::KMAX >= kDmmaMaxK && Slab<BN, BK, NT, B_MN>::KMAX >= kDmmaMaxK, "counts of slabs");
   const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
   const int wm = warp % NWM, wn = warp / NWM;
   const int fr = lane >> 2, fk = lane & 3;    // fragment row (m or n) and k within an 8x4 block
   Slab<BM, BK, NT, A_MN> ca;
   Slab<BN, BK, NT, B_MN> cb;
-  ca.init(A, m, k, lda, m0);
-  cb.init(B, n, k, ldb, n0);
+  ca.init(A, m, k, lda, m0, threadIdx.x);
+  cb.init(B, n, k, ldb, n0, threadIdx.x);
 
   double acc[MI][NI][2];
 #pragma unroll
@@ -170,12 +94,12 @@ __device__ __forceinline__ void dmma_tile(const double* __restrict__ A, const do
 #pragma unroll
     for (int j = 0; j < NI; ++j) acc[i][j][0] = acc[i][j][1] = 0.0;
 
-  const int ktiles = (int)((k + BK - 1) / BK);
+  const int ktiles = ca.slabs();
   const uint32_t smem0 = smem_addr(smem);
   auto issue = [&](int kt) {     // slabs in order, kt counts them
     const uint32_t sa = smem0 + 8u * (uint32_t)((kt % STAGES) * Sm::STAGE);
-    ca.copy(sa);
-    cb.copy(sa + 8u * Sm::A_MAX);
+    ca.copy(sa, CpAsync{});
+    cb.copy(sa + 8u * Sm::A_MAX, CpAsync{});
   };
 #pragma unroll
   for (int s = 0; s < STAGES - 1; ++s) {

@@ -348,7 +348,7 @@ cudaError_t plan_simt_grouped(const GroupedDesc& g, const std::vector<int>& memb
     iv.push_back(s);
     // plain fp64 on the FP64 tensor cores, as the batched call does, unless its DMMA configuration
     // for this shape is 2 (the DFMA kernel)
-    const bool dmma = x.row == ROW_F64 && choose_config(SSBLAS_PATH_DMMA, x.m, x.n, x.k, 1, 0) != 2;
+    const bool dmma = x.row == ROW_F64 && x.k < kDmmaMaxK && choose_config(SSBLAS_PATH_DMMA, x.m, x.n, x.k, 1, 0) != 2;
     // plain fp32 on the cp.async FFMA tiles unless the SIMT configuration for this shape is 0 or 1
     // (the register-tiled SIMT kernel)
     const bool sg = x.row == ROW_F32 && choose_config(SSBLAS_PATH_SIMT, x.m, x.n, x.k, 1, 3) >= 3;

@@ -110,7 +110,8 @@ cudaError_t launch_sgemm_async(const BatchDesc& d, int config, cudaStream_t stre
 // equally spaced with 16-byte-aligned bases, strides and leading dimensions
 bool sgemm_tma_fits(const BatchDesc& d);
 cudaError_t launch_sgemm_tma(const BatchDesc& d, int variant, cudaStream_t stream);
-// plain fp64 on the FP64 tensor cores (DMMA)
+// plain fp64 on the FP64 tensor cores (DMMA): k below kDmmaMaxK, whose slabs of 16 k it counts in 32 bits
+constexpr long kDmmaMaxK = 16 * 0x7ffffff0L;
 cudaError_t launch_dmma_f64(const BatchDesc& d, cudaStream_t stream);
 // int8 -> int32 on tcgen05; returns cudaErrorNotSupported when the layout is not eligible.
 cudaError_t launch_i8_tcgen05(const BatchDesc& d, cudaStream_t stream);
