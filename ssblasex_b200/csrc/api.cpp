@@ -155,6 +155,12 @@ int num_sms() {
   return sms[dev];
 }
 
+bool is_captured(cudaStream_t st) {
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(st, &cap) != cudaSuccess) cudaGetLastError();
+  return cap != cudaStreamCaptureStatusNone;
+}
+
 // ---------------------------------------------------------------- workspace ------------------
 struct DeviceWs {
   void* ptr[WS_NUM] = {};
@@ -211,12 +217,14 @@ static void release_workspace() {
 
 __device__ int g_device_error = 0;
 int* device_error_flag() {
-  int* p = nullptr;
-  if (cudaGetSymbolAddress((void**)&p, g_device_error) != cudaSuccess) {
+  static int* flag[kMaxDevices] = {};
+  const int dev = current_device();
+  if (dev < 0) return nullptr;
+  if (!flag[dev] && cudaGetSymbolAddress((void**)&flag[dev], g_device_error) != cudaSuccess) {
     cudaGetLastError();
-    return nullptr;
+    flag[dev] = nullptr;
   }
-  return p;
+  return flag[dev];
 }
 
 // ---------------------------------------------------------------- debug dump -----------------
@@ -357,21 +365,19 @@ static void pinned_done(cudaStream_t st) {
 // the arrays it had before: no host->device copy on the stream and no wait for a pinned slot, so
 // the calls of a loop queue up behind one another. Since the key is the values, memory freed and
 // allocated again at the same addresses is harmless. An entry is rewritten only after the last
-// call that read it has finished (its `used` event), and a call on another stream than the
-// entry's last user first waits for that use, so `used` always covers every earlier use.
+// call that read it has finished, and each call waits for the one before (StreamOrder), so the last
+// use covers every earlier one.
 struct PtrArrays {
   std::vector<const void*> key;   // A[0..batch), B[0..batch), C[0..batch)
   void** dev = nullptr;
   size_t cap = 0;                 // pointers the device buffer holds
-  cudaEvent_t used = nullptr;
-  cudaStream_t last_stream = nullptr;
-  bool in_use = false;
+  StreamOrder order;
   unsigned long tick = 0;
 };
 constexpr int kPtrEntries = 4;
 static PtrArrays g_ptr_arrays[kMaxDevices][kPtrEntries];
 static unsigned long g_ptr_tick = 0;
-static PtrArrays* g_ptr_current = nullptr;   // entry of the call in progress
+static PtrArrays* g_ptr_current = nullptr;   // entry of the call in progress (none: nothing to order)
 
 static bool same_key(const PtrArrays& e, const std::vector<void*>& a, const std::vector<void*>& b,
                      const std::vector<void*>& c) {
@@ -397,18 +403,14 @@ static cudaError_t device_pointer_arrays(const std::vector<void*>& a, const std:
     if (!victim || e.tick < victim->tick) victim = &e;
   }
   cudaError_t err;
+  const bool captured = is_captured(st);
   if (hit) {
-    if (hit->in_use && hit->last_stream != st && (err = cudaStreamWaitEvent(st, hit->used, 0)) != cudaSuccess)
-      return err;
+    if (!captured && (err = hit->order.begin(st)) != cudaSuccess) return err;
   } else {
     hit = victim;
-    if (hit->in_use) {
-      if ((err = cudaEventSynchronize(hit->used)) != cudaSuccess) return err;
-      hit->in_use = false;
-    }
+    if ((err = hit->order.idle()) != cudaSuccess) return err;
     hit->key.clear();   // no valid contents until the upload below is queued
-    if (!hit->used && (err = cudaEventCreateWithFlags(&hit->used, cudaEventDisableTiming)) != cudaSuccess)
-      return err;
+    if (!captured && (err = hit->order.begin(st)) != cudaSuccess) return err;
     if (hit->cap < 3 * n) {
       if (hit->dev) cudaFree(hit->dev);
       hit->dev = nullptr;
@@ -432,7 +434,7 @@ static cudaError_t device_pointer_arrays(const std::vector<void*>& a, const std:
     hit->key.assign((const void* const*)hp, (const void* const*)hp + 3 * n);
   }
   hit->tick = ++g_ptr_tick;
-  g_ptr_current = hit;
+  g_ptr_current = captured ? nullptr : hit;
   *out = hit->dev;
   return cudaSuccess;
 }
@@ -441,22 +443,14 @@ static cudaError_t device_pointer_arrays(const std::vector<void*>& a, const std:
 static void pointer_arrays_used(cudaStream_t st) {
   PtrArrays* e = g_ptr_current;
   g_ptr_current = nullptr;
-  if (!e) return;
-  if (cudaEventRecord(e->used, st) == cudaSuccess) {
-    e->in_use = true;
-    e->last_stream = st;
-  } else {
-    cudaGetLastError();
-    e->key.clear();   // cannot tell when its readers finish: never reused, rewritten after a sync
-    cudaStreamSynchronize(st);
-  }
+  if (e) e->order.end(st);
 }
 
 static void release_pointer_arrays(int dev) {
   if (!valid_device(dev)) return;
   for (PtrArrays& e : g_ptr_arrays[dev]) {
     if (e.dev) cudaFree(e.dev);
-    if (e.used) cudaEventDestroy(e.used);
+    e.order.destroy();
     e = PtrArrays{};
   }
 }

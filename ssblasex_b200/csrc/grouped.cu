@@ -431,8 +431,7 @@ using GCfgI8 = tc::Config<tc::KIND_I8, 1, 1, 128, 128, 6, 1, 2, tc::EPI_I32, 0>;
 }  // namespace
 
 // A prepared grouped call: device tables and packed buffers per kind, and the plain-instance batch.
-// The packed buffers are scratch of the calls that run it, so those are ordered: an event follows each
-// use, and a call on another stream waits for it.
+// The packed buffers are scratch of the calls that run it, so each call waits for the one before.
 struct GroupedPlan {
   std::vector<char> shapes;            // the argument arrays, back to back
   std::vector<uint64_t> scalars, settings;
@@ -445,13 +444,9 @@ struct GroupedPlan {
   long bf_tiles = 0;
   std::unique_ptr<GroupedSimt> simt;
   size_t scratch = 0;        // bytes of packed operand buffers
-  cudaEvent_t used = nullptr;
-  cudaStream_t last_stream = nullptr;
-  bool in_use = false;
+  StreamOrder order;
   unsigned long tick = 0;
-  ~GroupedPlan() {
-    if (used) cudaEventDestroy(used);
-  }
+  ~GroupedPlan() { order.destroy(); }
 };
 
 namespace {
@@ -590,7 +585,6 @@ cudaError_t grouped_make(const GroupedDesc& g, const GroupedArgs& a, cudaStream_
     pl->simt = std::make_unique<GroupedSimt>();
     if ((e = plan_simt_grouped(g, plain, *pl->simt, st))) return e;
   }
-  if ((e = cudaEventCreateWithFlags(&pl->used, cudaEventDisableTiming)) != cudaSuccess) return e;
   plans.push_back(std::move(pl));
   *out = plans.back().get();
   return cudaSuccess;
@@ -600,11 +594,8 @@ cudaError_t grouped_launch(GroupedPlan& pl, const GroupedPtrs& p, cudaStream_t s
   cudaError_t e;
   pl.tick = ++g_plan_tick;
   note_path(SSBLAS_PATH_GROUPED, (pl.oz.ninst || pl.oz_wide.ninst) ? 7 : 0);
-  // (a stream that is being captured runs later, and in the order that the caller gives its graph)
-  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-  if (cudaStreamIsCapturing(st, &cap) != cudaSuccess) cudaGetLastError();
-  const bool captured = cap != cudaStreamCaptureStatusNone;
-  if (!captured && pl.in_use && pl.last_stream != st && (e = cudaStreamWaitEvent(st, pl.used, 0)) != cudaSuccess) return e;
+  const bool captured = is_captured(st);
+  if (!captured && (e = pl.order.begin(st)) != cudaSuccess) return e;
   if ((e = launch_kind<GCfgOz, 2, 7>(pl.oz_wide, p, st, "grouped_ozaki_slice", "grouped_ozaki_gemm", pl.dynamic)))
     return e;
   if ((e = launch_kind<GCfgOz32, 2, 7>(pl.oz, p, st, "grouped_ozaki_slice", "grouped_ozaki_gemm", pl.dynamic)))
@@ -615,10 +606,7 @@ cudaError_t grouped_launch(GroupedPlan& pl, const GroupedPtrs& p, cudaStream_t s
   bool follows = false;
   if (pl.simt && (e = launch_dmma_grouped(*pl.simt, p, st, follows))) return e;
   if (pl.simt && (e = launch_sgemm_grouped(*pl.simt, p, st, follows))) return e;
-  if (captured) return cudaSuccess;
-  if ((e = cudaEventRecord(pl.used, st)) != cudaSuccess) return e;
-  pl.in_use = true;
-  pl.last_stream = st;
+  if (!captured) pl.order.end(st);
   return cudaSuccess;
 }
 

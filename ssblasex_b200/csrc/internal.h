@@ -11,6 +11,7 @@
 
 #include "../../include/ssblasBatch.h"
 #include "per_device.h"
+#include "use_order.h"
 
 namespace ssb {
 
@@ -94,6 +95,38 @@ void note_splits(int splits);
 
 // Device-side error flag (set by kernels whose bounded waits give up).
 int* device_error_flag();
+
+// UseOrder over CUDA events (use_order.h)
+struct CudaOrder {
+  using Stream = cudaStream_t;
+  using Event = cudaEvent_t;
+  using Error = cudaError_t;
+  static Error create(Event& e) { return cudaEventCreateWithFlags(&e, cudaEventDisableTiming); }
+  static Error wait(Stream s, Event e) { return cudaStreamWaitEvent(s, e, 0); }
+  static Error record(Event e, Stream s) {
+    const Error r = cudaEventRecord(e, s);
+    if (r != cudaSuccess) cudaGetLastError();
+    return r;
+  }
+  static Error sync(Event e) { return cudaEventSynchronize(e); }
+  static void sync_stream(Stream s) {
+    if (cudaStreamSynchronize(s) != cudaSuccess) cudaGetLastError();
+  }
+  static void destroy(Event e) { cudaEventDestroy(e); }
+  static uint64_t id(Stream s) {
+    unsigned long long id = 0;
+    if (s == cudaStreamPerThread) return 0;
+    if (cudaStreamGetId(s, &id) != cudaSuccess) {
+      cudaGetLastError();
+      return 0;
+    }
+    return (uint64_t)id + 1;
+  }
+};
+using StreamOrder = UseOrder<CudaOrder>;
+// whether `st` is being captured into a graph: its work runs later, in the order that the caller gives the graph
+bool is_captured(cudaStream_t st);
+
 
 // ---- kernel entry points (each returns a CUDA error code; launches on `stream`) ----
 cudaError_t launch_simt_gemm(const BatchDesc& d, cudaStream_t stream);

@@ -1,0 +1,60 @@
+"""Grouped calls that share a plan's scratch, or a kept pointer array, where the streams' handles do not tell
+the streams apart."""
+import threading
+
+import numpy as np
+import pytest
+
+from oracle import oracle as O
+
+pytestmark = pytest.mark.gpu
+PER_THREAD = 2   # cudaStreamPerThread: one handle, a stream per host thread
+
+
+@pytest.fixture
+def S():
+    import torch
+    assert torch.cuda.is_available()
+    import ssblasex_b200 as S
+    yield S
+    torch.cuda.synchronize()
+    S.set_stream(None)
+    S.set_sync_mode(True)
+    S.set_math_mode(S.SSBLAS_MATH_PLAIN)
+
+
+def problems(seed, count=40, row="f64"):
+    from ssblasex_b200 import workloads as W
+    rng = np.random.default_rng(5)
+    return [W.make_problem(row, i % 2, i // 2 % 2, *(int(x) for x in rng.integers(1, 200, 3)), 1, 1.0, 0.0,
+                           seed=1000 * seed + i) for i in range(count)]
+
+
+@pytest.mark.parametrize("device_arrays", [True])
+def test_two_threads_on_the_per_thread_stream(S, device_arrays):
+    import torch
+    from ssblasex_b200 import runner
+    S.set_math_mode(S.SSBLAS_MATH_FP64_OZAKI)
+    sets = [problems(1), problems(2)]
+    dev = [runner.GroupedDevice(p) for p in sets]
+    for d in dev:
+        d.reset_c()
+    torch.cuda.synchronize()
+    S.set_sync_mode(False)
+    S.set_stream(PER_THREAD)
+    status = [[], []]
+
+    def work(i):
+        for _ in range(20):
+            status[i].append(dev[i].call(device_arrays=device_arrays))
+
+    threads = [threading.Thread(target=work, args=(i,)) for i in range(2)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    torch.cuda.synchronize()
+    assert status == [[0] * 20, [0] * 20]
+    for p, d in zip(sets, dev):
+        for q, C in zip(p, d.results()):
+            np.testing.assert_array_equal(C.view(np.uint64), O.ozaki_f64(q, 7)[1].view(np.uint64))
