@@ -590,12 +590,9 @@ cudaError_t grouped_make(const GroupedDesc& g, const GroupedArgs& a, cudaStream_
   return cudaSuccess;
 }
 
-cudaError_t grouped_launch(GroupedPlan& pl, const GroupedPtrs& p, cudaStream_t st) {
+// The launches of one call, in order; what was queued before one that fails stays queued.
+static cudaError_t launch_all(GroupedPlan& pl, const GroupedPtrs& p, cudaStream_t st) {
   cudaError_t e;
-  pl.tick = ++g_plan_tick;
-  note_path(SSBLAS_PATH_GROUPED, (pl.oz.ninst || pl.oz_wide.ninst) ? 7 : 0);
-  const bool captured = is_captured(st);
-  if (!captured && (e = pl.order.begin(st)) != cudaSuccess) return e;
   if ((e = launch_kind<GCfgOz, 2, 7>(pl.oz_wide, p, st, "grouped_ozaki_slice", "grouped_ozaki_gemm", pl.dynamic)))
     return e;
   if ((e = launch_kind<GCfgOz32, 2, 7>(pl.oz, p, st, "grouped_ozaki_slice", "grouped_ozaki_gemm", pl.dynamic)))
@@ -606,8 +603,15 @@ cudaError_t grouped_launch(GroupedPlan& pl, const GroupedPtrs& p, cudaStream_t s
   bool follows = false;
   if (pl.simt && (e = launch_dmma_grouped(*pl.simt, p, st, follows))) return e;
   if (pl.simt && (e = launch_sgemm_grouped(*pl.simt, p, st, follows))) return e;
-  if (!captured) pl.order.end(st);
   return cudaSuccess;
+}
+
+cudaError_t grouped_launch(GroupedPlan& pl, const GroupedPtrs& p, cudaStream_t st) {
+  pl.tick = ++g_plan_tick;
+  note_path(SSBLAS_PATH_GROUPED, (pl.oz.ninst || pl.oz_wide.ninst) ? 7 : 0);
+  if (is_captured(st)) return launch_all(pl, p, st);
+  const Use<CudaOrder> use(pl.order, st);
+  return use.error() != cudaSuccess ? use.error() : launch_all(pl, p, st);
 }
 
 void grouped_release() { g_plans.clear(); }

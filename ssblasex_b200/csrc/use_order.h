@@ -59,4 +59,23 @@ struct UseOrder {
   }
 };
 
+// One call's use of a buffer: ended on every way out of the scope, also where a launch failed after others
+// were queued.
+template <class Api>
+class Use {
+ public:
+  Use(UseOrder<Api>& order, typename Api::Stream st) : order_(&order), st_(st), error_(order.begin(st)) {}
+  ~Use() {
+    if (error_ == typename Api::Error{}) order_->end(st_);
+  }
+  Use(const Use&) = delete;
+  Use& operator=(const Use&) = delete;
+  typename Api::Error error() const { return error_; }   // of the wait; nothing may be queued then
+
+ private:
+  UseOrder<Api>* order_;
+  typename Api::Stream st_;
+  typename Api::Error error_;
+};
+
 }  // namespace ssb

@@ -44,9 +44,9 @@ static bool was(const char* what) {
 '''
 
 
-def _run(tmp_path, body):
+def _run(tmp_path, body, before=""):
     src = tmp_path / "t.cpp"
-    src.write_text(FAKE + "int main() {\n" + body + '\n  std::puts("ok");\n  return 0;\n}\n')
+    src.write_text(FAKE + before + "int main() {\n" + body + '\n  std::puts("ok");\n  return 0;\n}\n')
     exe = tmp_path / "t"
     subprocess.run(["g++", "-std=c++17", "-O1", "-Wall", "-I", str(ROOT / "ssblasex_b200" / "csrc"), str(src), "-o",
                     str(exe)], check=True)
@@ -83,4 +83,28 @@ def test_a_call_waits_for_the_one_before(tmp_path):
   fail_create = 1;
   UseOrder<Fake> p;
   if (p.begin(5) != 2 || p.made) return 10;
+''')
+
+
+def test_a_use_ends_on_every_way_out(tmp_path):
+    """A call whose second launch fails has its first queued: the next call, on another stream, waits for it. A
+    call whose wait failed queued nothing."""
+    _run(tmp_path, r'''
+  UseOrder<Fake> o;
+  if (call(o, 5, 2) != 7 || !was("l l r5/1 ")) return 1;
+  if (call(o, 6, 9) != 0 || !was("w6/1 l l l r6/1 ")) return 2;
+  fail_create = 1;
+  UseOrder<Fake> p;
+  if (call(p, 5, 9) != 2 || !was("") || p.in_use) return 3;
+''', before=r'''
+// a call of three launches, of which number `bad` is refused
+static int call(UseOrder<Fake>& o, int st, int bad) {
+  const Use<Fake> use(o, st);
+  if (use.error()) return use.error();
+  for (int i = 1; i <= 3; ++i) {
+    said += "l ";
+    if (i == bad) return 7;
+  }
+  return 0;
+}
 ''')
