@@ -379,24 +379,23 @@ static PtrArrays g_ptr_arrays[kMaxDevices][kPtrEntries];
 static unsigned long g_ptr_tick = 0;
 static PtrArrays* g_ptr_current = nullptr;   // entry of the call in progress (none: nothing to order)
 
-static bool same_key(const PtrArrays& e, const std::vector<void*>& a, const std::vector<void*>& b,
-                     const std::vector<void*>& c) {
-  const size_t n = a.size();
+static bool same_key(const PtrArrays& e, const void* const* a, const void* const* b, const void* const* c, size_t n) {
   if (e.key.size() != 3 * n) return false;
   const void* const* k = e.key.data();
-  return memcmp(k, a.data(), n * sizeof(void*)) == 0 && memcmp(k + n, b.data(), n * sizeof(void*)) == 0 &&
-         memcmp(k + 2 * n, c.data(), n * sizeof(void*)) == 0;
+  return memcmp(k, a, n * sizeof(void*)) == 0 && memcmp(k + n, b, n * sizeof(void*)) == 0 &&
+         memcmp(k + 2 * n, c, n * sizeof(void*)) == 0;
 }
 
-static cudaError_t device_pointer_arrays(const std::vector<void*>& a, const std::vector<void*>& b,
-                                         const std::vector<void*>& c, cudaStream_t st, void*** out) {
+// The arrays a, b, c of n pointers each, back to back on the device; pointer_arrays_used() follows the
+// launches that read them.
+static cudaError_t device_pointer_arrays(const void* const* a, const void* const* b, const void* const* c, size_t n,
+                                         cudaStream_t st, void*** out) {
   const int dev = current_device();
   if (!valid_device(dev)) return cudaErrorInvalidDevice;
-  const size_t n = a.size();
   PtrArrays* hit = nullptr;
   PtrArrays* victim = nullptr;
   for (PtrArrays& e : g_ptr_arrays[dev]) {
-    if (same_key(e, a, b, c)) {
+    if (same_key(e, a, b, c, n)) {
       hit = &e;
       break;
     }
@@ -425,9 +424,9 @@ static cudaError_t device_pointer_arrays(const std::vector<void*>& a, const std:
     void* h = pinned(3 * n * sizeof(void*), &err);
     if (!h) return err;
     void** hp = (void**)h;
-    memcpy(hp, a.data(), n * sizeof(void*));
-    memcpy(hp + n, b.data(), n * sizeof(void*));
-    memcpy(hp + 2 * n, c.data(), n * sizeof(void*));
+    memcpy(hp, a, n * sizeof(void*));
+    memcpy(hp + n, b, n * sizeof(void*));
+    memcpy(hp + 2 * n, c, n * sizeof(void*));
     if ((err = cudaMemcpyAsync(hit->dev, hp, 3 * n * sizeof(void*), cudaMemcpyHostToDevice, st)) != cudaSuccess)
       return err;
     pinned_done(st);
@@ -684,6 +683,10 @@ static ssblasStatus_t grouped_device(GroupedArgs& args, const void* const alpha_
   cudaStream_t st = settings().stream;
   cudaError_t e;
   GroupedPtrs ptrs;
+  struct Used {   // of kept pointer arrays, if any: on every way out
+    cudaStream_t st;
+    ~Used() { pointer_arrays_used(st); }
+  } used{st};
   const bool dev_arrays = kind_of((const void*)A) == PK_DEVICE;
   if (dev_arrays) {
     if (kind_of((const void*)B) != PK_DEVICE || kind_of((const void*)C) != PK_DEVICE)
@@ -696,16 +699,8 @@ static ssblasStatus_t grouped_device(GroupedArgs& args, const void* const alpha_
     if (kind_of(B[0]) != PK_DEVICE || kind_of(C[0]) != PK_DEVICE) return SSBLAS_STATUS_INVALID_VALUE;
     long total = 0;
     for (SSINT gi = 0; gi < args.groups; ++gi) total += args.group_size[gi];
-    void* h = pinned(3 * sizeof(void*) * total, &e);
-    if (!h) return map_err(e);
-    void** hp = (void**)h;
-    memcpy(hp, A, sizeof(void*) * total);
-    memcpy(hp + total, B, sizeof(void*) * total);
-    memcpy(hp + 2 * total, C, sizeof(void*) * total);
-    void** dp = (void**)workspace(WS_PTRS, 3 * sizeof(void*) * total, &e);
-    if (!dp) return map_err(e);
-    if ((e = cudaMemcpyAsync(dp, hp, 3 * sizeof(void*) * total, cudaMemcpyHostToDevice, st))) return map_err(e);
-    pinned_done(st);
+    void** dp = nullptr;
+    if ((e = device_pointer_arrays(A, B, (const void* const*)C, (size_t)total, st, &dp)) != cudaSuccess) return map_err(e);
     ptrs = {(const void* const*)dp, (const void* const*)(dp + total), (void* const*)(dp + 2 * total)};
   }
   if (!plan && (e = grouped_make(g, args, st, &plan)) != cudaSuccess) return map_err(e);
@@ -927,7 +922,8 @@ static ssblasStatus_t gemm_batched(ssblasOperation_t transa, ssblasOperation_t t
     d.A0 = da[0]; d.B0 = db[0]; d.C0 = dc[0];
     // the three pointer arrays on the device (uploaded unless a recent call had the same)
     void** dp = nullptr;
-    if ((e = device_pointer_arrays(da, db, dc, st, &dp)) != cudaSuccess) return map_err(e);
+    if ((e = device_pointer_arrays(da.data(), db.data(), dc.data(), da.size(), st, &dp)) != cudaSuccess)
+      return map_err(e);
     d.A = (const void* const*)dp;
     d.B = (const void* const*)(dp + batchCount);
     d.C = (void* const*)(dp + 2 * batchCount);

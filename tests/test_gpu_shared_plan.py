@@ -30,7 +30,7 @@ def problems(seed, count=40, row="f64"):
                            seed=1000 * seed + i) for i in range(count)]
 
 
-@pytest.mark.parametrize("device_arrays", [True])
+@pytest.mark.parametrize("device_arrays", [True, False])
 def test_two_threads_on_the_per_thread_stream(S, device_arrays):
     import torch
     from ssblasex_b200 import runner
@@ -58,3 +58,26 @@ def test_two_threads_on_the_per_thread_stream(S, device_arrays):
     for p, d in zip(sets, dev):
         for q, C in zip(p, d.results()):
             np.testing.assert_array_equal(C.view(np.uint64), O.ozaki_f64(q, 7)[1].view(np.uint64))
+
+
+@pytest.mark.parametrize("same_shapes", [True, False])
+def test_host_arrays_on_two_streams(S, same_shapes):
+    """Asynchronous calls with host arrays of device pointers: each call's kernels read its own pointers, also
+    while another stream's call uploads others."""
+    import torch
+    from ssblasex_b200 import runner
+    sets = [problems(3, 60, "f32"), problems(4, 60 if same_shapes else 50, "f32")]
+    dev = [runner.GroupedDevice(p) for p in sets]
+    for d in dev:
+        d.reset_c()
+    streams = [torch.cuda.Stream() for _ in dev]
+    torch.cuda.synchronize()
+    S.set_sync_mode(False)
+    for _ in range(20):
+        for d, s in zip(dev, streams):
+            S.set_stream(s.cuda_stream)
+            assert d.call(device_arrays=False) == 0
+    torch.cuda.synchronize()
+    for p, d in zip(sets, dev):
+        for q, C in zip(p, d.results()):
+            assert O.normalized_error(q, C) <= 4 * q.k * 2.0 ** -24
