@@ -63,7 +63,17 @@ ssblasStatus_t ssblasGemmBatchedEx_64(ssblasOperation_t transa, ssblasOperation_
  * order. alpha_array[g]/beta_array[g] point to the group's host scalar of its scale type. The
  * per-group types must form one of the three rows (fp32, fp64, int8->int32); rows may differ
  * between groups, and all instances run in one persistent launch per phase. Pointer arrays
- * follow the same three conventions as ssblasGemmBatchedEx. */
+ * follow the same three conventions as ssblasGemmBatchedEx.
+ *
+ * A call whose shapes, scalars and settings equal those of one of the last four such calls reuses that
+ * call's plan (tables and scratch, at most 2 GiB kept together); any other makes a plan first, which
+ * allocates and waits for the stream. Asynchronous calls that share a plan are ordered by the library.
+ *
+ * Under stream capture the call must find a plan: make the same call once before the capture. The plan
+ * then belongs to CUDA graphs: it stays in place until
+ * ssblasReleaseWorkspace, after which the graph must not run, and ordinary calls of these shapes make
+ * another. Graphs that hold calls of the same shapes share its scratch: the caller runs them one
+ * after another. */
 ssblasStatus_t ssblasGemmGroupedBatchedEx(
     const ssblasOperation_t transa_array[], const ssblasOperation_t transb_array[],
     const SSINT m_array[], const SSINT n_array[], const SSINT k_array[],
@@ -224,7 +234,8 @@ typedef struct {
 ssblasStatus_t ssblasSetProfiling(int enable);
 ssblasStatus_t ssblasGetProfile(ssblasKernelProfile_t* out, int max_entries, int* entries);
 
-/* Frees the device workspace cached by the library (it is re-created on the next call). */
+/* Frees the device workspace cached by the library (it is re-created on the next call). CUDA graphs that hold
+ * calls captured before must not run after it. */
 ssblasStatus_t ssblasReleaseWorkspace(void);
 
 /* Kernel configuration (tile shape / pipeline depth) of one path (an ssblasPath_t value):

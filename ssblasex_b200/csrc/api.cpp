@@ -14,6 +14,7 @@
 #include <algorithm>
 #include <cstdio>
 #include <iostream>
+#include <memory>
 #include <mutex>
 #include <string>
 #include <vector>
@@ -366,16 +367,18 @@ static void pinned_done(cudaStream_t st) {
 // the calls of a loop queue up behind one another. Since the key is the values, memory freed and
 // allocated again at the same addresses is harmless. An entry is rewritten only after the last
 // call that read it has finished, and each call waits for the one before (StreamOrder), so the last
-// use covers every earlier one.
+// use covers every earlier one. An entry that a call under capture reads is never rewritten: the graph
+// holds its address, and its contents are uploaded before the capture goes on.
 struct PtrArrays {
   std::vector<const void*> key;   // A[0..batch), B[0..batch), C[0..batch)
   void** dev = nullptr;
   size_t cap = 0;                 // pointers the device buffer holds
   StreamOrder order;
   unsigned long tick = 0;
+  bool captured = false;          // a CUDA graph reads it
 };
-constexpr int kPtrEntries = 4;
-static PtrArrays g_ptr_arrays[kMaxDevices][kPtrEntries];
+constexpr int kPtrEntries = 4;    // that may be rewritten
+static std::vector<std::unique_ptr<PtrArrays>> g_ptr_arrays[kMaxDevices];
 static unsigned long g_ptr_tick = 0;
 static PtrArrays* g_ptr_current = nullptr;   // entry of the call in progress (none: nothing to order)
 
@@ -386,6 +389,17 @@ static bool same_key(const PtrArrays& e, const void* const* a, const void* const
          memcmp(k + 2 * n, c, n * sizeof(void*)) == 0;
 }
 
+// A copy on a stream of its own that has ended when this returns (a capture of other streams goes on).
+static cudaError_t upload_now(void* dst, const void* src, size_t bytes) {
+  cudaStream_t s;
+  cudaError_t e = cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking);
+  if (e != cudaSuccess) return e;
+  e = cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, s);
+  const cudaError_t w = cudaStreamSynchronize(s);
+  cudaStreamDestroy(s);
+  return e != cudaSuccess ? e : w;
+}
+
 // The arrays a, b, c of n pointers each, back to back on the device; pointer_arrays_used() follows the
 // launches that read them.
 static cudaError_t device_pointer_arrays(const void* const* a, const void* const* b, const void* const* c, size_t n,
@@ -394,22 +408,30 @@ static cudaError_t device_pointer_arrays(const void* const* a, const void* const
   if (!valid_device(dev)) return cudaErrorInvalidDevice;
   PtrArrays* hit = nullptr;
   PtrArrays* victim = nullptr;
-  for (PtrArrays& e : g_ptr_arrays[dev]) {
-    if (same_key(e, a, b, c, n)) {
-      hit = &e;
+  int free_to_rewrite = 0;
+  for (auto& e : g_ptr_arrays[dev]) {
+    if (same_key(*e, a, b, c, n)) {
+      hit = e.get();
       break;
     }
-    if (!victim || e.tick < victim->tick) victim = &e;
+    if (e->captured) continue;
+    ++free_to_rewrite;
+    if (!victim || e->tick < victim->tick) victim = e.get();
   }
   cudaError_t err;
   const bool captured = is_captured(st);
   if (hit) {
     if (!captured && (err = hit->order.begin(st)) != cudaSuccess) return err;
   } else {
+    if (captured || free_to_rewrite < kPtrEntries) {
+      g_ptr_arrays[dev].emplace_back(new PtrArrays);
+      victim = g_ptr_arrays[dev].back().get();
+    }
     hit = victim;
     if ((err = hit->order.idle()) != cudaSuccess) return err;
     hit->key.clear();   // no valid contents until the upload below is queued
     if (!captured && (err = hit->order.begin(st)) != cudaSuccess) return err;
+    const RelaxedCapture relaxed;
     if (hit->cap < 3 * n) {
       if (hit->dev) cudaFree(hit->dev);
       hit->dev = nullptr;
@@ -427,10 +449,20 @@ static cudaError_t device_pointer_arrays(const void* const* a, const void* const
     memcpy(hp, a, n * sizeof(void*));
     memcpy(hp + n, b, n * sizeof(void*));
     memcpy(hp + 2 * n, c, n * sizeof(void*));
-    if ((err = cudaMemcpyAsync(hit->dev, hp, 3 * n * sizeof(void*), cudaMemcpyHostToDevice, st)) != cudaSuccess)
-      return err;
-    pinned_done(st);
+    if (captured) {
+      // not by the graph, at whose launch the pinned slot holds something else
+      if ((err = upload_now(hit->dev, hp, 3 * n * sizeof(void*))) != cudaSuccess) return err;
+    } else {
+      if ((err = cudaMemcpyAsync(hit->dev, hp, 3 * n * sizeof(void*), cudaMemcpyHostToDevice, st)) != cudaSuccess)
+        return err;
+      pinned_done(st);
+    }
     hit->key.assign((const void* const*)hp, (const void* const*)hp + 3 * n);
+  }
+  if (captured && !hit->captured) {
+    const RelaxedCapture relaxed;
+    if ((err = hit->order.idle()) != cudaSuccess) return err;   // its upload, if an ordinary call made it
+    hit->captured = true;
   }
   hit->tick = ++g_ptr_tick;
   g_ptr_current = captured ? nullptr : hit;
@@ -447,11 +479,11 @@ static void pointer_arrays_used(cudaStream_t st) {
 
 static void release_pointer_arrays(int dev) {
   if (!valid_device(dev)) return;
-  for (PtrArrays& e : g_ptr_arrays[dev]) {
-    if (e.dev) cudaFree(e.dev);
-    e.order.destroy();
-    e = PtrArrays{};
+  for (auto& e : g_ptr_arrays[dev]) {
+    if (e->dev) cudaFree(e->dev);
+    e->order.destroy();
   }
+  g_ptr_arrays[dev].clear();
 }
 
 static ssblasStatus_t map_err(cudaError_t e) {
@@ -665,7 +697,8 @@ static ssblasStatus_t grouped_device(GroupedArgs& args, const void* const alpha_
                                      const void* const beta_array[], const void* const A[], const void* const B[],
                                      void* const C[]) {
   std::lock_guard<std::mutex> lock(g_mutex);
-  GroupedPlan* plan = grouped_scalars(alpha_array, beta_array, args) ? grouped_find(args) : nullptr;
+  const bool captured = is_captured(settings().stream);
+  GroupedPlan* plan = grouped_scalars(alpha_array, beta_array, args) ? grouped_find(args, captured) : nullptr;
   GroupedDesc g;
   if (!plan) {
     const ssblasStatus_t v = grouped_instances(args, alpha_array, beta_array, g);
@@ -704,7 +737,7 @@ static ssblasStatus_t grouped_device(GroupedArgs& args, const void* const alpha_
     ptrs = {(const void* const*)dp, (const void* const*)(dp + total), (void* const*)(dp + 2 * total)};
   }
   if (!plan && (e = grouped_make(g, args, st, &plan)) != cudaSuccess) return map_err(e);
-  if ((e = grouped_launch(*plan, ptrs, st)) != cudaSuccess) return map_err(e);
+  if ((e = grouped_launch(*plan, ptrs, st, captured)) != cudaSuccess) return map_err(e);
   if (settings().synchronous) {
     if ((e = cudaStreamSynchronize(st)) != cudaSuccess) return map_err(e);
     return check_device_error(st);

@@ -31,6 +31,7 @@
 
 #include "grouped.h"
 #include "internal.h"
+#include "plan_cache.h"
 #include "ozaki_digits.cuh"
 #include "tc_gemm.cuh"
 
@@ -446,17 +447,18 @@ struct GroupedPlan {
   size_t scratch = 0;        // bytes of packed operand buffers
   StreamOrder order;
   unsigned long tick = 0;
-  ~GroupedPlan() { order.destroy(); }
+  bool captured = false;     // a CUDA graph holds launches of it (plan_cache.h)
+  ~GroupedPlan() {
+    if (order.idle() != cudaSuccess) cudaGetLastError();
+    order.destroy();
+  }
 };
 
 namespace {
 
-// Cached plans per device: at most kMaxPlans, and beyond the newest one only as long as their scratch
-// stays within kMaxScratch. Host access is under the library lock.
-constexpr size_t kMaxPlans = 4;
-constexpr size_t kMaxScratch = (size_t)2 << 30;
-std::map<int, std::vector<std::unique_ptr<GroupedPlan>>> g_plans;
-unsigned long g_plan_tick = 0;
+// Plans kept per device. Host access is under the library lock.
+using Plans = PlanCache<GroupedPlan, 4, (size_t)2 << 30>;
+std::map<int, Plans> g_plans;
 
 // Tile shape of one Ozaki instance: 128 x 64 tiles with one accumulator read the slice planes from
 // shared memory a third more efficiently per product than 128 x 32 tiles with two, whose gain is
@@ -495,23 +497,22 @@ bool each_array(const GroupedArgs& a, F f) {
 
 }  // namespace
 
-GroupedPlan* grouped_find(const GroupedArgs& a) {
+GroupedPlan* grouped_find(const GroupedArgs& a, bool captured) {
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess) return nullptr;
   auto it = g_plans.find(dev);
   if (it == g_plans.end()) return nullptr;
   const std::vector<uint64_t> key = plan_settings();
-  for (auto& p : it->second) {
-    if (p->scalars != a.scalars || p->settings != key) continue;
+  return it->second.find(captured, [&](const GroupedPlan& p) {
+    if (p.scalars != a.scalars || p.settings != key) return false;
     size_t at = 0;
     const bool same = each_array(a, [&](const char* v, size_t n) {
-      if (at + n > p->shapes.size() || memcmp(p->shapes.data() + at, v, n) != 0) return false;
+      if (at + n > p.shapes.size() || memcmp(p.shapes.data() + at, v, n) != 0) return false;
       at += n;
       return true;
     });
-    if (same && at == p->shapes.size()) return p.get();
-  }
-  return nullptr;
+    return same && at == p.shapes.size();
+  });
 }
 
 bool grouped_has_f64(const GroupedPlan& plan) { return plan.has_f64; }
@@ -545,16 +546,6 @@ cudaError_t grouped_make(const GroupedDesc& g, const GroupedArgs& a, cudaStream_
     else if (in.row == ROW_F32 && (mode & SSBLAS_MATH_FP32_BF16X3) && f32_split_records(in, bf)) continue;
     else plain.push_back(i);
   }
-  // make room first: the evicted plans' buffers may be what the new one needs (cudaFree waits for
-  // the work that reads them)
-  auto& plans = g_plans[dev];
-  auto evict_oldest = [&] {
-    size_t old = 0;
-    for (size_t i = 1; i < plans.size(); ++i)
-      if (plans[i]->tick < plans[old]->tick) old = i;
-    plans.erase(plans.begin() + (long)old);
-  };
-  if (plans.size() >= kMaxPlans) evict_oldest();
   {
     KindPlan<GCfgOz32> k1;
     plan_kind(g, oz, k1);
@@ -563,12 +554,8 @@ cudaError_t grouped_make(const GroupedDesc& g, const GroupedArgs& a, cudaStream_
     KindPlan<GCfgI8> k3;
     plan_kind(g, i8, k3);
     pl->scratch = (size_t)(k0.bytesA + k0.bytesB + k1.bytesA + k1.bytesB + k3.bytesA + k3.bytesB);
-    auto total = [&] {
-      size_t s = pl->scratch;
-      for (auto& p : plans) s += p->scratch;
-      return s;
-    };
-    while (!plans.empty() && total() > kMaxScratch) evict_oldest();
+    // the dropped plans' buffers may be what the new one needs
+    g_plans[dev].make_room(pl->scratch);
     if ((e = upload_kind(k1, pl->oz, st))) return e;
     if ((e = upload_kind(k0, pl->oz_wide, st))) return e;
     if ((e = upload_kind(k3, pl->i8, st))) return e;
@@ -585,8 +572,7 @@ cudaError_t grouped_make(const GroupedDesc& g, const GroupedArgs& a, cudaStream_
     pl->simt = std::make_unique<GroupedSimt>();
     if ((e = plan_simt_grouped(g, plain, *pl->simt, st))) return e;
   }
-  plans.push_back(std::move(pl));
-  *out = plans.back().get();
+  *out = g_plans[dev].add(std::move(pl));
   return cudaSuccess;
 }
 
@@ -606,10 +592,21 @@ static cudaError_t launch_all(GroupedPlan& pl, const GroupedPtrs& p, cudaStream_
   return cudaSuccess;
 }
 
-cudaError_t grouped_launch(GroupedPlan& pl, const GroupedPtrs& p, cudaStream_t st) {
-  pl.tick = ++g_plan_tick;
+cudaError_t grouped_launch(GroupedPlan& pl, const GroupedPtrs& p, cudaStream_t st, bool captured) {
+  int dev = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e != cudaSuccess) return e;
+  g_plans[dev].use(pl);
   note_path(SSBLAS_PATH_GROUPED, (pl.oz.ninst || pl.oz_wide.ninst) ? 7 : 0);
-  if (is_captured(st)) return launch_all(pl, p, st);
+  if (captured) {
+    // from here on the plan belongs to graphs: the ordinary calls on its scratch end first, and none follows
+    if (!pl.captured) {
+      const RelaxedCapture relaxed;
+      if ((e = pl.order.idle()) != cudaSuccess) return e;
+      pl.captured = true;
+    }
+    return launch_all(pl, p, st);
+  }
   const Use<CudaOrder> use(pl.order, st);
   return use.error() != cudaSuccess ? use.error() : launch_all(pl, p, st);
 }

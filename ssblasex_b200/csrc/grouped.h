@@ -106,10 +106,11 @@ cudaError_t launch_f32_split_grouped(const SplitRec* recs, long tiles, const Gro
 // of the current device for these arguments (compared value by value), nullptr if there is none.
 // grouped_make: a new plan (the arguments were validated), cached in place of the least recently
 // used one. grouped_launch: all instances with device-resident operands, one pre-pass and one
-// persistent GEMM launch per kind. grouped_has_f64: whether any instance is fp64.
-GroupedPlan* grouped_find(const GroupedArgs& a);
+// persistent GEMM launch per kind. captured: the stream is being captured; the plan then stays until
+// grouped_release and serves graphs only. grouped_has_f64: whether any instance is fp64.
+GroupedPlan* grouped_find(const GroupedArgs& a, bool captured);
 cudaError_t grouped_make(const GroupedDesc& g, const GroupedArgs& a, cudaStream_t st, GroupedPlan** out);
-cudaError_t grouped_launch(GroupedPlan& plan, const GroupedPtrs& p, cudaStream_t st);
+cudaError_t grouped_launch(GroupedPlan& plan, const GroupedPtrs& p, cudaStream_t st, bool captured);
 bool grouped_has_f64(const GroupedPlan& plan);
 void grouped_release();
 

@@ -126,6 +126,21 @@ struct CudaOrder {
 using StreamOrder = UseOrder<CudaOrder>;
 // whether `st` is being captured into a graph: its work runs later, in the order that the caller gives the graph
 bool is_captured(cudaStream_t st);
+// While it lives, this thread may make calls (event waits, allocations, copies on streams of its own) that a
+// capture elsewhere in the process would otherwise forbid.
+class RelaxedCapture {
+ public:
+  RelaxedCapture() { ok_ = cudaThreadExchangeStreamCaptureMode(&mode_) == cudaSuccess; }
+  ~RelaxedCapture() {
+    if (ok_) cudaThreadExchangeStreamCaptureMode(&mode_);
+  }
+  RelaxedCapture(const RelaxedCapture&) = delete;
+  RelaxedCapture& operator=(const RelaxedCapture&) = delete;
+
+ private:
+  cudaStreamCaptureMode mode_ = cudaStreamCaptureModeRelaxed;
+  bool ok_;
+};
 
 
 // ---- kernel entry points (each returns a CUDA error code; launches on `stream`) ----
