@@ -166,6 +166,8 @@ bool is_captured(cudaStream_t st) {
 struct DeviceWs {
   void* ptr[WS_NUM] = {};
   size_t size[WS_NUM] = {};
+  bool captured[WS_NUM] = {};   // a CUDA graph holds the buffer's address
+  std::vector<void*> kept;      // such buffers that a larger one has replaced, until ssblasReleaseWorkspace
 };
 static std::vector<DeviceWs> g_ws;
 
@@ -182,13 +184,23 @@ void* workspace(WsSlot slot, size_t bytes, cudaError_t* err) {
     *err = cudaErrorMemoryAllocation;
     return nullptr;
   }
-  if (w.size[slot] >= bytes) return w.ptr[slot];
+  const bool captured = is_captured(settings().stream);
+  if (w.size[slot] >= bytes) {
+    w.captured[slot] |= captured;
+    return w.ptr[slot];
+  }
+  const RelaxedCapture relaxed;
   if (w.ptr[slot]) {
-    // the old buffer may still be read by work in flight
-    cudaStreamSynchronize(settings().stream);
-    cudaFree(w.ptr[slot]);
+    if (w.captured[slot] || captured) {   // (nothing can be waited for during a capture)
+      w.kept.push_back(w.ptr[slot]);
+    } else {
+      // the old buffer may still be read by work in flight
+      cudaStreamSynchronize(settings().stream);
+      cudaFree(w.ptr[slot]);
+    }
     w.ptr[slot] = nullptr;
     w.size[slot] = 0;
+    w.captured[slot] = false;
   }
   size_t grow = bytes + bytes / 4;
   grow = (grow + 4095) & ~(size_t)4095;
@@ -199,6 +211,7 @@ void* workspace(WsSlot slot, size_t bytes, cudaError_t* err) {
     return nullptr;
   }
   w.size[slot] = grow;
+  w.captured[slot] = captured;
   return w.ptr[slot];
 }
 
@@ -213,7 +226,10 @@ static void release_workspace() {
     if (g_ws[dev].ptr[s]) cudaFree(g_ws[dev].ptr[s]);
     g_ws[dev].ptr[s] = nullptr;
     g_ws[dev].size[s] = 0;
+    g_ws[dev].captured[s] = false;
   }
+  for (void* p : g_ws[dev].kept) cudaFree(p);
+  g_ws[dev].kept.clear();
 }
 
 __device__ int g_device_error = 0;

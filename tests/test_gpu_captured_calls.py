@@ -126,3 +126,42 @@ def test_batched_host_arrays_replay_after_other_calls(S, warm):
         graph.replay()
     s.synchronize()
     assert O.normalized_error(p, dp.C.cpu().numpy().reshape(p.C.shape)) <= 4 * p.k * 2.0 ** -53
+
+
+@pytest.mark.parametrize("row,mode", [("f64", "ozaki"), ("i8", "plain")])
+def test_batched_replay_after_larger_calls(S, row, mode):
+    """The scratch that a captured call reads is not freed when a larger call needs more."""
+    import torch
+    from ssblasex_b200 import runner, workloads as W
+    if mode == "ozaki":
+        S.set_math_mode(S.SSBLAS_MATH_FP64_OZAKI)
+    mk = lambda m, batch, seed: W.make_problem(row, 0, 1, m, 50, 61, batch, 1, 0, lda=m + 3, seed=seed)
+    want = lambda q: O.ozaki_f64(q, 7)[1] if row == "f64" else O.restated_gemm(q)[1]
+    p, fresh = mk(40, 3, 1), mk(40, 3, 2)
+    dp = runner.DeviceProblem(p)
+    assert runner.call(p, "device_array", dp)[0] == 0      # (synchronous: equal spacing is found)
+    s = torch.cuda.Stream()
+    S.set_sync_mode(False)
+    S.set_stream(s.cuda_stream)
+    arrays = dp.host_arrays()
+    al, be = np.array([p.alpha], p.scale_dtype), np.array([p.beta], p.scale_dtype)
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.stream(s):
+        with torch.cuda.graph(graph, stream=s):
+            assert S.lib().ssblasGemmBatchedEx(p.transa, p.transb, p.m, p.n, p.k, al.ctypes.data, arrays[0], p.types[0],
+                                               p.lda, arrays[1], p.types[1], p.ldb, be.ctypes.data, arrays[2],
+                                               p.types[2], p.ldc, p.batch, 0, 0) == 0
+    S.set_sync_mode(True)
+    for i in range(4):
+        q = mk(200 + 100 * i, 8, 10 + i)
+        st, C = runner.call(q, "host_array")
+        assert st == 0
+        np.testing.assert_array_equal(C.reshape(-1), want(q).reshape(-1))
+    dp.A.copy_(torch.from_numpy(fresh.A))
+    dp.B.copy_(torch.from_numpy(fresh.B))
+    dp.C.copy_(torch.from_numpy(fresh.C))
+    torch.cuda.synchronize()
+    with torch.cuda.stream(s):
+        graph.replay()
+    s.synchronize()
+    np.testing.assert_array_equal(dp.C.cpu().numpy().reshape(-1), want(fresh).reshape(-1))
