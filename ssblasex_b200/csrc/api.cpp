@@ -168,6 +168,8 @@ struct DeviceWs {
   size_t size[WS_NUM] = {};
   bool captured[WS_NUM] = {};   // a CUDA graph holds the buffer's address
   std::vector<void*> kept;      // such buffers that a larger one has replaced, until ssblasReleaseWorkspace
+  StreamOrder order;            // of the calls that use any of the buffers, whatever their streams
+  bool active = false;          // the call in progress is one of them
 };
 static std::vector<DeviceWs> g_ws;
 
@@ -185,6 +187,10 @@ void* workspace(WsSlot slot, size_t bytes, cudaError_t* err) {
     return nullptr;
   }
   const bool captured = is_captured(settings().stream);
+  if (!captured && !w.active) {
+    if ((*err = w.order.begin(settings().stream)) != cudaSuccess) return nullptr;
+    w.active = true;
+  }
   if (w.size[slot] >= bytes) {
     w.captured[slot] |= captured;
     return w.ptr[slot];
@@ -215,6 +221,16 @@ void* workspace(WsSlot slot, size_t bytes, cudaError_t* err) {
   return w.ptr[slot];
 }
 
+// At the end of each call, on every way out.
+struct WorkspaceUse {
+  ~WorkspaceUse() {
+    for (DeviceWs& w : g_ws) {
+      if (w.active) w.order.end(settings().stream);
+      w.active = false;
+    }
+  }
+};
+
 static void release_pointer_arrays(int dev);
 static void release_workspace() {
   int dev = 0;
@@ -230,6 +246,7 @@ static void release_workspace() {
   }
   for (void* p : g_ws[dev].kept) cudaFree(p);
   g_ws[dev].kept.clear();
+  g_ws[dev].order.destroy();
 }
 
 __device__ int g_device_error = 0;
@@ -894,6 +911,7 @@ static ssblasStatus_t gemm_batched(ssblasOperation_t transa, ssblasOperation_t t
   if (k > 0 && (lda < arows || ldb < brows)) return SSBLAS_STATUS_INVALID_VALUE;
 
   std::lock_guard<std::mutex> lock(g_mutex);
+  const WorkspaceUse workspace_use;
   g_info = ssblasRunInfo_t{};
   cudaStream_t st = settings().stream;
   cudaError_t e;

@@ -81,3 +81,30 @@ def test_host_arrays_on_two_streams(S, same_shapes):
     for p, d in zip(sets, dev):
         for q, C in zip(p, d.results()):
             assert O.normalized_error(q, C) <= 4 * q.k * 2.0 ** -24
+
+
+@pytest.mark.parametrize("row", ["f64", "i8"])
+def test_batched_scratch_on_two_streams(S, row):
+    """Asynchronous batched calls on two streams share the slices (fp64, Ozaki) or the aligned copies (int8)."""
+    import torch
+    from ssblasex_b200 import runner, workloads as W
+    S.set_math_mode(S.SSBLAS_MATH_FP64_OZAKI)
+    probs = [W.make_problem(row, 0, 1, 203, 190 - 50 * i, 301 + 70 * i, 6, 1, 0, lda=206, seed=i) for i in range(2)]
+    dev = [runner.DeviceProblem(p) for p in probs]
+    args = []
+    for p, d in zip(probs, dev):
+        a, t = d.host_arrays(), p.types
+        al, be = np.array([p.alpha], p.scale_dtype), np.array([p.beta], p.scale_dtype)
+        args.append((a, al, be, (p.transa, p.transb, p.m, p.n, p.k, al.ctypes.data, a[0], t[0], p.lda, a[1], t[1], p.ldb,
+                                 be.ctypes.data, a[2], t[2], p.ldc, p.batch, 0, 0)))
+    streams = [torch.cuda.Stream() for _ in dev]
+    torch.cuda.synchronize()
+    S.set_sync_mode(False)
+    for _ in range(20):
+        for a, s in zip(args, streams):
+            S.set_stream(s.cuda_stream)
+            assert S.lib().ssblasGemmBatchedEx(*a[3]) == 0
+    torch.cuda.synchronize()
+    for p, d in zip(probs, dev):
+        want = O.restated_gemm(p)[1] if row == "i8" else O.ozaki_f64(p, 7)[1]
+        np.testing.assert_array_equal(d.C.cpu().numpy().reshape(-1), want.reshape(-1))
