@@ -678,14 +678,13 @@ ssblasStatus_t check_device_error(cudaStream_t st) {
 static ssblasStatus_t map_err(cudaError_t e);
 static void* pinned(size_t bytes, cudaError_t* err);
 
-// The scalars of the groups by value; false where an alpha or beta is missing or C has a type that no row
-// has (the validation then answers).
+// The scalars of the groups by value, once the types are known to be one of the rows; false where an alpha or
+// beta is missing.
 static bool grouped_scalars(const void* const alpha_array[], const void* const beta_array[], GroupedArgs& a) {
   a.scalars.assign(2 * (size_t)a.groups, 0);
   for (SSINT gi = 0; gi < a.groups; ++gi) {
-    const ssblasDataType_t c = a.ctype[gi];
-    if (!alpha_array[gi] || !beta_array[gi] || (c != SSBLAS_R_64F && c != SSBLAS_R_32F && c != SSBLAS_R_32I)) return false;
-    const size_t bytes = c == SSBLAS_R_64F ? 8 : 4;
+    if (!alpha_array[gi] || !beta_array[gi]) return false;
+    const size_t bytes = a.ctype[gi] == SSBLAS_R_64F ? 8 : 4;
     memcpy(&a.scalars[2 * gi], alpha_array[gi], bytes);
     memcpy(&a.scalars[2 * gi + 1], beta_array[gi], bytes);
   }
@@ -731,11 +730,18 @@ static ssblasStatus_t grouped_device(GroupedArgs& args, const void* const alpha_
                                      void* const C[]) {
   std::lock_guard<std::mutex> lock(g_mutex);
   const bool captured = is_captured(settings().stream);
-  GroupedPlan* plan = grouped_scalars(alpha_array, beta_array, args) ? grouped_find(args, captured) : nullptr;
+  // (shapes and types that were valid for a plan tell how many bytes a scalar has; others may be refused unread)
+  bool read = false, have = false;
+  GroupedPlan* plan = grouped_find(args, captured, [&] {
+    if (!read) have = grouped_scalars(alpha_array, beta_array, args);
+    read = true;
+    return have;
+  });
   GroupedDesc g;
   if (!plan) {
     const ssblasStatus_t v = grouped_instances(args, alpha_array, beta_array, g);
     if (v != SSBLAS_STATUS_SUCCESS) return v;
+    if (!read) grouped_scalars(alpha_array, beta_array, args);
   }
   g_info = ssblasRunInfo_t{};
   if (settings().math_mode & SSBLAS_MATH_FP64_OZAKI) {

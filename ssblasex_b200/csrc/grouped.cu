@@ -497,21 +497,24 @@ bool each_array(const GroupedArgs& a, F f) {
 
 }  // namespace
 
-GroupedPlan* grouped_find(const GroupedArgs& a, bool captured) {
+static bool same_shapes(const GroupedPlan& p, const GroupedArgs& a) {
+  size_t at = 0;
+  const bool same = each_array(a, [&](const char* v, size_t n) {
+    if (at + n > p.shapes.size() || memcmp(p.shapes.data() + at, v, n) != 0) return false;
+    at += n;
+    return true;
+  });
+  return same && at == p.shapes.size();
+}
+
+GroupedPlan* grouped_find(const GroupedArgs& a, bool captured, const std::function<bool()>& read_scalars) {
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess) return nullptr;
   auto it = g_plans.find(dev);
   if (it == g_plans.end()) return nullptr;
   const std::vector<uint64_t> key = plan_settings();
   return it->second.find(captured, [&](const GroupedPlan& p) {
-    if (p.scalars != a.scalars || p.settings != key) return false;
-    size_t at = 0;
-    const bool same = each_array(a, [&](const char* v, size_t n) {
-      if (at + n > p.shapes.size() || memcmp(p.shapes.data() + at, v, n) != 0) return false;
-      at += n;
-      return true;
-    });
-    return same && at == p.shapes.size();
+    return p.settings == key && same_shapes(p, a) && read_scalars() && p.scalars == a.scalars;
   });
 }
 

@@ -4,6 +4,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <functional>
 #include <vector>
 
 #include "internal.h"
@@ -102,13 +103,14 @@ bool f32_split_records(const GroupedInst& in, std::vector<SplitRec>& out);
 cudaError_t launch_f32_split_grouped(const SplitRec* recs, long tiles, const GroupedPtrs& p, cudaStream_t st);
 
 // A grouped call's device tables depend on its shapes, scalars and the settings only, so a plan serves
-// every call that repeats those values, whatever matrices it points to. grouped_find: the cached plan
-// of the current device for these arguments (compared value by value), nullptr if there is none.
+// every call that repeats those values, whatever matrices it points to. grouped_find: the cached plan of the
+// current device for these arguments (compared value by value), nullptr if there is none; read_scalars fills
+// a.scalars, and is asked once the shapes and types are known to be a plan's (false: they cannot be read).
 // grouped_make: a new plan (the arguments were validated), cached in place of the least recently
 // used one. grouped_launch: all instances with device-resident operands, one pre-pass and one
 // persistent GEMM launch per kind. captured: the stream is being captured; the plan then stays until
 // grouped_release and serves graphs only. grouped_has_f64: whether any instance is fp64.
-GroupedPlan* grouped_find(const GroupedArgs& a, bool captured);
+GroupedPlan* grouped_find(const GroupedArgs& a, bool captured, const std::function<bool()>& read_scalars);
 cudaError_t grouped_make(const GroupedDesc& g, const GroupedArgs& a, cudaStream_t st, GroupedPlan** out);
 cudaError_t grouped_launch(GroupedPlan& plan, const GroupedPtrs& p, cudaStream_t st, bool captured);
 bool grouped_has_f64(const GroupedPlan& plan);

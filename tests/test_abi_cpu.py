@@ -357,3 +357,23 @@ def test_reference_arm_other_ranks_exit_quietly():
                         "--warmup", "0", "--workload", "fp32_batch64_128"], capture_output=True, text=True,
                        timeout=600, cwd=str(ROOT), env=env)
     assert r.returncode == 0 and r.stdout.strip() == "", (r.returncode, r.stdout[-500:], r.stderr[-500:])
+
+
+def test_grouped_scalars_are_not_read_before_the_arguments_are_checked():
+    """A group that is refused for its sizes or types never has its alpha or beta read: here they point to
+    unmapped memory."""
+    code = """
+import ctypes as ct
+import ssblasex_b200 as S
+L, I = (lambda v: (ct.c_long * 1)(v)), (lambda v: (ct.c_int * 1)(v))
+bad = (ct.c_void_p * 1)(64)
+p = (ct.c_void_p * 1)(4096)
+def call(m, a, c):
+    return S.lib().ssblasGemmGroupedBatchedEx(I(0), I(0), L(m), L(4), L(4), bad, p, I(a), L(4), p, I(a), L(4), bad, p,
+                                              I(c), L(4), 1, L(1), 0, 0)
+assert call(0, S.SSBLAS_R_64F, S.SSBLAS_R_64F) == S.SSBLAS_STATUS_INTERNAL_ERROR
+assert call(4, S.SSBLAS_R_32F, S.SSBLAS_R_64F) == S.SSBLAS_STATUS_INVALID_VALUE
+print("ok")
+"""
+    r = subprocess.run([sys.executable, "-c", code], capture_output=True, text=True, timeout=120, cwd=str(ROOT))
+    assert r.returncode == 0 and r.stdout.strip() == "ok", (r.returncode, r.stdout, r.stderr)
