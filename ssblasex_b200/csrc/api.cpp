@@ -173,6 +173,19 @@ struct DeviceWs {
 };
 static std::vector<DeviceWs> g_ws;
 
+static size_t workspace_growth(size_t bytes) { return (bytes + bytes / 4 + 4095) & ~(size_t)4095; }
+
+bool workspace_fits(WsSlot slot, size_t bytes) {
+  int dev = 0;
+  size_t left = 0, all = 0, has = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || cudaMemGetInfo(&left, &all) != cudaSuccess) {
+    cudaGetLastError();
+    return true;   // the allocation will tell
+  }
+  if ((int)g_ws.size() > dev) has = g_ws[dev].size[slot];
+  return has >= bytes || workspace_growth(bytes) <= left + has;
+}
+
 void* workspace(WsSlot slot, size_t bytes, cudaError_t* err) {
   int dev = 0;
   *err = cudaGetDevice(&dev);
@@ -208,8 +221,7 @@ void* workspace(WsSlot slot, size_t bytes, cudaError_t* err) {
     w.size[slot] = 0;
     w.captured[slot] = false;
   }
-  size_t grow = bytes + bytes / 4;
-  grow = (grow + 4095) & ~(size_t)4095;
+  const size_t grow = workspace_growth(bytes);
   *err = cudaMalloc(&w.ptr[slot], grow);
   if (*err != cudaSuccess) {
     cudaGetLastError();

@@ -87,6 +87,8 @@ bool tcgen05_available();
 enum WsSlot { WS_PTRS = 0, WS_PACK_A, WS_PACK_B, WS_EXP, WS_STAGE_A, WS_STAGE_B, WS_STAGE_C, WS_MISC, WS_SPLIT,
                WS_SPLIT_CNT, WS_ROWMAX, WS_NUM };
 void* workspace(WsSlot slot, size_t bytes, cudaError_t* err);
+// whether the slot has these bytes or the device's free memory has room for them
+bool workspace_fits(WsSlot slot, size_t bytes);
 
 // Launch bookkeeping for ssblasGetLastRunInfo and the benchmark's launch count.
 void note_launch(int count = 1);

@@ -399,13 +399,20 @@ cudaError_t launch_i8_tcgen05(const BatchDesc& d, cudaStream_t st) {
   const bool amn = d.transa == SSBLAS_OP_N, bmn = d.transb == SSBLAS_OP_T;
   // operands with odd leading dimensions or bases, or unevenly spaced instances, are first copied onto
   // the 16-byte grid, in the order in which they are stored
+  // A thin operand's lines grow to 16 bytes, up to 16 times what it has: where that does not fit the device any
+  // more, the SIMT kernel reads it as it is. (Asked only for 1 GiB and more, whose copy alone takes 0.3 ms.)
+  auto beyond_memory = [](WsSlot slot, long len, size_t bytes) {
+    return len < 16 && bytes >= ((size_t)1 << 30) && !workspace_fits(slot, bytes);
+  };
   BatchDesc x = d;
   LineCopy ca, cb;
   const LineCopy *pa = nullptr, *pb = nullptr;
   cudaError_t e;
   if (!operand_direct(d.A0, d.strideA, d.lda, d.batch, 1)) {
     const long len = amn ? d.m : d.k, lines = amn ? d.k : d.m, pitch = round_up(len, 16);
-    void* w = workspace(WS_PACK_A, (size_t)(lines * pitch) * (size_t)d.batch, &e);
+    const size_t bytes = (size_t)(lines * pitch) * (size_t)d.batch;
+    if (beyond_memory(WS_PACK_A, len, bytes)) return cudaErrorNotSupported;
+    void* w = workspace(WS_PACK_A, bytes, &e);
     if (!w) return e;
     ca = LineCopy{d.A, d.lda, lines, len, w, pitch};
     pa = &ca;
@@ -413,7 +420,9 @@ cudaError_t launch_i8_tcgen05(const BatchDesc& d, cudaStream_t st) {
   }
   if (!operand_direct(d.B0, d.strideB, d.ldb, d.batch, 1)) {
     const long len = bmn ? d.n : d.k, lines = bmn ? d.k : d.n, pitch = round_up(len, 16);
-    void* w = workspace(WS_PACK_B, (size_t)(lines * pitch) * (size_t)d.batch, &e);
+    const size_t bytes = (size_t)(lines * pitch) * (size_t)d.batch;
+    if (beyond_memory(WS_PACK_B, len, bytes)) return cudaErrorNotSupported;
+    void* w = workspace(WS_PACK_B, bytes, &e);
     if (!w) return e;
     cb = LineCopy{d.B, d.ldb, lines, len, w, pitch};
     pb = &cb;

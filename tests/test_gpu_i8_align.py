@@ -52,3 +52,38 @@ def test_align_copies(ta, tb, m, n, k, pads, shifts):
             np.testing.assert_array_equal(host[a: a + size], X[b].reshape(-1))
             keep[a: a + size] = False
         assert np.all(host[keep] == 77)
+
+
+@pytest.mark.parametrize("ta,tb", [(0, 0), (1, 1)])
+def test_thin_operand_beyond_the_memory_left(ta, tb):
+    """Lines of 3 bytes grow to 16 in the copy: where that does not fit the memory left, the call still runs."""
+    import torch
+    import ssblasex_b200 as S
+    S.set_sync_mode(True)
+    S.set_math_mode(S.SSBLAS_MATH_PLAIN)
+    S.release_workspace()
+    torch.cuda.empty_cache()
+    thin, other, k, batch = 3, 16, 16384, 4200      # 206 MB of operand, 1.1 GB of copy
+    g = torch.Generator(device="cuda").manual_seed(3)
+    X = torch.randint(-128, 128, (batch, k, thin), generator=g, device="cuda", dtype=torch.int8)
+    Y = torch.randint(-128, 128, (batch, other, k), generator=g, device="cuda", dtype=torch.int8)   # read in place
+    C = torch.zeros((batch, other, thin) if ta == 0 else (batch, thin, other), dtype=torch.int32, device="cuda")
+    px = torch.arange(batch, device="cuda") * X.stride(0) + X.data_ptr()
+    py = torch.arange(batch, device="cuda") * Y.stride(0) + Y.data_ptr()
+    pc = torch.arange(batch, device="cuda") * (C.stride(0) * 4) + C.data_ptr()
+    one, zero = np.array([1], np.int32), np.array([0], np.int32)
+    # op(A) op(B) with the thin operand, 3 x 16384 with its rows contiguous, as op(A) = A or as op(B) = B^T
+    a, b, lda, ldb, m, n = (px, py, thin, k, thin, other) if ta == 0 else (py, px, k, thin, other, thin)
+    left = torch.cuda.mem_get_info()[0]
+    hold = torch.empty(left - (600 << 20), dtype=torch.uint8, device="cuda")
+    torch.cuda.synchronize()
+    st = S.lib().ssblasGemmBatchedEx(ta, tb, m, n, k, one.ctypes.data, a.data_ptr(), S.SSBLAS_R_8I, lda, b.data_ptr(),
+                                     S.SSBLAS_R_8I, ldb, zero.ctypes.data, pc.data_ptr(), S.SSBLAS_R_32I, m, batch, 0, 0)
+    path = S.last_run_info()["path"]
+    del hold
+    torch.cuda.empty_cache()
+    assert st == 0 and path == "simt"
+    for i in (0, 1, batch // 2, batch - 1):
+        want = Y[i].double() @ X[i].double()             # other x thin, whole numbers below 2^28
+        got = C[i].double()
+        assert torch.equal(got, want if ta == 0 else want.T)
