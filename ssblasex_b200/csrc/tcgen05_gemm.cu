@@ -10,6 +10,7 @@
 #include "internal.h"
 #include "prepass.h"
 #include "tc_gemm.cuh"
+#include "tile_rules.h"
 
 namespace ssb {
 namespace {
@@ -384,17 +385,8 @@ cudaError_t launch_i8_tcgen05(const BatchDesc& d, cudaStream_t st) {
   if (!is_sm100() || !encoder()) return cudaErrorNotSupported;
   if (d.k > (1L << 31) || d.m > (1L << 31) || d.n > (1L << 31)) return cudaErrorNotSupported;
   CUtensorMap ta, tb;
-  // 128 x 128 tiles (configuration 1) or 128 x 256 (0). The wide tile reads a third less shared memory per
-  // product and is the faster one where the products bound the call (8 x 4096^3: 2570 TOPS against
-  // 1890); where bytes do, the narrow one is, whose shorter epilogues leave the memory idle for less. The
-  // line lies at 240 operations per byte of operands and C, between the measured sides (ms, narrow
-  // and wide): 512 x 512^3 beta = 1 (102 per byte) 0.221, 0.257; beta = 0 (171) 0.136, 0.145;
-  // 16 x 1024^3 off the 16-byte grid (341) 0.0424, 0.0408; 8 x 4096^3 (1365) 0.583, 0.429. Few wide
-  // tiles also take the narrow form.
-  const double ops = 2.0 * d.m * d.n * d.k;
-  const double bytes = (double)d.m * d.k + (double)d.n * d.k + (d.beta_i ? 8.0 : 4.0) * d.m * d.n;
-  const long wide = ((d.m + 127) / 128) * ((d.n + 255) / 256) * d.batch;
-  const bool narrow = d.n <= 128 || ops < 240.0 * bytes || wide < num_sms();
+  // 128 x 128 tiles (configuration 1) or 128 x 256 (0)
+  const bool narrow = i8_narrow_tiles(d.m, d.n, d.k, d.batch, d.beta_i != 0, num_sms());
   const int BN = choose_config(SSBLAS_PATH_I8_TCGEN05, d.m, d.n, d.k, d.batch, narrow ? 1 : 0) == 1 ? 128 : 256;
   const bool amn = d.transa == SSBLAS_OP_N, bmn = d.transb == SSBLAS_OP_T;
   // operands with odd leading dimensions or bases, or unevenly spaced instances, are first copied onto
