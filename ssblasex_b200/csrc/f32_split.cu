@@ -377,11 +377,16 @@ __global__ void __launch_bounds__(kSplitThreads, 1) f32_split_kernel(const Split
   ptx::grid_dep_wait();
   ptx::grid_dep_launch();
   const uint32_t nkc_all = (uint32_t)((a.k + kKC - 1) / kKC);   // chunks of every tile of a batched launch
+  // a wait that all lanes of a warp pass or all give up, converged: what follows is the whole warp's
+  // (tensor-memory loads, __syncwarp)
+  auto wait_warp = [&](uint64_t* bar, uint32_t parity, int code) -> bool {
+    return __all_sync(0xffffffffu, ptx::mbar_wait(ptx::smem_u32(bar), parity, err, code, wl));
+  };
   // the worker's i-th tile: whether there is one (grouped: once its record has arrived)
   auto tile_ready = [&](uint32_t i, int code) -> bool {
     if constexpr (GROUPED) {
       const uint32_t q = i % kRing;
-      return ptx::mbar_wait(ptx::smem_u32(&ring_full[q]), (i / kRing) & 1, err, code, wl) && ring[q].valid;
+      return wait_warp(&ring_full[q], (i / kRing) & 1, code) && ring[q].valid;
     } else {
       return me + i * workers < a.total;
     }
@@ -455,7 +460,7 @@ __global__ void __launch_bounds__(kSplitThreads, 1) f32_split_kernel(const Split
       for (uint32_t kc = 0; kc < nkc; ++kc, ++c) {
         // the stage is waited for before the next copies are queued: behind them the answer would take
         // hundreds of cycles
-        if (!ptx::mbar_wait(ptx::smem_u32(&empty[s]), ((c / F::STAGES) & 1) ^ 1, err, 81, wl)) {
+        if (!wait_warp(&empty[s], ((c / F::STAGES) & 1) ^ 1, 81)) {
           ok = false;
           break;
         }
@@ -645,7 +650,7 @@ __global__ void __launch_bounds__(kSplitThreads, 1) f32_split_kernel(const Split
       if constexpr (!F::PROMOTE) {
         // one accumulator per tile: groups of columns straight from it to C
         const uint32_t buf = q % F::NACC;
-        if (!ptx::mbar_wait(ptx::smem_u32(&acc_full[buf]), (q / F::NACC) & 1, err, 85, wl)) break;
+        if (!wait_warp(&acc_full[buf], (q / F::NACC) & 1, 85)) break;
         ptx::tc_fence_after();
         if (active && gi - lane < m) {
 #pragma unroll 1
@@ -659,17 +664,19 @@ __global__ void __launch_bounds__(kSplitThreads, 1) f32_split_kernel(const Split
               raw[j / 16][j % 16] =
                   __float_as_uint(fmaf(__uint_as_float(raw[j / 16][j % 16]), alpha, read_c ? beta * cv[j] : 0.0f));
             if (read_c && g + G < cols) load_c(g + G);
-            float* cp = C + (long)g * ldc;
-            asm volatile("" : "+l"(cp));
-            if (!row_ok) continue;
-            if (cols >= g + G) {
+            if (row_ok) {
+              float* cp = C + (long)g * ldc;
+              asm volatile("" : "+l"(cp));
+              if (cols >= g + G) {
 #pragma unroll
-              for (int j = 0; j < G; ++j, cp += ldc) __stcs(cp, __uint_as_float(raw[j / 16][j % 16]));
-            } else {
+                for (int j = 0; j < G; ++j, cp += ldc) __stcs(cp, __uint_as_float(raw[j / 16][j % 16]));
+              } else {
 #pragma unroll
-              for (int j = 0; j < G; ++j, cp += ldc)
-                if (g + j < cols) __stcs(cp, __uint_as_float(raw[j / 16][j % 16]));
+                for (int j = 0; j < G; ++j, cp += ldc)
+                  if (g + j < cols) __stcs(cp, __uint_as_float(raw[j / 16][j % 16]));
+              }
             }
+            __syncwarp();   // the next group's tensor-memory loads are the whole warp's
           }
         }
         ptx::tc_fence_before();
@@ -683,7 +690,7 @@ __global__ void __launch_bounds__(kSplitThreads, 1) f32_split_kernel(const Split
       for (int j = 0; j < HALF / 2; ++j) sum[j] = 0;
       for (uint32_t p = 0; p < nkc_all; ++p, ++q) {
         const uint32_t buf = q % F::NACC;
-        if (!ptx::mbar_wait(ptx::smem_u32(&acc_full[buf]), (q / F::NACC) & 1, err, 85, wl)) {
+        if (!wait_warp(&acc_full[buf], (q / F::NACC) & 1, 85)) {
           ok = false;
           break;
         }
