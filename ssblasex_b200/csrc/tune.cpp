@@ -10,6 +10,7 @@
 #include <stdlib.h>
 #include <string.h>
 
+#include <array>
 #include <map>
 #include <mutex>
 #include <string>
@@ -22,7 +23,10 @@ namespace {
 std::mutex g_tune_mutex;
 bool g_loaded = false;
 int g_generation = 0;   // how often the table was read again
-std::map<std::pair<int, std::string>, int> g_table;
+// path and the four size classes, as numbers: each call looks its configuration up, and the text of a bucket
+// took longer to write than the rest of the lookup
+using Bucket = std::array<int, 5>;
+std::map<Bucket, int> g_table;
 constexpr int kKeys = 16;
 int g_forced[kKeys] = {-1, -1, -1, -1, -1, -1, -1, -1, -1, -1, -1, -1, -1, -1, -1, -1};
 
@@ -49,30 +53,27 @@ void load_table() {
   if (!f) return;
   char line[512];
   while (fgets(line, sizeof(line), f)) {
-    int path = -1, cfg = -1;
+    int path = -1, cfg = -1, end = 0;
     char bucket[128] = {0};
+    Bucket b;
     const char* p = strstr(line, "\"path\"");
     if (!p) continue;
     if (sscanf(p, "\"path\": %d, \"bucket\": \"%127[^\"]\", \"config\": %d", &path, bucket, &cfg) == 3 && path >= 0 &&
-        cfg >= 0)
-      g_table[{path, std::string(bucket)}] = cfg;
+        cfg >= 0 && sscanf(bucket, "m%dn%dk%db%d%n", &b[1], &b[2], &b[3], &b[4], &end) == 4 && bucket[end] == 0) {
+      b[0] = path;
+      g_table[b] = cfg;
+    }
   }
   fclose(f);
 }
 
 }  // namespace
 
-std::string size_bucket(long m, long n, long k, long batch) {
-  char b[64];
-  snprintf(b, sizeof(b), "m%dn%dk%db%d", clog2(m), clog2(n), clog2(k), clog2(batch));
-  return b;
-}
-
 int choose_config(int path, long m, long n, long k, long batch, int fallback) {
   std::lock_guard<std::mutex> lock(g_tune_mutex);
   if (path >= 0 && path < kKeys && g_forced[path] >= 0) return g_forced[path];
   if (!g_loaded) load_table();
-  auto it = g_table.find({path, size_bucket(m, n, k, batch)});
+  auto it = g_table.find(Bucket{path, clog2(m), clog2(n), clog2(k), clog2(batch)});
   return it != g_table.end() ? it->second : fallback;
 }
 
