@@ -14,10 +14,12 @@
 // accumulator only lives for one chunk of 32 k -- the small products first, then the two steps of
 // hi hi, the only truncations at full magnitude -- and the epilogue warps add the chunks in
 // registers, rounding to nearest. The ends of the range: both operands are scaled by 2^24 before they
-// are split (exact, and the lo part of the smallest subnormal is then a BF16 number; the tensor
-// core takes and gives subnormals), and every sum that is not finite (Inf and NaN operands,
-// |x| >= 2^104, sums of 2^80 and more), or is below 2^-100 and not zero, is computed again by a chain
-// of fused multiply-adds over the operands, so those behave as FP32 arithmetic does.
+// are split (exact, and the lo part of the smallest subnormal is then a BF16 number). Small results need
+// nothing else: a sum of 2^-149 is 2^-101 on the accumulator, whose parts down to 2^-24 of it are still ordinary
+// FP32 numbers, and it is rounded to FP32's own subnormals once, at the end. Where a sum is not finite (Inf
+// and NaN operands, |x| >= 2^104, sums of 2^80 and more) its block of 32 rows is left as it is, and computed
+// once the CTA's tiles are done by chains of fused multiply-adds over the operands, so those behave as FP32
+// arithmetic does (split_redo).
 //
 // Design: persistent CTAs over (instance, tile) items, K in chunks of 32:
 //   warps 8-15   converters: each thread copies its own 16-byte units of op(A) and op(B), two to four chunks
@@ -48,6 +50,7 @@
 #include "grouped.h"
 #include "internal.h"
 #include "ptx.cuh"
+#include "sgemm_load.cuh"
 
 namespace ssb {
 namespace {
@@ -57,10 +60,10 @@ constexpr int kConvThreads = 256;            // warps 8-15
 constexpr int kSplitThreads = 32 * 20;       // the last warpgroup's first warp issues the MMAs
 constexpr int kIssueRegs = 32;               // registers per thread of that warpgroup
 constexpr int kUnitRow = 16 * kConvThreads;  // bytes of one unit of every converter thread
-// Plain form: scale of the operands, of their sums, and the magnitude below which a sum that is not
-// zero is computed again
-constexpr float kScale = 0x1p24f, kUnscale = 0x1p-48f;
-constexpr uint32_t kSmallestBits = 0x0d800000u;   // 2^-100
+constexpr float kScale = 0x1p24f, kUnscale = 0x1p-48f;   // plain form: of the operands, and of their sums
+// Plain form: tiles of a worker per launch, a byte each for the blocks to compute again. (Launches of so many
+// tiles take 10 ms and more.)
+constexpr uint32_t kRedoTiles = 4096;
 
 // NP parts per operand, AR rows of op(A) (64 when m <= 64) and BN columns of op(B) converted per CTA and
 // chunk. PAIR: two CTAs (a cluster) share a 256 x 256 tile -- each converts 128 of its rows and 128 of its
@@ -111,7 +114,7 @@ struct SplitArgs {
   float* const* C;
   float alpha, beta;
   int a_mn, b_mn;          // op(A) rows / op(B) columns contiguous in memory
-  uint32_t tiles_m, tiles_mn, total;
+  uint32_t tiles_m, tiles_mn, first, total;   // of this launch: tiles [first, first + total)
   int* err;
   uint32_t wait_limit;
   int skip;                // injected fault: CTA 0 never signals its first chunk
@@ -125,7 +128,7 @@ struct SplitTile {
 };
 template <class F>
 __device__ __forceinline__ SplitTile split_tile(const SplitArgs& a, uint32_t t) {
-  const uint32_t b = t / a.tiles_mn, r = t - b * a.tiles_mn;
+  const uint32_t b = (a.first + t) / a.tiles_mn, r = a.first + t - b * a.tiles_mn;
   const uint32_t nt = r / a.tiles_m;
   return {b, (long)(r - nt * a.tiles_m) * F::TM, (long)nt * F::TN};
 }
@@ -278,40 +281,68 @@ __device__ __forceinline__ void split_store(uint32_t raw, uint32_t dst, bool mn,
   }
 }
 
-// One lane's row of C again, for the columns of the mask among 16 from `C` on: C <- alpha * acc + beta * C
-// with acc a chain of fused multiply-adds over the operands in k order, op(A)(i, k) = pa[k * ak],
-// op(B)(k, j) = pb[j * bc + k * bk]; columns from n on repeat column n - 1. Eight k are in flight at a time,
-// so that this rare path runs near the speed of an ordinary FP32 kernel.
-__device__ __noinline__ void split_redo(const float* pa, long ak, const float* pb, long bc, long bk, int n, int k,
-                                        uint32_t mask, float* C, long ldc, float alpha, float beta) {
-  float acc[16];
-#pragma unroll
-  for (int j = 0; j < 16; ++j) acc[j] = 0.f;
-  int kk = 0;
+// The flagged blocks of one tile again, by the 256 epilogue threads: C <- alpha * acc + beta * C with acc a chain
+// of fused multiply-adds in k order. Block w (bit w of `flags`) is what epilogue warp w left unwritten: rows
+// 32 (w % 4) of the CTA's ROWS from m0 on, columns HALF (w / 4) from n0 on. FFMA tiles of ROWS x 128 (64) in the
+// shared memory that the tensor-core pipeline no longer uses, slabs of 32 k, four in flight; a thread has 8 (4)
+// columns and rows in groups of four, 64 apart.
+// Measured (us, the whole call; before: a chain per output in the epilogue, a load for every product): all of C out of
+// range 16 x 1024^3 7710 -> 1130 (the FFMA kernels 800, in range 152), 200 x (200 x 200 x 300) 1960 -> 460 (243, 74);
+// an Inf in one row of each matrix 16 x 1024^3 4300 -> 645. With 4 columns a thread everywhere 1435.
+template <int ROWS, int HALF>
+__device__ __forceinline__ void split_redo(const SplitArgs& a, uint32_t b, long m0, long n0, uint32_t flags, float* sm) {
+  constexpr int BK = 32, ST = 4, NC = HALF < 64 ? 64 : 128, TM = ROWS / 16, TN = NC / 16, PA = ROWS + 4, PB = NC + 4;
+  const int lane = threadIdx.x % 32, warp = threadIdx.x / 32;
+  const int tx = (warp % 2) * 8 + lane % 8, ty = (warp / 2) * 4 + lane / 8;   // a warp: 8 (rows) x 4 (columns)
+  const float *A = a.A[b], *B = a.B[b];
+  const bool vecA = (uintptr_t)A % 16 == 0 && a.lda % 4 == 0, vecB = (uintptr_t)B % 16 == 0 && a.ldb % 4 == 0;
+  const int slabs = (int)((a.k + BK - 1) / BK);
 #pragma unroll 1
-  for (; kk + 8 <= k; kk += 8, pa += 8 * ak, pb += 8 * bk) {
-    float x[8];
+  for (int c0 = 0; c0 < 2 * HALF; c0 += NC) {
+    if (HALF == NC && ((flags >> (4 * (c0 / HALF))) & 0xfu) == 0) continue;
+    auto load = [&](int i) {
+      float* sa = sm + (i % ST) * BK * (PA + PB);
+      if (a.a_mn) sload<ROWS, BK, 256, true>(sa, A, a.m, a.k, a.lda, m0, (long)i * BK, vecA);
+      else sload<ROWS, BK, 256, false>(sa, A, a.m, a.k, a.lda, m0, (long)i * BK, vecA);
+      if (a.b_mn) sload<NC, BK, 256, true>(sa + BK * PA, B, a.n, a.k, a.ldb, n0 + c0, (long)i * BK, vecB);
+      else sload<NC, BK, 256, false>(sa + BK * PA, B, a.n, a.k, a.ldb, n0 + c0, (long)i * BK, vecB);
+    };
+    uint64_t acc2[TM / 2][TN] = {};
+#pragma unroll 1
+    for (int i = 0; i < ST - 1; ++i) {
+      if (i < slabs) load(i);
+      commit_s();
+    }
+#pragma unroll 1
+    for (int i = 0; i < slabs; ++i) {
+      wait_s<ST - 2>();
+      asm volatile("bar.sync 1, 256;" ::: "memory");
+      if (i + ST - 1 < slabs) load(i + ST - 1);
+      commit_s();
+      const float* sa = sm + (i % ST) * BK * (PA + PB);
+      const float* sb = sa + BK * PA;
+#pragma unroll 4
+      for (int kk = 0; kk < BK; ++kk) outer2<TM, TN, 64>(acc2, sa + kk * PA + 4 * tx, sb + kk * PB + TN * ty);
+    }
+    wait_s<0>();
+    asm volatile("bar.sync 1, 256;" ::: "memory");   // the next columns' copies reuse the buffers
+    float acc[TM][TN];
+    unpack_acc<TM, TN>(acc2, acc);
 #pragma unroll
-    for (int u = 0; u < 8; ++u) x[u] = __ldg(pa + u * ak);
+    for (int h = 0; h < TM / 4; ++h) {
+      const int row = 64 * h + 4 * tx, col = c0 + TN * ty;
+      if (!((flags >> (4 * (col / HALF) + row / 32)) & 1u)) continue;
+      float* C = a.C[b] + m0 + row + (n0 + col) * a.ldc;
 #pragma unroll
-    for (int j = 0; j < 16; ++j) {
-      const float* q = pb + (j < n ? j : n - 1) * bc;
-      float y[8];
+      for (int j = 0; j < TN; ++j)
 #pragma unroll
-      for (int u = 0; u < 8; ++u) y[u] = __ldg(q + u * bk);
-#pragma unroll
-      for (int u = 0; u < 8; ++u) acc[j] = fmaf(x[u], y[u], acc[j]);
+        for (int i = 0; i < 4; ++i)
+          if (m0 + row + i < a.m && n0 + col + j < a.n) {
+            float* p = C + i + j * a.ldc;
+            *p = fmaf(acc[4 * h + i][j], a.alpha, a.beta != 0.0f ? a.beta * *p : 0.0f);
+          }
     }
   }
-#pragma unroll 1
-  for (; kk < k; ++kk, pa += ak, pb += bk) {
-    const float x = __ldg(pa);
-#pragma unroll
-    for (int j = 0; j < 16; ++j) acc[j] = fmaf(x, __ldg(pb + (j < n ? j : n - 1) * bc), acc[j]);
-  }
-#pragma unroll
-  for (int j = 0; j < 16; ++j)
-    if ((mask >> j) & 1u) C[j * ldc] = fmaf(acc[j], alpha, beta != 0.0f ? beta * C[j * ldc] : 0.0f);
 }
 
 // GROUPED: the tiles, their shapes and scalars come from a.recs. What bounds it on mixed small shapes (8 to 512
@@ -333,6 +364,7 @@ __global__ void __launch_bounds__(kSplitThreads, 1) f32_split_kernel(const Split
   uint64_t* ring_empty = ring_full + kRing;                      // [kRing] record read (17 warps)
   uint32_t* tmem_slot = (uint32_t*)(ring_empty + kRing);
   SplitItem* ring = (SplitItem*)((uint8_t*)full + 512);
+  uint32_t* redo = (uint32_t*)((uint8_t*)full + 512);            // plain form: a byte per tile of this worker
   static_assert((2 * F::STAGES + 2 * F::NACC + 1 + 2 * kRing) * 8 + 4 <= 512, "barrier area");
 
   const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
@@ -359,6 +391,10 @@ __global__ void __launch_bounds__(kSplitThreads, 1) f32_split_kernel(const Split
       }
     }
     ptx::fence_mbar_init();
+  }
+  if constexpr (F::PROMOTE) {
+    const uint32_t mine = (a.total - me + workers - 1) / workers;   // (a worker has a tile at least)
+    for (uint32_t i = threadIdx.x; i < (mine + 3) / 4; i += kSplitThreads) redo[i] = 0;
   }
   if (warp == 16) {
     if constexpr (F::PAIR) {
@@ -715,57 +751,47 @@ __global__ void __launch_bounds__(kSplitThreads, 1) f32_split_kernel(const Split
 #pragma unroll
       for (int j = 0; j < HALF / 2; ++j)
         unpack2(mul2(sum[j], pack2(kUnscale, kUnscale)), acc[2 * j], acc[2 * j + 1]);
-      // sums to compute again: not finite, or below the smallest and not zero (2 bits - 1
-      // drops the sign and wraps zero to the largest value)
-      constexpr uint32_t LO = 2u * kSmallestBits - 1u;
-      uint32_t low = 0xffffffffu;
       float high = 0.f;
 #pragma unroll
-      for (int j = 0; j < HALF; ++j) {
-        low = min(low, 2u * __float_as_uint(acc[j]) - 1u);
-        asm("max.NaN.f32 %0, %0, %1;" : "+f"(high) : "f"(fabsf(acc[j])));
+      for (int j = 0; j < HALF; ++j) asm("max.NaN.f32 %0, %0, %1;" : "+f"(high) : "f"(fabsf(acc[j])));
+      if (__any_sync(0xffffffffu, row_ok && cols > 0 && !(high < INFINITY))) {
+        if (lane == 0) atomicOr(&redo[i / 4], 1u << (8 * (i % 4) + warp));
+        continue;
       }
-      const bool redo = __any_sync(0xffffffffu, row_ok && (low < LO || !(high < INFINITY)));
-      if (!redo) {
 #pragma unroll
-        for (int g = 0; g < HALF; g += G) {
-          if (!EARLY_C && read_c) load_c(g);
-          float* cp = C + (long)g * ldc;
-          asm volatile("" : "+l"(cp));
+      for (int g = 0; g < HALF; g += G) {
+        if (!EARLY_C && read_c) load_c(g);
+        float* cp = C + (long)g * ldc;
+        asm volatile("" : "+l"(cp));
 #pragma unroll
-          for (int j = 0; j < G; ++j) acc[g + j] = fmaf(acc[g + j], alpha, read_c ? beta * cv[j] : 0.0f);
-          if (!row_ok) continue;
-          if (cols == HALF) {
+        for (int j = 0; j < G; ++j) acc[g + j] = fmaf(acc[g + j], alpha, read_c ? beta * cv[j] : 0.0f);
+        if (!row_ok) continue;
+        if (cols == HALF) {
 #pragma unroll
-            for (int j = 0; j < G; ++j, cp += ldc) __stcs(cp, acc[g + j]);
-          } else {
+          for (int j = 0; j < G; ++j, cp += ldc) __stcs(cp, acc[g + j]);
+        } else {
 #pragma unroll
-            for (int j = 0; j < G; ++j, cp += ldc)
-              if (g + j < cols) __stcs(cp, acc[g + j]);
-          }
-        }
-      } else if (row_ok) {
-        // the sound columns, then the others
-        uint32_t mask[HALF / 32] = {};
-#pragma unroll
-        for (int j = 0; j < HALF; ++j) {
-          if (j >= cols) break;
-          if (2u * __float_as_uint(acc[j]) - 1u < LO || !(fabsf(acc[j]) < INFINITY)) {
-            mask[j / 32] |= 1u << (j % 32);
-          } else {
-            float* cp = C + (long)j * ldc;
-            *cp = fmaf(acc[j], alpha, read_c ? beta * *cp : 0.0f);
-          }
-        }
-        const float* pa = a.A[b] + (a.a_mn ? gi : gi * a.lda);
-        const float* pb = a.B[b] + (a.b_mn ? gj0 : gj0 * a.ldb);
-        const long ak = a.a_mn ? a.lda : 1, bc = a.b_mn ? 1 : a.ldb, bk = a.b_mn ? a.ldb : 1;
-#pragma unroll
-        for (int g = 0; g < HALF; g += 16) {
-          const uint32_t mk = (mask[g / 32] >> (g % 32)) & 0xffffu;
-          if (mk) split_redo(pa, ak, pb + g * bc, bc, bk, cols - g, (int)a.k, mk, C + (long)g * ldc, ldc, alpha, beta);
+          for (int j = 0; j < G; ++j, cp += ldc)
+            if (g + j < cols) __stcs(cp, acc[g + j]);
         }
       }
+    }
+    if constexpr (F::PROMOTE) {
+      // (inside this branch, whose registers the FFMA tiles need) every other warp has arrived here when no
+      // copy or MMA is in flight in this CTA's shared memory any more, and none of them waits with a limit
+      asm volatile("bar.sync 2, %0;" ::"n"(kSplitThreads) : "memory");
+      for (uint32_t i = 0; me + i * workers < a.total; ++i) {
+        const uint32_t flags = (redo[i / 4] >> (8 * (i % 4))) & 0xffu;
+        if (!flags) continue;
+        const SplitTile ti = split_tile<F>(a, me + i * workers);
+        split_redo<F::AR, F::TN / 2>(a, ti.b, ti.m0 + rank * 128, ti.n0, flags, (float*)stages);
+      }
+    }
+  }
+  if constexpr (F::PROMOTE) {
+    if (warp >= 8) {
+      __syncwarp();
+      asm volatile("bar.arrive 2, %0;" ::"n"(kSplitThreads) : "memory");
     }
   }
   ptx::tc_fence_before();
@@ -789,7 +815,7 @@ cudaError_t launch_tiles(SplitArgs a, const char* name, cudaStream_t st) {
     a.wait_limit = 1u << 10;
   }
   auto kern = f32_split_kernel<F, GROUPED>;
-  constexpr int smem = F::SMEM + (GROUPED ? kRing * (int)sizeof(SplitItem) : 0);
+  constexpr int smem = F::SMEM + (GROUPED ? kRing * (int)sizeof(SplitItem) : F::PROMOTE ? (int)kRedoTiles : 0);
   static_assert(smem <= 232448, "shared memory");
   static bool attr[kMaxDevices] = {};
   if (cudaError_t e = smem_attr_once(attr, kern, smem)) return e;
@@ -828,8 +854,14 @@ cudaError_t launch_split(const BatchDesc& d, cudaStream_t st) {
   const long tm = (d.m + F::TM - 1) / F::TM, tn = (d.n + F::TN - 1) / F::TN;
   a.tiles_m = (uint32_t)tm;
   a.tiles_mn = (uint32_t)(tm * tn);
-  a.total = (uint32_t)(tm * tn * d.batch);
-  return launch_tiles<F, false>(a, F::NP == 3 ? "f32_split" : "bf16x3_split", st);
+  const long all = tm * tn * d.batch, most = F::PROMOTE ? (long)kRedoTiles * (num_sms() / (F::PAIR ? 2 : 1)) : all;
+  for (long t = 0; t < all; t += most) {
+    a.first = (uint32_t)t;
+    a.total = (uint32_t)(all - t < most ? all - t : most);
+    const cudaError_t e = launch_tiles<F, false>(a, F::NP == 3 ? "f32_split" : "bf16x3_split", st);
+    if (e != cudaSuccess) return e;
+  }
+  return cudaSuccess;
 }
 
 template <int NP>

@@ -175,3 +175,88 @@ def test_skipped_chunk_is_reported(S):
     C = run(S, p)
     ex, nrm = O.exact_f64(p, 0)
     assert np.all(np.abs(p.c_view(C, 0).astype(np.float64) - ex) <= (200 / 32 + 8) * U * nrm)
+
+
+# one shape for each form of the kernel: 64 x 64, 128 x 64, 128 x 128 tiles, and 256 x 256 by a pair of CTAs
+FORMS = {"64x64": (60, 50, 140, 3), "128x64": (120, 150, 140, 2), "128x128": (125, 127, 256, 140), "pair": (250, 255, 1000, 70)}
+
+
+@pytest.mark.parametrize("form", list(FORMS))
+@pytest.mark.parametrize("ta,tb,pad", [(0, 0, 1), (0, 1, 0), (1, 0, 4), (1, 1, 3)])
+@pytest.mark.parametrize("beta", [0.0, 0.25])
+def test_out_of_range_in_every_form(S, form, ta, tb, pad, beta):
+    """Inf, NaN, huge operands and sums that overflow on the scaled accumulators, in the first and the last rows and
+    columns of a tile and in between: what an FFMA kernel gives, and the rest within the FP32 bound. C is read once,
+    and nothing past the matrices is written."""
+    m, n, k, batch = FORMS[form]
+    p = problem(ta, tb, m, n, k, batch, beta, (pad, pad, pad), 7 + m)
+    last = batch - 1
+    for b in (0, last):
+        opa, opb = p.op_a(b), p.op_b(b)
+        opa[1, 3] = np.inf
+        opa[m - 1, k - 1] = -np.inf
+        opa[m // 2, :] *= np.float32(2.0 ** 90)          # sums beyond 2^80, finite
+        opb[k // 2, n - 1] = np.nan
+        if b == last:
+            opa[40, :] *= np.float32(2.0 ** 105)         # operands beyond 2^104
+            opb[5, n // 2] = np.inf
+            opa[17, 5] = 0.0                             # Inf * 0
+    C = run(S, p)
+    S.set_kernel_config("simt", 3)
+    try:
+        R = run(S, p)
+    finally:
+        S.set_kernel_config("simt", -1)
+    for b in sorted({0, 1, last}):
+        got, ref = p.c_view(C, b).astype(np.float64), p.c_view(R, b).astype(np.float64)
+        np.testing.assert_array_equal(np.isnan(got), np.isnan(ref))
+        ok = np.isfinite(ref)
+        np.testing.assert_array_equal(got[~ok & ~np.isnan(ref)], ref[~ok & ~np.isnan(ref)])
+        A, B = (np.where(np.isfinite(x), x, 0.0).astype(np.float64) for x in (p.op_a(b), p.op_b(b)))
+        C0 = beta * p.c_view(p.C, b).astype(np.float64)
+        ex, nrm = 0.75 * (A @ B) + C0, 0.75 * (np.abs(A) @ np.abs(B)) + np.abs(C0)
+        assert np.all(np.abs(got - ex)[ok] <= (4 * k * U * nrm)[ok])
+    np.testing.assert_array_equal(C.reshape(batch, n, -1)[:, :, m:], p.C.reshape(batch, n, -1)[:, :, m:])
+
+
+@pytest.mark.parametrize("form", list(FORMS))
+@pytest.mark.parametrize("ea,eb", [(-50, -52), (-60, -64), (-66, -70), (-72, -76), (30, -135), (100, -140)])
+def test_small_results(S, form, ea, eb):
+    """Results down to FP32's smallest subnormal, and subnormal operands, on the tensor cores: the plain bound, and
+    two roundings to FP32's subnormals (half of 2^-149 each) for the sum and for alpha."""
+    m, n, k, batch = FORMS[form]
+    p = problem(0, 0, m, n, k, batch, 0.0, (0, 0, 0), 3 + m)
+    p.A *= np.float32(2.0) ** np.float32(ea)
+    p.B[:] = np.ldexp(p.B.astype(np.float64), eb).astype(np.float32)
+    C = run(S, p)
+    assert S.last_run_info()["path"] == "f32_tcgen05"
+    for b in (0, batch - 1):
+        ex, nrm = O.exact_f64(p, b)
+        err = np.abs(p.c_view(C, b).astype(np.float64) - ex)
+        assert np.all(err <= (k / 32 + 8) * U * nrm + 2.0 ** -149)
+
+
+@pytest.mark.parametrize("ta,tb", [(0, 0), (1, 1)])
+def test_more_tiles_than_one_launch_holds(S, ta, tb):
+    """A launch holds 4096 tiles per worker; the tiles of the next launch go on where it ended, also those that
+    are computed again."""
+    m, n, k, batch = 1, 1, 128, 4096 * 148 + 300
+    import torch
+    g = torch.Generator(device="cuda").manual_seed(5)
+    A, B = (torch.rand((batch, k), generator=g, device="cuda") * 2 - 1 for _ in range(2))
+    bad = [0, 147, 148, 4096 * 148 - 1, 4096 * 148, batch - 1]
+    A[bad, 5] = 1e30
+    C = torch.full((batch,), float("nan"), device="cuda")
+    ptrs = [t.data_ptr() + torch.arange(batch, device="cuda") * (4 * s) for t, s in ((A, k), (B, k), (C, 1))]
+    al, be = np.array([1.0], np.float32), np.array([0.0], np.float32)
+    st = S.lib().ssblasGemmBatchedEx(ta, tb, m, n, k, al.ctypes.data, ptrs[0].data_ptr(), S.SSBLAS_R_32F, k if ta else 1,
+                                     ptrs[1].data_ptr(), S.SSBLAS_R_32F, 1 if tb else k, be.ctypes.data,
+                                     ptrs[2].data_ptr(), S.SSBLAS_R_32F, 1, batch, 0, 0)
+    info = S.last_run_info()
+    assert st == 0 and info["path"] == "f32_tcgen05" and info["kernel_launches"] == 2
+    ex, nrm = (A.double() * B.double()).sum(1), (A.double() * B.double()).abs().sum(1)
+    err = (C.double() - ex).abs()
+    plain = torch.ones(batch, dtype=torch.bool, device="cuda")
+    plain[bad] = False
+    assert bool((err <= (k / 32 + 8) * U * nrm)[plain].all())
+    assert bool((err <= 4 * k * U * nrm)[~plain].all())
