@@ -1,8 +1,8 @@
 // FP32 batched GEMM on the BF16 tensor cores (tcgen05.mma kind::f16), the operands split into BF16
 // parts inside the kernel. Two forms of the fp32 row share it:
 //   plain (NP = 3)    x = hi + mid + lo exactly (8 + 8 + 8 significand bits), six products
-//                     hi hi, hi mid, mid hi, mid mid, hi lo, lo hi: what is left out is below
-//                     2^-25 of a product, so the result is an FP32 GEMM's;
+//                     hi hi, hi mid, mid hi, mid mid, hi lo, lo hi: what is left out (mid lo and lo
+//                     mid, each up to 2^-25) is at most 2^-24 of a product;
 //   3xBF16 (NP = 2)   x ~ hi + lo, three products (the emulation mode of the fp32 row).
 // Semantics follow the reference (hirokitokura/ssblasEx): C <- beta*C, not read when beta == 0
 // (src/include/CScale/Xgemm_scale_kernel.hpp:164-176), then C <- C + acc*alpha with one fused
@@ -10,10 +10,16 @@
 //
 // Accuracy of the plain form. The tensor core adds a K step of 16 products and the accumulator
 // exactly enough, but truncates the sum to FP32: over a long K that bias would exceed the error of a
-// chain of fused multiply-adds (k = 1024, U[-1,1): 1.25e-6 against 5.6e-7 of the 2-norm). So an
-// accumulator only lives for one chunk of 32 k -- the small products first, then the two steps of
-// hi hi, the only truncations at full magnitude -- and the epilogue warps add the chunks in
-// registers, rounding to nearest. The ends of the range: both operands are scaled by 2^24 before they
+// chain of fused multiply-adds (k = 1024, U[-1,1): 1.25e-6 against 5.6e-7 of the 2-norm), and where a
+// result is one product, or a few, it would be twice the chain's. So hi hi, whose products have 16 bits, is
+// accumulated for one chunk of 32 k only, and the epilogue warps add the chunks in registers, rounding to
+// nearest; the smaller products, at most 2^-7 of the magnitudes' sum, have an accumulator of their own for up to
+// 32 chunks, which truncates at their magnitude. Measured, 2-norm of the error over that of the result in u =
+// 2^-24, a chain / this / all six products in the chunk's accumulator: k = 1024, U[-1,1) 9.6 / 1.9 / 2.0; with 1% of
+// outliers 3.3 / 1.9 / 1.9; one nonzero per row 0.42 / 0.43 / 0.76 (the largest error of a product 1.0 / 1.5 / 2.4 u);
+// two 0.52 / 0.44 / 0.88; four 0.67 / 0.45 / 1.0; four between 2^-12 and 2^12 0.68 / 0.71 / 1.0. With mid lo and lo
+// mid as well, one nonzero per row has the chain's error, and 16 x 1024^3 takes 185 us instead of 156.
+// The ends of the range: both operands are scaled by 2^24 before they
 // are split (exact, and the lo part of the smallest subnormal is then a BF16 number). Small results need
 // nothing else: a sum of 2^-149 is 2^-101 on the accumulator, whose parts down to 2^-24 of it are still ordinary
 // FP32 numbers, and it is rounded to FP32's own subnormals once, at the end. Where a sum is not finite (Inf
@@ -34,12 +40,13 @@
 // 128 of its rows and 128 of its columns, half as much per product as alone, and arrives on the leader's
 // barriers. Operands cross HBM once as fp32 and no plane is written back: the operands of a tile are split
 // again for every tile that shares them, which is cheaper than the 10 bytes per element of a split pass.
-// What bounds it (16 x 1024^3 plain, a pair's chunk of 1940 cycles): the 128 B per cycle of shared memory
+// What bounds it (16 x 1024^3 plain, a pair's chunk of 1820 cycles): the 128 B per cycle of shared memory
 // (units in and out 64 KB, parts in 48 KB, 12 MMAs reading 96 KB: 1660 cycles; the MMAs alone 1540). With
 // the units in registers, as before, the wait for a stage queued behind the loads and a chunk of a 128 x 128
 // tile took 1850 cycles; so did one of a pair while its arrivals asked for a cluster-wide release.
-// Measured (ms, FFMA kernels -> this one): 16 x 1024^3 NN 0.829 -> 0.166 (207 TFLOP/s); 4 x 2048^3 1.73 ->
-// 0.297; 64 x 128^3 NN 0.0145 -> 0.0125; 8 x (777 x 555 x 333) 0.103 -> 0.041; 2 x 128^2 x 4096 0.19 -> 0.094.
+// Measured in short bursts (us, FFMA kernels -> this one): 16 x 1024^3 NN 802 -> 154 (223 TFLOP/s; back to back
+// 165); 4 x 2048^3 1730 -> 305; 64 x 128^3 NN, beta = 0.5 16.7 -> 12; 200 x (200 x 200 x 300) TT, beta = 1 243 -> 73;
+// 2 x 128^2 x 4096 190 -> 99.
 // 3xBF16 (split pass and tiled GEMM -> this kernel): 256 x 256^3 0.130 -> 0.039, 16 x 1024^3 0.096; a grouped
 // call's 5000 instances of 8 to 512 each way 0.564 -> 0.39.
 #include <cuda_bf16.h>
@@ -58,12 +65,12 @@ namespace {
 constexpr int kKC = 32;                      // K elements per chunk
 constexpr int kConvThreads = 256;            // warps 8-15
 constexpr int kSplitThreads = 32 * 20;       // the last warpgroup's first warp issues the MMAs
-constexpr int kIssueRegs = 32;               // registers per thread of that warpgroup
 constexpr int kUnitRow = 16 * kConvThreads;  // bytes of one unit of every converter thread
 constexpr float kScale = 0x1p24f, kUnscale = 0x1p-48f;   // plain form: of the operands, and of their sums
 // Plain form: tiles of a worker per launch, a byte each for the blocks to compute again. (Launches of so many
 // tiles take 10 ms and more.)
 constexpr uint32_t kRedoTiles = 4096;
+constexpr uint32_t kSumChunks = 32;               // plain form: chunks of one accumulator of the smaller products
 
 // NP parts per operand, AR rows of op(A) (64 when m <= 64) and BN columns of op(B) converted per CTA and
 // chunk. PAIR: two CTAs (a cluster) share a 256 x 256 tile -- each converts 128 of its rows and 128 of its
@@ -82,17 +89,26 @@ struct Split {
   static constexpr int RAW = RAW_STAGE > 24 * 1024 ? (NP == 3 ? 2 : 3) : 4;
   static constexpr int STAGES = (224 * 1024 - RAW * RAW_STAGE) / STAGE > 6 ? 6 : (224 * 1024 - RAW * RAW_STAGE) / STAGE;
   static constexpr int TM = PAIR ? 256 : 128, TN = PAIR ? 2 * BN : BN;   // the tile
-  static constexpr int NACC = PAIR ? 2 : 4;  // accumulators in flight, TN columns each
-  static constexpr int TMEM_COLS = NACC * TN;
   static constexpr bool PROMOTE = NP == 3;
-  // registers of the converters and epilogue warps: 640 threads x 96 at launch = 61,440 = 256 x (conv +
-  // epilogue) + 128 x 32; the plain form's epilogue holds a sum per output, 128 a thread in a pair
-  static constexpr int CONV_REGS = PAIR && PROMOTE ? 56 : 104, EPI_REGS = 224 - CONV_REGS;
+  // accumulators in flight, TN columns each: NACC of a tile (3xBF16), or of a chunk's hi hi (plain), where NSUM more
+  // hold the smaller products. A pair's single ones cost nothing, since the smaller products of the next chunk run
+  // while hi hi is read; a 128 x 128 tile has three, so that the next tile is under way during this one's end
+  // (two and two: 100 x 256^3 31 -> 33 us, 74 x (256 x 256 x 128) 15.0 -> 15.7).
+  static constexpr int NACC = PROMOTE ? (PAIR ? 1 : TN == 128 ? 3 : 6) : PAIR ? 2 : 4;
+  static constexpr int NSUM = !PROMOTE ? 0 : TN == 64 ? 2 : 1;
+  static constexpr int TMEM_COLS = (NACC + NSUM) * TN;
+  // registers per thread: 640 threads x 96 at launch = 61,440 for 256 converters, 256 epilogue threads (the
+  // plain form's hold a sum per output, 128 a thread in a pair) and the 128 of the issuing warp's warpgroup (32
+  // made that warp's loop of the plain form spill: 2 x 128^2 x 4096 101 -> 107 us)
+  static constexpr int ISSUE_REGS = PROMOTE && !PAIR ? 40 : 32;
+  static constexpr int CONV_REGS = !PROMOTE ? 104 : PAIR ? 56 : TN == 128 ? 80 : 104;
+  static constexpr int EPI_REGS = (ISSUE_REGS > 32 ? 216 : 224) - CONV_REGS;
   // the MMA reads 128 rows of every A part: with AR = 64 the upper 64 come from whatever follows
   // (within the stage, since B follows A), and their products are never read
   static constexpr int SMEM = 1024 + STAGES * STAGE + RAW * RAW_STAGE + 512;
-  static_assert(STAGE % 1024 == 0 && NP * B_PLANE >= 4096 && SMEM <= 232448 && TMEM_COLS <= 512, "stages");
-  static_assert(256 * (CONV_REGS + EPI_REGS) + 128 * kIssueRegs <= kSplitThreads * 96, "registers");
+  static_assert(STAGE % 1024 == 0 && NP * B_PLANE >= 4096 && SMEM <= 232448, "stages");
+  static_assert(TMEM_COLS == 256 || TMEM_COLS == 512, "tensor memory comes in powers of two");
+  static_assert(256 * (CONV_REGS + EPI_REGS) + 128 * ISSUE_REGS <= kSplitThreads * 96, "registers");
 };
 
 // One tile of a grouped launch as a worker's warps see it: its record and its instance's matrices. A
@@ -309,16 +325,14 @@ __device__ __forceinline__ void split_redo(const SplitArgs& a, uint32_t b, long 
     };
     uint64_t acc2[TM / 2][TN] = {};
 #pragma unroll 1
-    for (int i = 0; i < ST - 1; ++i) {
-      if (i < slabs) load(i);
-      commit_s();
-    }
-#pragma unroll 1
-    for (int i = 0; i < slabs; ++i) {
-      wait_s<ST - 2>();
-      asm volatile("bar.sync 1, 256;" ::: "memory");
+    for (int i = 1 - ST; i < slabs; ++i) {     // (the loads once in the code)
+      if (i >= 0) {
+        wait_s<ST - 2>();
+        asm volatile("bar.sync 1, 256;" ::: "memory");
+      }
       if (i + ST - 1 < slabs) load(i + ST - 1);
       commit_s();
+      if (i < 0) continue;
       const float* sa = sm + (i % ST) * BK * (PA + PB);
       const float* sb = sa + BK * PA;
 #pragma unroll 4
@@ -350,7 +364,7 @@ __device__ __forceinline__ void split_redo(const SplitArgs& a, uint32_t b, long 
 // whole or not: a second group of converter warps (which took them below 64 registers) made it 1.8 times
 // as long, so the units of rows outside the matrix are left out instead (0.403 -> 0.390 ms).
 template <class F, bool GROUPED>
-__global__ void __launch_bounds__(kSplitThreads, 1) f32_split_kernel(const SplitArgs a) {
+__global__ void __launch_bounds__(kSplitThreads, 1) f32_split_kernel(const SplitArgs a, const SplitArgs again) {
   static_assert(!GROUPED || (!F::PAIR && !F::PROMOTE), "grouped launches: 3xBF16, one CTA per tile");
   extern __shared__ uint8_t smem_raw[];
   uint8_t* stages = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
@@ -359,13 +373,14 @@ __global__ void __launch_bounds__(kSplitThreads, 1) f32_split_kernel(const Split
   uint64_t* empty = full + F::STAGES;                            // parts read by the MMAs (commit)
   uint64_t* acc_full = empty + F::STAGES;                        // [NACC] sums complete (commit)
   uint64_t* acc_empty = acc_full + F::NACC;                      // [NACC] sums read (8 warps)
-  uint64_t* drain = acc_empty + F::NACC;
+  uint64_t* sum_empty = acc_empty + F::NACC;                     // [NSUM] smaller products read (8 warps)
+  uint64_t* drain = sum_empty + F::NSUM;
   uint64_t* ring_full = drain + 1;                               // [kRing] record written (scheduler)
   uint64_t* ring_empty = ring_full + kRing;                      // [kRing] record read (17 warps)
   uint32_t* tmem_slot = (uint32_t*)(ring_empty + kRing);
   SplitItem* ring = (SplitItem*)((uint8_t*)full + 512);
   uint32_t* redo = (uint32_t*)((uint8_t*)full + 512);            // plain form: a byte per tile of this worker
-  static_assert((2 * F::STAGES + 2 * F::NACC + 1 + 2 * kRing) * 8 + 4 <= 512, "barrier area");
+  static_assert((2 * F::STAGES + 2 * F::NACC + F::NSUM + 1 + 2 * kRing) * 8 + 4 <= 512, "barrier area");
 
   const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
   const uint32_t wl = a.wait_limit ? a.wait_limit : ptx::kWaitLimit;
@@ -383,6 +398,7 @@ __global__ void __launch_bounds__(kSplitThreads, 1) f32_split_kernel(const Split
       ptx::mbar_init(ptx::smem_u32(&acc_full[q]), 1);
       ptx::mbar_init(ptx::smem_u32(&acc_empty[q]), CT * 8);
     }
+    for (int q = 0; q < F::NSUM; ++q) ptx::mbar_init(ptx::smem_u32(&sum_empty[q]), CT * 8);
     ptx::mbar_init(ptx::smem_u32(drain), 1);
     if (GROUPED) {
       for (uint32_t q = 0; q < kRing; ++q) {
@@ -518,7 +534,7 @@ __global__ void __launch_bounds__(kSplitThreads, 1) f32_split_kernel(const Split
     asm volatile("cp.async.wait_group 0;" ::: "memory");   // no copy is in flight when the CTA exits
   } else if (warp >= 16) {
     // ------------------------------------------------------------------ MMA ---------------
-    asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kIssueRegs));
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(F::ISSUE_REGS));
     if (warp == 16 && rank == 0) {
       // descriptors of stage 0's first part, and their step along K: 16 k are 32 bytes of a K-major
       // line, 16 lines of an MN-major block (addresses count 16 bytes). The whole warp runs the loop
@@ -527,7 +543,7 @@ __global__ void __launch_bounds__(kSplitThreads, 1) f32_split_kernel(const Split
       const uint32_t lead = ptx::elect_one();
       const uint32_t st0 = ptx::smem_u32(stages);
       static_assert(kKC == 32, "two K steps per chunk");
-      uint32_t c = 0, q = 0;     // chunks, accumulators
+      uint32_t c = 0, q = 0, sq = 0;   // chunks, accumulators, accumulators of the smaller products
       bool ok = true;
       auto commit = [&](uint64_t* bar) {
         if constexpr (F::PAIR) ptx::mma_commit_pair_if(lead, ptx::smem_u32(bar));
@@ -547,38 +563,57 @@ __global__ void __launch_bounds__(kSplitThreads, 1) f32_split_kernel(const Split
         const uint64_t a0 = amn ? ptx::smem_desc_mnmajor(st0, kKC * 128) : ptx::smem_desc_kmajor(st0, 64);
         const uint64_t b0 = bmn ? ptx::smem_desc_mnmajor(st0 + F::NP * F::A_PLANE, kKC * 128)
                                 : ptx::smem_desc_kmajor(st0 + F::NP * F::A_PLANE, 64);
-        const uint64_t ka = amn ? 128 : 2, kb = bmn ? 128 : 2;
+        const uint32_t ka = amn ? 128 : 2, kb = bmn ? 128 : 2;
         for (uint32_t kc = 0; kc < nkc; ++kc, ++c) {
           const uint32_t s = c % F::STAGES;
-          if (F::PROMOTE || kc == 0) {
-            if (!ptx::mbar_wait(ptx::smem_u32(&acc_empty[q % F::NACC]), ((q / F::NACC) & 1) ^ 1, err, 82, wl)) {
-              ok = false;
-              break;
-            }
+          // (plain: the smaller products have accumulators of their own, read once in kSumChunks; the one
+          // accumulator of a pair for hi hi is waited for behind them)
+          bool free = true;
+          if (F::PROMOTE && kc % kSumChunks == 0)
+            free = ptx::mbar_wait(ptx::smem_u32(&sum_empty[sq % (F::PROMOTE ? F::NSUM : 1)]),
+                                  ((sq / (F::PROMOTE ? F::NSUM : 1)) & 1) ^ 1, err, 86, wl);
+          if (F::PROMOTE ? F::NACC > 1 : kc == 0)
+            free = free && ptx::mbar_wait(ptx::smem_u32(&acc_empty[q % F::NACC]), ((q / F::NACC) & 1) ^ 1, err, 82, wl);
+          if (!free) {
+            ok = false;
+            break;
           }
           if (!ptx::mbar_wait(ptx::smem_u32(&full[s]), (c / F::STAGES) & 1, err, 83, wl)) {
             ok = false;
             break;
           }
           ptx::tc_fence_after();
+          // (the low words: the addresses in them do not carry into the high ones)
+          const uint32_t sa = (uint32_t)a0 + s * (uint32_t)(F::STAGE >> 4), sb = (uint32_t)b0 + s * (uint32_t)(F::STAGE >> 4);
+          auto word = [](uint32_t lo, uint64_t base) { return (base & 0xffffffff00000000ull) | lo; };
           const uint32_t d = tmem + (q % F::NACC) * F::TN;
-          const uint64_t sa = a0 + (uint64_t)(s * (uint32_t)(F::STAGE >> 4)), sb = b0 + (uint64_t)(s * (uint32_t)(F::STAGE >> 4));
-          uint32_t acc = F::PROMOTE || kc == 0 ? 0u : 1u;
+          const uint32_t ds = F::PROMOTE ? tmem + (F::NACC + sq % (F::PROMOTE ? F::NSUM : 1)) * F::TN : d;
+          uint32_t acc = (F::PROMOTE ? kc % kSumChunks : kc) == 0 ? 0u : 1u;
           // smallest products first
 #pragma unroll
-          for (int sum = F::NP - 1; sum >= 0; --sum)
+          for (int sum = F::NP - 1; sum >= 0; --sum) {
+            if (F::PROMOTE && sum == 0) {
+              if constexpr (F::NACC == 1) {
+                if (!ptx::mbar_wait(ptx::smem_u32(&acc_empty[0]), (q & 1) ^ 1, err, 82, wl)) ok = false;
+                ptx::tc_fence_after();
+              }
+              acc = 0u;
+            }
 #pragma unroll
             for (int p = 0; p <= sum; ++p) {
-              const uint64_t ad = sa + (uint64_t)(p * (F::A_PLANE >> 4)), bd = sb + (uint64_t)((sum - p) * (F::B_PLANE >> 4));
+              const uint32_t ad = sa + (uint32_t)(p * (F::A_PLANE >> 4)), bd = sb + (uint32_t)((sum - p) * (F::B_PLANE >> 4));
               if constexpr (F::PAIR) {
-                ptx::mma_f16_pair_if(lead, d, ad, bd, idesc, acc);
-                ptx::mma_f16_pair_if(lead, d, ad + ka, bd + kb, idesc, 1u);
+                ptx::mma_f16_pair_if(lead, sum ? ds : d, word(ad, a0), word(bd, b0), idesc, acc);
+                ptx::mma_f16_pair_if(lead, sum ? ds : d, word(ad + ka, a0), word(bd + kb, b0), idesc, 1u);
               } else {
-                ptx::mma_f16_if(lead, d, ad, bd, idesc, acc);
-                ptx::mma_f16_if(lead, d, ad + ka, bd + kb, idesc, 1u);
+                ptx::mma_f16_if(lead, sum ? ds : d, word(ad, a0), word(bd, b0), idesc, acc);
+                ptx::mma_f16_if(lead, sum ? ds : d, word(ad + ka, a0), word(bd + kb, b0), idesc, 1u);
               }
               acc = 1u;
             }
+          }
+          if (F::PROMOTE && (kc % kSumChunks == kSumChunks - 1 || kc + 1 == nkc)) ++sq;
+          if (!ok) break;
           commit(&empty[s]);
           if (F::PROMOTE || kc + 1 == nkc) {
             commit(&acc_full[q % F::NACC]);
@@ -619,7 +654,7 @@ __global__ void __launch_bounds__(kSplitThreads, 1) f32_split_kernel(const Split
     const int quarter = warp % 4, half = warp / 4;
     const uint32_t t_row = tmem + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(half * HALF);
     const bool active = quarter * 32 < F::AR;      // rows past AR hold no results
-    uint32_t q = 0;
+    uint32_t q = 0, sq = 0;
     bool ok = true;
     for (uint32_t i = 0; ok && tile_ready(i, 90); ++i) {
       long gi = rank * 128 + quarter * 32 + lane, gj0 = half * HALF, m = a.m, n = a.n, ldc = a.ldc;
@@ -731,20 +766,28 @@ __global__ void __launch_bounds__(kSplitThreads, 1) f32_split_kernel(const Split
           break;
         }
         ptx::tc_fence_after();
-        if (active) {
+        // the smaller products' accumulator first, where it ends (the next chunk begins with them), then hi hi:
+        // added to the sums, rounding to nearest
+        const bool ends = p % kSumChunks == kSumChunks - 1 || p + 1 == nkc_all;
+#pragma unroll 1
+        for (int part = ends ? 0 : 1; part < 2; ++part) {
+          const uint32_t d = part ? buf : F::NACC + sq % F::NSUM;
+          if (active) {
 #pragma unroll
-          for (int g = 0; g < HALF; g += 16) {
-            uint32_t raw[16];
-            ptx::tmem_ld16(t_row + buf * F::TN + g, raw);
-            ptx::tmem_wait_ld();
+            for (int g = 0; g < HALF; g += 16) {
+              uint32_t raw[16];
+              ptx::tmem_ld16(t_row + d * F::TN + g, raw);
+              ptx::tmem_wait_ld();
 #pragma unroll
-            for (int j = 0; j < 8; ++j)
-              sum[g / 2 + j] = add2(sum[g / 2 + j], pack2(__uint_as_float(raw[2 * j]), __uint_as_float(raw[2 * j + 1])));
+              for (int j = 0; j < 8; ++j)
+                sum[g / 2 + j] = add2(sum[g / 2 + j], pack2(__uint_as_float(raw[2 * j]), __uint_as_float(raw[2 * j + 1])));
+            }
           }
+          ptx::tc_fence_before();
+          __syncwarp();
+          if (lane == 0) arrive(part ? &acc_empty[buf] : &sum_empty[sq % F::NSUM]);
         }
-        ptx::tc_fence_before();
-        __syncwarp();
-        if (lane == 0) arrive(&acc_empty[buf]);
+        if (ends) ++sq;
       }
       if (!ok) break;
       float acc[HALF];
@@ -778,13 +821,15 @@ __global__ void __launch_bounds__(kSplitThreads, 1) f32_split_kernel(const Split
     }
     if constexpr (F::PROMOTE) {
       // (inside this branch, whose registers the FFMA tiles need) every other warp has arrived here when no
-      // copy or MMA is in flight in this CTA's shared memory any more, and none of them waits with a limit
+      // copy or MMA is in flight in this CTA's shared memory any more, and none of them waits with a limit.
+      // `again` is `a` once more: with one copy of the arguments for both, the compiler spent the pipeline's
+      // registers on what this needs of them (128 x 64 tiles 5% slower)
       asm volatile("bar.sync 2, %0;" ::"n"(kSplitThreads) : "memory");
-      for (uint32_t i = 0; me + i * workers < a.total; ++i) {
+      for (uint32_t i = 0; me + i * workers < again.total; ++i) {
         const uint32_t flags = (redo[i / 4] >> (8 * (i % 4))) & 0xffu;
         if (!flags) continue;
-        const SplitTile ti = split_tile<F>(a, me + i * workers);
-        split_redo<F::AR, F::TN / 2>(a, ti.b, ti.m0 + rank * 128, ti.n0, flags, (float*)stages);
+        const SplitTile ti = split_tile<F>(again, me + i * workers);
+        split_redo<F::AR, F::TN / 2>(again, ti.b, ti.m0 + rank * 128, ti.n0, flags, (float*)stages);
       }
     }
   }
@@ -837,7 +882,7 @@ cudaError_t launch_tiles(SplitArgs a, const char* name, cudaStream_t st) {
   cfg.numAttrs = F::PAIR ? 2 : 1;
   ProfScope prof(name, st);
   note_launch();
-  return cudaLaunchKernelEx(&cfg, kern, a);
+  return cudaLaunchKernelEx(&cfg, kern, a, a);
 }
 
 template <class F>

@@ -260,3 +260,28 @@ def test_more_tiles_than_one_launch_holds(S, ta, tb):
     plain[bad] = False
     assert bool((err <= (k / 32 + 8) * U * nrm)[plain].all())
     assert bool((err <= 4 * k * U * nrm)[~plain].all())
+
+
+@pytest.mark.parametrize("form", list(FORMS))
+@pytest.mark.parametrize("ta,tb", [(0, 0), (1, 1)])
+def test_results_of_one_product(S, form, ta, tb):
+    """One nonzero per row of op(A): each result is one product. Its error, in u of the product: the sum of hi hi and
+    the smaller products is rounded once (1 u), mid lo and lo mid are left out (|mid| <= 2^-8 and |lo| <= 2^-17 of an
+    operand: 1 u), and the smaller products, at most 2^-7 (1 + 2^-8) of the product, are truncated five times (2 u
+    each at their magnitude: 0.08 u); alpha = 1 and beta = 0 round nothing: 2.1 u."""
+    m, n, k, batch = FORMS[form]
+    p = problem(ta, tb, m, n, k, batch, 0.0, (0, 0, 0), 21 + m)
+    p = dataclasses.replace(p, alpha=np.float32(1.0))
+    rng = np.random.default_rng(m)
+    for b in range(batch):
+        opa = p.op_a(b)
+        keep = rng.integers(0, k, m)
+        row = opa[np.arange(m), keep].copy()
+        opa[:] = 0.0
+        opa[np.arange(m), keep] = row
+    C = run(S, p)
+    assert S.last_run_info()["path"] == "f32_tcgen05"
+    for b in range(0, batch, max(1, batch // 8)):
+        ex, nrm = O.exact_f64(p, b)
+        err = np.abs(p.c_view(C, b).astype(np.float64) - ex)
+        assert np.all(err <= 2.1 * U * nrm)
