@@ -136,7 +136,8 @@ ssblasStatus_t ssblasGetOzakiSlices(int* slices);
  *     C) instead of leaving C untouched, and k < 0 returns SSBLAS_STATUS_INVALID_VALUE.
  *   SSBLAS_EXT_COMPUTE_TYPE: computeType is checked against the row and honoured:
  *     SSBLAS_COMPUTE_32I only with int8 operands; SSBLAS_COMPUTE_32F only on the fp32 and fp16 rows,
- *     where it asks for FP32 arithmetic (the fp32 row then never uses the 3xBF16 emulation); other
+ *     where it asks for FP32 arithmetic (the fp32 row then never uses the 3xBF16 emulation, nor the BF16
+ *     tensor cores on which it otherwise runs from k = 128 on, see SSBLAS_PATH_F32_TCGEN05, but FFMA); other
  *     combinations return SSBLAS_STATUS_INVALID_VALUE. Without the flag computeType is ignored.
  * The grouped entry point keeps the reference's three rows. Unknown flags return
  * SSBLAS_STATUS_INVALID_VALUE. */
@@ -211,8 +212,13 @@ typedef enum {
                                       8), 0 = automatic (none); the slicing of chunk c + 1 runs
                                       beside the GEMM of chunk c. */,
   SSBLAS_PATH_F16_TCGEN05 = 11,     /* fp16 inputs (SSBLAS_EXT_R16F row) on tcgen05.mma kind::f16 */
-  SSBLAS_PATH_F32_TCGEN05 = 13,    /* plain fp32 on tcgen05.mma kind::f16: three BF16 parts per operand
-                                      (exact), six products, FP32 sums of 32 k added in registers */
+  SSBLAS_PATH_F32_TCGEN05 = 13,    /* plain fp32, k >= 128, on tcgen05.mma kind::f16: three BF16 parts per
+                                      operand (exact), six of their nine products (what is left out is at
+                                      most 2^-24 of a product), FP32 sums of 32 k added in registers.
+                                      Closer to the exact result than an FFMA chain on dense operands;
+                                      a result that is a single product may be 2.1 * 2^-24 of it off (1.5
+                                      measured) instead of 2^-24. FFMA instead: SSBLAS_COMPUTE_32F under
+                                      SSBLAS_EXT_COMPUTE_TYPE, or ssblasSetKernelConfig(SSBLAS_PATH_SIMT, 3) */
   SSBLAS_PATH_GROUPED_OZAKI_TILE = 12 /* not a path: ssblasSetKernelConfig / tuning key of the tile
                                       shape of a grouped call's Ozaki instances per size bucket
                                       (batch 1): 0 = 128 x 64 tiles, one accumulator; 1 (default)

@@ -275,10 +275,11 @@ int simt_config(const BatchDesc& d) {
   const int short_k = area(64) >= 2 * area(32) ? 8 : 9;
   const int cores = d.row == ROW_F32 ? (d.k <= 64 ? short_k : big_default ? 4 : 3) : (big_default ? 1 : 0);
   // Plain fp32 takes the BF16 tensor cores from k = 128 on. Below, its error against 64 bits can be
-  // larger than that of the FFMA kernels (a truncated sum of 16 products against chains of so few
-  // rounded ones: entries with outliers, k = 64: 7.0e-8 against 6.4e-8; k = 128: 7.4e-8 against
-  // 8.0e-8; k = 1024: 1.2e-7 against 2.0e-7; U[-1,1), k = 1024: 1.2e-7 against 5.8e-7). The line
-  // depends on k alone, so a result does not depend on how many instances share the call.
+  // larger than that of the FFMA kernels on entries with outliers (a truncated sum of 16 products against chains
+  // of so few rounded ones). 2-norm of the error, tensor cores against FFMA: outliers, k = 32 5.9e-8, 4.4e-8;
+  // 64 6.2e-8, 5.6e-8; 96 6.6e-8, 6.8e-8; 128 6.9e-8, 7.6e-8; 1024 1.1e-7, 2.0e-7; U[-1,1), k = 64 4.6e-8, 1.4e-7;
+  // 1024 1.1e-7, 5.7e-7. The line depends on k alone, so a result does not depend on how many instances share
+  // the call. SSBLAS_COMPUTE_32F under SSBLAS_EXT_COMPUTE_TYPE (exact_f32) keeps FFMA.
   const int best = d.row == ROW_F32 && d.k >= 128 && !d.exact_f32 ? kSimtF32Split : cores;
   const int cfg = choose_config(SSBLAS_PATH_SIMT, d.m, d.n, d.k, d.batch, best);
   return cfg == kSimtF32Split && (d.row != ROW_F32 || d.exact_f32) ? cores : cfg;
@@ -395,11 +396,9 @@ cudaError_t plan_simt_grouped(const GroupedDesc& g, const std::vector<int>& memb
       return e;
   out.ntiles32 = (long)t32.size() / 3;
   out.ntiles64 = (long)t64.size() / 3;
-  out.launches = (out.ntiles32 ? 1 : 0) + (out.ntiles64 ? 1 : 0);
   for (int l = 0; l < 4; ++l) {
     out.ndmma[l] = (long)tdl[l].size() / 3;
     out.nsg[l] = (long)tsl[l].size() / 3;
-    out.launches += (out.ndmma[l] ? 1 : 0) + (out.nsg[l] ? 1 : 0);
   }
   return cudaStreamSynchronize(st);
 }

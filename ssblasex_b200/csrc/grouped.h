@@ -55,7 +55,6 @@ struct GroupedSimt {
   // fp32 tiles for the cp.async FFMA kernel (gemm_sgemm.cu), the same way; instances in inst32
   void* sg_tiles[4] = {};
   long nsg[4] = {};
-  int launches = 0;
   ~GroupedSimt();
 };
 cudaError_t plan_simt_grouped(const GroupedDesc& g, const std::vector<int>& members, GroupedSimt& out,

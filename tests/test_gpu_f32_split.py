@@ -285,3 +285,24 @@ def test_results_of_one_product(S, form, ta, tb):
         ex, nrm = O.exact_f64(p, b)
         err = np.abs(p.c_view(C, b).astype(np.float64) - ex)
         assert np.all(err <= 2.1 * U * nrm)
+
+
+def test_compute_type_keeps_ffma(S):
+    """SSBLAS_COMPUTE_32F, honoured under its extension, keeps plain fp32 off the tensor cores at any k."""
+    import torch
+    m, n, k = 70, 50, 300
+    g = torch.Generator(device="cuda").manual_seed(2)
+    A, B = (torch.rand(s, generator=g, device="cuda") * 2 - 1 for s in ((k, m), (n, k)))
+    C = torch.zeros((n, m), device="cuda")
+    ptrs = [(ct.c_void_p * 1)(t.data_ptr()) for t in (A, B, C)]
+    one, zero = np.array([1.0], np.float32), np.array([0.0], np.float32)
+    assert S.set_extensions(S.SSBLAS_EXT_COMPUTE_TYPE) == 0
+    try:
+        st = S.lib().ssblasGemmBatchedEx(0, 0, m, n, k, one.ctypes.data, ptrs[0], S.SSBLAS_R_32F, m, ptrs[1], S.SSBLAS_R_32F,
+                                         k, zero.ctypes.data, ptrs[2], S.SSBLAS_R_32F, m, 1, S.SSBLAS_COMPUTE_32F, 0)
+        assert st == 0 and S.last_run_info()["path"] == "simt"
+    finally:
+        S.set_extensions(S.SSBLAS_EXT_NONE)
+    ex = B.double() @ A.double()
+    nrm = B.double().abs() @ A.double().abs()
+    assert bool(((C.double() - ex).abs() <= k * U * nrm).all())
