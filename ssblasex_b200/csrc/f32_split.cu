@@ -58,6 +58,7 @@
 #include "internal.h"
 #include "ptx.cuh"
 #include "sgemm_load.cuh"
+#include "tile_rules.h"
 
 namespace ssb {
 namespace {
@@ -915,32 +916,12 @@ cudaError_t launch_split_np(const BatchDesc& d, cudaStream_t st) {
   if (d.k >= (1L << 31) || d.m >= (1L << 31) || d.n >= (1L << 31) || d.lda >= (1L << 25) || d.ldb >= (1L << 25))
     return cudaErrorNotSupported;
   if ((d.m + 127) / 128 * ((d.n + 63) / 64) * d.batch >= (1L << 31)) return cudaErrorNotSupported;
-  if (d.m <= 64 && d.n <= 64) return launch_split<Split<NP, 64, 64>>(d, st);
-  // 128 x 64, 128 x 128 or (a pair of CTAs) 256 x 256 tiles: the one whose waves end first, from the time
-  // of a chunk and of a tile's end that each was measured to take (ns; fitted to 16 x 1024^3 and
-  // 4 x 2048^3, checked on 16 other shapes). All give the same results bit for bit. Measured (us, 64 / 128 /
-  // pair): plain 16 x 1024^3 328 / 194 / 166, 256 x 256^3 98 / 62 / 74, 1 x 1024^3 32 / 34 / 47,
-  // 64 x (1024 x 64 x 512) 52 / 69 / 93; 3xBF16 16 x 1024^3 209 / 131 / 96, 256 x 256^3 65 / 44 / 39.
-  struct Cost {
-    long tm, tn, ctas, chunk, tile;
-  };
-  constexpr Cost cost[3] = {{128, 64, 1, NP == 3 ? 750 : 430, NP == 3 ? 300 : 1100},
-                            {128, 128, 1, NP == 3 ? 780 : 520, NP == 3 ? 2600 : 2100},
-                            {256, 256, 2, NP == 3 ? 1030 : 610, NP == 3 ? 8500 : 4400}};
-  const long nkc = (d.k + kKC - 1) / kKC;
-  int best = 0;
-  long least = 0;
-  for (int i = 0; i < 3; ++i) {
-    const Cost& c = cost[i];
-    const long tiles = (d.m + c.tm - 1) / c.tm * ((d.n + c.tn - 1) / c.tn) * d.batch, workers = num_sms() / c.ctas;
-    const long t = (tiles + workers - 1) / workers * (nkc * c.chunk + c.tile);
-    if (i == 0 || t < least) {
-      best = i;
-      least = t;
-    }
+  switch (split_form(NP, d.m, d.n, d.k, d.batch, num_sms()).form) {
+    case SPLIT_64: return launch_split<Split<NP, 64, 64>>(d, st);
+    case SPLIT_128_64: return launch_split<Split<NP, 128, 64>>(d, st);
+    case SPLIT_128_128: return launch_split<Split<NP, 128, 128>>(d, st);
+    default: return launch_split<Split<NP, 128, 128, true>>(d, st);
   }
-  if (best == 2) return launch_split<Split<NP, 128, 128, true>>(d, st);
-  return best == 1 ? launch_split<Split<NP, 128, 128>>(d, st) : launch_split<Split<NP, 128, 64>>(d, st);
 }
 
 }  // namespace

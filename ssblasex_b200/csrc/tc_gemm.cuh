@@ -765,6 +765,21 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
               }
             }
             }
+          } else if constexpr (Cfg::PAIRS == 1) {
+            // 3xBF16, in the order of the kernel that splits the operands itself (f32_split.cu): per 32 k hi lo, lo hi, hi
+            // hi, two steps of 16 k each, so that both give the same bits
+#pragma unroll
+            for (int h = 0; h < Cfg::KB / 64; ++h) {
+#pragma unroll
+              for (int t = 0; t < 3; ++t) {
+                const int p = t == 1 ? 1 : 0, q = t == 0 ? 1 : 0;
+#pragma unroll
+                for (int kk = 2 * h; kk < 2 * h + 2; ++kk)
+                  ptx::mma_f16(d_base, ptx::smem_desc_kmajor(sa + p * Cfg::BM * Cfg::KB + kk * 32, Cfg::KB),
+                               ptx::smem_desc_kmajor(sb + q * Cfg::BN * Cfg::KB + kk * 32, Cfg::KB), IDESC,
+                               (acc_k || h > 0 || t > 0 || kk > 0) ? 1u : 0u);
+              }
+            }
           } else {
 #pragma unroll
           for (int p = 0; p < Cfg::PA; ++p) {

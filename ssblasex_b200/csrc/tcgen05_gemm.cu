@@ -596,9 +596,15 @@ cudaError_t launch_bf16x3_f32(const BatchDesc& d, cudaStream_t st) {
   // fed by TMA that splits in shared memory, for equally spaced instances of at most 128 x 128 (the
   // others take configuration 0 / 1); 3 = one kernel that splits the tiles of any instances as it
   // loads them (f32_split.cu). Default: 2 where it applies (4096 x 64^3 TT: 0.057 ms against
-  // 0.084 + 0.072 ms for the split pass and the tiled GEMM), else 3 (256 x 256^3 NT: 0.039 against
-  // 0.130 ms).
-  const int fallback = bf16x3_small_fits(d) ? 2 : 3;
+  // 0.084 + 0.072 ms for the split pass and the tiled GEMM), else 3 or, with few tiles and a long K, 0 / 1
+  // (bf16x3_planes; the bits are the same).
+  auto on_grid = [](const void* X0, long stride, long ld) {
+    return ((uintptr_t)X0 % 16) == 0 && stride % 16 == 0 && ld % 4 == 0;   // (X0 is not known in every call)
+  };
+  const bool small = bf16x3_small_fits(d);
+  const bool planes = !small && bf16x3_planes(d.m, d.n, d.k, d.batch, d.transa == SSBLAS_OP_T, d.transb == SSBLAS_OP_N,
+                                              on_grid(d.A0, d.strideA, d.lda), on_grid(d.B0, d.strideB, d.ldb), num_sms());
+  const int fallback = small ? 2 : planes ? (d.n <= 64 ? 0 : 1) : 3;
   const int cfg = choose_config(SSBLAS_PATH_BF16X3_TCGEN05, d.m, d.n, d.k, d.batch, fallback);
   cudaError_t e;
   if (cfg == 2 && bf16x3_small_fits(d)) {
@@ -611,9 +617,10 @@ cudaError_t launch_bf16x3_f32(const BatchDesc& d, cudaStream_t st) {
   }
   const long Kp = round_up(d.k, 8);
   const long sa = d.m * Kp * 2, sb = d.n * Kp * 2;   // bytes per plane
+  const bool injected = settings().fault == SSBLAS_FAULT_ALLOC;
   void* pa = workspace(WS_PACK_A, (size_t)sa * 2 * d.batch, &e);
-  if (!pa) return e;
-  void* pb = workspace(WS_PACK_B, (size_t)sb * 2 * d.batch, &e);
+  void* pb = pa ? workspace(WS_PACK_B, (size_t)sb * 2 * d.batch, &e) : nullptr;
+  if (!pb && planes && cfg == fallback && !injected && e == cudaErrorMemoryAllocation) return launch_f32_split(d, 2, st);
   if (!pb) return e;
   PlaneArgs a{d.A, d.m, d.k, d.lda, d.transa == SSBLAS_OP_T, d.batch, pa, Kp, sa, sa * 2};
   PlaneArgs b{d.B, d.n, d.k, d.ldb, d.transb == SSBLAS_OP_N, d.batch, pb, Kp, sb, sb * 2};

@@ -306,3 +306,25 @@ def test_compute_type_keeps_ffma(S):
     ex = B.double() @ A.double()
     nrm = B.double().abs() @ A.double().abs()
     assert bool(((C.double() - ex).abs() <= k * U * nrm).all())
+
+
+@pytest.mark.parametrize("ta,tb", [(0, 0), (0, 1), (1, 0), (1, 1)])
+@pytest.mark.parametrize("shape", [(64, 64, 700, 1), (70, 33, 513, 3), (300, 200, 544, 2), (129, 257, 1000, 1)])
+@pytest.mark.parametrize("pad,beta", [(0, 0.25), (4, 0.0), (3, -1.5)])
+def test_bf16x3_planes_and_split_kernel_agree(S, ta, tb, shape, pad, beta):
+    """The split pass with the tiled GEMM (either tile width) and the split kernel: the same bits, so the choice between
+    them may follow the number of tiles."""
+    m, n, k, batch = shape
+    p = problem(ta, tb, m, n, k, batch, beta, (pad, pad, pad), 13 + m, "outliers")
+    S.set_math_mode(S.SSBLAS_MATH_FP32_BF16X3)
+    out = []
+    try:
+        # (by default instances of at most 128 x 128 may take a kernel of their own, with another order of sums)
+        for cfg in (3, 0, 1) if max(m, n) <= 128 else (3, 0, 1, -1):
+            S.set_kernel_config("bf16x3_tcgen05", cfg)
+            out.append(run(S, p, pad % 2).view(np.uint32))
+    finally:
+        S.set_kernel_config("bf16x3_tcgen05", -1)
+        S.set_math_mode(S.SSBLAS_MATH_PLAIN)
+    for o in out[1:]:
+        np.testing.assert_array_equal(o, out[0])
