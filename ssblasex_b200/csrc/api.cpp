@@ -158,7 +158,10 @@ int num_sms() {
 
 bool is_captured(cudaStream_t st) {
   cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-  if (cudaStreamIsCapturing(st, &cap) != cudaSuccess) cudaGetLastError();
+  if (cudaStreamIsCapturing(st, &cap) != cudaSuccess) {
+    cudaGetLastError();   // the legacy stream beside a capture: `cap` says nothing, and a launch there is refused
+    return false;
+  }
   return cap != cudaStreamCaptureStatusNone;
 }
 
