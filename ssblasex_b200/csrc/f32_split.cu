@@ -97,6 +97,7 @@ struct Split {
   // (two and two: 100 x 256^3 31 -> 33 us, 74 x (256 x 256 x 128) 15.0 -> 15.7).
   static constexpr int NACC = PROMOTE ? (PAIR ? 1 : TN == 128 ? 3 : 6) : PAIR ? 2 : 4;
   static constexpr int NSUM = !PROMOTE ? 0 : TN == 64 ? 2 : 1;
+  static constexpr int SUMS = PROMOTE ? NSUM : 1;   // (to count them by, also in code that does not run)
   static constexpr int TMEM_COLS = (NACC + NSUM) * TN;
   // registers per thread: 640 threads x 96 at launch = 61,440 for 256 converters, 256 epilogue threads (the
   // plain form's hold a sum per output, 128 a thread in a pair) and the 128 of the issuing warp's warpgroup (32
@@ -571,8 +572,8 @@ __global__ void __launch_bounds__(kSplitThreads, 1) f32_split_kernel(const Split
           // accumulator of a pair for hi hi is waited for behind them)
           bool free = true;
           if (F::PROMOTE && kc % kSumChunks == 0)
-            free = ptx::mbar_wait(ptx::smem_u32(&sum_empty[sq % (F::PROMOTE ? F::NSUM : 1)]),
-                                  ((sq / (F::PROMOTE ? F::NSUM : 1)) & 1) ^ 1, err, 86, wl);
+            free = ptx::mbar_wait(ptx::smem_u32(&sum_empty[sq % F::SUMS]),
+                                  ((sq / F::SUMS) & 1) ^ 1, err, 86, wl);
           if (F::PROMOTE ? F::NACC > 1 : kc == 0)
             free = free && ptx::mbar_wait(ptx::smem_u32(&acc_empty[q % F::NACC]), ((q / F::NACC) & 1) ^ 1, err, 82, wl);
           if (!free) {
@@ -588,7 +589,7 @@ __global__ void __launch_bounds__(kSplitThreads, 1) f32_split_kernel(const Split
           const uint32_t sa = (uint32_t)a0 + s * (uint32_t)(F::STAGE >> 4), sb = (uint32_t)b0 + s * (uint32_t)(F::STAGE >> 4);
           auto word = [](uint32_t lo, uint64_t base) { return (base & 0xffffffff00000000ull) | lo; };
           const uint32_t d = tmem + (q % F::NACC) * F::TN;
-          const uint32_t ds = F::PROMOTE ? tmem + (F::NACC + sq % (F::PROMOTE ? F::NSUM : 1)) * F::TN : d;
+          const uint32_t ds = F::PROMOTE ? tmem + (F::NACC + sq % F::SUMS) * F::TN : d;
           uint32_t acc = (F::PROMOTE ? kc % kSumChunks : kc) == 0 ? 0u : 1u;
           // smallest products first
 #pragma unroll
@@ -772,7 +773,7 @@ __global__ void __launch_bounds__(kSplitThreads, 1) f32_split_kernel(const Split
         const bool ends = p % kSumChunks == kSumChunks - 1 || p + 1 == nkc_all;
 #pragma unroll 1
         for (int part = ends ? 0 : 1; part < 2; ++part) {
-          const uint32_t d = part ? buf : F::NACC + sq % F::NSUM;
+          const uint32_t d = part ? buf : F::NACC + sq % F::SUMS;
           if (active) {
 #pragma unroll
             for (int g = 0; g < HALF; g += 16) {
@@ -786,7 +787,7 @@ __global__ void __launch_bounds__(kSplitThreads, 1) f32_split_kernel(const Split
           }
           ptx::tc_fence_before();
           __syncwarp();
-          if (lane == 0) arrive(part ? &acc_empty[buf] : &sum_empty[sq % F::NSUM]);
+          if (lane == 0) arrive(part ? &acc_empty[buf] : &sum_empty[sq % F::SUMS]);
         }
         if (ends) ++sq;
       }
