@@ -618,9 +618,10 @@ cudaError_t launch_bf16x3_f32(const BatchDesc& d, cudaStream_t st) {
   const long Kp = round_up(d.k, 8);
   const long sa = d.m * Kp * 2, sb = d.n * Kp * 2;   // bytes per plane
   const bool injected = settings().fault == SSBLAS_FAULT_ALLOC;
+  const bool by_rule = planes && cfg == fallback;   // the split kernel would run it too
   void* pa = workspace(WS_PACK_A, (size_t)sa * 2 * d.batch, &e);
   void* pb = pa ? workspace(WS_PACK_B, (size_t)sb * 2 * d.batch, &e) : nullptr;
-  if (!pb && planes && cfg == fallback && !injected && e == cudaErrorMemoryAllocation) return launch_f32_split(d, 2, st);
+  if (!pb && by_rule && !injected && e == cudaErrorMemoryAllocation) return launch_f32_split(d, 2, st);
   if (!pb) return e;
   PlaneArgs a{d.A, d.m, d.k, d.lda, d.transa == SSBLAS_OP_T, d.batch, pa, Kp, sa, sa * 2};
   PlaneArgs b{d.B, d.n, d.k, d.ldb, d.transb == SSBLAS_OP_N, d.batch, pb, Kp, sb, sb * 2};
@@ -629,7 +630,7 @@ cudaError_t launch_bf16x3_f32(const BatchDesc& d, cudaStream_t st) {
   CUtensorMap ta, tb;
   if (!make_map(&ta, pa, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, d.k, d.m, 2, d.batch, Kp * 2, sa, sa * 2, 64, 128, 2, 128) ||
       !make_map(&tb, pb, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, d.k, d.n, 2, d.batch, Kp * 2, sb, sb * 2, 64, BN, 2, 128))
-    return cudaErrorNotSupported;
+    return by_rule ? launch_f32_split(d, 2, st) : cudaErrorNotSupported;
   tc::Params prm = base_params(d);
   note_path(SSBLAS_PATH_BF16X3_TCGEN05);
   return BN == 64 ? run_gemm<CfgBf64>(ta, tb, prm, st, "bf16x3_gemm") : run_gemm<CfgBf128>(ta, tb, prm, st, "bf16x3_gemm");

@@ -328,3 +328,33 @@ def test_bf16x3_planes_and_split_kernel_agree(S, ta, tb, shape, pad, beta):
         S.set_math_mode(S.SSBLAS_MATH_PLAIN)
     for o in out[1:]:
         np.testing.assert_array_equal(o, out[0])
+
+
+def test_bf16x3_without_memory_for_planes(S):
+    """A call that would take the planes runs on the split kernel where their scratch cannot be had; an injected failure
+    of the allocation is reported."""
+    import torch
+    from ssblasex_b200 import runner
+    p = problem(0, 1, 1536, 1024, 4096, 1, 0.0, (3, 3, 3), 4)      # 31 MB for each plane pair and more
+    dp = runner.DeviceProblem(p)
+    S.set_math_mode(S.SSBLAS_MATH_FP32_BF16X3)
+    S.release_workspace()
+    torch.cuda.empty_cache()
+    try:
+        st, want = runner.call(p, "host_array", dp)
+        assert st == 0 and S.last_run_info()["kernel_launches"] == 2
+        S.release_workspace()
+        dp.reset_c()
+        hold = torch.empty(torch.cuda.mem_get_info()[0] - (24 << 20), dtype=torch.uint8, device="cuda")
+        st, got = runner.call(p, "host_array", dp)
+        launches = S.last_run_info()["kernel_launches"]
+        del hold
+        torch.cuda.empty_cache()
+        assert st == 0 and launches == 1
+        np.testing.assert_array_equal(got.view(np.uint32), want.view(np.uint32))
+        S.release_workspace()
+        assert S.set_fault_injection(S.SSBLAS_FAULT_ALLOC) == 0
+        assert runner.call(p, "host_array", dp)[0] == S.SSBLAS_STATUS_ALLOC_FAILED
+    finally:
+        S.set_math_mode(S.SSBLAS_MATH_PLAIN)
+        S.release_workspace()
